@@ -76,6 +76,14 @@ SIGNATURES = {
     "dlb_k_grouped_gemm_workspace_bytes": (c_i64, [c_i64, c_i64, c_i64, c_int, c_int]),
     "dlb_k_grouped_gemm_16bit": (c_int, [c_vp, c_vp, c_int, c_i64, c_i64, c_i64, c_vp, c_int, c_int, c_vp, c_i64, c_vp,
                                          c_vp, c_vp]),
+    "dlb_moe_build_tiles_sizes": (c_int, [c_vp, c_int, c_int, c_i64, c_int, c_vp, c_int, c_vp]),
+    "dlb_moe_plan": (c_int, [c_vp, c_int, c_i64, c_int, c_int, c_int, c_int, c_int, c_vp, c_vp, c_vp, c_int, c_vp, c_vp,
+                             c_vp, c_sz, c_vp]),
+    "dlb_moe_align_block_size": (c_int, [c_vp, c_int, c_i64, c_int, c_int, c_int, c_vp, c_i64, c_vp, c_int, c_vp, c_vp,
+                                         c_sz, c_vp]),
+    "dlb_permute_plan": (c_int, [c_vp, c_int, c_i64, c_int, c_int, c_i64, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_sz, c_vp]),
+    "dlb_unpermute_bwd_rows": (c_int, [c_vp, c_vp, c_int, c_vp, c_vp, c_i64, c_int, c_i64, c_i64, c_vp, c_int, c_vp, c_vp,
+                                       c_vp]),
     "dlb_moe_build_tiles_rows": (c_int, [c_vp, c_vp, c_int, c_int, c_int, c_vp, c_int, c_vp]),
     "dlb_unpermute": (c_int, [c_vp, c_int, c_vp, c_vp, c_i64, c_int, c_i64, c_vp, c_vp]),
     "dlb_unpermute_bwd": (c_int, [c_vp, c_vp, c_int, c_vp, c_vp, c_i64, c_int, c_i64, c_vp, c_vp, c_vp]),

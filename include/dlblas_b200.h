@@ -117,6 +117,25 @@ DLB_API int dlb_moe_build_tiles(const int64_t* exp_start, const int64_t* exp_end
 /* Same list with tiles of `tile_rows` rows (128 or 256). */
 DLB_API int dlb_moe_build_tiles_rows(const int64_t* exp_start, const int64_t* exp_end, int expert_offset,
                              int num_local_experts, int tile_rows, int32_t* tiles, int max_tiles, void* stream);
+/* The list for consecutive row groups of the given sizes (int32 or int64, on the device), clipped to total_rows rows. */
+DLB_API int dlb_moe_build_tiles_sizes(const void* sizes, int sizes_dtype, int num_groups, int64_t total_rows, int tile_rows,
+                              int32_t* tiles, int max_tiles, void* stream);
+/* Everything an expert layer needs to know about the routing before it touches a token: the stable sort of the
+ * [tokens, top_k] ids (sorted_idx and slot_pos as for dlb_sort_by_expert), the tile list over experts [expert_offset,
+ * expert_offset + num_local_experts) (as for dlb_moe_build_tiles_rows) and, when `weights` [tokens, top_k] is given, the
+ * weights divided by their sum over each token's slots (_renormalize, dlblas/kernels/moe.py:368-373).  Workspace as
+ * for dlb_sort_by_expert. */
+DLB_API int dlb_moe_plan(const void* ids, int ids_dtype, int64_t tokens, int top_k, int num_experts, int expert_offset,
+                 int num_local_experts, int tile_rows, int64_t* sorted_idx, int32_t* slot_pos, int32_t* tiles,
+                 int max_tiles, const float* weights, float* normalised, void* workspace, size_t workspace_bytes,
+                 void* stream);
+/* Block-aligned token layout (moe_align_block_size, dlblas/kernels/moe_align_block_size.py:138-210): every expert's slots
+ * in ascending order, padded with num_slots to whole blocks; the expert of every block, 0 behind the last; the padded
+ * total.  ids < 0 are replaced in place by `negative_as`; ids >= num_experts are ignored.  sorted_len >= num_slots +
+ * num_experts * (block_size - 1), num_blocks * block_size >= sorted_len.  Workspace as for dlb_sort_by_expert. */
+DLB_API int dlb_moe_align_block_size(void* ids, int ids_dtype, int64_t num_slots, int num_experts, int negative_as,
+                             int block_size, int32_t* sorted_ids, int64_t sorted_len, int32_t* expert_ids, int num_blocks,
+                             int32_t* num_padded, void* workspace, size_t workspace_bytes, void* stream);
 DLB_API int dlb_moe_build_tiles_masked(const int32_t* masked_m, int num_local_experts, int rows_per_expert,
                                int32_t* tiles, int max_tiles, void* stream);
 
@@ -330,6 +349,19 @@ DLB_API int dlb_unpermute(const void* in, int dtype, const int32_t* row_id_map, 
 DLB_API int dlb_unpermute_bwd(const void* grad_out, const void* fwd_in, int dtype, const int32_t* row_id_map,
                       const float* probs, int64_t tokens, int top_k, int64_t h, float* act_grad, float* prob_grad,
                       void* stream);
+/* The same with act_grad [rows, h] in fp32 or in the tensors' own type (act_dtype) and rows that no slot maps to set to
+ * zero; row_marks: `rows` bytes of workspace. */
+DLB_API int dlb_unpermute_bwd_rows(const void* grad_out, const void* fwd_in, int dtype, const int32_t* row_id_map,
+                           const float* probs, int64_t tokens, int top_k, int64_t h, int64_t rows, void* act_grad,
+                           int act_dtype, float* prob_grad, void* row_marks, void* stream);
+/* Routing side of the permutation (moe_permute_topk_op_triton, :62-137): dest int32 [tokens * top_k] = row of every slot
+ * (-1: no expert, or not below dest_limit) and row_id_map; sorted_idx (may be NULL) as for dlb_sort_by_expert.  ids lie
+ * below num_experts; stats int32 [3], if given, receives {largest id, ids equal to -1, ids below 0} in memory that the
+ * device can write (pinned host memory, for instance), and stats_event (cudaEvent_t, may be NULL) is recorded on the
+ * stream behind the kernel that writes it.  Workspace as for dlb_sort_by_expert. */
+DLB_API int dlb_permute_plan(const void* ids, int ids_dtype, int64_t tokens, int top_k, int num_experts, int64_t dest_limit,
+                     int64_t* sorted_idx, int32_t* dest, int32_t* row_id_map, int32_t* stats, void* stats_event,
+                     void* workspace, size_t workspace_bytes, void* stream);
 
 /* ---- expert-parallel load balancing ------------------------------------------------
  * map_logic_to_physical_idx_hash_random (dlblas/kernels/moe.py:524-579): every (token, slot) of topk_idx
