@@ -118,6 +118,28 @@ def lib():
     return _lib
 
 
+_host_module = None
+
+
+def host():
+    """The host side of the operators (csrc/host.cpp), bound to the library that `lib()` has loaded."""
+    global _host_module
+    if _host_module is None:
+        handle = lib()
+        with _lock:
+            if _host_module is None:
+                path = os.path.join(_HERE, "_host.so")
+                if not os.path.exists(path):
+                    raise RuntimeError(f"dlblas_b200: {path} is missing; build it with `python -m dlblas_b200.build`")
+                import importlib.util
+                spec = importlib.util.spec_from_file_location("dlblas_b200._host", path)
+                module = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(module)
+                module.bind({name: ctypes.cast(getattr(handle, name), ctypes.c_void_p).value for name in SIGNATURES})
+                _host_module = module
+    return _host_module
+
+
 def check(rc: int):
     """Maps a negative return code to the exception type the reference raises in that case:
     bad shapes / dtypes are `assert`s there, so DLB_ERR_INVALID becomes AssertionError."""
@@ -150,15 +172,9 @@ def require_cuda(*tensors):
             raise RuntimeError("dlblas_b200 runs on CUDA tensors only (B200, sm_100a); there is no CPU path")
 
 
-_status = {}
-
-
 def status_word(device) -> torch.Tensor:
     """Per-device int32 word the GEMM kernels set when a bounded wait gives up."""
-    key = torch.device(device).index or 0
-    if key not in _status:
-        _status[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _status[key]
+    return host().status_word(torch.device(device).index or 0)
 
 
 def check_status(device=None):

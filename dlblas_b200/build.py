@@ -1,9 +1,13 @@
-"""Builds the CUDA extension in-tree: dlblas_b200/_dlblas_b200.so (sm_100a only).
+"""Builds the native code in-tree (sm_100a only):
 
     python -m dlblas_b200.build [--force] [--verbose]
 
-Plain nvcc, no JIT at import time: the shared library is a C-ABI (include/dlblas_b200.h)
-loaded with ctypes, so it does not link against torch or Python.
+    dlblas_b200/_dlblas_b200.so   the CUDA library: a C ABI (include/dlblas_b200.h) that links against neither torch nor
+                                  Python (nvcc)
+    dlblas_b200/_host.so          the host side of the operators, a CPython extension on torch's C++ API that calls that
+                                  C ABI (g++)
+
+No JIT at import time.
 """
 import argparse
 import os
@@ -19,6 +23,25 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "--expt-relaxed-constexpr",
 ]
+
+
+HOST_OUT = os.path.join(PKG, "_host.so")
+HOST_SOURCE = "host.cpp"
+
+
+def _host_command(obj_source, out):
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(os.path.abspath(torch.__file__))
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    lib = os.path.join(root, "lib")
+    abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
+    return (["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
+             "-w"] + [f for d in inc for f in ("-isystem", d)] + [obj_source, "-o", out, "-L" + lib, "-Wl,-rpath," + lib,
+             "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"])
 
 
 def _nvcc():
@@ -40,6 +63,10 @@ def build(force=False, verbose=False):
     os.makedirs(objdir, exist_ok=True)
     hdrs = [os.path.normpath(os.path.join(CSRC, h)) for h in HEADERS]
     objs, procs = [], []
+    host = os.path.join(CSRC, HOST_SOURCE)
+    if force or _stale(HOST_OUT, [host, hdrs[-1]]):
+        procs.append((HOST_SOURCE, subprocess.Popen(_host_command(host, HOST_OUT), stdout=subprocess.PIPE,
+                                                    stderr=subprocess.STDOUT, text=True)))
     for src in SOURCES:
         s = os.path.join(CSRC, src)
         o = os.path.join(objdir, src.replace(".cu", ".o"))

@@ -1,0 +1,460 @@
+// Host side of the operators as a CPython extension (dlblas_b200/_host.so): argument checks, output and workspace
+// allocation, stream lookup and the calls into the C ABI (include/dlblas_b200.h), without a Python frame per tensor.
+//
+// A small expert layer is some thirty microseconds of kernels.  Through ctypes it spent 140 us on the host: every C call
+// converts up to twenty arguments, every torch.empty crosses the dispatcher, and a layer makes seven of the one and a dozen
+// of the other.  Here a layer is one call: one workspace for everything that does not leave it, one C++ call per kernel.
+//
+// The module binds to the C ABI by the addresses that the ctypes loader hands over (bind), so that there is one copy of the
+// library however it was located.  Errors of the C ABI become AssertionError (bad arguments, as the reference's
+// asserts) or RuntimeError.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Dtype.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <cstdlib>
+#include <mutex>
+#include <optional>
+#include <string>
+#include <vector>
+
+#include "../../include/dlblas_b200.h"
+
+namespace {
+
+using at::Tensor;
+
+// ---- the C ABI by address -----------------------------------------------------------------------------------------
+#define ABI_FUNCTIONS(X)                                                                                              \
+  X(dlb_last_error_string)                                                                                            \
+  X(dlb_sort_by_expert_workspace_size)                                                                                \
+  X(dlb_moe_plan)                                                                                                     \
+  X(dlb_quant_fp8)                                                                                                    \
+  X(dlb_permute_rows)                                                                                                 \
+  X(dlb_moe_grouped_gemm)                                                                                             \
+  X(dlb_silu_mul_quant)                                                                                               \
+  X(dlb_moe_sum_topk)                                                                                                 \
+  X(dlb_fp8_gemm)                                                                                                     \
+  X(dlb_route_softmax_topk)                                                                                           \
+  X(dlb_route_grouped_topk)
+
+struct Abi {
+#define X(name) decltype(&::name) name = nullptr;
+  ABI_FUNCTIONS(X)
+#undef X
+} abi;
+
+// ---- errors -------------------------------------------------------------------------------------------------------
+struct AssertionFailed : std::runtime_error {
+  using std::runtime_error::runtime_error;
+};
+void require(bool ok, const char* msg) {
+  if (!ok) throw AssertionFailed(msg);
+}
+void check(int rc) {
+  if (rc == DLB_OK) return;
+  const std::string msg = abi.dlb_last_error_string();
+  if (rc == DLB_ERR_INVALID) throw AssertionFailed(msg);
+  throw std::runtime_error("dlblas_b200 error " + std::to_string(rc) + ": " + msg);
+}
+
+// ---- arguments ----------------------------------------------------------------------------------------------------
+struct PyFailed {};   // a Python error is already set
+
+const Tensor& tensor(PyObject* o) {
+  if (!THPVariable_Check(o)) {
+    PyErr_SetString(PyExc_TypeError, "expected a torch.Tensor");
+    throw PyFailed{};
+  }
+  return THPVariable_Unpack(o);
+}
+std::optional<Tensor> opt_tensor(PyObject* o) {
+  if (o == Py_None) return std::nullopt;
+  return tensor(o);
+}
+int64_t integer(PyObject* o) {
+  const long long v = PyLong_AsLongLong(o);
+  if (v == -1 && PyErr_Occurred()) throw PyFailed{};
+  return v;
+}
+double real(PyObject* o) {
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred()) throw PyFailed{};
+  return v;
+}
+bool truth(PyObject* o) {
+  const int v = PyObject_IsTrue(o);
+  if (v < 0) throw PyFailed{};
+  return v != 0;
+}
+at::ScalarType dtype(PyObject* o) {
+  if (!THPDtype_Check(o)) {
+    PyErr_SetString(PyExc_TypeError, "expected a torch.dtype");
+    throw PyFailed{};
+  }
+  return reinterpret_cast<THPDtype*>(o)->scalar_type;
+}
+void need_args(Py_ssize_t n, Py_ssize_t want) {
+  if (n != want) {
+    PyErr_Format(PyExc_TypeError, "expected %zd arguments, got %zd", want, n);
+    throw PyFailed{};
+  }
+}
+PyObject* wrap(const Tensor& t) { return THPVariable_Wrap(t); }
+PyObject* wrap_tuple(std::initializer_list<const Tensor*> ts) {
+  PyObject* r = PyTuple_New((Py_ssize_t)ts.size());
+  Py_ssize_t i = 0;
+  for (const Tensor* t : ts) PyTuple_SET_ITEM(r, i++, wrap(*t));
+  return r;
+}
+
+// Runs the body of a method and turns C++ exceptions into Python ones.
+template <typename F> PyObject* guarded(F&& f) {
+  try {
+    return f();
+  } catch (const PyFailed&) {
+    return nullptr;
+  } catch (const AssertionFailed& e) {
+    PyErr_SetString(PyExc_AssertionError, e.what());
+  } catch (const c10::OutOfMemoryError& e) {
+    // the type that torch's own allocations raise
+    PyObject* torch = PyImport_ImportModule("torch");
+    PyObject* type = torch != nullptr ? PyObject_GetAttrString(torch, "OutOfMemoryError") : nullptr;
+    PyErr_Clear();
+    PyErr_SetString(type != nullptr ? type : PyExc_MemoryError, e.what_without_backtrace());
+    Py_XDECREF(type);
+    Py_XDECREF(torch);
+  } catch (const c10::Error& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+  }
+  return nullptr;
+}
+
+// ---- memory, streams ----------------------------------------------------------------------------------------------
+// The tensors' device made current, and its current stream.
+struct Call {
+  c10::cuda::CUDAGuard guard;
+  at::Device device;
+  cudaStream_t stream;
+  explicit Call(const Tensor& t) : guard(t.device()), device(t.device()), stream(at::cuda::getCurrentCUDAStream(t.device().index())) {}
+};
+
+void require_cuda(const Tensor& t) {
+  if (!t.is_cuda())
+    throw std::runtime_error("dlblas_b200 runs on CUDA tensors only (B200, sm_100a); there is no CPU path");
+}
+
+Tensor empty(at::IntArrayRef sizes, at::ScalarType dt, const Call& c) {
+  return at::detail::empty_cuda(sizes, dt, c.device, std::nullopt);
+}
+
+// Pieces of one allocation, each on a 256-byte boundary.
+struct Workspace {
+  size_t bytes = 0;
+  Tensor mem;
+  size_t take(size_t n) {
+    const size_t at = bytes;
+    bytes += (n + 255) / 256 * 256;
+    return at;
+  }
+  void allocate(const Call& c) { mem = empty({(int64_t)std::max<size_t>(bytes, 1)}, at::kByte, c); }
+  template <typename T> T* at(size_t off) const { return reinterpret_cast<T*>(static_cast<char*>(mem.data_ptr()) + off); }
+};
+
+int code(at::ScalarType t) {
+  switch (t) {
+    case at::kFloat: return DLB_F32;
+    case at::kBFloat16: return DLB_BF16;
+    case at::kHalf: return DLB_F16;
+    case at::kInt: return DLB_I32;
+    case at::kLong: return DLB_I64;
+    default: throw AssertionFailed(std::string("dlblas_b200: unsupported dtype ") + c10::toString(t));
+  }
+}
+
+// Per-device int32 word that the GEMM kernels set when a bounded wait gives up.
+Tensor status_word(at::DeviceIndex index) {
+  static std::mutex m;
+  static Tensor words[64];
+  require(index >= 0 && index < 64, "device index out of range");
+  std::lock_guard<std::mutex> lock(m);
+  if (!words[index].defined())
+    words[index] = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, index));
+  return words[index];
+}
+int32_t* status_ptr(const Call& c) { return status_word(c.device.index()).data_ptr<int32_t>(); }
+
+int env_int(const char* name, int fallback) {
+  const char* v = std::getenv(name);
+  return v != nullptr && *v != 0 ? std::atoi(v) : fallback;
+}
+
+// ---- quantisation and the dense GEMM ------------------------------------------------------------------------------
+// 1 x group quantisation of the rows of a 2-D tensor; with dst_pos, row t goes to rows dst_pos[t * fanout + j].
+std::pair<Tensor, Tensor> quant_fp8(const Tensor& x, int64_t group, int mode, double eps, bool column_major,
+                                    const std::optional<Tensor>& dst_pos, int64_t fanout, int64_t rows_out) {
+  require_cuda(x);
+  require(x.dim() == 2 && x.stride(1) == 1, "x must be 2-D with contiguous rows");
+  const int64_t m = x.size(0), k = x.size(1), rows = rows_out < 0 ? m : rows_out;
+  if (k % group != 0)
+    throw AssertionFailed("the last dimension of 'x' " + std::to_string(k) + " must be divisible by 'group_size' " +
+                          std::to_string(group));
+  Call c(x);
+  Tensor q = empty({rows, k}, at::kFloat8_e4m3fn, c);
+  Tensor s = column_major ? empty({k / group, rows}, at::kFloat, c).t() : empty({rows, k / group}, at::kFloat, c);
+  check(abi.dlb_quant_fp8(x.data_ptr(), code(x.scalar_type()), m, k, x.stride(0), (int)group, mode, (float)eps, q.data_ptr(),
+                          s.data_ptr<float>(), s.stride(0), s.stride(1), dst_pos ? dst_pos->data_ptr<int32_t>() : nullptr,
+                          (int)fanout, c.stream));
+  return {q, s};
+}
+
+PyObject* py_quant_fp8(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 8);
+    auto [q, s] = quant_fp8(tensor(a[0]), integer(a[1]), (int)integer(a[2]), real(a[3]), truth(a[4]), opt_tensor(a[5]),
+                            integer(a[6]), integer(a[7]));
+    return wrap_tuple({&q, &s});
+  });
+}
+
+// per_token_group_quant_fp8: any leading dimensions
+PyObject* py_group_quant_fp8(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 4);
+    const Tensor& x = tensor(a[0]);
+    const int64_t group = integer(a[1]);
+    const bool column_major = truth(a[3]);
+    if (x.dim() == 2) {
+      auto [q, s] = quant_fp8(x, group, DLB_QUANT_DIV_EPS, real(a[2]), column_major, std::nullopt, 1, -1);
+      return wrap_tuple({&q, &s});
+    }
+    require(!column_major, "column-major scales need a 2-D input");
+    auto [q, s] = quant_fp8(x.reshape({-1, x.size(-1)}), group, DLB_QUANT_DIV_EPS, real(a[2]), false, std::nullopt, 1, -1);
+    std::vector<int64_t> shape = x.sizes().vec();
+    Tensor qv = q.view(shape);
+    shape.back() /= group;
+    Tensor sv = s.view(shape);
+    return wrap_tuple({&qv, &sv});
+  });
+}
+
+Tensor fp8_gemm(const Tensor& a, const Tensor& b, const Tensor& a_s, const Tensor& b_s, at::ScalarType out_dtype,
+                int tile_rows) {
+  for (const Tensor* t : {&a, &b, &a_s, &b_s}) require_cuda(*t);
+  if (tile_rows < 0) tile_rows = env_int("DLBLAS_FP8_TILE_ROWS", 0);
+  if (out_dtype == at::kFloat) tile_rows = 128;
+  require(a.is_contiguous() && b.is_contiguous(), "Input tensors must be contiguous");
+  require(a_s.is_contiguous() && b_s.is_contiguous(), "Scaling factor tensors must be contiguous");
+  const int64_t k = a.size(-1), m = a.numel() / k, n = b.size(0), kb = k / 128;
+  require(a_s.numel() == m * kb && b_s.numel() == (n + 127) / 128 * kb, "scale shapes do not match a / b");
+  Call c(a);
+  Tensor out;
+  if (a.dim() == 2) {
+    out = empty({m, n}, out_dtype, c);
+  } else {
+    std::vector<int64_t> shape = a.sizes().vec();
+    shape.back() = n;
+    out = empty(shape, out_dtype, c);
+  }
+  check(abi.dlb_fp8_gemm(a.data_ptr(), b.data_ptr(), a_s.data_ptr<float>(), kb, 1, b_s.data_ptr<float>(), out.data_ptr(),
+                         code(out_dtype), m, n, k, tile_rows, status_ptr(c), c.stream));
+  return out;
+}
+
+PyObject* py_fp8_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 6);
+    return wrap(fp8_gemm(tensor(a[0]), tensor(a[1]), tensor(a[2]), tensor(a[3]), dtype(a[4]), (int)integer(a[5])));
+  });
+}
+
+// ---- routing ------------------------------------------------------------------------------------------------------
+PyObject* py_route_softmax_topk(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 4);
+    const Tensor& logits = tensor(a[0]);
+    const int64_t top_k = integer(a[1]);
+    const at::ScalarType ids_dtype = dtype(a[3]);
+    require_cuda(logits);
+    require(logits.dim() == 2 && logits.is_contiguous(), "logits must be a contiguous 2-D tensor");
+    Call c(logits);
+    const int64_t t = logits.size(0);
+    Tensor w = empty({t, top_k}, at::kFloat, c), ids = empty({t, top_k}, ids_dtype, c);
+    check(abi.dlb_route_softmax_topk(logits.data_ptr(), code(logits.scalar_type()), t, (int)logits.size(1), (int)top_k,
+                                     truth(a[2]), w.data_ptr<float>(), ids.data_ptr(), code(ids_dtype), c.stream));
+    return wrap_tuple({&w, &ids});
+  });
+}
+
+PyObject* py_route_grouped_topk(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 6);
+    const Tensor& given = tensor(a[0]);
+    const Tensor& given_bias = tensor(a[1]);
+    const int64_t top_k = integer(a[2]);
+    require_cuda(given);
+    require_cuda(given_bias);
+    require(given.dim() == 2, "logits must be 2-D");
+    Call c(given);
+    const Tensor logits = given.is_contiguous() ? given : given.contiguous();
+    Tensor bias = given_bias.scalar_type() == at::kFloat ? given_bias : given_bias.to(at::kFloat);
+    if (!bias.is_contiguous()) bias = bias.contiguous();
+    const int64_t t = logits.size(0), e = logits.size(1);
+    require(bias.numel() == e, "the bias must have one entry per expert");
+    Tensor w = empty({t, top_k}, at::kFloat, c), ids = empty({t, top_k}, at::kInt, c);
+    check(abi.dlb_route_grouped_topk(logits.data_ptr(), code(logits.scalar_type()), bias.data_ptr<float>(), t, (int)e,
+                                     (int)integer(a[4]), (int)integer(a[5]), (int)top_k, truth(a[3]), w.data_ptr<float>(),
+                                     ids.data_ptr<int32_t>(), c.stream));
+    return wrap_tuple({&w, &ids});
+  });
+}
+
+// ---- the FP8 expert layer -----------------------------------------------------------------------------------------
+// plan -> quantise + permute (or permute) -> w13 GEMM with the silu * up + quantise epilogue -> w2 GEMM scattered back to
+// (token, slot) order with the routed weight -> sum over the slots.
+struct MoeArgs {
+  std::optional<Tensor> hidden, x_q, x_s;   // unquantised rows, or quantised ones with their scales
+  Tensor w1, w1_s, w2, w2_s, weights, ids;
+  int64_t top_k;
+  at::ScalarType out_dtype;
+  int64_t expert_offset, num_experts;
+  int quant_mode;
+  bool skip_unrouted, renormalize, fuse_swiglu;
+};
+
+Tensor moe_forward(const MoeArgs& g) {
+  const Tensor& x = g.hidden ? *g.hidden : *g.x_q;
+  require_cuda(x);
+  require_cuda(g.w1);
+  for (const Tensor* t : {&g.w1, &g.w1_s, &g.w2, &g.w2_s}) require(t->is_contiguous(), "weights and scales must be contiguous");
+  require(g.ids.scalar_type() == at::kInt || g.ids.scalar_type() == at::kLong, "topk_ids must be int32 or int64");
+  require(x.dim() == 2 && x.stride(1) == 1, "x must be 2-D with contiguous rows");
+  Call c(x);
+  const int64_t e_local = g.w1.size(0), n = g.w1.size(1), h = g.w1.size(2), inter = n / 2;
+  const int64_t m = x.size(0), slots = m * g.top_k;
+  Tensor out = empty({m, h}, g.out_dtype, c);
+  if (m == 0) return out;
+  require(x.size(1) == h, "hidden size mismatch");
+  require(g.ids.numel() == slots && g.weights.numel() == slots, "topk_ids / topk_weights must be [tokens, top_k]");
+  const Tensor ids = g.ids.is_contiguous() ? g.ids : g.ids.contiguous();
+  Tensor weights = g.weights;
+  bool renormalize = g.renormalize;
+  if (weights.scalar_type() != at::kFloat) {
+    if (renormalize) weights = weights / weights.sum(-1, true);
+    renormalize = false;
+    weights = weights.to(at::kFloat);
+  }
+  if (!weights.is_contiguous()) weights = weights.contiguous();
+  int tile_rows = env_int("DLBLAS_FP8_TILE_ROWS", 0);
+  if (tile_rows == 0 || g.out_dtype == at::kFloat) tile_rows = 128;
+  const bool fused = g.fuse_swiglu && n % 256 == 0;
+  const int max_tiles = (int)(slots / tile_rows + e_local);
+  const size_t out_size = c10::elementSize(g.out_dtype);
+  const size_t sort_bytes = abi.dlb_sort_by_expert_workspace_size(slots, (int)g.num_experts);
+
+  Workspace ws;
+  const size_t o_sorted = ws.take(slots * 8), o_pos = ws.take(slots * 4), o_tiles = ws.take((max_tiles + 1) * 16),
+               o_w = ws.take(renormalize ? slots * 4 : 0), o_sort = ws.take(sort_bytes), o_a = ws.take(slots * h),
+               o_as = ws.take(slots * (h / 128) * 4), o_hq = ws.take(slots * inter), o_hs = ws.take(slots * (inter / 128) * 4),
+               o_c1 = ws.take(fused ? 0 : slots * n * out_size), o_y = ws.take(slots * h * out_size);
+  ws.allocate(c);
+  int64_t* sorted_idx = ws.at<int64_t>(o_sorted);
+  int32_t* pos = ws.at<int32_t>(o_pos);
+  int32_t* tiles = ws.at<int32_t>(o_tiles);
+  int32_t* status = status_ptr(c);
+  const float* w = renormalize ? ws.at<float>(o_w) : weights.data_ptr<float>();
+  check(abi.dlb_moe_plan(ids.data_ptr(), code(ids.scalar_type()), m, (int)g.top_k, (int)g.num_experts, (int)g.expert_offset,
+                         (int)e_local, tile_rows, sorted_idx, pos, tiles, max_tiles,
+                         renormalize ? weights.data_ptr<float>() : nullptr, renormalize ? ws.at<float>(o_w) : nullptr,
+                         ws.at<void>(o_sort), sort_bytes, c.stream));
+  if (g.hidden) {
+    check(abi.dlb_quant_fp8(x.data_ptr(), code(x.scalar_type()), m, h, x.stride(0), 128, g.quant_mode, 1e-10f,
+                            ws.at<void>(o_a), ws.at<float>(o_as), h / 128, 1, pos, (int)g.top_k, c.stream));
+  } else {
+    require(x.is_contiguous() && x.element_size() == 1, "quantised rows must be contiguous e4m3");
+    const Tensor x_s = g.x_s->is_contiguous() ? *g.x_s : g.x_s->contiguous();
+    require(x_s.scalar_type() == at::kFloat && x_s.numel() == m * (h / 128), "scales must be fp32 [tokens, hidden / 128]");
+    check(abi.dlb_permute_rows(x.data_ptr(), h, x_s.data_ptr<float>(), h / 128, m, pos, (int)g.top_k, ws.at<void>(o_a),
+                               ws.at<float>(o_as), c.stream));
+  }
+  auto gemm = [&](size_t a, size_t a_s, int64_t nn, int64_t kk, const Tensor& b, const Tensor& b_s, int epilogue, size_t dst,
+                  size_t q_scale, int64_t ldc) {
+    check(abi.dlb_moe_grouped_gemm(ws.at<void>(a), ws.at<float>(a_s), slots, b.data_ptr(), b_s.data_ptr<float>(), (int)e_local,
+                                   nn, kk, tiles, max_tiles, tile_rows, epilogue, ws.at<void>(dst), code(g.out_dtype), ldc,
+                                   epilogue == DLB_EPI_SWIGLU_QUANT ? ws.at<float>(q_scale) : nullptr, g.quant_mode, 1e-10f,
+                                   epilogue == DLB_EPI_SCATTER_WEIGHT ? sorted_idx : nullptr,
+                                   epilogue == DLB_EPI_SCATTER_WEIGHT ? w : nullptr, status, c.stream));
+  };
+  if (fused) {
+    gemm(o_a, o_as, n, h, g.w1, g.w1_s, DLB_EPI_SWIGLU_QUANT, o_hq, o_hs, inter);
+  } else {
+    gemm(o_a, o_as, n, h, g.w1, g.w1_s, DLB_EPI_STORE, o_c1, 0, n);
+    check(abi.dlb_silu_mul_quant(ws.at<void>(o_c1), code(g.out_dtype), slots, inter, g.quant_mode, 1e-10f, 0, nullptr, 0,
+                                 ws.at<void>(o_hq), ws.at<float>(o_hs), c.stream));
+  }
+  gemm(o_hq, o_hs, h, inter, g.w2, g.w2_s, DLB_EPI_SCATTER_WEIGHT, o_y, 0, h);
+  check(abi.dlb_moe_sum_topk(ws.at<void>(o_y), code(g.out_dtype), m, (int)g.top_k, h, ids.data_ptr(), code(ids.scalar_type()),
+                             g.expert_offset, g.expert_offset + e_local, g.skip_unrouted, out.data_ptr(), c.stream));
+  return out;
+}
+
+PyObject* py_moe_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 17);
+    MoeArgs g{opt_tensor(a[0]), opt_tensor(a[1]), opt_tensor(a[2]), tensor(a[3]), tensor(a[4]), tensor(a[5]), tensor(a[6]),
+              tensor(a[7]), tensor(a[8]), integer(a[9]), dtype(a[10]), integer(a[11]), integer(a[12]), (int)integer(a[13]),
+              truth(a[14]), truth(a[15]), truth(a[16])};
+    return wrap(moe_forward(g));
+  });
+}
+
+// ---- module -------------------------------------------------------------------------------------------------------
+// bind({name: address}): the C ABI to call
+PyObject* py_bind(PyObject*, PyObject* arg) {
+  return guarded([&]() -> PyObject* {
+    auto address = [&](const char* name) -> void* {
+      PyObject* v = PyDict_Check(arg) ? PyDict_GetItemString(arg, name) : nullptr;
+      if (v == nullptr) throw std::runtime_error(std::string("dlblas_b200: no address for ") + name);
+      void* p = PyLong_AsVoidPtr(v);
+      if (p == nullptr) throw PyFailed{};
+      return p;
+    };
+#define X(name) abi.name = reinterpret_cast<decltype(abi.name)>(address(#name));
+    ABI_FUNCTIONS(X)
+#undef X
+    Py_RETURN_NONE;
+  });
+}
+
+PyObject* py_status_word(PyObject*, PyObject* arg) {
+  return guarded([&] { return wrap(status_word((at::DeviceIndex)integer(arg))); });
+}
+
+#define FAST(name, fn) {name, (PyCFunction)(void (*)(void))fn, METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {
+    {"bind", py_bind, METH_O, nullptr},
+    {"status_word", py_status_word, METH_O, nullptr},
+    FAST("quant_fp8", py_quant_fp8),
+    FAST("group_quant_fp8", py_group_quant_fp8),
+    FAST("fp8_gemm", py_fp8_gemm),
+    FAST("route_softmax_topk", py_route_softmax_topk),
+    FAST("route_grouped_topk", py_route_grouped_topk),
+    FAST("moe_forward", py_moe_forward),
+    {nullptr, nullptr, 0, nullptr},
+};
+
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+extern "C" __attribute__((visibility("default"))) PyObject* PyInit__host(void) { return PyModule_Create(&module); }

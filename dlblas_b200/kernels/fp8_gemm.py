@@ -1,7 +1,7 @@
 """`dlblas.kernels.fp8_gemm` (dlblas/kernels/fp8_gemm.py:68-89 of the reference)."""
 import torch
 
-from .. import ops
+from .._C import host
 
 
 def fp8_gemm(a: torch.Tensor, b: torch.Tensor, a_s: torch.Tensor, b_s: torch.Tensor) -> torch.Tensor:
@@ -11,6 +11,4 @@ def fp8_gemm(a: torch.Tensor, b: torch.Tensor, a_s: torch.Tensor, b_s: torch.Ten
     b_s: [N/128, K/128] fp32.  As in the reference the output dtype is
     `torch.get_default_dtype()` (callers set bf16).  Runs the tcgen05 kernel of the CUDA extension.
     """
-    assert a.is_contiguous() and b.is_contiguous(), "Input tensors must be contiguous"
-    assert a_s.is_contiguous() and b_s.is_contiguous(), "Scaling factor tensors must be contiguous"
-    return ops.fp8_gemm(a, b, a_s, b_s, out_dtype=torch.get_default_dtype())
+    return host().fp8_gemm(a, b, a_s, b_s, torch.get_default_dtype(), -1)

@@ -48,8 +48,7 @@ def biased_grouped_topk(hidden_states: torch.Tensor, gating_output: torch.Tensor
     (:506-514) and is not offered here."""
     assert hidden_states.shape[0] == gating_output.shape[0], "Number of tokens mismatch"
     assert n_share_experts_fusion == 0, "n_share_experts_fusion is not supported"
-    return ops.route_grouped_topk(gating_output.contiguous(), correction_bias, topk, renormalize, num_expert_group,
-                                  topk_group)
+    return _C.host().route_grouped_topk(gating_output, correction_bias, topk, renormalize, num_expert_group, topk_group)
 
 
 def map_logic_to_physical_idx_hash_random(topk_idx: torch.Tensor, log2phy: torch.Tensor, logcnt: torch.Tensor,

@@ -1,8 +1,9 @@
 """`dlblas.layers.moe.kernels.blocked_fp8_fused_moe` (dlblas/layers/moe/kernels/blocked_fp8_fused_moe.py of
 the reference): the block-scaled FP8 fused MoE function (:261-338) and the grouped-GEMM launcher (:159-242).
 
-Pipeline of `moe_expert_forward` (all kernels from the CUDA extension, one launch each):
-  sort_by_expert -> build_tiles -> quantise+permute (or permute) the tokens into expert-contiguous order ->
+Pipeline of `moe_expert_forward` (all kernels from the CUDA extension; one call into csrc/host.cpp, except for the
+expert-parallel path that wants the slots' rows):
+  sort_by_expert + build_tiles -> quantise+permute (or permute) the tokens into expert-contiguous order ->
   grouped GEMM w13 with the silu*up + FP8 re-quantisation epilogue -> grouped GEMM w2 with the routed-weight
   epilogue scattered back to (token, slot) order -> sum over the top-k slots.
 """
@@ -29,17 +30,23 @@ def moe_expert_forward(hidden: Optional[torch.Tensor], x_q: Optional[torch.Tenso
                        quant_mode: int = _C.QUANT_RECIP_MUL, weighted_combine: bool = False,
                        fuse_swiglu: bool = True, group_size: int = 128,
                        skip_unrouted_rows: bool = False, return_slot_rows: bool = False,
-                       w2_column_parts: int = 1, on_columns_done=None, sm_margin: int = 0) -> torch.Tensor:
+                       w2_column_parts: int = 1, on_columns_done=None, sm_margin: int = 0,
+                       renormalize: bool = False) -> torch.Tensor:
     """Expert computation for tokens that are either unquantised (`hidden` [M, H]) or already
     quantised (`x_q` e4m3 [M, H], `x_s` fp32 [M, H/128]).  topk_ids are global ids in
     [expert_offset, expert_offset + E_local) for the experts held in w1/w2; any other id (e.g. -1)
-    contributes zero.  Returns [M, H] of out_dtype.
+    contributes zero; with `renormalize` a token's weights are divided by their sum first.  Returns [M, H] of out_dtype.
 
     With `return_slot_rows` and `w2_column_parts` > 1 the second GEMM runs in that many launches over windows of the
     hidden dimension; `on_columns_done(y, col_begin, col_count)` is called after each launch has been queued (the
     expert-parallel combine pushes those columns back from another stream), and every launch but the first leaves
     `sm_margin` SMs to that stream."""
     assert group_size == 128, "block size 128 is the only supported quantisation group"
+    if not return_slot_rows:
+        return _C.host().moe_forward(hidden, x_q, x_s, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids, topk, out_dtype,
+                                     expert_offset, w1.shape[0] if num_experts is None else num_experts, quant_mode,
+                                     skip_unrouted_rows, renormalize, fuse_swiglu)
+    topk_weights = _renormalize(topk_weights, renormalize)
     e_local, n, h = w1.shape
     inter = n // 2
     m = hidden.shape[0] if hidden is not None else x_q.shape[0]
@@ -76,7 +83,7 @@ def moe_expert_forward(hidden: Optional[torch.Tensor], x_q: Optional[torch.Tenso
         ops.grouped_gemm(a1, a1_s, w1, w1_scale, tiles, max_tiles, _C.EPI_STORE, c1, tile_rows=tile_rows)
         ops.silu_mul_quant(c1, quant_mode, 1e-10, False, None, h_q, h_s)
     y = torch.empty(s_rows, h, dtype=out_dtype, device=dev)
-    parts = w2_column_parts if (return_slot_rows and h % (256 * max(w2_column_parts, 1)) == 0) else 1
+    parts = w2_column_parts if h % (256 * max(w2_column_parts, 1)) == 0 else 1
     if parts > 1:
         step = h // parts
         for p in range(parts):
@@ -88,11 +95,9 @@ def moe_expert_forward(hidden: Optional[torch.Tensor], x_q: Optional[torch.Tenso
         return y
     ops.grouped_gemm(h_q, h_s, w2, w2_scale, tiles, max_tiles, _C.EPI_SCATTER_WEIGHT, y, sorted_idx=sorted_idx,
                      weights=weights, tile_rows=tile_rows)
-    if return_slot_rows:
-        # [M * topk, H] rows of the individual (token, slot) results, already weighted; the caller sums them
-        # (the expert-parallel combine does it while pushing the rows to their source rank)
-        return y
-    return ops.sum_topk(y, m, topk, ids, expert_offset, expert_offset + e_local, skip_unrouted_rows)
+    # [M * topk, H] rows of the individual (token, slot) results, already weighted; the caller sums them
+    # (the expert-parallel combine does it while pushing the rows to their source rank)
+    return y
 
 
 def fused_moe_blocked_fp8_kernel_launcher(A: torch.Tensor, A_scale: torch.Tensor, B: torch.Tensor,
@@ -140,8 +145,7 @@ def dlblas_fused_moe_blocked_fp8(input: torch.Tensor, input_scale: torch.Tensor,
         num_experts = e_local
         if ep_size > 1:
             num_experts = num_experts * ep_size
-    topk_weights = _renormalize(topk_weights, renormalize)
     if expert_offset != 0:
         topk_ids[topk_ids != -1] += expert_offset
     return moe_expert_forward(None, input, input_scale, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids, topk,
-                              out_dtype, expert_offset, num_experts)
+                              out_dtype, expert_offset, num_experts, renormalize=renormalize)

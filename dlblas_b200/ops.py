@@ -4,12 +4,10 @@ the CUDA extension.  The modules that mirror the reference's layout
 (`dlblas_b200.kernels.*`, `dlblas_b200.layers.moe.*`) are built on these."""
 from typing import Optional, Tuple
 
-import os
-
 import torch
 
 from . import _C
-from ._C import check, dtype_code, lib, ptr, require_cuda, stream
+from ._C import check, dtype_code, host, lib, ptr, require_cuda, stream
 
 FP8 = torch.float8_e4m3fn
 
@@ -68,21 +66,9 @@ def quant_fp8(x: torch.Tensor, group_size: int = 128, mode: int = _C.QUANT_RECIP
               column_major_scales: bool = False, dst_pos: Optional[torch.Tensor] = None, fanout: int = 1,
               rows_out: Optional[int] = None, out_dtype: torch.dtype = FP8):
     """1xG quantisation of a 2-D tensor; with dst_pos, row t is written to rows dst_pos[t*fanout + j]."""
-    require_cuda(x)
-    assert x.dim() == 2 and x.stride(-1) == 1, "x must be 2-D with contiguous rows"
     assert out_dtype == FP8, "only torch.float8_e4m3fn is supported"
-    m, k = x.shape
-    assert k % group_size == 0, f"the last dimension of 'x' {k} must be divisible by 'group_size' {group_size}"
-    rows = m if rows_out is None else rows_out
-    g = k // group_size
-    q = torch.empty(rows, k, dtype=FP8, device=x.device)
-    if column_major_scales:
-        s = torch.empty(g, rows, dtype=torch.float32, device=x.device).t()
-    else:
-        s = torch.empty(rows, g, dtype=torch.float32, device=x.device)
-    check(lib().dlb_quant_fp8(ptr(x), dtype_code(x.dtype), m, k, x.stride(0), group_size, mode, eps, ptr(q), ptr(s),
-                              s.stride(0), s.stride(1), ptr(dst_pos), fanout, stream(x.device)))
-    return q, s
+    return host().quant_fp8(x, group_size, mode, eps, column_major_scales, dst_pos, fanout,
+                            -1 if rows_out is None else rows_out)
 
 
 def permute_rows(q: torch.Tensor, scales: Optional[torch.Tensor], dst_pos: torch.Tensor, fanout: int, rows_out: int):
@@ -140,23 +126,7 @@ def silu_mul_quant(gate_up: torch.Tensor, mode: int = _C.QUANT_RECIP_MUL, eps: f
 def fp8_gemm(a: torch.Tensor, b: torch.Tensor, a_s: torch.Tensor, b_s: torch.Tensor,
              out_dtype: torch.dtype = torch.bfloat16, tile_rows: Optional[int] = None) -> torch.Tensor:
     """tile_rows: 128 / 256 (pairs of CTAs) / None = DLBLAS_FP8_TILE_ROWS or the library's choice."""
-    require_cuda(a, b, a_s, b_s)
-    if tile_rows is None:
-        tile_rows = int(os.environ.get("DLBLAS_FP8_TILE_ROWS", "0"))
-    if out_dtype == torch.float32:
-        tile_rows = 128
-    assert a.is_contiguous() and b.is_contiguous(), "Input tensors must be contiguous"
-    assert a_s.is_contiguous() and b_s.is_contiguous(), "Scaling factor tensors must be contiguous"
-    k = a.size(-1)
-    m = a.numel() // k
-    n = b.size(0)
-    c = torch.empty(*a.size()[:-1], n, dtype=out_dtype, device=a.device)
-    kb = k // 128
-    a_s2 = a_s.view(m, -1) if m > 0 else a_s
-    assert a_s.numel() == m * kb and b_s.numel() == ((n + 127) // 128) * kb, "scale shapes do not match a / b"
-    check(lib().dlb_fp8_gemm(ptr(a), ptr(b), ptr(a_s2), kb, 1, ptr(b_s), ptr(c), dtype_code(out_dtype), m, n, k,
-                             int(tile_rows), ptr(_C.status_word(a.device)), stream(a.device)))
-    return c
+    return host().fp8_gemm(a, b, a_s, b_s, out_dtype, -1 if tile_rows is None else tile_rows)
 
 
 def grouped_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Tensor, tiles: torch.Tensor,
@@ -272,28 +242,12 @@ def eplb_map_hash(topk_idx: torch.Tensor, log2phy: torch.Tensor, logcnt: torch.T
 
 
 def route_softmax_topk(logits: torch.Tensor, top_k: int, renormalize: bool = False, ids_dtype=torch.int64):
-    require_cuda(logits)
-    assert logits.dim() == 2 and logits.is_contiguous()
-    t, e = logits.shape
-    w = torch.empty(t, top_k, dtype=torch.float32, device=logits.device)
-    ids = torch.empty(t, top_k, dtype=ids_dtype, device=logits.device)
-    check(lib().dlb_route_softmax_topk(ptr(logits), dtype_code(logits.dtype), t, e, top_k, int(renormalize), ptr(w),
-                                       ptr(ids), dtype_code(ids_dtype), stream(logits.device)))
-    return w, ids
+    return host().route_softmax_topk(logits, top_k, renormalize, ids_dtype)
 
 
 def route_grouped_topk(logits: torch.Tensor, bias: torch.Tensor, top_k: int, renormalize: bool, num_expert_group: int,
                        topk_group: int):
-    require_cuda(logits, bias)
-    assert logits.dim() == 2 and logits.is_contiguous()
-    t, e = logits.shape
-    bias = bias.to(torch.float32).contiguous()
-    assert bias.numel() == e
-    w = torch.empty(t, top_k, dtype=torch.float32, device=logits.device)
-    ids = torch.empty(t, top_k, dtype=torch.int32, device=logits.device)
-    check(lib().dlb_route_grouped_topk(ptr(logits), dtype_code(logits.dtype), ptr(bias), t, e, num_expert_group,
-                                       topk_group, top_k, int(renormalize), ptr(w), ptr(ids), stream(logits.device)))
-    return w, ids
+    return host().route_grouped_topk(logits, bias, top_k, renormalize, num_expert_group, topk_group)
 
 
 def topk_gating_bwd(ws: torch.Tensor, dtype, tokens: int, experts: int, k: int, capacity: int, grad_l_aux: torch.Tensor,
