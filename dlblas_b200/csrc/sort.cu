@@ -35,7 +35,7 @@ struct IdStats {
 };
 
 template <typename IdT, bool STATS = false>
-__device__ __forceinline__ int bucket_of(const IdT* __restrict__ ids, long long f, long long end, int num_experts,
+__device__ __forceinline__ int bucket_of(const IdT* __restrict__ ids, unsigned f, unsigned end, int num_experts,
                                          int negative_as, IdStats* st = nullptr) {
   if (f >= end) return num_experts + 2;  // spare slot for idle lanes
   long long v = (long long)ids[f];
@@ -76,10 +76,10 @@ __host__ __device__ constexpr int hist_stride(int num_experts) {   // 32-bit wor
 // distinct values one after another, and with some thirty different experts in a warp that was most of the kernel.
 __device__ __forceinline__ int warp_rank_step(Count* hist, int bucket, int lane, int bits) {
   unsigned peers = 0xffffffffu;
+#pragma unroll 4
   for (int i = 0; i < bits; ++i) {
-    const bool one = (bucket >> i) & 1;
-    const unsigned m = __ballot_sync(0xffffffffu, one);
-    peers &= one ? m : ~m;
+    const unsigned one = (bucket >> i) & 1u;
+    peers &= __ballot_sync(0xffffffffu, one) ^ (one - 1u);
   }
   const int rank = __popc(peers & ((1u << lane) - 1u));
   const int old = hist[bucket];
@@ -117,33 +117,40 @@ __device__ __forceinline__ void scan_and_write_segments(const int* total, int* b
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   unsigned long long carry = 0;      // high half: tiles, low half: slots
   for (int b0 = 0; b0 < nb; b0 += blockDim.x) {
+    const int busy = min(warps, (nb - b0 + 31) / 32);   // warps that hold buckets of this pass
     const int b = b0 + threadIdx.x;
-    unsigned long long v = 0;
-    if (b < nb) {
-      v = (unsigned)total[b];
-      const int e = b - 1 - o.expert_offset;
-      if (o.tile_rows > 0 && e >= 0 && e < o.num_local && b < nb - 1)
-        v |= (unsigned long long)((total[b] + o.tile_rows - 1) / o.tile_rows) << 32;
+    unsigned long long v = 0, inc = 0;
+    if (warp < busy) {
+      if (b < nb) {
+        v = (unsigned)total[b];
+        const int e = b - 1 - o.expert_offset;
+        if (o.tile_rows > 0 && e >= 0 && e < o.num_local && b < nb - 1)
+          v |= (unsigned long long)((unsigned)(total[b] + o.tile_rows - 1) / (unsigned)o.tile_rows) << 32;
+      }
+      inc = v;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, inc, d);
+        if (lane >= d) inc += y;
+      }
+      if (lane == 31) warp_sums[warp] = inc;
     }
-    unsigned long long inc = v;
+    __syncthreads();
+    // the sums of the (at most 32) warps, added up by every warp for itself
+    const unsigned long long s = lane < busy ? warp_sums[lane] : 0ull;
+    unsigned long long incl = s;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-      const unsigned long long y = __shfl_up_sync(0xffffffffu, inc, d);
-      if (lane >= d) inc += y;
+      if (d >= busy) break;
+      const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += y;
     }
-    if (lane == 31) warp_sums[warp] = inc;
-    __syncthreads();
-    unsigned long long before = carry, all = 0;
-    for (int w = 0; w < warps; ++w) {
-      const unsigned long long s = warp_sums[w];
-      if (w < warp) before += s;
-      all += s;
-    }
+    const unsigned long long before = carry + __shfl_sync(0xffffffffu, incl - s, min(warp, busy - 1)) + inc - v;
     if (b < nb) {
-      base[b] = (int)(unsigned)(before + inc - v);
-      if (o.tile_rows > 0) tile_first[b] = (int)((before + inc - v) >> 32);
+      base[b] = (int)(unsigned)before;
+      if (o.tile_rows > 0) tile_first[b] = (int)(before >> 32);
     }
-    carry += all;
+    carry += __shfl_sync(0xffffffffu, incl, busy - 1);
     __syncthreads();
   }
   for (int e = part * blockDim.x + threadIdx.x; e < num_experts; e += parts * blockDim.x) {
@@ -184,7 +191,7 @@ __device__ __forceinline__ void scan_and_write_segments(const int* total, int* b
 
 // Output of slot f, which is at place `pos` of the sorted order.
 template <typename IdT>
-__device__ __forceinline__ void write_slot(long long f, long long n, int bucket, int pos, const int* base,
+__device__ __forceinline__ void write_slot(unsigned f, unsigned n, int bucket, int pos, const int* base,
                                            const int* tile_first, int num_experts, const SortOut& o) {
   const bool expert = bucket >= 1 && bucket <= num_experts;
   if (o.sorted_idx) o.sorted_idx[pos] = f;
@@ -199,12 +206,12 @@ __device__ __forceinline__ void write_slot(long long f, long long n, int bucket,
     const int d = pos - base[1];                      // base[1]: slots without an expert, which sort first
     const int out = expert && d < o.dest_limit ? d : -1;
     o.dest[f] = out;
-    const unsigned t = (unsigned)f / (unsigned)o.top_k, j = (unsigned)f - t * (unsigned)o.top_k;
-    o.row_map[(long long)j * (n / o.top_k) + t] = out;
+    const unsigned t = f / (unsigned)o.top_k, j = f - t * (unsigned)o.top_k;
+    o.row_map[j * (n / (unsigned)o.top_k) + t] = out;
   }
   if (o.w_out) {
     // weights of a token divided by their sum (added up in slot order)
-    const float* w = o.w_in + (unsigned)f / (unsigned)o.top_k * (unsigned)o.top_k;
+    const float* w = o.w_in + f / (unsigned)o.top_k * (unsigned)o.top_k;
     float sum = 0.f;
     for (int j = 0; j < o.top_k; ++j) sum += __ldg(w + j);
     o.w_out[f] = __ldg(o.w_in + f) / sum;
@@ -213,7 +220,7 @@ __device__ __forceinline__ void write_slot(long long f, long long n, int bucket,
 
 // ---- one block ---------------------------------------------------------------------
 template <typename IdT, int ITEMS>
-__global__ void __launch_bounds__(MAX_WARPS * 32) sort_one_block_kernel(const IdT* __restrict__ ids, long long n,
+__global__ void __launch_bounds__(MAX_WARPS * 32) sort_one_block_kernel(const IdT* __restrict__ ids, unsigned n,
                                                                         int num_experts, SortOut o) {
   extern __shared__ int sm[];
   const int nb = num_experts + 2;
@@ -225,7 +232,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32) sort_one_block_kernel(const Id
   int* tile_first = base + nb;             // [nb]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int bits = 32 - __clz(nb);         // buckets 0 ... nb, the last one for idle lanes
-  const long long begin = (long long)warp * ITEMS * 32;
+  const unsigned begin = warp * ITEMS * 32;
   int bucket[ITEMS], before[ITEMS];
   IdStats st;
 #pragma unroll
@@ -250,7 +257,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32) sort_one_block_kernel(const Id
   scan_and_write_segments(total, base, tile_first, num_experts, o, 0, 1);
 #pragma unroll
   for (int i = 0; i < ITEMS; ++i) {
-    const long long f = begin + i * 32 + lane;
+    const unsigned f = begin + i * 32 + lane;
     if (f < n)
       write_slot<IdT>(f, n, bucket[i], base[bucket[i]] + my[bucket[i]] + before[i], base, tile_first, num_experts, o);
   }
@@ -260,8 +267,8 @@ __global__ void __launch_bounds__(MAX_WARPS * 32) sort_one_block_kernel(const Id
 // stats: the caller's {largest, equal to -1, below 0}; run[0..2] holds the running values and run[3] counts the blocks
 // that are done (the last one, which waits for nobody, hands the values over), all of it {-1, 0, 0, 0} before the launch.
 template <typename IdT>
-__global__ void __launch_bounds__(512) sort_count_kernel(const IdT* __restrict__ ids, long long n, int num_experts,
-                                                         long long chunk, int negative_as, int* __restrict__ cnt,
+__global__ void __launch_bounds__(512) sort_count_kernel(const IdT* __restrict__ ids, unsigned n, int num_experts,
+                                                         unsigned chunk, int negative_as, int* __restrict__ cnt,
                                                          int* __restrict__ stats, int* __restrict__ run) {
   extern __shared__ int sm[];
   __shared__ int stats_s[3];
@@ -269,15 +276,16 @@ __global__ void __launch_bounds__(512) sort_count_kernel(const IdT* __restrict__
   for (int b = threadIdx.x; b < nb + 1; b += blockDim.x) sm[b] = 0;
   if (threadIdx.x < 3) stats_s[threadIdx.x] = threadIdx.x == 0 ? -1 : 0;
   __syncthreads();
-  const long long begin = blockIdx.x * chunk, end = min(begin + chunk, n);
+  const unsigned begin = blockIdx.x * chunk, end = min(begin + chunk, n);   // n < 2^31
   IdStats st;
-  for (long long f0 = begin; f0 < end; f0 += 4 * 512) {
+  for (unsigned f0 = begin; f0 < end; f0 += 4 * 512) {
     int b[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
       b[i] = bucket_of<IdT, true>(ids, f0 + i * 512 + threadIdx.x, end, num_experts, negative_as, &st);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) atomicAdd(sm + b[i], 1);
+    for (int i = 0; i < 4; ++i)
+      if (b[i] < nb) atomicAdd(sm + b[i], 1);
   }
   if (stats != nullptr) add_stats(st, stats_s);
   __syncthreads();
@@ -326,8 +334,8 @@ __global__ void __launch_bounds__(256) sort_scan_chunks_kernel(int* cnt, int num
 
 // total != nullptr: cnt already holds prefixes over the chunks (sort_scan_chunks_kernel); otherwise plain histograms.
 template <typename IdT>
-__global__ void __launch_bounds__(MAX_WARPS * 32) sort_scatter_kernel(const IdT* __restrict__ ids, long long n,
-                                                                      int num_experts, long long chunk,
+__global__ void __launch_bounds__(MAX_WARPS * 32) sort_scatter_kernel(const IdT* __restrict__ ids, unsigned n,
+                                                                      int num_experts, unsigned chunk,
                                                                       const int* __restrict__ cnt,
                                                                       const int* __restrict__ total_in, SortOut o) {
   extern __shared__ int sm[];
@@ -365,10 +373,10 @@ __global__ void __launch_bounds__(MAX_WARPS * 32) sort_scatter_kernel(const IdT*
   }
   __syncthreads();
   scan_and_write_segments(total, base, tile_first, num_experts, o, c, gridDim.x);
-  const long long begin = (long long)c * chunk, end = min(begin + chunk, n);
+  const unsigned begin = c * chunk, end = min(begin + chunk, n);
   Count* my = reinterpret_cast<Count*>(hist + warp * stride);
-  for (long long p0 = begin; p0 < end; p0 += CHUNK_STEP) {
-    const long long first = p0 + (long long)warp * CHUNK_ITEMS * 32;
+  for (unsigned p0 = begin; p0 < end; p0 += CHUNK_STEP) {
+    const unsigned first = p0 + warp * CHUNK_ITEMS * 32;
     int bucket[CHUNK_ITEMS], before[CHUNK_ITEMS];
 #pragma unroll
     for (int i = 0; i < CHUNK_ITEMS; ++i)
@@ -383,7 +391,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32) sort_scatter_kernel(const IdT*
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < CHUNK_ITEMS; ++i) {
-      const long long f = first + i * 32 + lane;
+      const unsigned f = first + i * 32 + lane;
       const int b = bucket[i];
       if (f < end) write_slot<IdT>(f, n, b, base[b] + mine[b] + my[b] + before[i], base, tile_first, num_experts, o);
     }
@@ -449,7 +457,7 @@ int launch_one_block(const IdT* ids, long long n, int num_experts, const SortOut
                         "cudaFuncSetAttribute(sort_one_block_kernel)");
     if (rc != DLB_OK) return rc;
   }
-  sort_one_block_kernel<IdT, ITEMS><<<1, p.warps * 32, p.smem, st>>>(ids, n, num_experts, o);
+  sort_one_block_kernel<IdT, ITEMS><<<1, p.warps * 32, p.smem, st>>>(ids, (unsigned)n, num_experts, o);
   count_launch();
   DLB_CHECK_LAUNCH("sort_one_block_kernel");
   if (o.stats_event != nullptr) return check_cuda(cudaEventRecord((cudaEvent_t)o.stats_event, st), "cudaEventRecord");
@@ -481,7 +489,7 @@ int run_sort(const IdT* ids, long long n, int num_experts, const SortOut& o, voi
     cudaMemsetAsync(run, 0xff, 4, st);
     cudaMemsetAsync(run + 1, 0, 12, st);
   }
-  sort_count_kernel<IdT><<<p.num_chunks, 512, (size_t)(nb + 1) * 4, st>>>(ids, n, num_experts, p.chunk, o.negative_as, cnt,
+  sort_count_kernel<IdT><<<p.num_chunks, 512, (size_t)(nb + 1) * 4, st>>>(ids, (unsigned)n, num_experts, (unsigned)p.chunk, o.negative_as, cnt,
                                                                          o.stats, run);
   count_launch();
   DLB_CHECK_LAUNCH("sort_count_kernel");
@@ -501,7 +509,7 @@ int run_sort(const IdT* ids, long long n, int num_experts, const SortOut& o, voi
                         "cudaFuncSetAttribute(sort_scatter_kernel)");
     if (rc != DLB_OK) return rc;
   }
-  sort_scatter_kernel<IdT><<<p.num_chunks, MAX_WARPS * 32, p.smem, st>>>(ids, n, num_experts, p.chunk, cnt,
+  sort_scatter_kernel<IdT><<<p.num_chunks, MAX_WARPS * 32, p.smem, st>>>(ids, (unsigned)n, num_experts, (unsigned)p.chunk, cnt,
                                                                         scan ? total : nullptr, o);
   count_launch();
   DLB_CHECK_LAUNCH("sort_scatter_kernel");
