@@ -1,5 +1,7 @@
-// Routing kernels: one warp per token row, scores in registers, warp-shuffle arg-max with
-// a deterministic tie-break (lowest expert index wins).
+// Routing kernels: one warp per token row, scores in registers, arg-max over the warp with a deterministic
+// tie-break (lowest expert index wins).  What bounds them is the chain of arg-max rounds, not memory: a round is two integer
+// warp reductions (redux) on an order-preserving key and on the index, where a butterfly of shuffles took ten of them and
+// ten compare-and-selects.
 #include "common.cuh"
 #include "sort.cuh"
 
@@ -17,15 +19,19 @@ struct ArgMax {
 __device__ __forceinline__ ArgMax better(ArgMax a, ArgMax b) {
   return (b.v > a.v || (b.v == a.v && b.i < a.i)) ? b : a;
 }
+// fp32 as an unsigned integer of the same order; -0 counts as +0, and a NaN comes last (it is never chosen)
+__device__ __forceinline__ uint32_t order_key(float v) {
+  const uint32_t b = __float_as_uint(v + 0.f);
+  return v != v ? 0u : b ^ ((uint32_t)((int32_t)b >> 31) | 0x80000000u);
+}
+__device__ __forceinline__ float key_value(uint32_t k) {
+  return k == 0u ? -__builtin_huge_valf() : __uint_as_float((k & 0x80000000u) ? k ^ 0x80000000u : ~k);
+}
 __device__ __forceinline__ ArgMax warp_argmax(ArgMax a) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    ArgMax b;
-    b.v = __shfl_xor_sync(0xffffffffu, a.v, o);
-    b.i = __shfl_xor_sync(0xffffffffu, a.i, o);
-    a = better(a, b);
-  }
-  return a;
+  const uint32_t key = order_key(a.v);
+  const uint32_t best = __reduce_max_sync(0xffffffffu, key);
+  const unsigned at = __reduce_min_sync(0xffffffffu, key == best ? (unsigned)a.i : 0x7fffffffu);
+  return ArgMax{key_value(best), (int)at};
 }
 
 constexpr float NEG_INF = -__builtin_huge_valf();
@@ -207,6 +213,104 @@ __global__ void __launch_bounds__(WARPS * 32) grouped_topk_kernel(const T* __res
       my_id = a.i;
     }
     knock_out<VPT>(ch, a.i, lane);
+  }
+  if (lane < top_k) {
+    weights[t * top_k + lane] = renorm ? my_w / wsum : my_w;
+    ids[t * top_k + lane] = my_id;
+  }
+}
+
+// The same for 32 * VPT experts in groups of whole lanes: lane l holds experts [l * VPT, (l + 1) * VPT), so that a group is a
+// power of two of neighbouring lanes (`group_lanes`).  All groups' two largest scores then come out of one butterfly over
+// group_lanes lanes (the kernel above takes two arg-max rounds per group: 16 of its 28 rounds with 8 groups), a lane's
+// position is its experts' position, so the lowest index among equal scores is the lowest lane of a ballot, and a round only
+// touches the winner's registers.
+template <typename T, int VPT, bool VEC>
+__global__ void __launch_bounds__(WARPS * 32) grouped_topk_lanes_kernel(const T* __restrict__ logits,
+                                                                        const float* __restrict__ bias, long long tokens,
+                                                                        int num_groups, int group_lanes, int topk_group,
+                                                                        int top_k, int renorm, float* __restrict__ weights,
+                                                                        int* __restrict__ ids) {
+  const int lane = threadIdx.x & 31;
+  const long long t = (long long)blockIdx.x * WARPS + (threadIdx.x >> 5);
+  if (t >= tokens) return;
+  float sc[VPT], ch[VPT];
+  {
+    const T* row = logits + t * (32 * VPT) + lane * VPT;
+    constexpr int BYTES = VPT * sizeof(T);
+    alignas(16) T x[VPT];
+    if constexpr (VEC && BYTES % 16 == 0) {
+#pragma unroll
+      for (int i = 0; i < BYTES / 16; ++i) reinterpret_cast<uint4*>(x)[i] = __ldg(reinterpret_cast<const uint4*>(row) + i);
+    } else if constexpr (VEC && BYTES % 8 == 0) {
+#pragma unroll
+      for (int i = 0; i < BYTES / 8; ++i) reinterpret_cast<uint2*>(x)[i] = __ldg(reinterpret_cast<const uint2*>(row) + i);
+    } else {
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) x[i] = row[i];
+    }
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      sc[i] = sigmoid_exact(to_f32<T>(x[i]));
+      ch[i] = sc[i] + __ldg(bias + lane * VPT + i);
+    }
+  }
+  // the two largest scores of the lane, then of its group
+  float v1 = ch[0], v2 = NEG_INF;
+#pragma unroll
+  for (int i = 1; i < VPT; ++i) {
+    v2 = fmaxf(v2, fminf(v1, ch[i]));
+    v1 = fmaxf(v1, ch[i]);
+  }
+  for (int o = 1; o < group_lanes; o <<= 1) {
+    const float w1 = __shfl_xor_sync(0xffffffffu, v1, o), w2 = __shfl_xor_sync(0xffffffffu, v2, o);
+    v2 = fmaxf(fminf(v1, w1), fmaxf(v2, w2));
+    v1 = fmaxf(v1, w1);
+  }
+  const float gscore = v1 + v2;
+  const int my_group = lane / group_lanes;
+  int better_groups = 0;
+  for (int g = 0; g < num_groups; ++g) {
+    const float s = __shfl_sync(0xffffffffu, gscore, g * group_lanes);
+    better_groups += (s > gscore || (s == gscore && g < my_group)) ? 1 : 0;
+  }
+  const bool kept = better_groups < topk_group;
+  // best remaining expert of the lane
+  float best = NEG_INF, best_score = 0.f;
+  int best_at = 0;
+  auto scan = [&] {
+    best = NEG_INF;
+    best_at = 0;
+    best_score = sc[0];
+#pragma unroll
+    for (int i = 0; i < VPT; ++i)
+      if (ch[i] > best) {
+        best = ch[i];
+        best_at = i;
+        best_score = sc[i];
+      }
+  };
+  if (kept) scan();
+  uint32_t key = kept ? order_key(best) : 0u;
+  float wsum = 0.f, my_w = 0.f;
+  int my_id = 0;
+  for (int j = 0; j < top_k; ++j) {
+    const uint32_t top = __reduce_max_sync(0xffffffffu, key);
+    const int owner = __ffs(__ballot_sync(0xffffffffu, key == top)) - 1;
+    const float w = __shfl_sync(0xffffffffu, best_score, owner);
+    const int at = __shfl_sync(0xffffffffu, best_at, owner);
+    wsum += w;
+    if (lane == j) {
+      my_w = w;
+      my_id = owner * VPT + at;
+    }
+    if (lane == owner) {
+#pragma unroll
+      for (int i = 0; i < VPT; ++i)
+        if (i == best_at) ch[i] = NEG_INF;
+      scan();
+      key = order_key(best);
+    }
   }
   if (lane < top_k) {
     weights[t * top_k + lane] = renorm ? my_w / wsum : my_w;
@@ -397,6 +501,20 @@ struct GroupedArgs {
 };
 template <int VPT> struct GroupedLauncher {
   template <typename T> static void go(const GroupedArgs& a) {
+    const int per_group = a.experts / a.num_groups;
+    const int lanes = per_group / VPT;
+    if (a.experts == 32 * VPT && per_group % VPT == 0 && (lanes & (lanes - 1)) == 0) {
+      const int grid = (int)ceil_div(a.tokens, WARPS);
+      if ((uintptr_t)a.logits % 16 == 0)   // every row then is, too
+        grouped_topk_lanes_kernel<T, VPT, true><<<grid, WARPS * 32, 0, a.st>>>(
+            reinterpret_cast<const T*>(a.logits), a.bias, a.tokens, a.num_groups, lanes, a.topk_group, a.top_k, a.renorm,
+            a.weights, a.ids);
+      else
+        grouped_topk_lanes_kernel<T, VPT, false><<<grid, WARPS * 32, 0, a.st>>>(
+            reinterpret_cast<const T*>(a.logits), a.bias, a.tokens, a.num_groups, lanes, a.topk_group, a.top_k, a.renorm,
+            a.weights, a.ids);
+      return;
+    }
     grouped_topk_kernel<T, VPT><<<(int)ceil_div(a.tokens, WARPS), WARPS * 32, 0, a.st>>>(
         reinterpret_cast<const T*>(a.logits), a.bias, a.tokens, a.experts, a.num_groups, a.topk_group, a.top_k, a.renorm,
         a.weights, a.ids);
@@ -612,6 +730,7 @@ extern "C" int dlb_route_grouped_topk(const void* logits, int dtype, const float
   DLB_REQUIRE(logits && bias && weights && ids, DLB_ERR_INVALID, "route_grouped_topk: null pointer");
   GroupedArgs a = {logits, dtype, bias, tokens, experts, num_groups, topk_group, top_k, renormalize, weights, ids,
                    (cudaStream_t)stream};
+  if (experts == 160) return GroupedLauncher<5>::run(a);   // 32 lanes of 5 experts
   return dispatch_vpt<GroupedLauncher>(experts, a);
 }
 
