@@ -320,130 +320,176 @@ __global__ void __launch_bounds__(WARPS * 32) grouped_topk_lanes_kernel(const T*
 
 // ---- capacity-limited gating (dlblas.topk_gating) -----------------------------------
 // part 1: gates = exp(x) / sum(exp(x)) (no max subtraction, topk_gating_fwd_part1.py:38-41),
-// k rounds of arg-max on the gates; ids and chosen gates are written k-major.
+// k rounds of arg-max on the gates; ids and chosen gates are written k-major.  The block also adds up its tokens' gates and
+// first choices per expert (psum, pcnt [blocks][experts]): the column sums over all tokens then only have the blocks to add.
+// (A kernel of its own for them, one warp row per 32 experts, was two blocks walking 4096 tokens: 70 of the forward's 105 us.)
+// Fixed summation order, no atomics on the sums.
+constexpr int GATING_TOKENS = 4;   // tokens per warp, one after the other
 template <typename T, int VPT>
 __global__ void __launch_bounds__(WARPS * 32) gating_part1_kernel(const T* __restrict__ logits, long long tokens,
                                                                   int experts, int top_k, float* __restrict__ gates,
-                                                                  int* __restrict__ ids_km, float* __restrict__ gate_km) {
-  const int lane = threadIdx.x & 31;
-  const long long t = (long long)blockIdx.x * WARPS + (threadIdx.x >> 5);
-  if (t >= tokens) return;
-  float x[VPT];
-  load_row<T, VPT>(logits + t * experts, experts, lane, x);
-  float sum = 0.f;
+                                                                  int* __restrict__ ids_km, float* __restrict__ gate_km,
+                                                                  float* __restrict__ psum, int* __restrict__ pcnt,
+                                                                  int* __restrict__ ticket) {
+  extern __shared__ float sm[];
+  float* s_sum = sm;                                            // [WARPS][experts]
+  int* s_cnt = reinterpret_cast<int*>(sm + WARPS * experts);    // [experts]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int e = threadIdx.x; e < experts; e += blockDim.x) s_cnt[e] = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0;
+  __syncthreads();
+  float col[VPT];
 #pragma unroll
-  for (int s = 0; s < VPT; ++s) {
-    x[s] = (s * 32 + lane < experts) ? expf(x[s]) : NEG_INF;
-    sum += (s * 32 + lane < experts) ? x[s] : 0.f;
-  }
-  sum = warp_sum(sum);
+  for (int s = 0; s < VPT; ++s) col[s] = 0.f;
+  const long long first = ((long long)blockIdx.x * WARPS + warp) * GATING_TOKENS;
+  for (long long t = first; t < min(first + GATING_TOKENS, tokens); ++t) {
+    float x[VPT];
+    load_row<T, VPT>(logits + t * experts, experts, lane, x);
+    float sum = 0.f;
 #pragma unroll
-  for (int s = 0; s < VPT; ++s) {
-    const int e = s * 32 + lane;
-    if (e < experts) {
-      x[s] = x[s] / sum;
-      gates[t * experts + e] = x[s];
+    for (int s = 0; s < VPT; ++s) {
+      x[s] = (s * 32 + lane < experts) ? expf(x[s]) : NEG_INF;
+      sum += (s * 32 + lane < experts) ? x[s] : 0.f;
+    }
+    sum = warp_sum(sum);
+#pragma unroll
+    for (int s = 0; s < VPT; ++s) {
+      const int e = s * 32 + lane;
+      if (e < experts) {
+        x[s] = x[s] / sum;
+        gates[t * experts + e] = x[s];
+        col[s] += x[s];
+      }
+    }
+    for (int j = 0; j < top_k; ++j) {
+      const ArgMax a = row_argmax<VPT>(x, lane);
+      if (lane == 0) {
+        ids_km[(long long)j * tokens + t] = a.i;
+        gate_km[(long long)j * tokens + t] = a.v;
+        if (j == 0 && a.i < experts) atomicAdd(s_cnt + a.i, 1);
+      }
+      knock_out<VPT>(x, a.i, lane);
     }
   }
-  for (int j = 0; j < top_k; ++j) {
-    const ArgMax a = row_argmax<VPT>(x, lane);
-    if (lane == 0) {
-      ids_km[(long long)j * tokens + t] = a.i;
-      gate_km[(long long)j * tokens + t] = a.v;
-    }
-    knock_out<VPT>(x, a.i, lane);
+#pragma unroll
+  for (int s = 0; s < VPT; ++s)
+    if (s * 32 + lane < experts) s_sum[warp * experts + s * 32 + lane] = col[s];
+  __syncthreads();
+  for (int e = threadIdx.x; e < experts; e += blockDim.x) {
+    float sum = 0.f;
+    for (int w = 0; w < WARPS; ++w) sum += s_sum[w * experts + e];
+    psum[(long long)blockIdx.x * experts + e] = sum;
+    pcnt[(long long)blockIdx.x * experts + e] = s_cnt[e];
   }
 }
 
-// part 2: per expert, me = mean of gates, ce = share of tokens whose first choice it is
-// (topk_gating_fwd_part2.py:31-36); fixed summation order, no atomics.
-__global__ void __launch_bounds__(256) gating_colsum_kernel(const float* __restrict__ gates,
-                                                            const int* __restrict__ ids_km, long long tokens,
-                                                            int experts, float* __restrict__ res,
-                                                            float* __restrict__ ce_out) {
-  __shared__ float s_sum[8][33];
-  __shared__ int s_cnt[8][33];
-  const int ex = threadIdx.x & 31, y = threadIdx.x >> 5;
-  const int e = blockIdx.x * 32 + ex;
-  float sum = 0.f;
-  int cnt = 0;
+// part 2, in the blocks behind the tokens' of part 3, one warp per expert: me = mean of gates, ce = share of tokens whose
+// first choice it is (topk_gating_fwd_part2.py:31-36), and, for an expert with fewer than `capacity` tokens, the remaining
+// slots of expert_select_token_idx: the tokens that did not choose it, in ascending order (what a stable descending sort of
+// the reference's int mask gives).  The last of these blocks (it waits for nobody) adds up the auxiliary loss.
+template <typename T>
+__device__ void gating_expert_part(const int* __restrict__ ids_km, const int* __restrict__ counts,
+                                   const float* __restrict__ psum, const int* __restrict__ pcnt, int part_blocks,
+                                   long long tokens, int experts, int top_k, long long capacity, int block, int blocks,
+                                   float* __restrict__ res, float* __restrict__ ce_out, int* __restrict__ ticket,
+                                   T* __restrict__ l_aux, long long* __restrict__ select) {
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31;
+  const int e = block * (int)(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (e < experts) {
-    for (long long t = y; t < tokens; t += 8) {
-      sum += gates[t * experts + e];
-      cnt += (ids_km[t] == e) ? 1 : 0;
+    float sum = 0.f;
+    int cnt = 0;
+#pragma unroll 4
+    for (int b = lane; b < part_blocks; b += 32) {
+      sum += psum[(long long)b * experts + e];
+      cnt += pcnt[(long long)b * experts + e];
+    }
+    sum = warp_sum(sum);
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if (lane == 0) {
+      const float me = sum / (float)tokens;
+      const float ce = (float)cnt / (float)tokens;
+      res[e] = me * ce * (float)experts * (float)experts;
+      ce_out[e] = ce;                                     // kept for the backward pass
+    }
+    long long filled = counts[e];
+    for (long long t0 = 0; t0 < tokens && filled < capacity; t0 += 32) {
+      const long long t = t0 + lane;
+      bool free_tok = t < tokens;
+#pragma unroll 8
+      for (int j = 0; j < top_k; ++j) free_tok = free_tok & (t < tokens && ids_km[(long long)j * tokens + t] != e);
+      const unsigned m = __ballot_sync(0xffffffffu, free_tok);
+      const long long pos = filled + __popc(m & ((1u << lane) - 1u));
+      if (free_tok && pos < capacity) select[(long long)e * capacity + pos] = t;
+      filled += __popc(m);
     }
   }
-  s_sum[y][ex] = sum;
-  s_cnt[y][ex] = cnt;
+  __threadfence();
   __syncthreads();
-  if (y == 0 && e < experts) {
-    float tot = 0.f;
-    int c = 0;
-    for (int i = 0; i < 8; ++i) {
-      tot += s_sum[i][ex];
-      c += s_cnt[i][ex];
-    }
-    const float me = tot / (float)tokens;
-    const float ce = (float)c / (float)tokens;
-    res[e] = me * ce * (float)experts * (float)experts;
-    ce_out[e] = ce;                                     // kept for the backward pass
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1) == blocks - 1;
+  __syncthreads();
+  if (last && threadIdx.x < 32) {
+    __threadfence();
+    float s = 0.f;
+    for (int i = lane; i < experts; i += 32) s += __ldcg(res + i);
+    s = warp_sum(s);
+    if (lane == 0) *l_aux = from_f32<T>(s / (float)experts);
   }
 }
 
 // part 3: drop entries beyond the capacity, renormalise the kept gates, emit the indices
 // (topk_gating_fwd_part3.py:9-61) and the kept part of expert_select_token_idx.
+constexpr int GATING_SLOTS = 8;   // slots of a token whose loads are in flight together
 template <typename T>
-__global__ void __launch_bounds__(256) gating_part3_kernel(const int* __restrict__ ids_km,
-                                                           const float* __restrict__ gate_km,
-                                                           const int* __restrict__ rank, const float* __restrict__ res,
-                                                           long long tokens, int experts, int top_k, long long capacity,
-                                                           T* __restrict__ l_aux, int* __restrict__ ec_idx,
-                                                           T* __restrict__ out_w, long long* __restrict__ select) {
-  const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    float s = 0.f;
-    for (int e = 0; e < experts; ++e) s += res[e];
-    *l_aux = from_f32<T>(s / (float)experts);
+__global__ void __launch_bounds__(64) gating_part3_kernel(const int* __restrict__ ids_km,
+                                                          const float* __restrict__ gate_km,
+                                                          const int* __restrict__ rank, const int* __restrict__ counts,
+                                                          const float* __restrict__ psum, const int* __restrict__ pcnt,
+                                                          int part_blocks, long long tokens, int experts, int top_k,
+                                                          long long capacity, int token_blocks, float* __restrict__ res,
+                                                          float* __restrict__ ce_out, int* __restrict__ ticket,
+                                                          T* __restrict__ l_aux, int* __restrict__ ec_idx,
+                                                          T* __restrict__ out_w, long long* __restrict__ select) {
+  if ((int)blockIdx.x >= token_blocks) {
+    gating_expert_part<T>(ids_km, counts, psum, pcnt, part_blocks, tokens, experts, top_k, capacity,
+                          blockIdx.x - token_blocks, gridDim.x - token_blocks, res, ce_out, ticket, l_aux, select);
+    return;
   }
+  const long long t = (long long)blockIdx.x * 64 + threadIdx.x;
   if (t >= tokens) return;
   float denom = 0.f;
-  for (int j = 0; j < top_k; ++j) {
-    const long long f = (long long)j * tokens + t;
-    if (rank[f] < capacity) denom += gate_km[f];
+  int loc[GATING_SLOTS];
+  float gate[GATING_SLOTS];
+  auto fetch = [&](int j0) {
+#pragma unroll
+    for (int j = 0; j < GATING_SLOTS; ++j) {
+      const long long f = (long long)(j0 + j) * tokens + t;
+      loc[j] = j0 + j < top_k ? __ldg(rank + f) : 0x7fffffff;
+      gate[j] = j0 + j < top_k ? __ldg(gate_km + f) : 0.f;
+    }
+  };
+  for (int j0 = 0; j0 < top_k; j0 += GATING_SLOTS) {
+    fetch(j0);
+#pragma unroll
+    for (int j = 0; j < GATING_SLOTS; ++j)
+      if (loc[j] < capacity) denom += gate[j];
   }
   const float eps = sizeof(T) == 2 ? 9.765625e-4f : 1.1920929e-7f;   // torch.finfo(dtype).eps
   denom = denom < eps ? eps : denom;
-  for (int j = 0; j < top_k; ++j) {
-    const long long f = (long long)j * tokens + t;
-    const int loc = rank[f];
-    const bool kept = loc < capacity;
-    out_w[f] = from_f32<T>(kept ? gate_km[f] / denom : 0.f);
-    ec_idx[f] = kept ? (int)((long long)ids_km[f] * capacity + loc) : 0;
-    if (kept) select[(long long)ids_km[f] * capacity + loc] = t;
-  }
-}
-
-// Experts with fewer than `capacity` tokens: the remaining slots of expert_select_token_idx
-// take the tokens that did not choose the expert, in ascending order (what a stable
-// descending sort of the reference's int mask gives).  One warp per expert.
-__global__ void __launch_bounds__(WARPS * 32) gating_fill_kernel(const int* __restrict__ ids_km,
-                                                                 const int* __restrict__ counts, long long tokens,
-                                                                 int experts, int top_k, long long capacity,
-                                                                 long long* __restrict__ select) {
-  const int lane = threadIdx.x & 31;
-  const int e = blockIdx.x * WARPS + (threadIdx.x >> 5);
-  if (e >= experts) return;
-  long long filled = counts[e];
-  if (filled >= capacity) return;
-  for (long long t0 = 0; t0 < tokens && filled < capacity; t0 += 32) {
-    const long long t = t0 + lane;
-    bool free_tok = t < tokens;
-    if (free_tok)
-      for (int j = 0; j < top_k; ++j) free_tok = free_tok && (ids_km[(long long)j * tokens + t] != e);
-    const unsigned m = __ballot_sync(0xffffffffu, free_tok);
-    const long long pos = filled + __popc(m & ((1u << lane) - 1u));
-    if (free_tok && pos < capacity) select[(long long)e * capacity + pos] = t;
-    filled += __popc(m);
+  for (int j0 = 0; j0 < top_k; j0 += GATING_SLOTS) {
+    if (top_k > GATING_SLOTS) fetch(j0);
+    int id[GATING_SLOTS];
+#pragma unroll
+    for (int j = 0; j < GATING_SLOTS; ++j) id[j] = j0 + j < top_k ? __ldg(ids_km + (long long)(j0 + j) * tokens + t) : 0;
+#pragma unroll
+    for (int j = 0; j < GATING_SLOTS; ++j) {
+      if (j0 + j >= top_k) break;
+      const long long f = (long long)(j0 + j) * tokens + t;
+      const bool kept = loc[j] < capacity;
+      out_w[f] = from_f32<T>(kept ? gate[j] / denom : 0.f);
+      ec_idx[f] = kept ? (int)((long long)id[j] * capacity + loc[j]) : 0;
+      if (kept) select[(long long)id[j] * capacity + loc[j]] = t;
+    }
   }
 }
 
@@ -537,17 +583,24 @@ struct GatingArgs {
   float* gates;
   int* ids_km;
   float* gate_km;
+  float* psum;
+  int* pcnt;
+  int* ticket;
   cudaStream_t st;
 };
+int gating_blocks(long long tokens) { return (int)ceil_div(tokens, (int64_t)(WARPS * GATING_TOKENS)); }
 template <int VPT> struct GatingLauncher {
   static int run(GatingArgs a) {
-    const int grid = (int)ceil_div(a.tokens, WARPS);
+    const int grid = gating_blocks(a.tokens);
+    const size_t smem = (size_t)(WARPS + 1) * a.experts * 4;    // at most 36 KB
     if (a.dtype == DLB_F32)
-      gating_part1_kernel<float, VPT><<<grid, WARPS * 32, 0, a.st>>>(reinterpret_cast<const float*>(a.logits), a.tokens,
-                                                                    a.experts, a.top_k, a.gates, a.ids_km, a.gate_km);
+      gating_part1_kernel<float, VPT><<<grid, WARPS * 32, smem, a.st>>>(
+          reinterpret_cast<const float*>(a.logits), a.tokens, a.experts, a.top_k, a.gates, a.ids_km, a.gate_km, a.psum,
+          a.pcnt, a.ticket);
     else
-      gating_part1_kernel<__half, VPT><<<grid, WARPS * 32, 0, a.st>>>(reinterpret_cast<const __half*>(a.logits), a.tokens,
-                                                                     a.experts, a.top_k, a.gates, a.ids_km, a.gate_km);
+      gating_part1_kernel<__half, VPT><<<grid, WARPS * 32, smem, a.st>>>(
+          reinterpret_cast<const __half*>(a.logits), a.tokens, a.experts, a.top_k, a.gates, a.ids_km, a.gate_km, a.psum,
+          a.pcnt, a.ticket);
     count_launch();
     DLB_CHECK_LAUNCH("gating_part1_kernel");
     return DLB_OK;
@@ -559,8 +612,9 @@ template <int VPT> struct GatingLauncher {
 //           + sum over kept slots j with ids[j] == e of
 //             ( gw[j] / D + [D not clamped] * sum_i(-gw[i] * g[i] / D^2) )   (w[j] = g[j] / D, D = sum of kept gates)
 //   grad[e] = gates[e] * (add[e] - sum_i gates[i] * add[i])                (softmax backward, :40-44)
-// One warp per token; reads what the forward left in its workspace.
-template <typename T>
+// One warp per token; reads what the forward left in its workspace.  Lane j looks after slot j of the token (32 slots at a
+// time): the slots' terms are formed once, in registers, and handed to the lanes that hold the experts' gates.
+template <typename T, int VPT>
 __global__ void __launch_bounds__(WARPS * 32) gating_bwd_kernel(const float* __restrict__ gates,
                                                                 const float* __restrict__ ce,
                                                                 const int* __restrict__ ids_km,
@@ -572,53 +626,90 @@ __global__ void __launch_bounds__(WARPS * 32) gating_bwd_kernel(const float* __r
   const int lane = threadIdx.x & 31;
   const long long t = (long long)blockIdx.x * WARPS + (threadIdx.x >> 5);
   if (t >= tokens) return;
+  float g[VPT], add[VPT];
   const float gl = to_f32<T>(*grad_l_aux) * (float)experts / (float)tokens;
-  const float eps = sizeof(T) == 2 ? 9.765625e-4f : 1.1920929e-7f;   // torch.finfo(dtype).eps
-  float denom = 0.f, coupling = 0.f;
+#pragma unroll
+  for (int s = 0; s < VPT; ++s) {
+    const int e = s * 32 + lane;
+    g[s] = e < experts ? __ldg(gates + t * experts + e) : 0.f;
+    add[s] = e < experts ? __ldg(ce + e) * gl : 0.f;
+  }
   if (grad_w != nullptr) {
-    for (int j = 0; j < top_k; ++j) {
-      const long long f = (long long)j * tokens + t;
-      if (rank[f] < capacity) denom += gate_km[f];
+    const float eps = sizeof(T) == 2 ? 9.765625e-4f : 1.1920929e-7f;   // torch.finfo(dtype).eps
+    float denom = 0.f, weighted = 0.f;
+    int id = -1;
+    float gate = 0.f, gw = 0.f;
+    bool kept = false;
+    auto fetch = [&](int j0) {
+      const long long f = (long long)(j0 + lane) * tokens + t;
+      kept = j0 + lane < top_k && __ldg(rank + f) < capacity;
+      id = kept ? __ldg(ids_km + f) : -1;
+      gate = kept ? __ldg(gate_km + f) : 0.f;
+      gw = kept ? to_f32<T>(grad_w[f]) : 0.f;
+    };
+    for (int j0 = 0; j0 < top_k; j0 += 32) {
+      fetch(j0);
+      denom += warp_sum(gate);
+      weighted += warp_sum(gw * gate);
     }
     const bool clamped = denom < eps;
-    const float cd = clamped ? eps : denom;
-    if (!clamped) {
-      for (int j = 0; j < top_k; ++j) {
-        const long long f = (long long)j * tokens + t;
-        if (rank[f] < capacity) coupling -= to_f32<T>(grad_w[f]) * gate_km[f] / (cd * cd);
+    if (clamped) denom = eps;
+    const float coupling = clamped ? 0.f : -weighted / (denom * denom);
+    for (int j0 = 0; j0 < top_k; j0 += 32) {
+      if (top_k > 32) fetch(j0);
+      const float term = gw / denom + coupling;
+      for (int j = 0; j < min(32, top_k - j0); ++j) {
+        const int e = __shfl_sync(0xffffffffu, id, j);
+        const float v = __shfl_sync(0xffffffffu, term, j);
+        if (e >= 0 && (e & 31) == lane) {
+#pragma unroll
+          for (int s = 0; s < VPT; ++s)
+            if (s == (e >> 5)) add[s] += v;
+        }
       }
     }
-    denom = cd;
   }
-  const float* g_row = gates + t * experts;
   float dot = 0.f;
-  for (int e = lane; e < experts; e += 32) {
-    float add = ce[e] * gl;
-    if (grad_w != nullptr) {
-      for (int j = 0; j < top_k; ++j) {
-        const long long f = (long long)j * tokens + t;
-        if (ids_km[f] == e && rank[f] < capacity) add += to_f32<T>(grad_w[f]) / denom + coupling;
-      }
-    }
-    dot += g_row[e] * add;
-  }
+#pragma unroll
+  for (int s = 0; s < VPT; ++s) dot += g[s] * add[s];
   dot = warp_sum(dot);
-  for (int e = lane; e < experts; e += 32) {
-    float add = ce[e] * gl;
-    if (grad_w != nullptr) {
-      for (int j = 0; j < top_k; ++j) {
-        const long long f = (long long)j * tokens + t;
-        if (ids_km[f] == e && rank[f] < capacity) add += to_f32<T>(grad_w[f]) / denom + coupling;
-      }
-    }
-    grad_logits[t * experts + e] = from_f32<T>(g_row[e] * (add - dot));
-  }
+#pragma unroll
+  for (int s = 0; s < VPT; ++s)
+    if (s * 32 + lane < experts) grad_logits[t * experts + s * 32 + lane] = from_f32<T>(g[s] * (add[s] - dot));
 }
 
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
+struct GatingBwdArgs {
+  const float *gates, *ce;
+  const int* ids_km;
+  const float* gate_km;
+  const int* rank;
+  int dtype;
+  long long tokens;
+  int experts, top_k;
+  long long capacity;
+  const void *grad_l_aux, *grad_w;
+  void* grad_logits;
+  cudaStream_t st;
+};
+template <int VPT> struct GatingBwdLauncher {
+  template <typename T> static void go(const GatingBwdArgs& a) {
+    gating_bwd_kernel<T, VPT><<<(int)ceil_div(a.tokens, WARPS), WARPS * 32, 0, a.st>>>(
+        a.gates, a.ce, a.ids_km, a.gate_km, a.rank, a.tokens, a.experts, a.top_k, a.capacity,
+        reinterpret_cast<const T*>(a.grad_l_aux), reinterpret_cast<const T*>(a.grad_w), reinterpret_cast<T*>(a.grad_logits));
+  }
+  static int run(GatingBwdArgs a) {
+    if (a.dtype == DLB_F32) go<float>(a);
+    else go<__half>(a);
+    count_launch();
+    DLB_CHECK_LAUNCH("gating_bwd_kernel");
+    return DLB_OK;
+  }
+};
+
 struct GatingWs {
-  size_t gates, ids_km, gate_km, rank, res, ce, counts, sort, bytes;
+  size_t gates, ids_km, gate_km, rank, res, ce, counts, psum, pcnt, ticket, sort, bytes;
 };
 GatingWs gating_ws(long long tokens, int experts, int top_k) {
   GatingWs w;
@@ -630,6 +721,9 @@ GatingWs gating_ws(long long tokens, int experts, int top_k) {
   w.res = off; off += align256((size_t)experts * 4);
   w.ce = off; off += align256((size_t)experts * 4);
   w.counts = off; off += align256((size_t)experts * 4);
+  w.psum = off; off += align256((size_t)gating_blocks(tokens) * experts * 4);
+  w.pcnt = off; off += align256((size_t)gating_blocks(tokens) * experts * 4);
+  w.ticket = off; off += 256;
   w.sort = off; off += sort_workspace_size(tokens * top_k, experts);
   w.bytes = off;
   return w;
@@ -760,35 +854,27 @@ extern "C" int dlb_topk_gating(const void* logits, int dtype, int64_t tokens, in
   float* res = reinterpret_cast<float*>(ws + w.res);
   int* counts = reinterpret_cast<int*>(ws + w.counts);
   cudaStream_t st = (cudaStream_t)stream;
-  GatingArgs a = {logits, dtype, tokens, experts, top_k, gates, ids_km, gate_km, st};
+  float* psum = reinterpret_cast<float*>(ws + w.psum);
+  int* pcnt = reinterpret_cast<int*>(ws + w.pcnt);
+  int* ticket = reinterpret_cast<int*>(ws + w.ticket);
+  GatingArgs a = {logits, dtype, tokens, experts, top_k, gates, ids_km, gate_km, psum, pcnt, ticket, st};
   int rc = dispatch_vpt<GatingLauncher>(experts, a);
   if (rc != DLB_OK) return rc;
-  gating_colsum_kernel<<<(int)ceil_div(experts, 32), 256, 0, st>>>(gates, ids_km, tokens, experts, res,
-                                                                   reinterpret_cast<float*>(ws + w.ce));
-  count_launch();
-  DLB_CHECK_LAUNCH("gating_colsum_kernel");
   // position of every (slot, token) entry inside its expert, in k-major / token-minor order:
   // the cumulative sum of the one-hot masks of the reference (topk_gating_fwd_part2.py:31)
   rc = sort_by_expert(ids_km, DLB_I32, tokens * top_k, experts, nullptr, nullptr, nullptr, nullptr, rank, counts,
                       ws + w.sort, workspace_bytes - w.sort, st);
   if (rc != DLB_OK) return rc;
-  const int grid3 = (int)ceil_div(tokens, 256);
-  if (dtype == DLB_F32)
-    gating_part3_kernel<float><<<grid3, 256, 0, st>>>(ids_km, gate_km, rank, res, tokens, experts, top_k, capacity,
-                                                     reinterpret_cast<float*>(l_aux), ec_idx,
-                                                     reinterpret_cast<float*>(gate_weights),
-                                                     reinterpret_cast<long long*>(select));
-  else
-    gating_part3_kernel<__half><<<grid3, 256, 0, st>>>(ids_km, gate_km, rank, res, tokens, experts, top_k, capacity,
-                                                      reinterpret_cast<__half*>(l_aux), ec_idx,
-                                                      reinterpret_cast<__half*>(gate_weights),
-                                                      reinterpret_cast<long long*>(select));
+  const int token_blocks = (int)ceil_div(tokens, 64), expert_blocks = (int)ceil_div(experts, 2);
+  auto part3 = [&](auto* out_l_aux, auto* out_w) {
+    gating_part3_kernel<<<token_blocks + expert_blocks, 64, 0, st>>>(
+        ids_km, gate_km, rank, counts, psum, pcnt, gating_blocks(tokens), tokens, experts, top_k, capacity, token_blocks, res,
+        reinterpret_cast<float*>(ws + w.ce), ticket, out_l_aux, ec_idx, out_w, reinterpret_cast<long long*>(select));
+  };
+  if (dtype == DLB_F32) part3(reinterpret_cast<float*>(l_aux), reinterpret_cast<float*>(gate_weights));
+  else part3(reinterpret_cast<__half*>(l_aux), reinterpret_cast<__half*>(gate_weights));
   count_launch();
   DLB_CHECK_LAUNCH("gating_part3_kernel");
-  gating_fill_kernel<<<(int)ceil_div(experts, WARPS), WARPS * 32, 0, st>>>(ids_km, counts, tokens, experts, top_k,
-                                                                          capacity, reinterpret_cast<long long*>(select));
-  count_launch();
-  DLB_CHECK_LAUNCH("gating_fill_kernel");
   return DLB_OK;
 }
 
@@ -808,19 +894,7 @@ extern "C" int dlb_topk_gating_bwd(const void* workspace, size_t workspace_bytes
   const int* ids_km = reinterpret_cast<const int*>(ws + w.ids_km);
   const float* gate_km = reinterpret_cast<const float*>(ws + w.gate_km);
   const int* rank = reinterpret_cast<const int*>(ws + w.rank);
-  cudaStream_t st = (cudaStream_t)stream;
-  const int grid = (int)ceil_div(tokens, WARPS);
-  if (dtype == DLB_F32)
-    gating_bwd_kernel<float><<<grid, WARPS * 32, 0, st>>>(gates, ce, ids_km, gate_km, rank, tokens, experts, top_k,
-                                                          capacity, reinterpret_cast<const float*>(grad_l_aux),
-                                                          reinterpret_cast<const float*>(grad_weights),
-                                                          reinterpret_cast<float*>(grad_logits));
-  else
-    gating_bwd_kernel<__half><<<grid, WARPS * 32, 0, st>>>(gates, ce, ids_km, gate_km, rank, tokens, experts, top_k,
-                                                           capacity, reinterpret_cast<const __half*>(grad_l_aux),
-                                                           reinterpret_cast<const __half*>(grad_weights),
-                                                           reinterpret_cast<__half*>(grad_logits));
-  count_launch();
-  DLB_CHECK_LAUNCH("gating_bwd_kernel");
-  return DLB_OK;
+  GatingBwdArgs a = {gates, ce, ids_km, gate_km, rank, dtype, tokens, experts, top_k, capacity, grad_l_aux, grad_weights,
+                     grad_logits, (cudaStream_t)stream};
+  return dispatch_vpt<GatingBwdLauncher>(experts, a);
 }
