@@ -44,7 +44,15 @@ using at::Tensor;
   X(dlb_moe_sum_topk)                                                                                                 \
   X(dlb_fp8_gemm)                                                                                                     \
   X(dlb_route_softmax_topk)                                                                                           \
-  X(dlb_route_grouped_topk)
+  X(dlb_route_grouped_topk)                                                                                           \
+  X(dlb_moe_grouped_gemm_window)                                                                                      \
+  X(dlb_ep_gather)                                                                                                    \
+  X(dlb_moe_build_tiles_sizes)                                                                                        \
+  X(dlb_grouped_gemm_16bit)                                                                                           \
+  X(dlb_grouped_gemm_16bit_b_kn)                                                                                      \
+  X(dlb_k_grouped_gemm_workspace_bytes)                                                                               \
+  X(dlb_k_grouped_gemm_16bit)                                                                                         \
+  X(dlb_silu_and_mul)
 
 struct Abi {
 #define X(name) decltype(&::name) name = nullptr;
@@ -418,6 +426,199 @@ PyObject* py_moe_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+// The decode step of FusedMoELowLatency on one rank.  Rounding points of the masked-layout path (w13 rows rounded to
+// out_dtype, silu rounded before the product, scales max(absmax, eps) / 448, the weights applied in fp32 in the gather), on the
+// rows that exist: with a single rank the exchange is a permutation, so the rows go straight into expert order instead of a
+// [experts, max tokens, hidden] layout, and the layer is six launches of which two stream the weights.
+Tensor low_latency_forward(const Tensor& x, const Tensor& topk_weights, const Tensor& topk_ids, const Tensor& w1,
+                           const Tensor& w1_s, const Tensor& w2, const Tensor& w2_s, at::ScalarType out_dtype) {
+  require_cuda(x);
+  require_cuda(w1);
+  for (const Tensor* t : {&w1, &w1_s, &w2, &w2_s}) require(t->is_contiguous(), "weights and scales must be contiguous");
+  require(x.dim() == 2 && x.stride(1) == 1, "hidden states must be 2-D with contiguous rows");
+  Call c(x);
+  const int64_t e = w1.size(0), n = w1.size(1), h = w1.size(2), inter = n / 2;
+  const int64_t m = x.size(0), top_k = topk_ids.size(1), slots = m * top_k;
+  require(x.size(1) == h, "hidden size mismatch");
+  Tensor out = empty({m, h}, out_dtype, c);
+  if (m == 0) return out;
+  Tensor ids = topk_ids.scalar_type() == at::kInt || topk_ids.scalar_type() == at::kLong ? topk_ids : topk_ids.to(at::kLong);
+  if (!ids.is_contiguous()) ids = ids.contiguous();
+  Tensor weights = topk_weights.scalar_type() == at::kFloat ? topk_weights : topk_weights.to(at::kFloat);
+  if (!weights.is_contiguous()) weights = weights.contiguous();
+  const int max_tiles = (int)(slots / 128 + e);
+  const size_t size = c10::elementSize(out_dtype);
+  const size_t sort_bytes = abi.dlb_sort_by_expert_workspace_size(slots, (int)e);
+  Workspace ws;
+  const size_t o_pos = ws.take(slots * 4), o_tiles = ws.take((max_tiles + 1) * 16), o_sort = ws.take(sort_bytes),
+               o_a = ws.take(slots * h), o_as = ws.take(slots * (h / 128) * 4), o_c1 = ws.take(slots * n * size),
+               o_hq = ws.take(slots * inter), o_hs = ws.take(slots * (inter / 128) * 4), o_y = ws.take(slots * h * size);
+  ws.allocate(c);
+  int32_t *pos = ws.at<int32_t>(o_pos), *tiles = ws.at<int32_t>(o_tiles), *status = status_ptr(c);
+  check(abi.dlb_moe_plan(ids.data_ptr(), code(ids.scalar_type()), m, (int)top_k, (int)e, 0, (int)e, 128, nullptr, pos, tiles,
+                         max_tiles, nullptr, nullptr, ws.at<void>(o_sort), sort_bytes, c.stream));
+  check(abi.dlb_quant_fp8(x.data_ptr(), code(x.scalar_type()), m, h, x.stride(0), 128, DLB_QUANT_DIV_EPS, 1e-10f,
+                          ws.at<void>(o_a), ws.at<float>(o_as), h / 128, 1, pos, (int)top_k, c.stream));
+  // SMs left to kernels of other streams (a shared expert's small GEMMs): the weights stream at the memory rate from fewer
+  const int margin = env_int("DLBLAS_DECODE_SM_MARGIN", 0);
+  auto gemm = [&](size_t a, size_t a_s, int64_t nn, int64_t kk, const Tensor& b, const Tensor& b_s, size_t dst) {
+    check(abi.dlb_moe_grouped_gemm_window(ws.at<void>(a), ws.at<float>(a_s), slots, b.data_ptr(), b_s.data_ptr<float>(),
+                                          (int)e, nn, kk, tiles, max_tiles, 128, DLB_EPI_STORE, ws.at<void>(dst),
+                                          code(out_dtype), nn, nullptr, DLB_QUANT_RECIP_MUL, 1e-10f, nullptr, nullptr, status,
+                                          c.stream, 0, nn, margin));
+  };
+  gemm(o_a, o_as, n, h, w1, w1_s, o_c1);
+  check(abi.dlb_silu_mul_quant(ws.at<void>(o_c1), code(out_dtype), slots, inter, DLB_QUANT_DIV_EPS, 1e-10f, 1, nullptr, 0,
+                               ws.at<void>(o_hq), ws.at<float>(o_hs), c.stream));
+  gemm(o_hq, o_hs, h, inter, w2, w2_s, o_y);
+  check(abi.dlb_ep_gather(ws.at<void>(o_y), code(out_dtype), h, pos, pos, DLB_I32, weights.data_ptr<float>(), m, (int)top_k,
+                          out.data_ptr(), c.stream));
+  return out;
+}
+
+PyObject* py_low_latency_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 8);
+    return wrap(low_latency_forward(tensor(a[0]), tensor(a[1]), tensor(a[2]), tensor(a[3]), tensor(a[4]), tensor(a[5]),
+                                    tensor(a[6]), dtype(a[7])));
+  });
+}
+
+// ---- 16-bit grouped GEMMs and the unquantised expert layer --------------------------------------------------------
+// pairs of CTAs on 256-row tiles when the groups are large enough to fill them (decided from the shapes, no look at the
+// group sizes on the host); DLBLAS_GEMM16_TILE_ROWS = 128 / 256 overrides
+int gemm16_tile_rows(int64_t rows, int64_t groups) {
+  return env_int("DLBLAS_GEMM16_TILE_ROWS", rows >= 512 * groups ? 256 : 128);
+}
+
+Tensor group_sizes(const Tensor& sizes) {
+  Tensor s = sizes.scalar_type() == at::kInt || sizes.scalar_type() == at::kLong ? sizes : sizes.to(at::kLong);
+  return s.is_contiguous() ? s : s.contiguous();
+}
+
+Tensor m_grouped_gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& sizes_in, bool trans_b) {
+  require(a_in.dim() == 2, "A must be 2-D");
+  require(b_in.dim() == 3, "B must be 3-D");
+  for (const Tensor* t : {&a_in, &b_in, &sizes_in}) require_cuda(*t);
+  require(a_in.stride(1) == 1, "Please make sure A is K-major");
+  require(a_in.scalar_type() == b_in.scalar_type() &&
+              (a_in.scalar_type() == at::kBFloat16 || a_in.scalar_type() == at::kHalf),
+          "A and B must both be bf16 or fp16");
+  Call c(a_in);
+  const int64_t m = a_in.size(0), k = a_in.size(1), groups = b_in.size(0);
+  const int64_t n = trans_b ? b_in.size(1) : b_in.size(2), bk = trans_b ? b_in.size(2) : b_in.size(1);
+  require(bk == k, "K of A should be equal to K of B");
+  require(sizes_in.numel() == groups, "one size per group");
+  const bool b_kn = !trans_b && k % 64 == 0;
+  const Tensor a = a_in.is_contiguous() ? a_in : a_in.contiguous();
+  Tensor b = trans_b || b_kn ? b_in : b_in.transpose(1, 2);
+  if (!b.is_contiguous()) b = b.contiguous();
+  Tensor out = empty({m, n}, a.scalar_type(), c);
+  if (m == 0) return out;
+  const Tensor sizes = group_sizes(sizes_in);
+  const int tile_rows = gemm16_tile_rows(m, groups);
+  const int max_tiles = (int)(m / tile_rows + groups);
+  Workspace ws;
+  ws.take((size_t)(max_tiles + 1) * 16);
+  ws.allocate(c);
+  int32_t* tiles = ws.at<int32_t>(0);
+  check(abi.dlb_moe_build_tiles_sizes(sizes.data_ptr(), code(sizes.scalar_type()), (int)groups, m, tile_rows, tiles, max_tiles,
+                                      c.stream));
+  auto gemm = b_kn ? abi.dlb_grouped_gemm_16bit_b_kn : abi.dlb_grouped_gemm_16bit;
+  check(gemm(a.data_ptr(), b.data_ptr(), code(a.scalar_type()), m, (int)groups, n, k, tiles, max_tiles, tile_rows,
+             out.data_ptr(), n, status_ptr(c), c.stream));
+  return out;
+}
+
+PyObject* py_m_grouped_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 4);
+    return wrap(m_grouped_gemm(tensor(a[0]), tensor(a[1]), tensor(a[2]), truth(a[3])));
+  });
+}
+
+Tensor k_grouped_gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& sizes_in) {
+  require(a_in.dim() == 2, "A must be 2-D");
+  require(b_in.dim() == 2, "B must be 2-D");
+  for (const Tensor* t : {&a_in, &b_in, &sizes_in}) require_cuda(*t);
+  require(a_in.stride(1) == 1, "Please make sure A is K-major");
+  require(b_in.stride(1) == 1, "Please make sure B is K-major");
+  require(a_in.size(0) == b_in.size(0), "Please make sure that A and B have the same seqlen");
+  if (a_in.scalar_type() != b_in.scalar_type() || (a_in.scalar_type() != at::kBFloat16 && a_in.scalar_type() != at::kHalf))
+    throw AssertionFailed(std::string("data type ") + c10::toString(a_in.scalar_type()) + " not supported");
+  Call c(a_in);
+  const Tensor a = a_in.is_contiguous() ? a_in : a_in.contiguous(), b = b_in.is_contiguous() ? b_in : b_in.contiguous();
+  const int64_t k = a.size(0), m = a.size(1), n = b.size(1), groups = sizes_in.size(0);
+  Tensor out = empty({groups, m, n}, a.scalar_type(), c);
+  if (groups == 0 || m == 0 || n == 0) return out;
+  Tensor sizes = group_sizes(sizes_in);
+  if (sizes.scalar_type() != at::kLong) sizes = sizes.to(at::kLong);
+  // pairs of CTAs on 256-row tiles of C unless M is smaller than one; DLBLAS_GEMM16_TILE_ROWS = 128 / 256 overrides
+  const int tile_rows = env_int("DLBLAS_GEMM16_TILE_ROWS", m >= 256 ? 256 : 128);
+  const int64_t need = abi.dlb_k_grouped_gemm_workspace_bytes(k, m, n, (int)groups, tile_rows);
+  require(need > 0, "k_grouped_gemm: bad sizes");
+  const Tensor work = empty({need}, at::kByte, c);
+  check(abi.dlb_k_grouped_gemm_16bit(a.data_ptr(), b.data_ptr(), code(a.scalar_type()), k, m, n, sizes.data_ptr<int64_t>(),
+                                     (int)groups, tile_rows, work.data_ptr(), need, out.data_ptr(), status_ptr(c), c.stream));
+  return out;
+}
+
+PyObject* py_k_grouped_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 3);
+    return wrap(k_grouped_gemm(tensor(a[0]), tensor(a[1]), tensor(a[2])));
+  });
+}
+
+// rows copied into expert order -> w1 GEMM -> silu(gate) * up -> w2 GEMM -> fp32 weighted sum over the slots
+Tensor moe_forward_16bit(const Tensor& x, const Tensor& w1_in, const Tensor& w2_in, const Tensor& weights_in,
+                         const Tensor& ids_in) {
+  require(x.scalar_type() == at::kBFloat16 || x.scalar_type() == at::kHalf,
+          "the unquantised mode takes bf16 or fp16 activations");
+  require(w1_in.scalar_type() == x.scalar_type() && w2_in.scalar_type() == x.scalar_type(),
+          "weights must have the activations' type");
+  require_cuda(x);
+  require_cuda(w1_in);
+  Call c(x);
+  const int64_t m = x.size(0), h = x.size(1), e = w1_in.size(0), n2 = w1_in.size(1), inter = n2 / 2;
+  require(w2_in.dim() == 3 && w2_in.size(0) == e && w2_in.size(1) == h && w2_in.size(2) == inter, "w2 must be [E, H, I]");
+  Tensor out = empty({m, h}, x.scalar_type(), c);
+  if (m == 0) return out;
+  const int64_t top_k = ids_in.size(1), slots = m * top_k;
+  require(ids_in.scalar_type() == at::kInt || ids_in.scalar_type() == at::kLong, "topk_ids must be int32 or int64");
+  const Tensor ids = ids_in.is_contiguous() ? ids_in : ids_in.contiguous();
+  const Tensor w1 = w1_in.is_contiguous() ? w1_in : w1_in.contiguous(), w2 = w2_in.is_contiguous() ? w2_in : w2_in.contiguous();
+  Tensor weights = weights_in.scalar_type() == at::kFloat ? weights_in : weights_in.to(at::kFloat);
+  if (!weights.is_contiguous()) weights = weights.contiguous();
+  const int tile_rows = gemm16_tile_rows(slots, e), max_tiles = (int)(slots / tile_rows + e), dt = code(x.scalar_type());
+  const size_t sort_bytes = abi.dlb_sort_by_expert_workspace_size(slots, (int)e);
+  Workspace ws;
+  const size_t o_pos = ws.take(slots * 4), o_tiles = ws.take((max_tiles + 1) * 16), o_sort = ws.take(sort_bytes),
+               o_a = ws.take(slots * h * 2), o_c1 = ws.take(slots * n2 * 2), o_act = ws.take(slots * inter * 2),
+               o_y = ws.take(slots * h * 2);
+  ws.allocate(c);
+  int32_t *pos = ws.at<int32_t>(o_pos), *tiles = ws.at<int32_t>(o_tiles), *status = status_ptr(c);
+  check(abi.dlb_moe_plan(ids.data_ptr(), code(ids.scalar_type()), m, (int)top_k, (int)e, 0, (int)e, tile_rows, nullptr, pos,
+                         tiles, max_tiles, nullptr, nullptr, ws.at<void>(o_sort), sort_bytes, c.stream));
+  check(abi.dlb_permute_rows(x.data_ptr(), 2 * h, nullptr, 0, m, pos, (int)top_k, ws.at<void>(o_a), nullptr, c.stream));
+  check(abi.dlb_grouped_gemm_16bit(ws.at<void>(o_a), w1.data_ptr(), dt, slots, (int)e, n2, h, tiles, max_tiles, tile_rows,
+                                   ws.at<void>(o_c1), n2, status, c.stream));
+  check(abi.dlb_silu_and_mul(ws.at<void>(o_c1), dt, slots, inter, n2, ws.at<void>(o_act), inter, c.stream));
+  check(abi.dlb_grouped_gemm_16bit(ws.at<void>(o_act), w2.data_ptr(), dt, slots, (int)e, h, inter, tiles, max_tiles, tile_rows,
+                                   ws.at<void>(o_y), h, status, c.stream));
+  // slots of other ranks' experts have a negative position and are left out of the sum
+  check(abi.dlb_ep_gather(ws.at<void>(o_y), dt, h, pos, pos, DLB_I32, weights.data_ptr<float>(), m, (int)top_k, out.data_ptr(),
+                          c.stream));
+  return out;
+}
+
+PyObject* py_moe_forward_16bit(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 5);
+    return wrap(moe_forward_16bit(tensor(a[0]), tensor(a[1]), tensor(a[2]), tensor(a[3]), tensor(a[4])));
+  });
+}
+
 // ---- module -------------------------------------------------------------------------------------------------------
 // bind({name: address}): the C ABI to call
 PyObject* py_bind(PyObject*, PyObject* arg) {
@@ -450,6 +651,10 @@ PyMethodDef methods[] = {
     FAST("route_softmax_topk", py_route_softmax_topk),
     FAST("route_grouped_topk", py_route_grouped_topk),
     FAST("moe_forward", py_moe_forward),
+    FAST("low_latency_forward", py_low_latency_forward),
+    FAST("m_grouped_gemm", py_m_grouped_gemm),
+    FAST("k_grouped_gemm", py_k_grouped_gemm),
+    FAST("moe_forward_16bit", py_moe_forward_16bit),
     {nullptr, nullptr, 0, nullptr},
 };
 

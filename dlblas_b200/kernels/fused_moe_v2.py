@@ -64,30 +64,5 @@ def _fused_moe_16bit(hidden: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, t
     activations' 16-bit type): rows copied into expert order -> w1 grouped GEMM -> silu(gate) * up -> w2 grouped GEMM
     -> sum over top-k of weight * row in fp32, one rounding.  Both GEMMs run on the 16-bit tcgen05 kernel; ids outside
     [0, E) (other ranks' experts under `expert_map`) contribute nothing."""
-    import os
-    from .. import ops
-    assert hidden.dtype in (torch.bfloat16, torch.float16), "the unquantised mode takes bf16 or fp16 activations"
-    assert w1.dtype == hidden.dtype and w2.dtype == hidden.dtype, "weights must have the activations' type"
-    m, h = hidden.shape
-    e, n2, _ = w1.shape
-    assert w2.shape == (e, h, n2 // 2), "w2 must be [E, H, I]"
-    top_k = ids.shape[1]
-    out_dtype = out_dtype or hidden.dtype
-    if m == 0:
-        return torch.empty(0, h, dtype=out_dtype, device=hidden.device)
-    s_rows = m * top_k
-    ids = ids.contiguous()
-    _, exp_start, exp_end, pos = ops.sort_by_expert(ids, e, want_pos=True)
-    tile_rows = int(os.environ.get("DLBLAS_GEMM16_TILE_ROWS", "256" if s_rows >= 512 * e else "128"))
-    max_tiles = ops.max_tiles_for(s_rows, e, tile_rows)
-    tiles = ops.build_tiles(exp_start, exp_end, 0, e, max_tiles, tile_rows)
-    a1, _ = ops.permute_rows(hidden, None, pos, top_k, s_rows)
-    c1 = torch.empty(s_rows, n2, dtype=hidden.dtype, device=hidden.device)
-    ops.grouped_gemm_16bit(a1, w1.contiguous(), tiles, max_tiles, tile_rows, c1)
-    act = ops.silu_and_mul(c1)
-    y = torch.empty(s_rows, h, dtype=hidden.dtype, device=hidden.device)
-    ops.grouped_gemm_16bit(act, w2.contiguous(), tiles, max_tiles, tile_rows, y)
-    out = torch.empty(m, h, dtype=hidden.dtype, device=hidden.device)
-    weights = topk_weights.contiguous().float()
-    ops.ep_gather(y, ids.to(torch.int32), weights, pos.view(m, top_k), out)
-    return out if out_dtype == hidden.dtype else out.to(out_dtype)
+    out = _C.host().moe_forward_16bit(hidden, w1, w2, topk_weights, ids)
+    return out if out_dtype in (None, out.dtype) else out.to(out_dtype)
