@@ -13,6 +13,7 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -20,6 +21,7 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <cmath>
 #include <cstdlib>
 #include <mutex>
 #include <optional>
@@ -52,7 +54,14 @@ using at::Tensor;
   X(dlb_grouped_gemm_16bit_b_kn)                                                                                      \
   X(dlb_k_grouped_gemm_workspace_bytes)                                                                               \
   X(dlb_k_grouped_gemm_16bit)                                                                                         \
-  X(dlb_silu_and_mul)
+  X(dlb_silu_and_mul)                                                                                                 \
+  X(dlb_moe_align_block_size)                                                                                         \
+  X(dlb_topk_gating_workspace_size)                                                                                   \
+  X(dlb_topk_gating)                                                                                                  \
+  X(dlb_topk_gating_bwd)                                                                                              \
+  X(dlb_permute_plan)                                                                                                 \
+  X(dlb_unpermute)                                                                                                    \
+  X(dlb_unpermute_bwd_rows)
 
 struct Abi {
 #define X(name) decltype(&::name) name = nullptr;
@@ -619,6 +628,346 @@ PyObject* py_moe_forward_16bit(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+// ---- block-aligned token layout -----------------------------------------------------------------------------------
+PyObject* py_moe_align_block_size(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 6);
+    Tensor given = tensor(a[0]);
+    const int64_t block = integer(a[1]), experts = integer(a[2]), local = integer(a[3]);
+    const std::optional<Tensor> expert_map = opt_tensor(a[4]);
+    require_cuda(given);
+    require(given.scalar_type() == at::kInt || given.scalar_type() == at::kLong, "topk_ids must be int32 or int64");
+    Call c(given);
+    Tensor ids = given.is_contiguous() ? given : given.contiguous();
+    const int64_t slots = ids.numel();
+    int64_t padded = slots + experts * (block - 1);
+    if (truth(a[5])) padded = (padded + block - 1) / block * block;
+    const int64_t blocks = (padded + block - 1) / block;
+    Tensor sorted = empty({padded}, at::kInt, c), owner = empty({blocks}, at::kInt, c), total = empty({1}, at::kInt, c);
+    const size_t sort_bytes = abi.dlb_sort_by_expert_workspace_size(slots, (int)experts);
+    Workspace ws;
+    ws.take(sort_bytes);
+    ws.allocate(c);
+    check(abi.dlb_moe_align_block_size(ids.data_ptr(), code(ids.scalar_type()), slots, (int)experts, (int)local, (int)block,
+                                       sorted.data_ptr<int32_t>(), padded, owner.data_ptr<int32_t>(), (int)blocks,
+                                       total.data_ptr<int32_t>(), ws.at<void>(0), sort_bytes, c.stream));
+    if (!ids.is_same(given)) given.copy_(ids);      // negative ids are replaced in the caller's tensor
+    if (expert_map) owner = expert_map->index({owner.to(at::kLong)});
+    return wrap_tuple({&sorted, &owner, &total});
+  });
+}
+
+// ---- capacity-limited gating --------------------------------------------------------------------------------------
+// ceil(T / E * capacity_factor), at least min_capacity, from the single-precision product that the reference forms
+int64_t gating_capacity(int64_t tokens, int64_t experts, double factor, int64_t min_capacity) {
+  const float per_expert = (float)((double)tokens / (double)experts), f = (float)factor;
+  return std::max<int64_t>((int64_t)std::ceil(per_expert * f), min_capacity);
+}
+
+PyObject* py_gating_capacity(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 4);
+    return PyLong_FromLongLong(gating_capacity(integer(a[0]), integer(a[1]), real(a[2]), integer(a[3])));
+  });
+}
+
+struct Gating {
+  Tensor l_aux, ec_idx, weights, select, ws;
+};
+Gating gating_forward(const Tensor& given, int64_t k, int64_t capacity) {
+  require_cuda(given);
+  require(given.dim() == 2, "logits must be 2-D");
+  Call c(given);
+  const Tensor logits = given.is_contiguous() ? given : given.contiguous();
+  const int64_t t = logits.size(0), e = logits.size(1);
+  const size_t bytes = abi.dlb_topk_gating_workspace_size(t, (int)e, (int)k);
+  Gating g{empty({}, logits.scalar_type(), c), empty({k * t}, at::kInt, c), empty({k * t}, logits.scalar_type(), c),
+           empty({e * capacity}, at::kLong, c), empty({(int64_t)std::max<size_t>(bytes, 1)}, at::kByte, c)};
+  check(abi.dlb_topk_gating(logits.data_ptr(), code(logits.scalar_type()), t, (int)e, (int)k, capacity, g.l_aux.data_ptr(),
+                            g.ec_idx.data_ptr<int32_t>(), g.weights.data_ptr(), g.select.data_ptr<int64_t>(),
+                            g.ws.data_ptr(), bytes, c.stream));
+  return g;
+}
+
+Tensor gating_backward(const Tensor& ws, at::ScalarType dt, int64_t tokens, int64_t experts, int64_t k, int64_t capacity,
+                       const Tensor& grad_l_aux, const Tensor& grad_weights) {
+  require_cuda(ws);
+  Call c(ws);
+  auto ready = [&](const Tensor& g) {
+    Tensor r = g.scalar_type() == dt ? g : g.to(dt);
+    return r.is_contiguous() ? r : r.contiguous();
+  };
+  const Tensor gl = grad_l_aux.defined() ? ready(grad_l_aux) : at::zeros({}, ws.options().dtype(dt));
+  const Tensor gw = grad_weights.defined() ? ready(grad_weights) : Tensor();
+  Tensor out = empty({tokens, experts}, dt, c);
+  check(abi.dlb_topk_gating_bwd(ws.data_ptr(), ws.numel(), code(dt), tokens, (int)experts, (int)k, capacity, gl.data_ptr(),
+                                gw.defined() ? gw.data_ptr() : nullptr, out.data_ptr(), c.stream));
+  return out;
+}
+
+// dlblas/kernels/topk_gating.py:245-285.  The backward differentiates the auxiliary loss (topk_gating_bwd.py:13-68) and,
+// with `higher_precision`, the weights too.
+struct GatingFunction : torch::autograd::Function<GatingFunction> {
+  static torch::autograd::variable_list forward(torch::autograd::AutogradContext* ctx, const Tensor& logits, int64_t k,
+                                                int64_t capacity, bool higher_precision) {
+    Gating g = gating_forward(logits, k, capacity);
+    ctx->set_materialize_grads(false);
+    ctx->saved_data["k"] = k;
+    ctx->saved_data["capacity"] = capacity;
+    ctx->saved_data["hp"] = higher_precision;
+    ctx->saved_data["t"] = logits.size(0);
+    ctx->saved_data["e"] = logits.size(1);
+    ctx->saved_data["dtype"] = (int64_t)logits.scalar_type();
+    ctx->save_for_backward({g.ws});
+    ctx->mark_non_differentiable({g.ec_idx, g.select});
+    return {g.l_aux, g.ec_idx, g.weights, g.select};
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    auto& s = ctx->saved_data;
+    const Tensor ws = ctx->get_saved_variables()[0];
+    return {gating_backward(ws, (at::ScalarType)s["dtype"].toInt(), s["t"].toInt(), s["e"].toInt(), s["k"].toInt(),
+                            s["capacity"].toInt(), grads[0], s["hp"].toBool() ? grads[2] : Tensor()),
+            Tensor(), Tensor(), Tensor()};
+  }
+};
+
+// (logits, k, capacity, with workspace) -> (l_aux, ec_idx, weights, select[, workspace])
+PyObject* py_gating_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 4);
+    Gating g = gating_forward(tensor(a[0]), integer(a[1]), integer(a[2]));
+    return truth(a[3]) ? wrap_tuple({&g.l_aux, &g.ec_idx, &g.weights, &g.select, &g.ws})
+                       : wrap_tuple({&g.l_aux, &g.ec_idx, &g.weights, &g.select});
+  });
+}
+
+PyObject* py_gating_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 8);
+    const std::optional<Tensor> gw = opt_tensor(a[7]);
+    return wrap(gating_backward(tensor(a[0]), dtype(a[1]), integer(a[2]), integer(a[3]), integer(a[4]), integer(a[5]),
+                                tensor(a[6]), gw ? *gw : Tensor()));
+  });
+}
+
+// (logits, k, capacity_factor, min_capacity, higher_precision): differentiable in the logits
+PyObject* py_topk_gating(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 5);
+    const Tensor& logits = tensor(a[0]);
+    const int64_t k = integer(a[1]);
+    require(logits.dim() == 2, "logits must be 2-D");
+    const int64_t capacity = gating_capacity(logits.size(0), logits.size(1), real(a[2]) * (double)k, integer(a[3]));
+    if (logits.requires_grad() && at::GradMode::is_enabled()) {
+      auto r = GatingFunction::apply(logits, k, capacity, truth(a[4]));
+      return wrap_tuple({&r[0], &r[1], &r[2], &r[3]});
+    }
+    Gating g = gating_forward(logits, k, capacity);
+    return wrap_tuple({&g.l_aux, &g.ec_idx, &g.weights, &g.select});
+  });
+}
+
+// ---- training-side permutation (dlblas/kernels/permute/moe_triton_kernels.py) -------------------------------------
+// Ids below this bound are sorted without a look at them on the host.
+constexpr int PERMUTE_EXPERTS = 1024;
+
+struct PermutePlan {
+  Tensor sorted_idx, dest, row_map;   // sorted flat slots; row of every slot; the same, top_k-major
+  int64_t minus_one = 0, negative = 0;
+};
+
+// The output of a permutation has as many rows as slots are routed, so one value has to reach the host.  The kernel that
+// counts the ids hands their statistics over in pinned memory behind an event; the placement of the rows is queued before
+// the host waits for that event, so the GPU works while the host looks.
+PermutePlan permute_plan(const Tensor& indices, int64_t dest_limit, bool want_sorted) {
+  require_cuda(indices);
+  require(indices.dim() == 2, "indices must be [tokens, top_k]");
+  require(indices.scalar_type() == at::kInt || indices.scalar_type() == at::kLong, "topk_ids must be int32 or int64");
+  Call c(indices);
+  const Tensor ids = indices.is_contiguous() ? indices : indices.contiguous();
+  const int64_t t = ids.size(0), k = ids.size(1), slots = t * k;
+  PermutePlan p;
+  if (want_sorted) p.sorted_idx = empty({slots}, at::kLong, c);
+  p.dest = empty({slots}, at::kInt, c);
+  p.row_map = empty({slots}, at::kInt, c);
+  // one event and twelve bytes per thread and device: both are used up before this function returns
+  thread_local at::cuda::CUDAEvent events[16];
+  thread_local Tensor stats_mem[16];
+  const int dev = c.device.index();
+  require(dev < 16, "device index out of range");
+  if (!stats_mem[dev].defined()) {
+    stats_mem[dev] = at::empty({4}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+    events[dev].record(at::cuda::getCurrentCUDAStream(c.device.index()));   // creates the event
+  }
+  int32_t* stats = stats_mem[dev].data_ptr<int32_t>();
+  auto plan = [&](int64_t experts, bool with_stats) {
+    const size_t bytes = abi.dlb_sort_by_expert_workspace_size(slots, (int)experts);
+    Workspace ws;
+    ws.take(bytes);
+    ws.allocate(c);
+    check(abi.dlb_permute_plan(ids.data_ptr(), code(ids.scalar_type()), t, (int)k, (int)experts, dest_limit,
+                               want_sorted ? p.sorted_idx.data_ptr<int64_t>() : nullptr, p.dest.data_ptr<int32_t>(),
+                               p.row_map.data_ptr<int32_t>(), with_stats ? stats : nullptr,
+                               with_stats ? (void*)events[dev].event() : nullptr, ws.at<void>(0), bytes, c.stream));
+  };
+  plan(PERMUTE_EXPERTS, true);
+  PyThreadState* others = PyGILState_Check() ? PyEval_SaveThread() : nullptr;   // the host may wait here: let others run
+  const cudaError_t waited = cudaEventSynchronize(events[dev].event());
+  if (others != nullptr) PyEval_RestoreThread(others);
+  if (waited != cudaSuccess) throw std::runtime_error(std::string("permute: ") + cudaGetErrorString(waited));
+  const int64_t largest = stats[0];
+  p.minus_one = stats[1];
+  p.negative = stats[2];
+  if (largest >= PERMUTE_EXPERTS) plan(largest + 1, false);
+  return p;
+}
+
+// Copies the rows of x to their places in `out`; rows that no slot fills become zero.
+void permute_rows(const Tensor& x, const PermutePlan& p, int64_t k, const Tensor& out) {
+  Call c(x);
+  const int64_t t = x.size(0), routed = t * k - p.negative, row_bytes = x.size(1) * x.element_size();
+  if (out.size(0) > routed) out.narrow(0, routed, out.size(0) - routed).zero_();
+  check(abi.dlb_permute_rows(x.data_ptr(), row_bytes, nullptr, 0, t, p.dest.data_ptr<int32_t>(), (int)k, out.data_ptr(),
+                             nullptr, c.stream));
+}
+
+// moe_permute_topk_op_triton: (indices, rows wanted) -> (sorted_idx, dest, row_id_map, ids equal to -1, ids below 0)
+PyObject* py_permute_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 2);
+    PermutePlan p = permute_plan(tensor(a[0]), integer(a[1]), true);
+    return Py_BuildValue("(NNNLL)", wrap(p.sorted_idx), wrap(p.dest), wrap(p.row_map), (long long)p.minus_one,
+                         (long long)p.negative);
+  });
+}
+
+Tensor unpermute_rows(const Tensor& x_in, const Tensor& row_map_in, const Tensor& probs_in, int64_t tokens, int64_t k) {
+  require_cuda(x_in);
+  require_cuda(row_map_in);
+  Call c(x_in);
+  const Tensor x = x_in.is_contiguous() ? x_in : x_in.contiguous();
+  const Tensor row_map = row_map_in.is_contiguous() ? row_map_in : row_map_in.contiguous();
+  Tensor probs;
+  if (probs_in.defined()) {
+    probs = probs_in.scalar_type() == at::kFloat ? probs_in : probs_in.to(at::kFloat);
+    if (!probs.is_contiguous()) probs = probs.contiguous();
+  }
+  Tensor out = empty({tokens, x.size(1)}, x.scalar_type(), c);
+  check(abi.dlb_unpermute(x.data_ptr(), code(x.scalar_type()), row_map.data_ptr<int32_t>(),
+                          probs.defined() ? probs.data_ptr<float>() : nullptr, tokens, (int)k, x.size(1), out.data_ptr(),
+                          c.stream));
+  return out;
+}
+
+PyObject* py_unpermute_rows(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 5);
+    const std::optional<Tensor> probs = opt_tensor(a[2]);
+    return wrap(unpermute_rows(tensor(a[0]), tensor(a[1]), probs ? *probs : Tensor(), integer(a[3]), integer(a[4])));
+  });
+}
+
+// (gradient of the rows in act_dtype, gradient of the probabilities in fp32)
+std::pair<Tensor, Tensor> unpermute_backward(const Tensor& grad_in, const Tensor& fwd_in, const Tensor& row_map_in,
+                                             const Tensor& probs_in, at::ScalarType act_dtype) {
+  require_cuda(grad_in);
+  require_cuda(fwd_in);
+  Call c(grad_in);
+  require(grad_in.scalar_type() == fwd_in.scalar_type(), "gradient and rows must have one type");
+  const int64_t t = probs_in.size(0), k = probs_in.size(1), h = grad_in.size(1), rows = fwd_in.size(0);
+  const Tensor grad = grad_in.is_contiguous() ? grad_in : grad_in.contiguous();
+  const Tensor fwd = fwd_in.is_contiguous() ? fwd_in : fwd_in.contiguous();
+  const Tensor row_map = row_map_in.is_contiguous() ? row_map_in : row_map_in.contiguous();
+  Tensor probs = probs_in.scalar_type() == at::kFloat ? probs_in : probs_in.to(at::kFloat);
+  if (!probs.is_contiguous()) probs = probs.contiguous();
+  Tensor act = empty({rows, fwd.size(1)}, act_dtype, c), prob_grad = empty({t, k}, at::kFloat, c);
+  Workspace ws;
+  ws.take(rows);
+  ws.allocate(c);
+  check(abi.dlb_unpermute_bwd_rows(grad.data_ptr(), fwd.data_ptr(), code(grad.scalar_type()), row_map.data_ptr<int32_t>(),
+                                   probs.data_ptr<float>(), t, (int)k, h, rows, act.data_ptr(), code(act_dtype),
+                                   prob_grad.data_ptr<float>(), ws.at<void>(0), c.stream));
+  return {act, prob_grad};
+}
+
+PyObject* py_unpermute_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 5);
+    auto [act, prob] = unpermute_backward(tensor(a[0]), tensor(a[1]), tensor(a[2]), tensor(a[3]), dtype(a[4]));
+    return wrap_tuple({&act, &prob});
+  });
+}
+
+struct PermuteFunction : torch::autograd::Function<PermuteFunction> {
+  static torch::autograd::variable_list forward(torch::autograd::AutogradContext* ctx, const Tensor& x_in,
+                                                const Tensor& indices) {
+    const Tensor x = x_in.is_contiguous() ? x_in : x_in.contiguous();
+    const int64_t t = x.size(0), k = indices.size(1);
+    PermutePlan p = permute_plan(indices, t * k, false);
+    Call c(x);
+    Tensor out = empty({t * k - p.minus_one, x.size(1)}, x.scalar_type(), c);
+    permute_rows(x, p, k, out);
+    ctx->set_materialize_grads(false);
+    ctx->save_for_backward({p.row_map});
+    ctx->saved_data["t"] = t;
+    ctx->saved_data["k"] = k;
+    ctx->mark_non_differentiable({p.row_map});
+    return {out, p.row_map};
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    if (!grads[0].defined() || grads[0].numel() == 0) return {grads[0], Tensor()};
+    return {unpermute_rows(grads[0], ctx->get_saved_variables()[0], Tensor(), ctx->saved_data["t"].toInt(),
+                           ctx->saved_data["k"].toInt()),
+            Tensor()};
+  }
+};
+
+PyObject* py_permute(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need_args(n, 2);
+    const Tensor& x = tensor(a[0]);
+    Tensor indices = tensor(a[1]);
+    if (x.numel() == 0) return Py_BuildValue("(NO)", wrap(x), Py_None);
+    if (indices.dim() == 1) indices = indices.view({-1, 1});
+    if (!x.is_cuda() || !indices.is_cuda()) throw std::runtime_error("permute needs CUDA tensors");
+    if (x.size(0) != indices.size(0))
+      throw std::runtime_error("token count mismatch: " + std::to_string(x.size(0)) + " vs " + std::to_string(indices.size(0)));
+    auto r = PermuteFunction::apply(x, indices);
+    return wrap_tuple({&r[0], &r[1]});
+  });
+}
+
+struct UnpermuteFunction : torch::autograd::Function<UnpermuteFunction> {
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const Tensor& row_map,
+                        const std::optional<Tensor>& probs) {
+    const int64_t t = probs ? probs->size(0) : row_map.numel(), k = probs ? probs->size(1) : 1;
+    ctx->save_for_backward({x, row_map, probs ? *probs : Tensor()});
+    ctx->saved_data["with_probs"] = probs.has_value();
+    return unpermute_rows(x, row_map, probs ? *probs : Tensor(), t, k);
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &row_map = saved[1];
+    if (!ctx->saved_data["with_probs"].toBool()) {
+      const Tensor ones = at::ones({row_map.numel(), 1}, row_map.options().dtype(at::kFloat));
+      return {unpermute_backward(grads[0], x, row_map, ones, x.scalar_type()).first, Tensor(), Tensor()};
+    }
+    auto [act, prob] = unpermute_backward(grads[0], x, row_map, saved[2], x.scalar_type());
+    if (!ctx->needs_input_grad(2)) prob = Tensor();
+    else if (prob.scalar_type() != saved[2].scalar_type()) prob = prob.to(saved[2].scalar_type());
+    return {act, Tensor(), prob};
+  }
+};
+
+PyObject* py_unpermute(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    need_args(n, 3);
+    const Tensor& x = tensor(a[0]);
+    if (x.numel() == 0) return wrap(x);
+    return wrap(UnpermuteFunction::apply(x, tensor(a[1]), opt_tensor(a[2])));
+  });
+}
+
 // ---- module -------------------------------------------------------------------------------------------------------
 // bind({name: address}): the C ABI to call
 PyObject* py_bind(PyObject*, PyObject* arg) {
@@ -655,6 +1004,16 @@ PyMethodDef methods[] = {
     FAST("m_grouped_gemm", py_m_grouped_gemm),
     FAST("k_grouped_gemm", py_k_grouped_gemm),
     FAST("moe_forward_16bit", py_moe_forward_16bit),
+    FAST("moe_align_block_size", py_moe_align_block_size),
+    FAST("gating_capacity", py_gating_capacity),
+    FAST("gating_forward", py_gating_forward),
+    FAST("gating_backward", py_gating_backward),
+    FAST("topk_gating", py_topk_gating),
+    FAST("permute_plan", py_permute_plan),
+    FAST("unpermute_rows", py_unpermute_rows),
+    FAST("unpermute_backward", py_unpermute_backward),
+    FAST("permute", py_permute),
+    FAST("unpermute", py_unpermute),
     {nullptr, nullptr, 0, nullptr},
 };
 

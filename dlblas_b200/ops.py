@@ -253,32 +253,11 @@ def route_grouped_topk(logits: torch.Tensor, bias: torch.Tensor, top_k: int, ren
 def topk_gating_bwd(ws: torch.Tensor, dtype, tokens: int, experts: int, k: int, capacity: int, grad_l_aux: torch.Tensor,
                     grad_weights):
     """grad of (l_aux, token_exp_weights) w.r.t. the logits from the forward's workspace `ws`."""
-    require_cuda(ws, grad_l_aux)
-    dev = ws.device
-    grad_l_aux = grad_l_aux.to(dtype).contiguous()
-    gw = None if grad_weights is None else grad_weights.to(dtype).contiguous()
-    out = torch.empty(tokens, experts, dtype=dtype, device=dev)
-    check(lib().dlb_topk_gating_bwd(ptr(ws), ws.numel(), dtype_code(dtype), tokens, experts, k, capacity,
-                                    ptr(grad_l_aux), 0 if gw is None else ptr(gw), ptr(out), stream(dev)))
-    return out
+    return host().gating_backward(ws, dtype, tokens, experts, k, capacity, grad_l_aux, grad_weights)
 
 
 def topk_gating(logits: torch.Tensor, k: int, capacity: int, return_workspace: bool = False):
-    require_cuda(logits)
-    assert logits.dim() == 2 and logits.is_contiguous()
-    t, e = logits.shape
-    dev = logits.device
-    l_aux = torch.empty((), dtype=logits.dtype, device=dev)
-    ec_idx = torch.empty(k * t, dtype=torch.int32, device=dev)
-    w = torch.empty(k * t, dtype=logits.dtype, device=dev)
-    sel = torch.empty(e * capacity, dtype=torch.int64, device=dev)
-    ws_bytes = lib().dlb_topk_gating_workspace_size(t, e, k)
-    ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=dev)
-    check(lib().dlb_topk_gating(ptr(logits), dtype_code(logits.dtype), t, e, k, capacity, ptr(l_aux), ptr(ec_idx), ptr(w),
-                                ptr(sel), ptr(ws), ws_bytes, stream(dev)))
-    if return_workspace:
-        return l_aux, ec_idx, w, sel, ws
-    return l_aux, ec_idx, w, sel
+    return host().gating_forward(logits, k, capacity, return_workspace)
 
 
 def ep_dest_ranks(topk_ids: torch.Tensor, num_local_experts: int, world_size: int) -> torch.Tensor:
