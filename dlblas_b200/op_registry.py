@@ -5,6 +5,8 @@ op_registry.py:124-136); the first matching candidate is taken, and nothing impo
 from dataclasses import dataclass, field
 from typing import Optional
 
+import torch
+
 from .cache import Cache
 from .op_struct import OpImpl, match, parse_args
 
@@ -13,6 +15,8 @@ from .op_struct import OpImpl, match, parse_args
 class OpRegistry:
     ops: dict = field(default_factory=dict)
     cache: Cache = field(default_factory=Cache)
+    # what the text key of `Cache.gen_key` says, as a tuple: building the text takes longer than a small operator
+    quick: dict = field(default_factory=dict)
 
     def register(self, name, spaces, args, call, bench_fn, kernel):
         params = parse_args(args)
@@ -37,6 +41,21 @@ class OpRegistry:
         return self.cache.get(op_name, args, cache_key)
 
     def get_op(self, op_name: str, args: tuple, configs=None, cache_key=None) -> OpImpl:
+        key = None
+        if cache_key is None and isinstance(args, tuple):
+            try:
+                key = (op_name, *[(a.dtype, a.shape) if isinstance(a, torch.Tensor) else (type(a), a) for a in args])
+                op = self.quick.get(key)
+                if op is not None:
+                    return op
+            except TypeError:      # an argument that cannot be hashed
+                key = None
+        op = self._get_op(op_name, args, cache_key)
+        if key is not None:
+            self.quick[key] = op
+        return op
+
+    def _get_op(self, op_name: str, args: tuple, cache_key) -> OpImpl:
         if op_name not in self.ops:
             raise NameError(f"op {op_name} not found")
         op = self.look_up_cache(op_name, args, cache_key)
