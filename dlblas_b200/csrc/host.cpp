@@ -21,6 +21,9 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <cctype>
+#include <cerrno>
+#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <mutex>
@@ -171,6 +174,20 @@ void require_cuda(const Tensor& t) {
     throw std::runtime_error("dlblas_b200 runs on CUDA tensors only (B200, sm_100a); there is no CPU path");
 }
 
+// Every tensor whose memory a kernel reads: a host address would fault the device.
+void require_cuda(std::initializer_list<const Tensor*> ts) {
+  for (const Tensor* t : ts) require_cuda(*t);
+}
+
+// Weights [experts, n, k] of an FP8 layer and one scale per 128 x 128 block: the kernels take the sizes from here, so a
+// tensor of another shape would be read past its end.
+void require_fp8_weights(const Tensor& w, const Tensor& w_s, int64_t e, int64_t n, int64_t k) {
+  require(w.dim() == 3 && w.size(0) == e && w.size(1) == n && w.size(2) == k && w.element_size() == 1,
+          "expert weights must be e4m3 [experts, n, k] with matching sizes");
+  require(w_s.numel() == e * ((n + 127) / 128) * (k / 128), "one weight scale per 128 x 128 block");
+  require(w.is_contiguous() && w_s.is_contiguous(), "weights and scales must be contiguous");
+}
+
 Tensor empty(at::IntArrayRef sizes, at::ScalarType dt, const Call& c) {
   return at::detail::empty_cuda(sizes, dt, c.device, std::nullopt);
 }
@@ -211,9 +228,24 @@ Tensor status_word(at::DeviceIndex index) {
 }
 int32_t* status_ptr(const Call& c) { return status_word(c.device.index()).data_ptr<int32_t>(); }
 
+// A whole number from the environment; text that is none is an error, as Python's int() makes it.
 int env_int(const char* name, int fallback) {
   const char* v = std::getenv(name);
-  return v != nullptr && *v != 0 ? std::atoi(v) : fallback;
+  if (v == nullptr) return fallback;
+  char* end = nullptr;
+  errno = 0;
+  const long n = std::strtol(v, &end, 10);
+  while (end != v && std::isspace((unsigned char)*end)) ++end;
+  if (end == v || *end != 0 || errno != 0 || n < INT_MIN || n > INT_MAX) {
+    PyErr_Format(PyExc_ValueError, "%s must be a whole number, got '%s'", name, v);
+    throw PyFailed{};
+  }
+  return (int)n;
+}
+int tile_rows_env(const char* name, int fallback) {
+  const int rows = env_int(name, fallback);
+  if (rows != 128 && rows != 256) throw AssertionFailed(std::string(name) + " must be 128 or 256");
+  return rows;
 }
 
 // ---- quantisation and the dense GEMM ------------------------------------------------------------------------------
@@ -223,6 +255,8 @@ std::pair<Tensor, Tensor> quant_fp8(const Tensor& x, int64_t group, int mode, do
   require_cuda(x);
   require(x.dim() == 2 && x.stride(1) == 1, "x must be 2-D with contiguous rows");
   const int64_t m = x.size(0), k = x.size(1), rows = rows_out < 0 ? m : rows_out;
+  require(group > 0, "group_size must be positive");
+  if (dst_pos) require_cuda(*dst_pos);
   if (k % group != 0)
     throw AssertionFailed("the last dimension of 'x' " + std::to_string(k) + " must be divisible by 'group_size' " +
                           std::to_string(group));
@@ -251,6 +285,7 @@ PyObject* py_group_quant_fp8(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor& x = tensor(a[0]);
     const int64_t group = integer(a[1]);
     const bool column_major = truth(a[3]);
+    require(x.dim() > 0 && x.stride(-1) == 1, "groups must be contiguous");
     if (x.dim() == 2) {
       auto [q, s] = quant_fp8(x, group, DLB_QUANT_DIV_EPS, real(a[2]), column_major, std::nullopt, 1, -1);
       return wrap_tuple({&q, &s});
@@ -272,7 +307,9 @@ Tensor fp8_gemm(const Tensor& a, const Tensor& b, const Tensor& a_s, const Tenso
   if (out_dtype == at::kFloat) tile_rows = 128;
   require(a.is_contiguous() && b.is_contiguous(), "Input tensors must be contiguous");
   require(a_s.is_contiguous() && b_s.is_contiguous(), "Scaling factor tensors must be contiguous");
+  require(a.dim() > 0 && a.size(-1) > 0, "a must have a last dimension of at least 128");
   const int64_t k = a.size(-1), m = a.numel() / k, n = b.size(0), kb = k / 128;
+  require(b.numel() == n * k, "b must be [n, k]");
   require(a_s.numel() == m * kb && b_s.numel() == (n + 127) / 128 * kb, "scale shapes do not match a / b");
   Call c(a);
   Tensor out;
@@ -351,14 +388,16 @@ struct MoeArgs {
 
 Tensor moe_forward(const MoeArgs& g) {
   const Tensor& x = g.hidden ? *g.hidden : *g.x_q;
-  require_cuda(x);
-  require_cuda(g.w1);
-  for (const Tensor* t : {&g.w1, &g.w1_s, &g.w2, &g.w2_s}) require(t->is_contiguous(), "weights and scales must be contiguous");
+  require_cuda({&x, &g.w1, &g.w1_s, &g.w2, &g.w2_s, &g.weights, &g.ids});
+  if (g.x_s) require_cuda(*g.x_s);
+  require(g.w1.dim() == 3, "w1 must be [experts, 2 * intermediate, hidden]");
   require(g.ids.scalar_type() == at::kInt || g.ids.scalar_type() == at::kLong, "topk_ids must be int32 or int64");
   require(x.dim() == 2 && x.stride(1) == 1, "x must be 2-D with contiguous rows");
   Call c(x);
   const int64_t e_local = g.w1.size(0), n = g.w1.size(1), h = g.w1.size(2), inter = n / 2;
   const int64_t m = x.size(0), slots = m * g.top_k;
+  require_fp8_weights(g.w1, g.w1_s, e_local, n, h);
+  require_fp8_weights(g.w2, g.w2_s, e_local, h, inter);
   Tensor out = empty({m, h}, g.out_dtype, c);
   if (m == 0) return out;
   require(x.size(1) == h, "hidden size mismatch");
@@ -374,6 +413,7 @@ Tensor moe_forward(const MoeArgs& g) {
   if (!weights.is_contiguous()) weights = weights.contiguous();
   int tile_rows = env_int("DLBLAS_FP8_TILE_ROWS", 0);
   if (tile_rows == 0 || g.out_dtype == at::kFloat) tile_rows = 128;
+  require(tile_rows == 128 || tile_rows == 256, "DLBLAS_FP8_TILE_ROWS must be 0, 128 or 256");
   const bool fused = g.fuse_swiglu && n % 256 == 0;
   const int max_tiles = (int)(slots / tile_rows + e_local);
   const size_t out_size = c10::elementSize(g.out_dtype);
@@ -441,20 +481,23 @@ PyObject* py_moe_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // [experts, max tokens, hidden] layout, and the layer is six launches of which two stream the weights.
 Tensor low_latency_forward(const Tensor& x, const Tensor& topk_weights, const Tensor& topk_ids, const Tensor& w1,
                            const Tensor& w1_s, const Tensor& w2, const Tensor& w2_s, at::ScalarType out_dtype) {
-  require_cuda(x);
-  require_cuda(w1);
-  for (const Tensor* t : {&w1, &w1_s, &w2, &w2_s}) require(t->is_contiguous(), "weights and scales must be contiguous");
+  require_cuda({&x, &w1, &w1_s, &w2, &w2_s, &topk_weights, &topk_ids});
+  require(topk_weights.scalar_type() == at::kFloat, "topk_weights must be fp32");
+  require(w1.dim() == 3, "w1 must be [experts, 2 * intermediate, hidden]");
+  require(topk_ids.dim() == 2, "topk_ids must be [tokens, top_k]");
   require(x.dim() == 2 && x.stride(1) == 1, "hidden states must be 2-D with contiguous rows");
   Call c(x);
   const int64_t e = w1.size(0), n = w1.size(1), h = w1.size(2), inter = n / 2;
   const int64_t m = x.size(0), top_k = topk_ids.size(1), slots = m * top_k;
   require(x.size(1) == h, "hidden size mismatch");
+  require(topk_ids.size(0) == m && topk_weights.numel() == slots, "topk_ids / topk_weights must be [tokens, top_k]");
+  require_fp8_weights(w1, w1_s, e, n, h);
+  require_fp8_weights(w2, w2_s, e, h, inter);
   Tensor out = empty({m, h}, out_dtype, c);
   if (m == 0) return out;
   Tensor ids = topk_ids.scalar_type() == at::kInt || topk_ids.scalar_type() == at::kLong ? topk_ids : topk_ids.to(at::kLong);
   if (!ids.is_contiguous()) ids = ids.contiguous();
-  Tensor weights = topk_weights.scalar_type() == at::kFloat ? topk_weights : topk_weights.to(at::kFloat);
-  if (!weights.is_contiguous()) weights = weights.contiguous();
+  const Tensor weights = topk_weights.is_contiguous() ? topk_weights : topk_weights.contiguous();
   const int max_tiles = (int)(slots / 128 + e);
   const size_t size = c10::elementSize(out_dtype);
   const size_t sort_bytes = abi.dlb_sort_by_expert_workspace_size(slots, (int)e);
@@ -497,7 +540,7 @@ PyObject* py_low_latency_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // pairs of CTAs on 256-row tiles when the groups are large enough to fill them (decided from the shapes, no look at the
 // group sizes on the host); DLBLAS_GEMM16_TILE_ROWS = 128 / 256 overrides
 int gemm16_tile_rows(int64_t rows, int64_t groups) {
-  return env_int("DLBLAS_GEMM16_TILE_ROWS", rows >= 512 * groups ? 256 : 128);
+  return tile_rows_env("DLBLAS_GEMM16_TILE_ROWS", rows >= 512 * groups ? 256 : 128);
 }
 
 Tensor group_sizes(const Tensor& sizes) {
@@ -563,7 +606,7 @@ Tensor k_grouped_gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& size
   Tensor sizes = group_sizes(sizes_in);
   if (sizes.scalar_type() != at::kLong) sizes = sizes.to(at::kLong);
   // pairs of CTAs on 256-row tiles of C unless M is smaller than one; DLBLAS_GEMM16_TILE_ROWS = 128 / 256 overrides
-  const int tile_rows = env_int("DLBLAS_GEMM16_TILE_ROWS", m >= 256 ? 256 : 128);
+  const int tile_rows = tile_rows_env("DLBLAS_GEMM16_TILE_ROWS", m >= 256 ? 256 : 128);
   const int64_t need = abi.dlb_k_grouped_gemm_workspace_bytes(k, m, n, (int)groups, tile_rows);
   require(need > 0, "k_grouped_gemm: bad sizes");
   const Tensor work = empty({need}, at::kByte, c);
@@ -586,8 +629,11 @@ Tensor moe_forward_16bit(const Tensor& x, const Tensor& w1_in, const Tensor& w2_
           "the unquantised mode takes bf16 or fp16 activations");
   require(w1_in.scalar_type() == x.scalar_type() && w2_in.scalar_type() == x.scalar_type(),
           "weights must have the activations' type");
-  require_cuda(x);
-  require_cuda(w1_in);
+  require_cuda({&x, &w1_in, &w2_in, &weights_in, &ids_in});
+  require(x.dim() == 2 && x.is_contiguous(), "activations must be contiguous [tokens, hidden]");
+  require(w1_in.dim() == 3 && w1_in.size(2) == x.size(1), "w1 must be [E, 2 I, H]");
+  require(ids_in.dim() == 2 && ids_in.size(0) == x.size(0) && weights_in.numel() == ids_in.numel(),
+          "topk_ids / topk_weights must be [tokens, top_k]");
   Call c(x);
   const int64_t m = x.size(0), h = x.size(1), e = w1_in.size(0), n2 = w1_in.size(1), inter = n2 / 2;
   require(w2_in.dim() == 3 && w2_in.size(0) == e && w2_in.size(1) == h && w2_in.size(2) == inter, "w2 must be [E, H, I]");
@@ -637,6 +683,7 @@ PyObject* py_moe_align_block_size(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const std::optional<Tensor> expert_map = opt_tensor(a[4]);
     require_cuda(given);
     require(given.scalar_type() == at::kInt || given.scalar_type() == at::kLong, "topk_ids must be int32 or int64");
+    require(block > 0 && experts > 0, "block_size and num_experts must be positive");
     Call c(given);
     Tensor ids = given.is_contiguous() ? given : given.contiguous();
     const int64_t slots = ids.numel();
@@ -660,6 +707,7 @@ PyObject* py_moe_align_block_size(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // ---- capacity-limited gating --------------------------------------------------------------------------------------
 // ceil(T / E * capacity_factor), at least min_capacity, from the single-precision product that the reference forms
 int64_t gating_capacity(int64_t tokens, int64_t experts, double factor, int64_t min_capacity) {
+  require(experts > 0, "logits must have at least one expert");
   const float per_expert = (float)((double)tokens / (double)experts), f = (float)factor;
   return std::max<int64_t>((int64_t)std::ceil(per_expert * f), min_capacity);
 }
@@ -842,8 +890,8 @@ PyObject* py_permute_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 Tensor unpermute_rows(const Tensor& x_in, const Tensor& row_map_in, const Tensor& probs_in, int64_t tokens, int64_t k) {
-  require_cuda(x_in);
-  require_cuda(row_map_in);
+  require_cuda({&x_in, &row_map_in});
+  if (probs_in.defined()) require_cuda(probs_in);
   Call c(x_in);
   const Tensor x = x_in.is_contiguous() ? x_in : x_in.contiguous();
   const Tensor row_map = row_map_in.is_contiguous() ? row_map_in : row_map_in.contiguous();
@@ -870,8 +918,7 @@ PyObject* py_unpermute_rows(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // (gradient of the rows in act_dtype, gradient of the probabilities in fp32)
 std::pair<Tensor, Tensor> unpermute_backward(const Tensor& grad_in, const Tensor& fwd_in, const Tensor& row_map_in,
                                              const Tensor& probs_in, at::ScalarType act_dtype) {
-  require_cuda(grad_in);
-  require_cuda(fwd_in);
+  require_cuda({&grad_in, &fwd_in, &row_map_in, &probs_in});
   Call c(grad_in);
   require(grad_in.scalar_type() == fwd_in.scalar_type(), "gradient and rows must have one type");
   const int64_t t = probs_in.size(0), k = probs_in.size(1), h = grad_in.size(1), rows = fwd_in.size(0);

@@ -10,6 +10,9 @@ import torch
 from .cache import Cache
 from .op_struct import OpImpl, match, parse_args
 
+_PLAIN = (int, float, bool, str)
+_QUICK_MAX = 1024      # batch sizes vary without end in a serving process
+
 
 @dataclass
 class OpRegistry:
@@ -43,15 +46,24 @@ class OpRegistry:
     def get_op(self, op_name: str, args: tuple, configs=None, cache_key=None) -> OpImpl:
         key = None
         if cache_key is None and isinstance(args, tuple):
-            try:
-                key = (op_name, *[(a.dtype, a.shape) if isinstance(a, torch.Tensor) else (type(a), a) for a in args])
+            key = [op_name]
+            for a in args:
+                if isinstance(a, torch.Tensor):
+                    key.append((a.dtype, a.shape))
+                elif a is None or type(a) in _PLAIN:
+                    key.append((type(a), a))
+                else:              # what else there is goes by its text: nothing of the caller's is kept
+                    key = None
+                    break
+            if key is not None:
+                key = tuple(key)
                 op = self.quick.get(key)
                 if op is not None:
                     return op
-            except TypeError:      # an argument that cannot be hashed
-                key = None
         op = self._get_op(op_name, args, cache_key)
         if key is not None:
+            if len(self.quick) >= _QUICK_MAX:
+                self.quick.clear()
             self.quick[key] = op
         return op
 

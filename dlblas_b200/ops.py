@@ -247,6 +247,7 @@ def route_softmax_topk(logits: torch.Tensor, top_k: int, renormalize: bool = Fal
 
 def route_grouped_topk(logits: torch.Tensor, bias: torch.Tensor, top_k: int, renormalize: bool, num_expert_group: int,
                        topk_group: int):
+    assert logits.is_contiguous(), "logits must be contiguous"
     return host().route_grouped_topk(logits, bias, top_k, renormalize, num_expert_group, topk_group)
 
 
@@ -257,6 +258,7 @@ def topk_gating_bwd(ws: torch.Tensor, dtype, tokens: int, experts: int, k: int, 
 
 
 def topk_gating(logits: torch.Tensor, k: int, capacity: int, return_workspace: bool = False):
+    assert logits.is_contiguous(), "logits must be contiguous"
     return host().gating_forward(logits, k, capacity, return_workspace)
 
 
