@@ -60,6 +60,7 @@ struct Args16 {
   const int4* kseg;
   int group_m_tiles;   // m tiles per group when kseg is given
   int band;            // n tiles per band of the tile order when kseg is given
+  int m_band;          // order of the tiles when it is not, see tile_at
   // Per-worker tile lists (a worker is a CTA or a pair): worker w runs tiles sched[w * sched_stride + i] for
   // i < sched_count[w].  Null: worker w runs tiles w, w + workers, ...
   const int* sched;
@@ -127,10 +128,9 @@ struct Tile16 {
 };
 constexpr int KG_BAND = 4;   // default n tiles per band in the tile order of k-grouped launches
 
-template <int CTAS> __device__ __forceinline__ Tile16 decode16(const Args16& g, int t) {
+template <int CTAS> __device__ __forceinline__ Tile16 decode16(const Args16& g, int num_m_tiles, int t) {
   Tile16 ti;
-  int m_tile = t / g.num_n_tiles;
-  int n_tile = t - m_tile * g.num_n_tiles;
+  int m_tile, n_tile;
   if (g.kseg != nullptr) {
     // Every group has the same m x n grid of tiles.  Walk it in bands of `band` n tiles, m tile by m tile inside a
     // band, so that the tiles in flight at one time share rows of both operands and a band of B can stay in L2 while
@@ -143,6 +143,8 @@ template <int CTAS> __device__ __forceinline__ Tile16 decode16(const Args16& g, 
     const int mt = li / width;
     m_tile = grp * g.group_m_tiles + mt;
     n_tile = band * g.band + (li - mt * width);
+  } else {
+    tile_at(t, num_m_tiles, g.num_n_tiles, g.m_band, m_tile, n_tile);
   }
   if (g.tiles != nullptr) {
     const int4 v = __ldg(g.tiles + 1 + m_tile);
@@ -202,7 +204,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
   const int my_tiles = g.sched != nullptr ? __ldg(g.sched_count + worker)
                                           : (worker < total_tiles ? (total_tiles - worker + workers - 1) / workers : 0);
   const int* my_sched = g.sched != nullptr ? g.sched + (long long)worker * g.sched_stride : nullptr;
-  auto tile_at = [&](int i) { return my_sched != nullptr ? __ldg(my_sched + i) : worker + i * workers; };
+  auto nth_tile = [&](int i) { return my_sched != nullptr ? __ldg(my_sched + i) : worker + i * workers; };
   const unsigned long long limit = g.timeout_cycles;
 
   if (threadIdx.x == 0) {
@@ -248,8 +250,8 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     uint32_t it = 0;
     bool ok = true;
     for (int i = 0; i < my_tiles && ok; ++i) {
-      const int t = tile_at(i);
-      const Tile16 ti = decode16<CTAS>(g, t);
+      const int t = nth_tile(i);
+      const Tile16 ti = decode16<CTAS>(g, num_m_tiles, t);
       const bool mn = g.kseg != nullptr;
       const int4 ks = mn ? __ldg(g.kseg + ti.e) : make_int4(0, kblocks, 64, 0);
       for (int kb = 0; kb < ks.y; ++kb, ++it) {
@@ -344,7 +346,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     // every use of every stage's barrier, block by block: a parity wait only tells the current phase from the one
     // before it, so a waiter that skipped uses could take an earlier phase for the one it wants.
     for (int i = 0; PAIR && mn && rank != 0 && i < my_tiles && ok; ++i) {
-      const int4 ks = __ldg(g.kseg + decode16<CTAS>(g, tile_at(i)).e);
+      const int4 ks = __ldg(g.kseg + decode16<CTAS>(g, num_m_tiles, nth_tile(i)).e);
       for (int kb = 0; kb < ks.y; ++kb, ++it) {
         const int s = it % STAGES;
         if (!mbar_wait(land_bar(s), (it / STAGES) & 1u, abort_flag, limit)) {
@@ -360,14 +362,14 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
       }
     }
     for (int i = 0; i < my_tiles && ok && rank == 0; ++i, ++tile_no) {
-      const int t = tile_at(i);
+      const int t = nth_tile(i);
       const int b = tile_no % TMEM_BUFS;
       if (!mbar_wait(tempty_bar(b), ((tile_no / TMEM_BUFS) & 1u) ^ 1u, abort_flag, limit)) {
         ok = false;
         break;
       }
       const uint32_t d_tmem = tmem_base + (uint32_t)(b * BN);
-      const int4 ks = mn ? __ldg(g.kseg + decode16<CTAS>(g, t).e) : make_int4(0, kblocks, 64, 0);
+      const int4 ks = mn ? __ldg(g.kseg + decode16<CTAS>(g, num_m_tiles, t).e) : make_int4(0, kblocks, 64, 0);
       const int nkb = ks.y;
       for (int kb = 0; kb < nkb; ++kb, ++it) {
         const int s = it % STAGES;
@@ -428,8 +430,8 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     uint32_t tile_no = 0;
     bool ok = true;
     for (int i = 0; i < my_tiles && ok; ++i, ++tile_no) {
-      const int t = tile_at(i);
-      const Tile16 ti = decode16<CTAS>(g, t);
+      const int t = nth_tile(i);
+      const Tile16 ti = decode16<CTAS>(g, num_m_tiles, t);
       if (!mbar_wait(staged_bar, tile_no & 1u, abort_flag, limit)) {
         ok = false;
         break;
@@ -460,7 +462,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     uint32_t tile_no = 0;
     bool ok = true;
     for (int i = 0; i < my_tiles && ok; ++i, ++tile_no) {
-      const int t = tile_at(i);
+      const int t = nth_tile(i);
       const int b = tile_no % TMEM_BUFS;
       if (!mbar_wait(tfull_bar(b), (tile_no / TMEM_BUFS) & 1u, abort_flag, limit) ||
           !mbar_wait(sfree_bar, (tile_no & 1u) ^ 1u, abort_flag, limit)) {
@@ -709,6 +711,7 @@ static int run_gemm16(const void* a, int64_t a_map_rows, int64_t a_row_bytes, in
   if (kseg != nullptr || b_mn) g.idesc |= 1u << 16;    // B MN-major
   g.status = status;
   g.timeout_cycles = wait_limit_cycles(DEFAULT_TIMEOUT_CYCLES);
+  g.m_band = tile_band(tile_rows, g.num_n_tiles);
   const int workers = sm_count() / ctas;
   const long long total = (long long)(tiles != nullptr ? max_tiles : g.num_m_tiles_static) * g.num_n_tiles;
   const int grid = ctas * (int)(total < workers ? total : workers);

@@ -66,6 +66,7 @@ struct GemmArgs {
   int n_half;                 // SWIGLU_QUANT: intermediate size (n / 2)
   int num_m_tiles_static;
   int num_n_tiles;
+  int m_band;    // order of the tiles, see tile_at
   int n_tile0;   // first n tile of the launch (a launch may cover a window of the columns; 0 otherwise)
   const long long* sorted_idx;
   const float* weights;
@@ -106,10 +107,10 @@ struct Tile {
 // The part of tile t that CTA `rank` of a pair works on (CTAS = 2: rows [rank * 128, rank * 128 + 128) of the
 // 256-row tile; its `rows` is 0 when the tile ends before them).
 template <int BN, int MODE, int CTAS = 1>
-__device__ __forceinline__ Tile decode_tile(const GemmArgs& g, int t, int rank = 0) {
+__device__ __forceinline__ Tile decode_tile(const GemmArgs& g, int num_m_tiles, int t, int rank = 0) {
   Tile ti;
-  const int m_tile = t / g.num_n_tiles;
-  const int n_tile = t - m_tile * g.num_n_tiles;
+  int m_tile, n_tile;
+  tile_at(t, num_m_tiles, g.num_n_tiles, g.m_band, m_tile, n_tile);
   if (g.tiles != nullptr) {
     const int4 v = __ldg(g.tiles + 1 + m_tile);
     ti.e = v.x;
@@ -251,7 +252,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       uint32_t it = 0;
       bool ok = true;
       for (int t = worker; t < total_tiles && ok; t += workers) {
-        const Tile ti = decode_tile<BN, MODE, CTAS>(g, t, (int)rank);
+        const Tile ti = decode_tile<BN, MODE, CTAS>(g, num_m_tiles, t, (int)rank);
         for (int kb = 0; kb < kblocks; ++kb, ++it) {
           const int s = it % C::STAGES;
           const uint32_t ph = (it / C::STAGES) & 1u;
@@ -356,7 +357,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     uint32_t tile_no = 0;
     bool ok = true;
     for (int t = worker; t < total_tiles && ok; t += workers, ++tile_no) {
-      const Tile ti = decode_tile<BN, MODE, CTAS>(g, t, (int)rank);
+      const Tile ti = decode_tile<BN, MODE, CTAS>(g, num_m_tiles, t, (int)rank);
       if constexpr (MODE == DLB_EPI_SWIGLU_QUANT) {
         // A staging row holds the tile's 128 gate columns, then its 128 up columns, already
         // rounded to OutT.  Reference rounding points: silu(gate)*up -> OutT, then
@@ -454,7 +455,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     uint32_t tile_no = 0;
     bool ok = true;
     for (int t = worker; t < total_tiles && ok; t += workers, ++tile_no) {
-      const Tile ti = decode_tile<BN, MODE, CTAS>(g, t, (int)rank);
+      const Tile ti = decode_tile<BN, MODE, CTAS>(g, num_m_tiles, t, (int)rank);
       const bool row_ok = r < ti.rows;
       const long long p = (long long)ti.row0 + r;          // row of A / sorted position
       // threads without a row read the scales of a row that exists (a pair's second CTA can hold an empty
@@ -757,6 +758,7 @@ extern "C" int dlb_fp8_gemm(const void* a, const void* b, const float* a_s, int6
   g.status = status;
   g.timeout_cycles = wait_limit_cycles(DEFAULT_TIMEOUT_CYCLES);
   g.withhold_loads = withhold_loads() ? 1 : 0;
+  g.m_band = tile_band(BM * ctas, g.num_n_tiles);
   const long long total = (long long)m_tiles * g.num_n_tiles;
   const int workers = sms / ctas;
   const int grid = ctas * (int)(total < workers ? total : workers);
@@ -836,6 +838,7 @@ static int moe_grouped_gemm(const void* a, const float* a_s, int64_t rows_a, con
     g.num_n_tiles = (int)ceil_div(n_count, bn);
     g.n_tile0 = (int)(n_begin / bn);
   }
+  g.m_band = tile_band(BM * ctas, g.num_n_tiles);
   const long long total = (long long)max_tiles * g.num_n_tiles;
   const int workers = sms / ctas;
   const int grid = ctas * (int)(total < workers ? total : workers);

@@ -64,6 +64,31 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
+// Order of the tiles of a persistent launch.  band = 1: n tile by n tile, then the next m tile.  band > 1: bands of that
+// many m tiles, each walked n tile by n tile with the m tiles innermost, so that the tiles in flight share their operands: in
+// the first order a launch of 112 n tiles holds one or two m tiles at a time, and the weights (117 MB an expert) come from
+// DRAM again for every 128 rows.
+__device__ __forceinline__ void tile_at(int t, int num_m_tiles, int num_n_tiles, int band, int& m_tile, int& n_tile) {
+  if (band <= 1) {
+    m_tile = t / num_n_tiles;
+    n_tile = t - m_tile * num_n_tiles;
+    return;
+  }
+  const int per_band = band * num_n_tiles;
+  const int m0 = t / per_band * band;
+  const int l = t - m0 * num_n_tiles;
+  const int height = min(band, num_m_tiles - m0);
+  n_tile = l / height;
+  m_tile = m0 + (l - n_tile * height);
+}
+// Bands of 4096 rows where a row of tiles has more than 16: 32 m tiles and four or five n tiles in flight, whose rows of A
+// (29 MB at k = 7168) stay in L2 while B passes once per band.  Times before -> with bands, repeated passes at the power
+// limit: 8192 x 24576 x 4096 FP8 with its quantiser 1280 -> 1056 us, 1000 x 24576 x 7168 291 -> 247, expert layer of 4096
+// tokens, 8 experts, 4096 x 14336, 2386 -> 2157, 16-bit groups 32768 x 7168 x 4096 1645 -> 1560.  Bands of 2048 rows are up
+// to 3 % slower, of 8192 rows up to 10 % (16-bit: A no longer fits); with 16 n tiles or fewer the first order already holds
+// five or more m tiles, and bands measured the same or 4 % slower (16384 x 4096 x 3072).
+inline int tile_band(int tile_rows, int num_n_tiles) { return num_n_tiles > 16 ? 4096 / tile_rows : 1; }
+
 // True in exactly one lane of a converged warp.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;

@@ -317,3 +317,27 @@ def test_grouped_gemm_over_column_windows_equals_one_launch():
     assert torch.equal(whole, halves)
     with pytest.raises(AssertionError):
         ops.grouped_gemm(a, a_s, b, b_s, tiles, mt, _C.EPI_STORE, halves, n_begin=128, n_count=256)
+
+
+@pytest.mark.parametrize("m,n", [(4096 + 133, 4360), (4096, 4352), (100, 4360), (1, 8192)])
+def test_fp8_gemm_tile_bands(m, n):
+    """More than 16 tiles of columns: the tiles are walked in bands of 32 tiles of rows, the last band may be lower."""
+    from dlblas_b200 import ops
+    g = torch.Generator().manual_seed(m + n)
+    a, a_s = O.quant_fp8(torch.randn(m, 128, generator=g).to(torch.bfloat16), 128)
+    b = torch.randn(n, 128, generator=g).to(FP8)
+    b_s = torch.rand((n + 127) // 128, 1, generator=g) + 0.5
+    c = ops.fp8_gemm(a.to(DEV), b.to(DEV), a_s.to(DEV), b_s.to(DEV), torch.bfloat16)
+    _status_ok()
+    assert O.rel_frobenius(c.cpu(), O.fp8_gemm(a, b, a_s, b_s, torch.float32)) < 4e-3   # one rounding to bf16: 2^-8
+
+
+def test_layer_tile_bands():
+    """The same over ragged experts: 18 tiles of columns in the first GEMM, more than 32 tiles of rows."""
+    from dlblas_b200.layers.moe.ep_moe import DlblasTritonFusedMoEBlockedF8Impl
+    x, logits, w13, w13s, w2, w2s = O.make_layer_inputs(600, 256, 2304, 40, seed=9)
+    w, ids = O.softmax_topk(logits, 2, True)
+    layer = DlblasTritonFusedMoEBlockedF8Impl(top_k=2, num_experts=40, out_dtype=torch.bfloat16)
+    out = layer.forward(*(t.to(DEV) for t in (x, w, ids, w13, w13s, w2, w2s)))
+    _status_ok()
+    assert O.rel_frobenius(out.cpu(), O.moe_layer(x, w, ids, w13, w13s, w2, w2s, top_k=2)) < 2e-2

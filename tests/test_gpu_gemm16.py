@@ -125,3 +125,20 @@ def test_k_grouped_gemm_sizes_that_do_not_add_up():
         ref = O.k_grouped_gemm(a, b, torch.tensor(clipped, dtype=torch.int64))
         assert O.rel_frobenius(out.cpu(), ref) < 2e-3
         assert not out[-1].any() or clipped[-1] > 0
+
+
+@pytest.mark.parametrize("tile_rows", [128, 256])
+@pytest.mark.parametrize("trans_b", [True, False])
+def test_m_grouped_gemm_tile_bands(tile_rows, trans_b, monkeypatch):
+    """More than 16 tiles of columns: bands of 4096 rows of tiles, the last one lower; groups end inside a band."""
+    monkeypatch.setenv("DLBLAS_GEMM16_TILE_ROWS", str(tile_rows))
+    from dlblas_b200 import _C
+    from dlblas_b200.kernels.grouped_gemm.BF16 import m_grouped_gemm, utils
+    g = torch.Generator(device=DEV).manual_seed(29)
+    sizes = torch.tensor([1000, 0, 3300, 17, 513], device=DEV)
+    a = torch.randn(4830, 64, generator=g, device=DEV, dtype=torch.bfloat16)
+    b = torch.randn(5, 4360, 64, generator=g, device=DEV, dtype=torch.bfloat16)
+    out = m_grouped_gemm(a, b if trans_b else b.transpose(1, 2).contiguous(), sizes, trans_b=trans_b)
+    _C.check_status()
+    ref = utils.gmm(a.float(), b.float(), sizes.cpu(), trans_b=True)
+    assert float((out.float() - ref).norm() / ref.norm()) < 3e-3
