@@ -140,12 +140,15 @@ template <int CTAS> __device__ __forceinline__ Tile16 decode16(const Args16& g, 
     const int grp = t / per_group, l = t - grp * per_group;
     const int band = l / (g.group_m_tiles * g.band), li = l - band * g.group_m_tiles * g.band;
     const int width = min(g.band, g.num_n_tiles - band * g.band);
-    const int mt = li / width;
-    m_tile = grp * g.group_m_tiles + mt;
-    n_tile = band * g.band + (li - mt * width);
-  } else {
-    tile_at(t, num_m_tiles, g.num_n_tiles, g.m_band, m_tile, n_tile);
+    m_tile = li / width;
+    n_tile = band * g.band + (li - m_tile * width);
+    ti.e = grp;
+    ti.row0 = m_tile * CTAS * BM;
+    ti.rows = min(CTAS * BM, g.m - ti.row0);
+    ti.n0 = n_tile * BN;
+    return ti;
   }
+  tile_at(t, num_m_tiles, g.num_n_tiles, g.m_band, m_tile, n_tile);
   if (g.tiles != nullptr) {
     const int4 v = __ldg(g.tiles + 1 + m_tile);
     ti.e = v.x;
@@ -567,111 +570,100 @@ int launch16(const CUtensorMap& ma, const CUtensorMap& mb, const Args16& g, int 
 // any row; its last 64-row block may run into the next group's rows, which the MMA warp clears in shared memory.  An
 // empty group gets one block with no valid row so that its tiles still run and write zeros.
 
-// One block.  Thread 0 scans the group sizes; all threads then write the tile list {group, row0, rows}.
-__global__ void k_group_plan_kernel(const long long* __restrict__ sizes, int groups, long long k_total, int m,
-                                    int tile_rows, int4* __restrict__ kseg, int4* __restrict__ tiles) {
-  if (threadIdx.x == 0) {
-    long long run = 0;
-    for (int g = 0; g < groups; ++g) {
-      long long sz = sizes[g];
-      sz = sz < 0 ? 0 : sz;
-      sz = sz > k_total - run ? k_total - run : sz;
-      const long long nkb = sz == 0 ? 1 : (sz + 63) / 64;
-      kseg[g] = make_int4((int)run, (int)nkb, (int)(sz - 64 * (nkb - 1)), 0);
-      run += sz;
-    }
-  }
-  const int m_tiles = (m + tile_rows - 1) / tile_rows;
-  if (threadIdx.x == 0) tiles[0] = make_int4(groups * m_tiles, 0, 0, 0);
-  for (int i = threadIdx.x; i < groups * m_tiles; i += blockDim.x) {
-    const int g = i / m_tiles, t = i - g * m_tiles;
-    tiles[1 + i] = make_int4(g, t * tile_rows, min(tile_rows, m - t * tile_rows), 0);
-  }
-}
-
-// Tile lists for the workers of the GEMM, built in two steps.  Tiles are handed out in tile order,
-// group by group, each to the worker that a greedy scheduler would find free first, with a tile's cost taken as its
-// K blocks (at least KG_MIN_COST, the part of a tile that does not shrink with K).  All tiles of a group cost the same,
-// so inside a group the order of the workers by the time they become free does not change: tile l of the group goes to
-// the worker of rank l mod workers, and the order is updated once per group.  Tiles that follow one another in tile
-// order (and share rows of A or B) thus start at about the same time whatever the K ranges of the groups before them;
-// handing tile t to worker t mod workers lets the workers drift apart by whole tiles once the groups differ in K, and
-// the operands were then read from DRAM 4.4 times instead of 2 (32 groups, K ranges uniform in 0 ... 10 k).
+// Plan of a launch, one small block: the groups' K ranges (kseg) and the workers' tile lists.
+//
+// Tiles are handed out in tile order, group by group, each to the worker that a greedy scheduler would find free first,
+// with a tile's cost taken as its K blocks (at least KG_MIN_COST, the part of a tile that does not shrink with K).  All
+// tiles of a group cost the same, so inside a group the order of the workers by the time they become free does not change:
+// tile l of the group goes to the worker of rank l mod workers, and the order is updated once per group.  Tiles that follow
+// one another in tile order (and share rows of A or B) thus start at about the same time whatever the K ranges of the
+// groups before them; handing tile t to worker t mod workers lets the workers drift apart by whole tiles once the groups
+// differ in K, and the operands were then read from DRAM 4.4 times instead of 2 (32 groups, K ranges uniform in 0 ... 10 k).
+//
+// Bound by latency: the groups follow one another, and each costs one search in shared memory and one block barrier.  So
+// the block holds one thread per worker and no more; the thread of a rank writes that worker's tiles itself, which needs
+// nothing from the other threads.  Plan of 32 groups, three kernels before, 35 -> 11 us (call of 40001 x 1536 x 2048
+// 274 -> 252 us).
 constexpr int KG_MIN_COST = 8;
+constexpr int KG_MAX_WORKERS = 256;
+constexpr int KG_CHUNK = 1024;   // groups whose K ranges are worked out at a time
 
-// Step 1, one small block (the loop over the groups is sequential and pays one block barrier per group, so the block is
-// no larger than the workers need): for every group the workers in the order in which they become free (who_of) and
-// how many tiles each already holds (held_before); at the end every worker's tile count.
-__global__ void __launch_bounds__(256)
-k_group_schedule_kernel(const int4* __restrict__ kseg, int groups, int tiles_per_group, int workers,
-                        int* __restrict__ who_of, int* __restrict__ held_before, int* __restrict__ sched_count) {
-  // free_at[b][r] and who[b][r] for rank r, double-buffered so that a group needs one barrier
-  __shared__ long long free_at[2][256];
-  __shared__ int who[2][256];
-  __shared__ int held_of[2][256]; // a worker changes rank from group to group: its tile count travels with it
-  __shared__ int cost_of[1024];   // the groups' tile costs, 1024 groups at a time (one global load per group would
-                                  // sit on the critical path of the loop below)
-  const int r = threadIdx.x;
+__global__ void __launch_bounds__(KG_MAX_WORKERS)
+k_group_plan_kernel(const long long* __restrict__ sizes, int groups, long long k_total, int tiles_per_group, int workers,
+                    int4* __restrict__ kseg, int* __restrict__ sched, int sched_stride, int* __restrict__ sched_count) {
+  // per rank, double-buffered so that a group needs one barrier: when the worker becomes free, which one it is, and the
+  // tiles it holds (a worker changes rank from group to group, its tile count travels with it)
+  __shared__ long long free_at[2][KG_MAX_WORKERS];
+  __shared__ int who[2][KG_MAX_WORKERS], held_of[2][KG_MAX_WORKERS];
+  __shared__ int cost_of[KG_CHUNK];
+  const int r = threadIdx.x, lane = r & 31;
   if (r < workers) {
     free_at[0][r] = 0;
     who[0][r] = r;
     held_of[0][r] = 0;
   }
-  __syncthreads();
   const int full = tiles_per_group / workers, rest = tiles_per_group - full * workers;
+  const bool front = r < rest;       // the first `rest` ranks take one tile more than the others
+  const int got = full + (front ? 1 : 0);
+  long long before = 0;              // rows of the groups before the chunk (kept by the first warp)
   int cur = 0;
   for (int g = 0; g < groups; ++g, cur ^= 1) {
-    if ((g & 1023) == 0) {
-      for (int j = threadIdx.x; j < min(1024, groups - g); j += blockDim.x)
-        cost_of[j] = max(KG_MIN_COST, __ldg(&kseg[g + j]).y);
+    if (g % KG_CHUNK == 0) {
+      __syncthreads();               // the chunk before is used up, the first order is in place
+      if (r < 32) {
+        const int n = min(KG_CHUNK, groups - g);
+        for (int j0 = 0; j0 < n; j0 += 32) {
+          const int j = j0 + lane;
+          long long own = j < n ? sizes[g + j] : 0;
+          own = own < 0 ? 0 : (own > k_total ? k_total : own);
+          long long end = own;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const long long v = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += v;
+          }
+          end += before;
+          before = __shfl_sync(0xffffffffu, end, 31);
+          // sizes that add up to more than there is are cut at the end of the operands
+          const long long first = min(end - own, k_total), rows = min(end, k_total) - first;
+          const int blocks = rows == 0 ? 1 : (int)((rows + 63) / 64);
+          if (j < n) {
+            kseg[g + j] = make_int4((int)first, blocks, (int)(rows - 64ll * (blocks - 1)), 0);
+            cost_of[j] = max(KG_MIN_COST, blocks);
+          }
+        }
+      }
       __syncthreads();
     }
-    // The first `rest` workers take one tile more than the others.  Both parts stay sorted, so the new order is a merge
-    // of the two: each worker finds its new rank with one binary search in the other part.
-    const long long cost = cost_of[g & 1023];
     if (r < workers) {
+      const long long cost = cost_of[g % KG_CHUNK];
       const int me = who[cur][r], held = held_of[cur][r];
-      who_of[(long long)g * workers + r] = me;
-      held_before[(long long)g * workers + r] = held;      // indexed by rank, like who_of
-      const int got = full + (r < rest ? 1 : 0);
       const long long mine = free_at[cur][r] + got * cost;
-      int lo, hi, new_rank;
-      if (r < rest) {   // after the workers of the other part that are free no later
-        lo = rest, hi = workers;
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          if (free_at[cur][mid] + full * cost <= mine) lo = mid + 1; else hi = mid;
-        }
-        new_rank = r + (lo - rest);
-      } else {          // after the workers of the other part that are free strictly earlier
-        lo = 0, hi = rest;
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          if (free_at[cur][mid] + (full + 1) * cost < mine) lo = mid + 1; else hi = mid;
-        }
-        new_rank = (r - rest) + lo;
+      int* list = sched + (long long)me * sched_stride + held;
+      for (int i = 0; i < got; ++i) list[i] = g * tiles_per_group + r + i * workers;
+      // Both parts stay sorted, so the new order is a merge of the two, and a worker finds its rank by counting the workers
+      // of the other part that are free before it (ties: the front part first).  Three probes at a time: the loads do not
+      // wait for one another.
+      const long long add = (front ? full : full + 1) * cost, bound = front ? mine + 1 : mine;
+      int at = front ? rest : 0, n = front ? workers - rest : rest;
+      const int base = at;
+      while (n > 0) {
+        const int step = (n + 3) >> 2;
+        const long long* p = &free_at[cur][at];
+        const long long v0 = p[step - 1], v1 = p[min(2 * step, n) - 1], v2 = p[min(3 * step, n) - 1];
+        const int c0 = v0 + add < bound, c1 = 2 * step <= n && v1 + add < bound, c2 = 3 * step <= n && v2 + add < bound;
+        const int c = c0 + c1 + c2;              // the probes rise: c0 >= c1 >= c2
+        at += c * step;
+        n = min(c < 3 ? step - 1 : n, n - c * step);
       }
-      free_at[cur ^ 1][new_rank] = mine;
-      who[cur ^ 1][new_rank] = me;
-      held_of[cur ^ 1][new_rank] = held + got;
+      const int rank = (front ? r : r - rest) + (at - base);
+      free_at[cur ^ 1][rank] = mine;
+      who[cur ^ 1][rank] = me;
+      held_of[cur ^ 1][rank] = held + got;
     }
     __syncthreads();
   }
   if (r < workers) sched_count[who[cur][r]] = held_of[cur][r];
-}
-
-// Step 2, one thread per tile: tile l of group g goes to the worker at rank l mod workers of that group's order, behind
-// the tiles the worker already holds.
-__global__ void __launch_bounds__(256)
-k_group_tile_lists_kernel(const int* __restrict__ who_of, const int* __restrict__ held_before, int groups,
-                          int tiles_per_group, int workers, int* __restrict__ sched, int sched_stride) {
-  const long long total = (long long)groups * tiles_per_group;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int g = (int)(t / tiles_per_group), l = (int)(t - (long long)g * tiles_per_group);
-    const int round = l / workers, rank = l - round * workers;
-    const long long at = (long long)g * workers + rank;
-    sched[(long long)__ldg(who_of + at) * sched_stride + __ldg(held_before + at) + round] = (int)t;
-  }
 }
 
 // Maps, arguments and launch shared by the two entry points.  The tensor maps see a as [a_map_rows, a_row_bytes] and b
@@ -680,7 +672,7 @@ static int run_gemm16(const void* a, int64_t a_map_rows, int64_t a_row_bytes, in
                       int64_t b_map_rows, int64_t b_row_bytes, int b_box_rows, int dtype, int64_t m, int64_t n, int64_t k,
                       const int4* kseg, bool b_mn, int b_group_rows, long long c_group_rows, const int32_t* tiles,
                       int max_tiles, int tile_rows, void* c, int64_t ldc, int32_t* status, void* stream,
-                      const int* sched = nullptr, const int* sched_count = nullptr, int sched_stride = 0) {
+                      int k_groups = 1, const int* sched = nullptr, const int* sched_count = nullptr, int sched_stride = 0) {
   int rc = check_device();
   if (rc != DLB_OK) return rc;
   CUtensorMap ma, mb;
@@ -704,7 +696,7 @@ static int run_gemm16(const void* a, int64_t a_map_rows, int64_t a_row_bytes, in
   g.b_mn = b_mn;
   g.c_group_rows = c_group_rows;
   const int ctas = tile_rows / BM;
-  g.num_m_tiles_static = (int)ceil_div(m, (int64_t)tile_rows);
+  g.num_m_tiles_static = k_groups * (int)ceil_div(m, (int64_t)tile_rows);
   g.num_n_tiles = (int)ceil_div(n, (int64_t)BN);
   g.idesc = make_idesc16(dtype == DLB_BF16 ? 1u : 0u, ctas);
   if (kseg != nullptr) g.idesc |= 1u << 15;            // A MN-major
@@ -774,16 +766,13 @@ extern "C" int dlb_grouped_gemm_16bit_b_kn(const void* a, const void* b, int dty
                             stream);
 }
 
-// Workspace of dlb_k_grouped_gemm_16bit, in bytes: the tile list, the K ranges and the workers' tile lists.
+// Workspace of dlb_k_grouped_gemm_16bit, in bytes: the K ranges and the workers' tile lists.
 extern "C" int64_t dlb_k_grouped_gemm_workspace_bytes(int64_t k_total, int64_t m, int64_t n, int num_groups,
                                                       int tile_rows) {
   if (k_total < 0 || m <= 0 || n <= 0 || num_groups <= 0 || (tile_rows != 128 && tile_rows != 256)) return -1;
-  const int64_t m_tiles = ceil_div(m, (int64_t)tile_rows);
-  const int64_t per_group = m_tiles * ceil_div(n, (int64_t)BN);
-  // tile lists: at most per_group / workers + 1 tiles per group and worker; sized for any worker count up to 256
-  // + per group the workers' order and their tile counts before the group (two ints per worker, up to 256 workers)
-  const int64_t sched_ints = 256 + num_groups * (per_group + 256) + 2 * (int64_t)num_groups * 256;
-  return 16 * (1 + num_groups * m_tiles) + 16 * (int64_t)num_groups + 4 * sched_ints;
+  const int64_t per_group = ceil_div(m, (int64_t)tile_rows) * ceil_div(n, (int64_t)BN);
+  // at most per_group / workers + 1 tiles per group and worker; sized for any worker count up to KG_MAX_WORKERS
+  return 16 * (int64_t)num_groups + 4 * (KG_MAX_WORKERS + num_groups * (per_group + KG_MAX_WORKERS));
 }
 
 extern "C" int dlb_k_grouped_gemm_16bit(const void* a, const void* b, int dtype, int64_t k_total, int64_t m, int64_t n,
@@ -796,8 +785,7 @@ extern "C" int dlb_k_grouped_gemm_16bit(const void* a, const void* b, int dtype,
   DLB_REQUIRE(m % 8 == 0 && n % 8 == 0, DLB_ERR_INVALID,
               "k_grouped_gemm_16bit: m=%lld and n=%lld must be multiples of 8 (16-byte rows)", (long long)m, (long long)n);
   DLB_REQUIRE(tile_rows == 128 || tile_rows == 256, DLB_ERR_INVALID, "k_grouped_gemm_16bit: tile_rows must be 128 or 256");
-  const int64_t m_tiles = ceil_div(m, (int64_t)tile_rows);
-  const int64_t per_group = m_tiles * ceil_div(n, (int64_t)BN);
+  const int64_t per_group = ceil_div(m, (int64_t)tile_rows) * ceil_div(n, (int64_t)BN);
   const int64_t all_tiles = per_group * num_groups;
   DLB_REQUIRE(k_total < (1ll << 31) - 64 && 2 * m < (1ll << 31) && 2 * n < (1ll << 31) && all_tiles < (1ll << 30),
               DLB_ERR_INVALID, "k_grouped_gemm_16bit: size too large");
@@ -814,31 +802,18 @@ extern "C" int dlb_k_grouped_gemm_16bit(const void* a, const void* b, int dtype,
               "k_grouped_gemm_16bit: workspace of %lld bytes is too small", (long long)workspace_bytes);
   int rc = check_device();
   if (rc != DLB_OK) return rc;
-  int4* tiles = reinterpret_cast<int4*>(workspace);
-  int4* kseg = tiles + 1 + num_groups * m_tiles;
+  int4* kseg = reinterpret_cast<int4*>(workspace);
   int* sched_count = reinterpret_cast<int*>(kseg + num_groups);
-  int* sched = sched_count + 256;
+  int* sched = sched_count + KG_MAX_WORKERS;
   const int max_workers = sm_count() / (tile_rows / BM);
   const int workers = (int)(all_tiles < max_workers ? all_tiles : max_workers);   // as run_gemm16 sizes its grid
-  DLB_REQUIRE(workers <= 256, DLB_ERR_INVALID, "k_grouped_gemm_16bit: more than 256 workers");
+  DLB_REQUIRE(workers <= KG_MAX_WORKERS, DLB_ERR_INVALID, "k_grouped_gemm_16bit: more than %d workers", KG_MAX_WORKERS);
   const int sched_stride = (int)(num_groups * (per_group / workers + 1));
-  cudaStream_t st = (cudaStream_t)stream;
-  k_group_plan_kernel<<<1, 256, 0, st>>>(reinterpret_cast<const long long*>(group_sizes), num_groups, k_total, (int)m,
-                                         tile_rows, kseg, tiles);
+  k_group_plan_kernel<<<1, (workers + 31) / 32 * 32, 0, (cudaStream_t)stream>>>(
+      reinterpret_cast<const long long*>(group_sizes), num_groups, k_total, (int)per_group, workers, kseg, sched,
+      sched_stride, sched_count);
   if ((rc = check_cuda(cudaGetLastError(), "k_group_plan_kernel")) != DLB_OK) return rc;
   count_launch();
-  int* who_of = sched + (long long)num_groups * (per_group + 256);
-  int* held_before = who_of + (long long)num_groups * 256;
-  const int sched_threads = (workers + 31) / 32 * 32;
-  k_group_schedule_kernel<<<1, sched_threads, 0, st>>>(kseg, num_groups, (int)per_group, workers, who_of, held_before,
-                                                       sched_count);
-  if ((rc = check_cuda(cudaGetLastError(), "k_group_schedule_kernel")) != DLB_OK) return rc;
-  count_launch();
-  k_group_tile_lists_kernel<<<(unsigned)min((long long)ceil_div(all_tiles, (int64_t)256), 1024ll), 256, 0, st>>>(
-      who_of, held_before, num_groups, (int)per_group, workers, sched, sched_stride);
-  if ((rc = check_cuda(cudaGetLastError(), "k_group_tile_lists_kernel")) != DLB_OK) return rc;
-  count_launch();
   return run_gemm16(a, k_total, 2 * m, 64, b, k_total, 2 * n, 64, dtype, m, n, 64, kseg, false, 0, m,
-                    reinterpret_cast<const int32_t*>(tiles), (int)(num_groups * m_tiles), tile_rows, c, n, status, stream,
-                    sched, sched_count, sched_stride);
+                    nullptr, 0, tile_rows, c, n, status, stream, num_groups, sched, sched_count, sched_stride);
 }

@@ -142,3 +142,21 @@ def test_m_grouped_gemm_tile_bands(tile_rows, trans_b, monkeypatch):
     _C.check_status()
     ref = utils.gmm(a.float(), b.float(), sizes.cpu(), trans_b=True)
     assert float((out.float() - ref).norm() / ref.norm()) < 3e-3
+
+
+@pytest.mark.parametrize("groups,m,n", [(1100, 8, 8), (1025, 264, 520), (40, 1536, 2048), (3, 8, 8), (2, 2560, 4096)])
+@pytest.mark.parametrize("tile_rows", [128, 256])
+def test_k_grouped_gemm_plan(groups, m, n, tile_rows, monkeypatch):
+    """Fewer tiles than workers, many more, whole numbers of tiles per worker, and more groups than the plan takes at a time."""
+    monkeypatch.setenv("DLBLAS_GEMM16_TILE_ROWS", str(tile_rows))
+    from dlblas_b200 import _C
+    from dlblas_b200.kernels.grouped_gemm.BF16 import k_grouped_gemm, utils
+    g = torch.Generator().manual_seed(groups)
+    sizes = torch.randint(0, 8 if groups > 1000 else 700, (groups,), generator=g)
+    k = int(sizes.sum())
+    a = torch.randn(k, m, generator=g).to(torch.bfloat16).to(DEV)
+    b = torch.randn(k, n, generator=g).to(torch.bfloat16).to(DEV)
+    out = k_grouped_gemm(a, b, sizes.to(DEV))
+    _C.check_status()
+    ref = utils.gmm_dw(a.float(), b.float(), sizes)
+    assert float((out.float() - ref.float()).norm() / ref.float().norm()) < 3e-3
