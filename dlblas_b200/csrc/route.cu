@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(WARPS * 32) softmax_topk_kernel(const T* __res
 // torch's fp32 sigmoid by at most one unit in the last place.
 __device__ __forceinline__ double pow2_exact(int n) { return __longlong_as_double((long long)(n + 1023) << 52); }
 
-__device__ __forceinline__ float sigmoid_exact(float x) {
+__device__ __noinline__ float sigmoid_exact(float x) {
   double z = -(double)x;
   z = fmin(fmax(z, -750.0), 750.0);
   const double n = rint(__dmul_rn(z, 1.4426950408889634));
@@ -134,6 +134,56 @@ __device__ __forceinline__ float sigmoid_exact(float x) {
   return __double2float_rn(__ddiv_rn(1.0, __dadd_rn(1.0, e)));
 }
 
+// The same bits for a third of the fp64 operations: the polynomial stops at degree 10 and uses fused operations, the
+// quotient is a reciprocal estimate with one cubic step, and both conversions are integer arithmetic.  The value is then
+// within 2^-41 of the logistic function (truncation 3.2e-13), sigmoid_exact within 2^-46; where the fp32 rounding boundary
+// is more than 2^-40 away both round alike.  False otherwise (one value in 10^4 at most), and for |x| >= 80, where exp
+// leaves the range of normal floats, and NaN.
+__device__ __forceinline__ bool sigmoid_quick(float x, float& s) {
+  const uint32_t u = __float_as_uint(x);
+  // -x; zeros and subnormals become +-2^-127 or so, which gives the same 0.5
+  const double z = __hiloint2double((int)((((u & 0x7fffffffu) >> 3) + 0x38000000u) | (~u & 0x80000000u)), (int)(u << 29));
+  const double t = __fma_rn(z, 1.4426950408889634, 6755399441055744.0);   // 1.5 * 2^52: n in the low word
+  const int n = __double2loint(t);
+  const double nd = __dsub_rn(t, 6755399441055744.0);
+  double r = __fma_rn(nd, -0.6931471803691238, z);
+  r = __fma_rn(nd, -1.9082149292705877e-10, r);
+  double p = 2.755731922398589e-07;
+  p = __fma_rn(p, r, 2.7557319223985893e-06);
+  p = __fma_rn(p, r, 2.48015873015873e-05);
+  p = __fma_rn(p, r, 0.0001984126984126984);
+  p = __fma_rn(p, r, 0.001388888888888889);
+  p = __fma_rn(p, r, 0.008333333333333333);
+  p = __fma_rn(p, r, 0.041666666666666664);
+  p = __fma_rn(p, r, 0.16666666666666666);
+  p = __fma_rn(p, r, 0.5);
+  p = __fma_rn(p, r, 1.0);
+  p = __fma_rn(p, r, 1.0);
+  const double d = __dadd_rn(1.0, __hiloint2double(__double2hiint(p) + (n << 20), __double2loint(p)));
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  double e = __fma_rn(-d, y, 1.0);
+  e = __fma_rn(e, e, e);
+  y = __fma_rn(y, e, y);
+  const uint32_t hi = (uint32_t)__double2hiint(y), lo = (uint32_t)__double2loint(y);
+  const uint32_t tail = lo & 0x1fffffffu;                                  // the bits below the float's last place
+  s = __uint_as_float((((hi - 0x38000000u) << 3) | (lo >> 29)) + (tail >> 28));
+  return fabsf(x) < 80.f && tail - (0x10000000u - 0x2000u) >= 0x4000u;     // 2^13 units of 2^-53 around the tie
+}
+
+// A lane's scores.  fp64 runs at half the rate of fp32, and 256 of the full evaluations per token were a third of the routing
+// kernel: 20000 x 256 fp32 logits with the aligned layout 53 -> 45 us.
+template <int VPT> __device__ __forceinline__ void sigmoid_row(const float (&x)[VPT], float (&s)[VPT]) {
+  uint32_t unsure = 0;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) unsure |= (sigmoid_quick(x[i], s[i]) ? 0u : 1u) << i;
+  if (unsure != 0) {
+#pragma unroll
+    for (int i = 0; i < VPT; ++i)
+      if ((unsure >> i) & 1u) s[i] = sigmoid_exact(x[i]);
+  }
+}
+
 // DeepSeek-V3 style grouped routing (dlblas/kernels/moe.py:477-521).
 template <typename T, int VPT>
 __global__ void __launch_bounds__(WARPS * 32) grouped_topk_kernel(const T* __restrict__ logits,
@@ -151,10 +201,13 @@ __global__ void __launch_bounds__(WARPS * 32) grouped_topk_kernel(const T* __res
     float x[VPT];
     load_row<T, VPT>(logits + t * experts, experts, lane, x);
 #pragma unroll
+    for (int s = 0; s < VPT; ++s)
+      if (s * 32 + lane >= experts) x[s] = 0.f;   // the filling's minus infinity would take the slow way
+    sigmoid_row<VPT>(x, sc);
+#pragma unroll
     for (int s = 0; s < VPT; ++s) {
       const int e = s * 32 + lane;
       if (e < experts) {
-        sc[s] = sigmoid_exact(x[s]);
         ch[s] = sc[s] + __ldg(bias + e);
       } else {
         sc[s] = 0.f;
@@ -249,11 +302,12 @@ __global__ void __launch_bounds__(WARPS * 32) grouped_topk_lanes_kernel(const T*
 #pragma unroll
       for (int i = 0; i < VPT; ++i) x[i] = row[i];
     }
+    float xf[VPT];
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      sc[i] = sigmoid_exact(to_f32<T>(x[i]));
-      ch[i] = sc[i] + __ldg(bias + lane * VPT + i);
-    }
+    for (int i = 0; i < VPT; ++i) xf[i] = to_f32<T>(x[i]);
+    sigmoid_row<VPT>(xf, sc);
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) ch[i] = sc[i] + __ldg(bias + lane * VPT + i);
   }
   // the two largest scores of the lane, then of its group
   float v1 = ch[0], v2 = NEG_INF;

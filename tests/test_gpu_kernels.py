@@ -437,3 +437,17 @@ def test_topk_gating_backward(golden, higher_precision):
     assert x.grad.dtype == torch.float16
     tol = 2e-2 * float(ref.abs().max()) + 1e-6
     assert float((x.grad.cpu().float() - ref).abs().max()) <= tol
+
+
+@pytest.mark.parametrize("experts", [8, 32])          # the general kernel, and the one for whole lanes
+def test_scores_are_the_oracles_bits(experts):
+    """All experts chosen, so the weights are the scores: both ways of working them out, over the whole range."""
+    from dlblas_b200 import ops
+    g = torch.Generator().manual_seed(experts)
+    x = torch.cat([torch.randn(60000, experts, generator=g) * 3, torch.randn(20000, experts, generator=g) * 40,
+                   (torch.rand(20000, experts, generator=g) * 2 - 1) * torch.logspace(-40, 2, 20000)[:, None]])
+    x[-1, :8] = torch.tensor([float("-inf"), -200.0, -80.0, -79.99999, -1e-45, -0.0, 1e-40, 79.99999])
+    x[-2, :8] = torch.tensor([float("inf"), 104.0, 80.0, 90.0, 16.64, 17.33, 1.0, -103.97])
+    w, ids = ops.route_grouped_topk(x.to(DEV), torch.zeros(experts, device=DEV), experts, False, 1, 1)
+    got = torch.empty_like(x).scatter_(1, ids.cpu().long(), w.cpu())
+    assert torch.equal(got.view(torch.int32), O.sigmoid_exact(x).view(torch.int32))
