@@ -173,16 +173,17 @@ template <int N>
 __device__ __forceinline__ void div_to_e4m3(const float (&v)[N], float scale, bool regular, uint32_t (&out)[N / 4]) {
   if (regular) {
     const float inv = __frcp_rn(scale);
-    const uint64_t y = pack_f32x2(inv, inv), ns = pack_f32x2(-scale, -scale);
+    const uint64_t ny = pack_f32x2(-inv, -inv), s = pack_f32x2(scale, scale);
 #pragma unroll
     for (int i = 0; i < N; i += 4) {
       uint32_t half[2];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const uint64_t a = pack_f32x2(v[i + 2 * h], v[i + 2 * h + 1]);
-        uint64_t q = mul_f32x2(a, y);
-        q = fma_f32x2(fma_f32x2(q, ns, a), y, q);
-        q = fma_f32x2(fma_f32x2(q, ns, a), y, q);
+        // with -v and -1 / scale: the remainder of a zero is then +0, and the correction -0 keeps the quotient's sign
+        const uint64_t na = pack_f32x2(-v[i + 2 * h], -v[i + 2 * h + 1]);
+        uint64_t q = mul_f32x2(na, ny);
+        q = fma_f32x2(fma_f32x2(q, s, na), ny, q);
+        q = fma_f32x2(fma_f32x2(q, s, na), ny, q);
         uint16_t r;
         asm("{\n\t.reg .f32 lo, hi;\n\tmov.b64 {lo, hi}, %1;\n\tcvt.rn.satfinite.e4m3x2.f32 %0, hi, lo;\n\t}"
             : "=h"(r)
