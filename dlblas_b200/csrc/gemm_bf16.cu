@@ -22,15 +22,15 @@ namespace dlb {
 namespace {
 
 constexpr int BM = 128;
-constexpr int BN = 256;
 constexpr int A_STAGE_BYTES = BM * UMMA_BK_BYTES;
 // per CTA: the whole B tile (CTAS = 1) or its half (CTAS = 2)
-template <int CTAS> struct Geo {
+template <int CTAS, int BN> struct Geo {
   static constexpr int B_STAGE_BYTES = (BN / CTAS) * UMMA_BK_BYTES;
   static constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
-  static constexpr int STAGES = CTAS == 1 ? 3 : 4;
+  static constexpr int STAGES = BN == 128 ? 5 : CTAS == 1 ? 3 : 4;
+  static constexpr int STAGING_ROW_BYTES = BN * 2 + 16;
   static constexpr int STAGING_OFF = STAGES * STAGE_BYTES;
-  static constexpr int BAR_OFF = STAGING_OFF + BM * (BN * 2 + 16);
+  static constexpr int BAR_OFF = STAGING_OFF + BM * STAGING_ROW_BYTES;
   static constexpr int NUM_BARS = 3 * STAGES + 2 * 2 + 3;
   static constexpr int MISC_OFF = BAR_OFF + NUM_BARS * 8;
   static constexpr int SMEM_BYTES = MISC_OFF + 16 + 1024;
@@ -43,7 +43,6 @@ constexpr int STORE_WARPS = 2;
 constexpr int NUM_THREADS = 384;
 constexpr int TMEM_COLS = 512;
 constexpr int TMEM_BUFS = 2;
-constexpr int STAGING_ROW_BYTES = BN * 2 + 16;
 
 struct Args16 {
   void* c;
@@ -74,9 +73,9 @@ struct Args16 {
   unsigned long long timeout_cycles;
 };
 
-// kind::f16: fp32 accumulate, A and B K-major, both of format `fmt` (0 = fp16, 1 = bf16), M = 128, N = BN
-constexpr uint32_t make_idesc16(uint32_t fmt, int ctas) {
-  return (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((ctas * BM) >> 4) << 24);
+// kind::f16: fp32 accumulate, A and B K-major, both of format `fmt` (0 = fp16, 1 = bf16), M = 128 per CTA, N = bn
+constexpr uint32_t make_idesc16(uint32_t fmt, int ctas, int bn) {
+  return (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)((ctas * BM) >> 4) << 24);
 }
 
 __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
@@ -128,7 +127,7 @@ struct Tile16 {
 };
 constexpr int KG_BAND = 4;   // default n tiles per band in the tile order of k-grouped launches
 
-template <int CTAS> __device__ __forceinline__ Tile16 decode16(const Args16& g, int num_m_tiles, int t) {
+template <int CTAS, int BN> __device__ __forceinline__ Tile16 decode16(const Args16& g, int num_m_tiles, int t) {
   Tile16 ti;
   int m_tile, n_tile;
   if (g.kseg != nullptr) {
@@ -173,14 +172,15 @@ template <> __device__ __forceinline__ uint32_t pack16<__half>(float a, float b)
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-template <typename T, int CTAS>
+template <typename T, int CTAS, int BN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const Args16 g) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  using G = Geo<CTAS>;
+  using G = Geo<CTAS, BN>;
   constexpr int STAGES = G::STAGES;
   constexpr int STAGE_BYTES = G::STAGE_BYTES;
+  constexpr int STAGING_ROW_BYTES = G::STAGING_ROW_BYTES;
   constexpr bool PAIR = CTAS == 2;
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t bar_base = smem_base + G::BAR_OFF;
@@ -254,7 +254,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     bool ok = true;
     for (int i = 0; i < my_tiles && ok; ++i) {
       const int t = nth_tile(i);
-      const Tile16 ti = decode16<CTAS>(g, num_m_tiles, t);
+      const Tile16 ti = decode16<CTAS, BN>(g, num_m_tiles, t);
       const bool mn = g.kseg != nullptr;
       const int4 ks = mn ? __ldg(g.kseg + ti.e) : make_int4(0, kblocks, 64, 0);
       for (int kb = 0; kb < ks.y; ++kb, ++it) {
@@ -328,8 +328,9 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
 #pragma unroll
             for (int c = 0; c < BN / 64; ++c) tma_load_2d(b_dst + c * 8192, &tmap_b, bx + 128 * c, by, full_bar(s));
           } else {
-            tma_load_2d(b_dst, &tmap_b, kx, b_row, full_bar(s));
-            tma_load_2d(b_dst + 128 * UMMA_BK_BYTES, &tmap_b, kx, b_row + 128, full_bar(s));
+#pragma unroll
+            for (int h = 0; h < BN / 128; ++h)
+              tma_load_2d(b_dst + h * 128 * UMMA_BK_BYTES, &tmap_b, kx, b_row + h * 128, full_bar(s));
           }
         }
         __syncwarp();
@@ -349,7 +350,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     // every use of every stage's barrier, block by block: a parity wait only tells the current phase from the one
     // before it, so a waiter that skipped uses could take an earlier phase for the one it wants.
     for (int i = 0; PAIR && mn && rank != 0 && i < my_tiles && ok; ++i) {
-      const int4 ks = __ldg(g.kseg + decode16<CTAS>(g, num_m_tiles, nth_tile(i)).e);
+      const int4 ks = __ldg(g.kseg + decode16<CTAS, BN>(g, num_m_tiles, nth_tile(i)).e);
       for (int kb = 0; kb < ks.y; ++kb, ++it) {
         const int s = it % STAGES;
         if (!mbar_wait(land_bar(s), (it / STAGES) & 1u, abort_flag, limit)) {
@@ -372,7 +373,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         break;
       }
       const uint32_t d_tmem = tmem_base + (uint32_t)(b * BN);
-      const int4 ks = mn ? __ldg(g.kseg + decode16<CTAS>(g, num_m_tiles, t).e) : make_int4(0, kblocks, 64, 0);
+      const int4 ks = mn ? __ldg(g.kseg + decode16<CTAS, BN>(g, num_m_tiles, t).e) : make_int4(0, kblocks, 64, 0);
       const int nkb = ks.y;
       for (int kb = 0; kb < nkb; ++kb, ++it) {
         const int s = it % STAGES;
@@ -434,7 +435,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     bool ok = true;
     for (int i = 0; i < my_tiles && ok; ++i, ++tile_no) {
       const int t = nth_tile(i);
-      const Tile16 ti = decode16<CTAS>(g, num_m_tiles, t);
+      const Tile16 ti = decode16<CTAS, BN>(g, num_m_tiles, t);
       if (!mbar_wait(staged_bar, tile_no & 1u, abort_flag, limit)) {
         ok = false;
         break;
@@ -461,7 +462,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     const int quad = warp & 3;
     const int r = quad * 32 + lane;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
-    uint8_t* srow = staging + r * STAGING_ROW_BYTES + wg * 128 * 2;
+    uint8_t* srow = staging + r * STAGING_ROW_BYTES + wg * BN;   // this warpgroup's half of the columns
     uint32_t tile_no = 0;
     bool ok = true;
     for (int i = 0; i < my_tiles && ok; ++i, ++tile_no) {
@@ -473,14 +474,14 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         break;
       }
       tc_fence_after();
-      const uint32_t col0 = lane_addr + (uint32_t)(b * BN + wg * 128);
+      const uint32_t col0 = lane_addr + (uint32_t)(b * BN + wg * (BN / 2));
       uint32_t s0[32], s1[32];
       tmem_ld32(col0, s0);
       tmem_ld32(col0 + 32, s1);
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
+      for (int q = 0; q < BN / 128; ++q) {
         tmem_ld_wait(s0, s1);
-        if (q == 1) {
+        if (q == BN / 128 - 1) {
           // the whole accumulator is in registers: the MMA warp may reuse it
           tc_fence_before();
           __syncwarp();
@@ -502,7 +503,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
             *reinterpret_cast<uint4*>(srow + ((2 * q + half) * 32 + j) * 2) = v;
           }
         }
-        if (q == 0) {
+        if (q + 1 < BN / 128) {
           tmem_ld32(col0 + 64, s0);
           tmem_ld32(col0 + 96, s1);
         }
@@ -527,10 +528,10 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
   }
 }
 
-template <typename T, int CTAS>
+template <typename T, int CTAS, int BN>
 int launch16(const CUtensorMap& ma, const CUtensorMap& mb, const Args16& g, int grid, cudaStream_t st) {
-  auto kern = gemm16_kernel<T, CTAS>;
-  constexpr int SMEM_BYTES = Geo<CTAS>::SMEM_BYTES;
+  auto kern = gemm16_kernel<T, CTAS, BN>;
+  constexpr int SMEM_BYTES = Geo<CTAS, BN>::SMEM_BYTES;
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -671,7 +672,7 @@ k_group_plan_kernel(const long long* __restrict__ sizes, int groups, long long k
 static int run_gemm16(const void* a, int64_t a_map_rows, int64_t a_row_bytes, int a_box_rows, const void* b,
                       int64_t b_map_rows, int64_t b_row_bytes, int b_box_rows, int dtype, int64_t m, int64_t n, int64_t k,
                       const int4* kseg, bool b_mn, int b_group_rows, long long c_group_rows, const int32_t* tiles,
-                      int max_tiles, int tile_rows, void* c, int64_t ldc, int32_t* status, void* stream,
+                      int max_tiles, int tile_rows, int bn, void* c, int64_t ldc, int32_t* status, void* stream,
                       int k_groups = 1, const int* sched = nullptr, const int* sched_count = nullptr, int sched_stride = 0) {
   int rc = check_device();
   if (rc != DLB_OK) return rc;
@@ -697,8 +698,8 @@ static int run_gemm16(const void* a, int64_t a_map_rows, int64_t a_row_bytes, in
   g.c_group_rows = c_group_rows;
   const int ctas = tile_rows / BM;
   g.num_m_tiles_static = k_groups * (int)ceil_div(m, (int64_t)tile_rows);
-  g.num_n_tiles = (int)ceil_div(n, (int64_t)BN);
-  g.idesc = make_idesc16(dtype == DLB_BF16 ? 1u : 0u, ctas);
+  g.num_n_tiles = (int)ceil_div(n, (int64_t)bn);
+  g.idesc = make_idesc16(dtype == DLB_BF16 ? 1u : 0u, ctas, bn);
   if (kseg != nullptr) g.idesc |= 1u << 15;            // A MN-major
   if (kseg != nullptr || b_mn) g.idesc |= 1u << 16;    // B MN-major
   g.status = status;
@@ -709,11 +710,15 @@ static int run_gemm16(const void* a, int64_t a_map_rows, int64_t a_row_bytes, in
   const int grid = ctas * (int)(total < workers ? total : workers);
   cudaStream_t st = (cudaStream_t)stream;
   if (ctas == 2) {
-    if (dtype == DLB_BF16) return launch16<__nv_bfloat16, 2>(ma, mb, g, grid, st);
-    return launch16<__half, 2>(ma, mb, g, grid, st);
+    if (dtype == DLB_BF16) return launch16<__nv_bfloat16, 2, 256>(ma, mb, g, grid, st);
+    return launch16<__half, 2, 256>(ma, mb, g, grid, st);
   }
-  if (dtype == DLB_BF16) return launch16<__nv_bfloat16, 1>(ma, mb, g, grid, st);
-  return launch16<__half, 1>(ma, mb, g, grid, st);
+  if (bn == 128) {
+    if (dtype == DLB_BF16) return launch16<__nv_bfloat16, 1, 128>(ma, mb, g, grid, st);
+    return launch16<__half, 1, 128>(ma, mb, g, grid, st);
+  }
+  if (dtype == DLB_BF16) return launch16<__nv_bfloat16, 1, 256>(ma, mb, g, grid, st);
+  return launch16<__half, 1, 256>(ma, mb, g, grid, st);
 }
 
 }  // namespace
@@ -745,11 +750,15 @@ static int grouped_gemm_16bit(const void* a, const void* b, bool b_kn, int dtype
   DLB_REQUIRE(((uintptr_t)a % 16 == 0) && ((uintptr_t)b % 16 == 0) && ((uintptr_t)c % 16 == 0) &&
                   ((uintptr_t)tiles % 16 == 0),
               DLB_ERR_INVALID, "grouped_gemm_16bit: a, b, c and tiles must be 16-byte aligned");
+  // Tiles of 128 columns only where those of 256 leave SMs idle: 128 rows in 3 groups, 1536 x 7168, 56.6 -> 45.1 us, 800 rows
+  // in 2 groups, 1536 x 3072, 28.7 -> 26.6.  With enough tiles they cost 7 to 30 % (A is fetched twice as often).
+  const int64_t most_tiles = tiles != nullptr ? max_tiles : ceil_div(rows, (int64_t)tile_rows);
+  const int bn = tile_rows == 128 && most_tiles * ceil_div(n, (int64_t)256) < sm_count() ? 128 : 256;
   if (b_kn)
     return run_gemm16(a, rows, 2 * k, 128, b, (int64_t)num_groups * k, 2 * n, 64, dtype, rows, n, k, nullptr, true, (int)k,
-                      0, tiles, max_tiles, tile_rows, c, ldc, status, stream);
+                      0, tiles, max_tiles, tile_rows, bn, c, ldc, status, stream);
   return run_gemm16(a, rows, 2 * k, 128, b, (int64_t)num_groups * n, 2 * k, 128, dtype, rows, n, k, nullptr, false, (int)n,
-                    0, tiles, max_tiles, tile_rows, c, ldc, status, stream);
+                    0, tiles, max_tiles, tile_rows, bn, c, ldc, status, stream);
 }
 
 extern "C" int dlb_grouped_gemm_16bit(const void* a, const void* b, int dtype, int64_t rows, int num_groups, int64_t n,
@@ -770,7 +779,7 @@ extern "C" int dlb_grouped_gemm_16bit_b_kn(const void* a, const void* b, int dty
 extern "C" int64_t dlb_k_grouped_gemm_workspace_bytes(int64_t k_total, int64_t m, int64_t n, int num_groups,
                                                       int tile_rows) {
   if (k_total < 0 || m <= 0 || n <= 0 || num_groups <= 0 || (tile_rows != 128 && tile_rows != 256)) return -1;
-  const int64_t per_group = ceil_div(m, (int64_t)tile_rows) * ceil_div(n, (int64_t)BN);
+  const int64_t per_group = ceil_div(m, (int64_t)tile_rows) * ceil_div(n, (int64_t)256);
   // at most per_group / workers + 1 tiles per group and worker; sized for any worker count up to KG_MAX_WORKERS
   return 16 * (int64_t)num_groups + 4 * (KG_MAX_WORKERS + num_groups * (per_group + KG_MAX_WORKERS));
 }
@@ -785,7 +794,7 @@ extern "C" int dlb_k_grouped_gemm_16bit(const void* a, const void* b, int dtype,
   DLB_REQUIRE(m % 8 == 0 && n % 8 == 0, DLB_ERR_INVALID,
               "k_grouped_gemm_16bit: m=%lld and n=%lld must be multiples of 8 (16-byte rows)", (long long)m, (long long)n);
   DLB_REQUIRE(tile_rows == 128 || tile_rows == 256, DLB_ERR_INVALID, "k_grouped_gemm_16bit: tile_rows must be 128 or 256");
-  const int64_t per_group = ceil_div(m, (int64_t)tile_rows) * ceil_div(n, (int64_t)BN);
+  const int64_t per_group = ceil_div(m, (int64_t)tile_rows) * ceil_div(n, (int64_t)256);
   const int64_t all_tiles = per_group * num_groups;
   DLB_REQUIRE(k_total < (1ll << 31) - 64 && 2 * m < (1ll << 31) && 2 * n < (1ll << 31) && all_tiles < (1ll << 30),
               DLB_ERR_INVALID, "k_grouped_gemm_16bit: size too large");
@@ -815,5 +824,5 @@ extern "C" int dlb_k_grouped_gemm_16bit(const void* a, const void* b, int dtype,
   if ((rc = check_cuda(cudaGetLastError(), "k_group_plan_kernel")) != DLB_OK) return rc;
   count_launch();
   return run_gemm16(a, k_total, 2 * m, 64, b, k_total, 2 * n, 64, dtype, m, n, 64, kseg, false, 0, m,
-                    nullptr, 0, tile_rows, c, n, status, stream, num_groups, sched, sched_count, sched_stride);
+                    nullptr, 0, tile_rows, 256, c, n, status, stream, num_groups, sched, sched_count, sched_stride);
 }

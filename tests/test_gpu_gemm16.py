@@ -160,3 +160,20 @@ def test_k_grouped_gemm_plan(groups, m, n, tile_rows, monkeypatch):
     _C.check_status()
     ref = utils.gmm_dw(a.float(), b.float(), sizes)
     assert float((out.float() - ref.float()).norm() / ref.float().norm()) < 3e-3
+
+
+@pytest.mark.parametrize("groups,n", [(5, 8), (5, 120), (5, 128), (5, 136), (5, 392), (73, 256), (73, 264), (147, 256), (148, 256)])
+def test_m_grouped_gemm_narrow_tiles(groups, n):
+    """Tiles of 128 columns where there are fewer tiles of 256 than SMs (148): both sides of the line, ragged columns."""
+    from dlblas_b200 import _C
+    from dlblas_b200.kernels.grouped_gemm.BF16 import m_grouped_gemm, utils
+    g = torch.Generator(device=DEV).manual_seed(31)
+    sizes = torch.tensor([1, 130, 0, 257, 128] if groups == 5 else [1] * groups, device=DEV)
+    m, k = int(sizes.sum()), 192
+    a = torch.randn(m, k, generator=g, device=DEV, dtype=torch.float16)
+    for trans_b in (True, False):
+        b = torch.randn(groups, n, k, generator=g, device=DEV, dtype=torch.float16)
+        out = m_grouped_gemm(a, b if trans_b else b.transpose(1, 2).contiguous(), sizes, trans_b=trans_b)
+        _C.check_status()
+        ref = utils.gmm(a.float(), b.float(), sizes.cpu(), trans_b=True)
+        assert float((out.float() - ref).norm() / ref.norm()) < 1e-3     # one rounding to fp16
