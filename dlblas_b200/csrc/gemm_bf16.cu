@@ -27,13 +27,17 @@ constexpr int A_STAGE_BYTES = BM * UMMA_BK_BYTES;
 template <int CTAS, int BN> struct Geo {
   static constexpr int B_STAGE_BYTES = (BN / CTAS) * UMMA_BK_BYTES;
   static constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
-  static constexpr int STAGES = BN == 128 ? 5 : CTAS == 1 ? 3 : 4;
+  static constexpr int STAGES = BN == 128 || CTAS == 2 ? 5 : 3;
   static constexpr int STAGING_ROW_BYTES = BN * 2 + 16;
   static constexpr int STAGING_OFF = STAGES * STAGE_BYTES;
-  static constexpr int BAR_OFF = STAGING_OFF + BM * STAGING_ROW_BYTES;
   static constexpr int NUM_BARS = 3 * STAGES + 2 * 2 + 3;
-  static constexpr int MISC_OFF = BAR_OFF + NUM_BARS * 8;
-  static constexpr int SMEM_BYTES = MISC_OFF + 16 + 1024;
+  // The barriers and the misc words lie in the padding of the staging rows: five stages of the pair variant then just fit.
+  // Four stages -> five: 16384 rows in 16 groups, 4096 x 3072, 372 -> 361 us; weight gradient of 40001 rows in 32 groups,
+  // 1536 x 2048, 252.5 -> 245 us.
+  static constexpr int BAR_OFF = STAGING_OFF + BN * 2;
+  static constexpr int MISC_OFF = BAR_OFF + NUM_BARS * STAGING_ROW_BYTES;
+  static constexpr int SMEM_BYTES = STAGING_OFF + BM * STAGING_ROW_BYTES + 1024;   // + slack for 1024-byte alignment
+  static_assert(SMEM_BYTES <= 227 * 1024 && NUM_BARS < BM, "shared memory of one CTA");
 };
 constexpr int DRAIN_WARPS = 8;
 constexpr int PRODUCER_WARP = 8;
@@ -183,15 +187,15 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
   constexpr int STAGING_ROW_BYTES = G::STAGING_ROW_BYTES;
   constexpr bool PAIR = CTAS == 2;
   const uint32_t smem_base = smem_u32(smem);
-  const uint32_t bar_base = smem_base + G::BAR_OFF;
-  auto full_bar = [&](int s) { return bar_base + 8u * s; };
-  auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
-  auto tfull_bar = [&](int b) { return bar_base + 8u * (2 * STAGES + b); };
-  auto tempty_bar = [&](int b) { return bar_base + 8u * (2 * STAGES + TMEM_BUFS + b); };
-  const uint32_t drain_bar = bar_base + 8u * (2 * STAGES + 2 * TMEM_BUFS);
-  const uint32_t staged_bar = drain_bar + 8u;
-  const uint32_t sfree_bar = drain_bar + 16u;
-  auto land_bar = [&](int s) { return drain_bar + 24u + 8u * s; };   // k-grouped launches: this CTA's loads of a stage
+  auto bar = [&](int i) { return smem_base + (uint32_t)(G::BAR_OFF + i * G::STAGING_ROW_BYTES); };
+  auto full_bar = [&](int s) { return bar(s); };
+  auto empty_bar = [&](int s) { return bar(STAGES + s); };
+  auto land_bar = [&](int s) { return bar(2 * STAGES + s); };   // k-grouped launches: this CTA's loads of a stage
+  auto tfull_bar = [&](int b) { return bar(3 * STAGES + b); };
+  auto tempty_bar = [&](int b) { return bar(3 * STAGES + TMEM_BUFS + b); };
+  const uint32_t drain_bar = bar(3 * STAGES + 2 * TMEM_BUFS);
+  const uint32_t staged_bar = bar(3 * STAGES + 2 * TMEM_BUFS + 1);
+  const uint32_t sfree_bar = bar(3 * STAGES + 2 * TMEM_BUFS + 2);
   uint8_t* staging = smem + G::STAGING_OFF;
   volatile uint32_t* tmem_holder = reinterpret_cast<volatile uint32_t*>(smem + G::MISC_OFF);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + G::MISC_OFF + 4);
