@@ -341,3 +341,17 @@ def test_layer_tile_bands():
     out = layer.forward(*(t.to(DEV) for t in (x, w, ids, w13, w13s, w2, w2s)))
     _status_ok()
     assert O.rel_frobenius(out.cpu(), O.moe_layer(x, w, ids, w13, w13s, w2, w2s, top_k=2)) < 2e-2
+
+
+@pytest.mark.parametrize("m,n,k", [(100, 7168, 256), (1, 64, 128), (33, 72, 384), (128, 9472, 128), (129, 4736, 128), (97, 136, 1152)])
+def test_fp8_gemm_narrow_tiles(m, n, k):
+    """Tiles of 64 columns where they make one wave (148 tiles at most), ragged columns."""
+    from dlblas_b200 import ops
+    g = torch.Generator().manual_seed(m + n)
+    a, a_s = O.quant_fp8(torch.randn(m, k, generator=g).to(torch.bfloat16), 128)
+    b = torch.randn(n, k, generator=g).to(FP8)
+    b_s = torch.rand((n + 127) // 128, k // 128, generator=g) + 0.5
+    for dtype in (torch.bfloat16, torch.float16):
+        c = ops.fp8_gemm(a.to(DEV), b.to(DEV), a_s.to(DEV), b_s.to(DEV), dtype)
+        _status_ok()
+        assert O.rel_frobenius(c.cpu(), O.fp8_gemm(a, b, a_s, b_s, torch.float32)) < 4e-3
