@@ -587,8 +587,8 @@ int launch16(const CUtensorMap& ma, const CUtensorMap& mb, const Args16& g, int 
 //
 // Bound by latency: the groups follow one another, and each costs one search in shared memory and one block barrier.  So
 // the block holds one thread per worker and no more; the thread of a rank writes that worker's tiles itself, which needs
-// nothing from the other threads.  Plan of 32 groups, three kernels before, 35 -> 11 us (call of 40001 x 1536 x 2048
-// 274 -> 252 us).
+// nothing from the other threads.  Call of 40001 x 1536 x 2048 in 32 groups,
+// with three kernels for the plan before: 274 -> 252 us.
 constexpr int KG_MIN_COST = 8;
 constexpr int KG_MAX_WORKERS = 256;
 constexpr int KG_CHUNK = 1024;   // groups whose K ranges are worked out at a time

@@ -355,3 +355,27 @@ def test_fp8_gemm_narrow_tiles(m, n, k):
         c = ops.fp8_gemm(a.to(DEV), b.to(DEV), a_s.to(DEV), b_s.to(DEV), dtype)
         _status_ok()
         assert O.rel_frobenius(c.cpu(), O.fp8_gemm(a, b, a_s, b_s, torch.float32)) < 4e-3
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("fuse", [True, False])
+def test_layer_tiles_of_few_rows(dtype, fuse):
+    """At most 32 rows per expert on average: tiles of at most 32 rows exchange the operands.  Segments around the 16-row
+    chunks, the 32-row line and whole tiles, every expert with one row, and both sides of the line of the rule."""
+    from dlblas_b200.layers.moe.kernels.blocked_fp8_fused_moe import moe_expert_forward
+    g = torch.Generator().manual_seed(41)
+    for counts in ([1, 0, 15, 16, 17, 31, 32, 33, 49, 63, 64, 65, 127, 128, 129, 192, 193, 0, 2] + [0] * 20, [1] * 160, [32, 32],
+                   [32, 33], [0, 5, 0]):
+        e, t, h, inter = len(counts), sum(counts), 384, 256
+        x, _, w13, w13s, w2, w2s = O.make_layer_inputs(t, h, inter, e, seed=e)
+        x = x.to(dtype)
+        ids = torch.repeat_interleave(torch.arange(e), torch.tensor(counts))[torch.randperm(t, generator=g)].view(t, 1)
+        w = torch.rand(t, 1, generator=g) + 0.5
+        out = moe_expert_forward(x.to(DEV), None, None, *(v.to(DEV) for v in (w13, w13s, w2, w2s, w, ids)), 1, dtype,
+                                 fuse_swiglu=fuse).cpu()
+        _status_ok()
+        ref = O.moe_layer(x, w, ids, w13, w13s, w2, w2s, top_k=1)
+        for k in range(e):
+            rows = ids[:, 0] == k
+            if bool(rows.any()):
+                assert O.rel_frobenius(out[rows], ref[rows]) < 2e-2, (e, k)
