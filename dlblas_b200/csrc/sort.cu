@@ -645,15 +645,22 @@ int sort_by_expert(const void* ids, int ids_dtype, long long n, int num_experts,
   DLB_REQUIRE(n >= 0 && n < (1ll << 31) && num_experts > 0, DLB_ERR_INVALID,
               "sort_by_expert: bad sizes num_slots=%lld num_experts=%d", n, num_experts);
   DLB_REQUIRE(ids_dtype == DLB_I32 || ids_dtype == DLB_I64, DLB_ERR_INVALID, "sort_by_expert: ids must be int32/int64");
-  if (n == 0 && o.aligned == nullptr) {
-    // no slots: every expert is empty
-    if (o.exp_start) cudaMemsetAsync(o.exp_start, 0, sizeof(long long) * num_experts, st);
-    if (o.exp_end) cudaMemsetAsync(o.exp_end, 0, sizeof(long long) * num_experts, st);
-    if (o.counts) cudaMemsetAsync(o.counts, 0, sizeof(int) * num_experts, st);
-    if (o.tiles) cudaMemsetAsync(o.tiles, 0, sizeof(int4), st);
+  if (n == 0) {
+    // no slots: every expert is empty, and so is the block-aligned layout (padding only: its filling is the number of slots)
+    auto clear = [&](void* p, size_t bytes) {
+      return p == nullptr || bytes == 0 ? DLB_OK : check_cuda(cudaMemsetAsync(p, 0, bytes, st), "cudaMemsetAsync(sort_by_expert)");
+    };
+    const struct { void* p; size_t bytes; } outputs[] = {
+        {o.exp_start, sizeof(long long) * num_experts}, {o.exp_end, sizeof(long long) * num_experts},
+        {o.counts, sizeof(int) * num_experts}, {o.tiles, sizeof(int4)}, {o.aligned, sizeof(int) * o.aligned_len},
+        {o.block_expert, sizeof(int) * o.num_blocks}, {o.padded_total, sizeof(int)}};
+    for (const auto& out : outputs) {
+      const int rc = clear(out.p, out.bytes);
+      if (rc != DLB_OK) return rc;
+    }
     return DLB_OK;
   }
-  DLB_REQUIRE(ids != nullptr || n == 0, DLB_ERR_INVALID, "sort_by_expert: null ids");
+  DLB_REQUIRE(ids != nullptr, DLB_ERR_INVALID, "sort_by_expert: null ids");
   if (ids_dtype == DLB_I32) return run_sort<int>(reinterpret_cast<const int*>(ids), n, num_experts, o, ws, ws_bytes, st);
   return run_sort<long long>(reinterpret_cast<const long long*>(ids), n, num_experts, o, ws, ws_bytes, st);
 }
@@ -830,7 +837,8 @@ extern "C" int dlb_moe_align_block_size(void* ids, int ids_dtype, int64_t num_sl
   DLB_REQUIRE(num_slots >= 0 && num_experts > 0 && sorted_len >= num_slots + (int64_t)num_experts * (block_size - 1) &&
                   sorted_len < (1ll << 31) && (int64_t)num_blocks * block_size >= sorted_len,
               DLB_ERR_INVALID, "moe_align_block_size: outputs too small");
-  DLB_REQUIRE(sorted_ids && expert_ids && num_padded, DLB_ERR_INVALID, "moe_align_block_size: null pointer");
+  DLB_REQUIRE((sorted_ids || sorted_len == 0) && (expert_ids || num_blocks == 0) && num_padded, DLB_ERR_INVALID,
+              "moe_align_block_size: null pointer");
   SortOut o = {};
   o.tile_rows = block_size;
   o.num_local = num_experts;

@@ -1,0 +1,47 @@
+"""Calls at the far ends of what the entry points take: no slots or tokens, rows without a finite score, 16-bit routing
+weights, expert counts at the edge of the default shared-memory limit, shapes that do not fit together."""
+import subprocess
+import sys
+
+import pytest
+import torch
+
+from oracle import moe_oracle as O
+
+DEV = "cuda"
+
+
+def _child(code):
+    """A process of its own: for calls that would end it, and for limits that an earlier call would have raised."""
+    return subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+
+
+# ---- no slots ----------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("block", [1, 16])
+def test_align_without_slots_reaches_the_launch(block):
+    """Without a device the call ends in a CUDA error; it must not end the process before that."""
+    r = _child(f"""
+from dlblas_b200 import _C
+import ctypes
+out = (ctypes.c_int32 * 64)()
+p = ctypes.addressof(out)
+n = 4 * ({block} - 1)
+rc = _C.lib().dlb_moe_align_block_size(p, _C.DLB_I32, 0, 4, 4, {block}, p if n else None, n, p if n else None,
+                                       -(-n // {block}), p, None, 0, None) if not __import__('torch').cuda.is_available() else 0
+print('rc', rc)
+""")
+    assert r.returncode == 0 and "rc" in r.stdout, (r.returncode, r.stderr[-500:])
+    assert "rc -1" not in r.stdout                                             # nor be refused
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("experts,block", [(3, 1), (3, 16), (256, 64), (9000, 2)])
+@pytest.mark.parametrize("pad", [False, True])
+def test_align_without_slots(experts, block, pad):
+    from dlblas_b200.kernels.moe_align_block_size import moe_align_block_size
+    ids = torch.empty(0, 2, dtype=torch.int64, device=DEV)
+    slots, owner, total = moe_align_block_size(ids, block, experts, experts, None, pad)
+    n = experts * (block - 1)
+    n = -(-n // block) * block if pad else n
+    assert slots.shape == (n,) and owner.shape == (-(-n // block),)
+    assert not slots.any() and not owner.any() and total.tolist() == [0]      # the filling is the number of slots
