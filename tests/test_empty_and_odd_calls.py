@@ -45,3 +45,16 @@ def test_align_without_slots(experts, block, pad):
     n = -(-n // block) * block if pad else n
     assert slots.shape == (n,) and owner.shape == (-(-n // block),)
     assert not slots.any() and not owner.any() and total.tolist() == [0]      # the filling is the number of slots
+
+
+# ---- one-rank decode layer ---------------------------------------------------------------------------------------
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float64])
+def test_decode_takes_weights_of_any_type(dtype):
+    from dlblas_b200.layers.moe.ep_moe import FusedMoELowLatency
+    x, logits, w13, w13s, w2, w2s = (t.to(DEV) for t in O.make_layer_inputs(24, 256, 256, 8, seed=5))
+    w, ids = O.softmax_topk(logits.cpu(), 2, True)
+    layer = FusedMoELowLatency(1, None, 8, 256, 0)
+    w = w.to(DEV).to(dtype)
+    out = layer.forward(x, w, ids.to(DEV), w13, w13s, w2, w2s)
+    assert torch.equal(out, layer.forward(x, w.float(), ids.to(DEV), w13, w13s, w2, w2s))

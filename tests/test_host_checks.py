@@ -78,7 +78,7 @@ def test_refused_on_the_device(monkeypatch):
     for host_side in ({"w": w.cpu()}, {"ids": ids.cpu()}):
         with pytest.raises(RuntimeError, match="CUDA"):
             layer(**host_side)
-    with pytest.raises(AssertionError):                          # the exchange takes fp32 weights only
+    with pytest.raises(AssertionError):                          # the layer has converted the weights by then
         step(x, w.half(), ids, w13, s13, w2, s2, torch.bfloat16)
     b = torch.zeros(1, 64, 64, dtype=torch.bfloat16, device=DEV)
     size = torch.tensor([8], device=DEV)
