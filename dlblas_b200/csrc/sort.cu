@@ -28,6 +28,8 @@ constexpr int CHUNK_ITEMS = 2;               // ids per lane and pass of the chu
 constexpr int CHUNK_STEP = MAX_WARPS * 32 * CHUNK_ITEMS;   // 2048
 constexpr int DIRECT_CHUNKS = 160;
 constexpr int SMEM_LIMIT = 220 * 1024;
+// Without cudaFuncSetAttribute a block has 48 KB, and its static arrays (warp_sums, stats_s: 272 bytes) count towards them.
+constexpr int SMEM_DEFAULT = 48 * 1024 - 512;
 
 // Largest id and numbers of ids equal to -1 and below 0 seen by one thread (SortOut::stats).
 struct IdStats {
@@ -451,7 +453,7 @@ int allow_smem(const void* kernel, bool (&configured)[64], const char* what) {
 
 template <typename IdT, int ITEMS>
 int launch_one_block(const IdT* ids, long long n, int num_experts, const SortOut& o, const Plan& p, cudaStream_t st) {
-  if (p.smem > 48 * 1024) {
+  if (p.smem > (size_t)SMEM_DEFAULT) {
     static bool configured[64] = {};
     int rc = allow_smem(reinterpret_cast<const void*>(sort_one_block_kernel<IdT, ITEMS>), configured,
                         "cudaFuncSetAttribute(sort_one_block_kernel)");
@@ -503,7 +505,7 @@ int run_sort(const IdT* ids, long long n, int num_experts, const SortOut& o, voi
     count_launch();
     DLB_CHECK_LAUNCH("sort_scan_chunks_kernel");
   }
-  if (p.smem > 48 * 1024) {
+  if (p.smem > (size_t)SMEM_DEFAULT) {
     static bool configured[64] = {};
     int rc = allow_smem(reinterpret_cast<const void*>(sort_scatter_kernel<IdT>), configured,
                         "cudaFuncSetAttribute(sort_scatter_kernel)");
