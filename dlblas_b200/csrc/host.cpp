@@ -838,6 +838,7 @@ PermutePlan permute_plan(const Tensor& indices, int64_t dest_limit, bool want_so
   if (want_sorted) p.sorted_idx = empty({slots}, at::kLong, c);
   p.dest = empty({slots}, at::kInt, c);
   p.row_map = empty({slots}, at::kInt, c);
+  if (t == 0) return p;      // nothing to place
   // one event and twelve bytes per thread and device: both are used up before this function returns
   thread_local at::cuda::CUDAEvent events[16];
   thread_local Tensor stats_mem[16];

@@ -47,6 +47,16 @@ def test_align_without_slots(experts, block, pad):
     assert not slots.any() and not owner.any() and total.tolist() == [0]      # the filling is the number of slots
 
 
+@pytest.mark.gpu
+def test_permute_plan_without_tokens():
+    from dlblas_b200.kernels.permute.moe_triton_kernels import moe_permute_topk_op_triton
+    x = torch.empty(0, 64, dtype=torch.bfloat16, device=DEV)
+    rmap = torch.empty(0, dtype=torch.int32, device=DEV)
+    for ids in (torch.empty(0, 2, dtype=t, device=DEV) for t in (torch.int32, torch.int64)):
+        out, got, order, _ = moe_permute_topk_op_triton(x, ids, 0, [], 0, 0, torch.empty_like(x), rmap)
+        assert out.shape == (0, 64) and got.shape == (0,) and order.shape == (0,) and order.dtype == torch.int64
+
+
 # ---- one-rank decode layer ---------------------------------------------------------------------------------------
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float64])
