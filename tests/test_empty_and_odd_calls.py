@@ -70,6 +70,61 @@ def test_decode_takes_weights_of_any_type(dtype):
     assert torch.equal(out, layer.forward(x, w.float(), ids.to(DEV), w13, w13s, w2, w2s))
 
 
+def _decode_layer(dispatcher_class, layer_class=None):
+    """A one-rank layer without its device buffers."""
+    from dlblas_b200.layers.moe.ep_moe import FusedMoELowLatency
+    layer_class = layer_class or FusedMoELowLatency
+    d = dispatcher_class.__new__(dispatcher_class)
+    d.world_size, d.num_max_dispatch_tokens_per_rank, d.max_top_k, d.handle = 1, 128, 8, None
+    layer = layer_class.__new__(layer_class)
+    layer.num_experts, layer.layer_index, layer.out_dtype, layer.token_dispatcher = 4, 0, torch.bfloat16, d
+    return layer
+
+
+def test_decode_calls_replaced_steps(monkeypatch):
+    from dlblas_b200.layers.moe.ep_moe import FusedMoELowLatency
+    from dlblas_b200.layers.moe.token_dispatcher import TokenDispatcherLowLatencyP2P as P2P
+    called = []
+    x, w, ids = torch.zeros(2, 128), torch.ones(2, 2), torch.zeros(2, 2, dtype=torch.int64)
+    steps = {n: (lambda *a, n=n, r=r, **k: called.append(n) or r)
+             for n, r in (("dispatch", (None,) * 5), ("experts", None), ("combine", x))}
+    layer = _decode_layer(type("Exchange", (P2P,), {n: steps[n] for n in ("dispatch", "combine")}),
+                          type("Layer", (FusedMoELowLatency,), {"experts": steps["experts"]}))
+    layer.forward(x, w, ids, torch.zeros(4, 256, 128), None, None, None)
+    assert called == ["dispatch", "experts", "combine"]
+
+
+@pytest.mark.parametrize("name", ["experts", "dispatch", "dispatch_async", "combine", "combine_async"])
+@pytest.mark.parametrize("where", ["object", "class", "subclass"])
+def test_decode_is_direct_with_its_own_steps_only(name, where, monkeypatch):
+    from dlblas_b200.layers.moe.ep_moe import FusedMoELowLatency
+    from dlblas_b200.layers.moe.token_dispatcher import TokenDispatcherLowLatencyP2P as P2P
+    assert _decode_layer(P2P)._direct()
+    hook = lambda *a, **k: None  # noqa: E731
+    if where == "subclass":
+        kinds = (P2P, type("L", (FusedMoELowLatency,), {name: hook})) if name == "experts" else (type("D", (P2P,), {name: hook}),)
+        layer = _decode_layer(*kinds)
+    else:
+        layer = _decode_layer(P2P)
+        owner = layer if name == "experts" else layer.token_dispatcher
+        monkeypatch.setattr(owner if where == "object" else type(owner), name, hook, raising=False)
+    assert not layer._direct()
+
+
+@pytest.mark.gpu
+def test_decode_direct_and_step_by_step_agree():
+    """Ids of no expert among them; a method on the object sends the call through the three steps."""
+    from dlblas_b200.layers.moe.ep_moe import FusedMoELowLatency
+    x, logits, w13, w13s, w2, w2s = (t.to(DEV) for t in O.make_layer_inputs(100, 384, 256, 16, seed=6))
+    w, ids = (t.to(DEV) for t in O.softmax_topk(logits.cpu(), 4, True))
+    ids[::7, 1] = -1
+    ids[5] = -1
+    layer = FusedMoELowLatency(1, None, 16, 384, 0)
+    out = layer.forward(x, w, ids, w13, w13s, w2, w2s)
+    layer.token_dispatcher.dispatch = layer.token_dispatcher.dispatch
+    assert torch.equal(out, layer.forward(x, w, ids, w13, w13s, w2, w2s)) and layer.token_dispatcher.handle is not None
+
+
 # ---- expert counts whose histograms just fill the default shared memory -------------------------------------------
 @pytest.mark.gpu
 def test_sort_at_the_default_shared_memory_limit():
