@@ -492,7 +492,9 @@ __device__ void gating_expert_part(const int* __restrict__ ids_km, const int* __
 }
 
 // part 3: drop entries beyond the capacity, renormalise the kept gates, emit the indices
-// (topk_gating_fwd_part3.py:9-61) and the kept part of expert_select_token_idx.
+// (topk_gating_fwd_part3.py:9-61) and the kept part of expert_select_token_idx.  An entry without an expert is dropped
+// as well: a row whose gates are all NaN (a NaN logit, or every exp of it 0) has none, the sort gives it rank -1.
+__device__ __forceinline__ bool gating_kept(int rank, long long capacity) { return rank >= 0 && rank < capacity; }
 constexpr int GATING_SLOTS = 8;   // slots of a token whose loads are in flight together
 template <typename T>
 __global__ void __launch_bounds__(64) gating_part3_kernel(const int* __restrict__ ids_km,
@@ -526,7 +528,7 @@ __global__ void __launch_bounds__(64) gating_part3_kernel(const int* __restrict_
     fetch(j0);
 #pragma unroll
     for (int j = 0; j < GATING_SLOTS; ++j)
-      if (loc[j] < capacity) denom += gate[j];
+      if (gating_kept(loc[j], capacity)) denom += gate[j];
   }
   const float eps = sizeof(T) == 2 ? 9.765625e-4f : 1.1920929e-7f;   // torch.finfo(dtype).eps
   denom = denom < eps ? eps : denom;
@@ -539,7 +541,7 @@ __global__ void __launch_bounds__(64) gating_part3_kernel(const int* __restrict_
     for (int j = 0; j < GATING_SLOTS; ++j) {
       if (j0 + j >= top_k) break;
       const long long f = (long long)(j0 + j) * tokens + t;
-      const bool kept = loc[j] < capacity;
+      const bool kept = gating_kept(loc[j], capacity);
       out_w[f] = from_f32<T>(kept ? gate[j] / denom : 0.f);
       ec_idx[f] = kept ? (int)((long long)id[j] * capacity + loc[j]) : 0;
       if (kept) select[(long long)id[j] * capacity + loc[j]] = t;
@@ -696,7 +698,7 @@ __global__ void __launch_bounds__(WARPS * 32) gating_bwd_kernel(const float* __r
     bool kept = false;
     auto fetch = [&](int j0) {
       const long long f = (long long)(j0 + lane) * tokens + t;
-      kept = j0 + lane < top_k && __ldg(rank + f) < capacity;
+      kept = j0 + lane < top_k && gating_kept(__ldg(rank + f), capacity);
       id = kept ? __ldg(ids_km + f) : -1;
       gate = kept ? __ldg(gate_km + f) : 0.f;
       gw = kept ? to_f32<T>(grad_w[f]) : 0.f;

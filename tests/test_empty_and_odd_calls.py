@@ -143,3 +143,31 @@ for n, experts in ((1024, 640), (2048, 641), (4096, 642), (4097, 609)):
 print("done")
 """)
     assert r.returncode == 0 and "done" in r.stdout, r.stderr[-800:]
+
+
+# ---- gating rows without a finite gate ----------------------------------------------------------------------------
+@pytest.mark.gpu
+@pytest.mark.parametrize("experts", [32, 40])             # whole lanes, and lanes with filling
+@pytest.mark.parametrize("bad", [-200.0, float("nan")])   # every exp is 0, so 0 / 0; or a NaN to begin with
+def test_gating_drops_rows_without_a_gate(experts, bad):
+    import dlblas_b200
+    good, top_k, capacity = 64, 2, 6                      # the capacity is the least one, whatever the number of tokens
+    x = torch.randn(good, experts, generator=torch.Generator().manual_seed(experts))
+    rows = torch.arange(good + 2)
+    keep = (rows != 3) & (rows != good + 1)
+    full = torch.full((good + 2, experts), bad)
+    full[keep] = x
+    logits = full.to(DEV).requires_grad_(True)
+    l_aux, ec_idx, weights, select = dlblas_b200.topk_gating(logits, top_k, 1.0, capacity, True)
+    _, want_idx, want_w, _ = O.topk_gating(x, top_k, 1.0, capacity)
+    idx, w = ec_idx.cpu().view(top_k, -1), weights.detach().cpu().view(top_k, -1)
+    assert torch.equal(idx[:, keep], want_idx.view(top_k, -1))
+    torch.testing.assert_close(w[:, keep], want_w.view(top_k, -1), rtol=1e-5, atol=1e-6)
+    assert not idx[:, ~keep].any() and not w[:, ~keep].any()
+    place, live = idx[:, keep].flatten().long(), w[:, keep].flatten() > 0
+    assert torch.equal(select.cpu()[place[live]], rows[keep].repeat(top_k)[live])
+    assert int(select.min()) >= 0 and int(select.max()) < good + 2
+    grad = torch.rand(top_k, good + 2, generator=torch.Generator().manual_seed(1))
+    weights.backward(grad.flatten().to(DEV))
+    ref = O.topk_gating_grad(x, top_k, 1.0, capacity, 0.0, grad[:, keep])
+    torch.testing.assert_close(logits.grad.cpu()[keep], ref, rtol=1e-4, atol=1e-6)
