@@ -256,7 +256,12 @@ std::pair<Tensor, Tensor> quant_fp8(const Tensor& x, int64_t group, int mode, do
   require(x.dim() == 2 && x.stride(1) == 1, "x must be 2-D with contiguous rows");
   const int64_t m = x.size(0), k = x.size(1), rows = rows_out < 0 ? m : rows_out;
   require(group > 0, "group_size must be positive");
-  if (dst_pos) require_cuda(*dst_pos);
+  if (dst_pos) {
+    require_cuda(*dst_pos);
+    require(fanout > 0 && dst_pos->numel() >= m * fanout, "dst_pos must have `fanout` entries per row");
+  } else {
+    require(rows >= m, "fewer rows wanted than there are");
+  }
   if (k % group != 0)
     throw AssertionFailed("the last dimension of 'x' " + std::to_string(k) + " must be divisible by 'group_size' " +
                           std::to_string(group));
@@ -747,6 +752,7 @@ Tensor gating_backward(const Tensor& ws, at::ScalarType dt, int64_t tokens, int6
   };
   const Tensor gl = grad_l_aux.defined() ? ready(grad_l_aux) : at::zeros({}, ws.options().dtype(dt));
   const Tensor gw = grad_weights.defined() ? ready(grad_weights) : Tensor();
+  require(gl.numel() >= 1 && (!gw.defined() || gw.numel() >= tokens * k), "gradients smaller than the outputs they belong to");
   Tensor out = empty({tokens, experts}, dt, c);
   check(abi.dlb_topk_gating_bwd(ws.data_ptr(), ws.numel(), code(dt), tokens, (int)experts, (int)k, capacity, gl.data_ptr(),
                                 gw.defined() ? gw.data_ptr() : nullptr, out.data_ptr(), c.stream));
@@ -893,6 +899,8 @@ PyObject* py_permute_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
 Tensor unpermute_rows(const Tensor& x_in, const Tensor& row_map_in, const Tensor& probs_in, int64_t tokens, int64_t k) {
   require_cuda({&x_in, &row_map_in});
   if (probs_in.defined()) require_cuda(probs_in);
+  require(row_map_in.numel() >= tokens * k, "the row map must have an entry for every token and slot");
+  require(!probs_in.defined() || probs_in.numel() >= tokens * k, "one probability per token and slot");
   Call c(x_in);
   const Tensor x = x_in.is_contiguous() ? x_in : x_in.contiguous();
   const Tensor row_map = row_map_in.is_contiguous() ? row_map_in : row_map_in.contiguous();
@@ -922,6 +930,9 @@ std::pair<Tensor, Tensor> unpermute_backward(const Tensor& grad_in, const Tensor
   require_cuda({&grad_in, &fwd_in, &row_map_in, &probs_in});
   Call c(grad_in);
   require(grad_in.scalar_type() == fwd_in.scalar_type(), "gradient and rows must have one type");
+  require(probs_in.dim() == 2 && grad_in.dim() == 2 && fwd_in.dim() == 2, "gradient, rows and probabilities must be 2-D");
+  require(grad_in.size(0) >= probs_in.size(0) && grad_in.size(1) == fwd_in.size(1), "gradient and rows do not fit together");
+  require(row_map_in.numel() >= probs_in.numel(), "the row map must have an entry for every token and slot");
   const int64_t t = probs_in.size(0), k = probs_in.size(1), h = grad_in.size(1), rows = fwd_in.size(0);
   const Tensor grad = grad_in.is_contiguous() ? grad_in : grad_in.contiguous();
   const Tensor fwd = fwd_in.is_contiguous() ? fwd_in : fwd_in.contiguous();

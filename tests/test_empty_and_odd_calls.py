@@ -171,3 +171,40 @@ def test_gating_drops_rows_without_a_gate(experts, bad):
     weights.backward(grad.flatten().to(DEV))
     ref = O.topk_gating_grad(x, top_k, 1.0, capacity, 0.0, grad[:, keep])
     torch.testing.assert_close(logits.grad.cpu()[keep], ref, rtol=1e-4, atol=1e-6)
+
+
+# ---- shapes that do not fit together: the kernels would read or write past the smaller tensor -----------------------
+@pytest.mark.gpu
+def test_shapes_that_do_not_fit_are_refused():
+    from dlblas_b200 import ops
+    from dlblas_b200.kernels.permute.moe_triton_kernels import (moe_recover_topk_bwd_op_triton, moe_recover_topk_op_triton,
+                                                                unpermute)
+    rows = torch.zeros(12, 64, dtype=torch.bfloat16, device=DEV)
+    rmap = torch.arange(12, dtype=torch.int32, device=DEV)
+    probs, grad = torch.ones(6, 2, device=DEV), torch.zeros(6, 64, dtype=torch.bfloat16, device=DEV)
+    unpermute(rows, rmap, probs)
+    moe_recover_topk_bwd_op_triton(grad, rows, rmap, probs)
+    for bad in (torch.ones(7, 2, device=DEV), torch.ones(6, 3, device=DEV)):
+        with pytest.raises(AssertionError):
+            unpermute(rows, rmap, bad)
+        with pytest.raises(AssertionError):
+            moe_recover_topk_bwd_op_triton(grad, rows, rmap, bad)
+    with pytest.raises(AssertionError):
+        moe_recover_topk_op_triton(rows, rmap, probs[:5], 6, 2)
+    with pytest.raises(AssertionError):
+        moe_recover_topk_op_triton(rows, rmap[:11], None, 6, 2)
+    for bad in (grad[:5], grad[:, :32], torch.zeros(6, 128, dtype=torch.bfloat16, device=DEV)):
+        with pytest.raises(AssertionError):
+            moe_recover_topk_bwd_op_triton(bad, rows, rmap, probs)
+    x = torch.zeros(4, 128, dtype=torch.bfloat16, device=DEV)
+    pos = torch.arange(8, dtype=torch.int32, device=DEV)
+    ops.quant_fp8(x, 128, dst_pos=pos, fanout=2, rows_out=8)
+    with pytest.raises(AssertionError):
+        ops.quant_fp8(x, 128, dst_pos=pos[:7], fanout=2, rows_out=8)
+    with pytest.raises(AssertionError):
+        ops.quant_fp8(x, 128, rows_out=3)
+    _, _, _, _, ws = ops.topk_gating(torch.zeros(6, 8, device=DEV), 2, 3, return_workspace=True)
+    one = torch.ones((), device=DEV)
+    ops.topk_gating_bwd(ws, torch.float32, 6, 8, 2, 3, one, torch.ones(12, device=DEV))
+    with pytest.raises(AssertionError):
+        ops.topk_gating_bwd(ws, torch.float32, 6, 8, 2, 3, one, torch.ones(11, device=DEV))
