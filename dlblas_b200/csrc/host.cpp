@@ -410,7 +410,8 @@ Tensor moe_forward(const MoeArgs& g) {
   const Tensor ids = g.ids.is_contiguous() ? g.ids : g.ids.contiguous();
   Tensor weights = g.weights;
   bool renormalize = g.renormalize;
-  if (weights.scalar_type() != at::kFloat) {
+  if (weights.scalar_type() != at::kFloat || !weights.is_contiguous()) {
+    // in the weights' own type, and in the order that torch adds such a layout up
     if (renormalize) weights = weights / weights.sum(-1, true);
     renormalize = false;
     weights = weights.to(at::kFloat);

@@ -191,6 +191,23 @@ __device__ __forceinline__ void scan_and_write_segments(const int* total, int* b
   }
 }
 
+// Sum of a token's weights.  The expert-parallel path divides by torch's sum over the last dimension; the result here has the
+// same bits: the upper half of the slots is added to the lower one until one is left (slots that do not exist count as zero).
+__device__ __forceinline__ float slot_weight_sum(const float* __restrict__ w, int top_k) {
+  auto at = [&](int j) { return j < top_k ? __ldg(w + j) : 0.f; };
+  float v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = at(i);
+  if (top_k > 8) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = (v[i] + at(i + 16)) + (at(i + 8) + at(i + 24));
+    for (int j0 = 32; j0 < top_k; j0 += 8)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] += at(j0 + i);
+  }
+  return ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7]));
+}
+
 // Output of slot f, which is at place `pos` of the sorted order.
 template <typename IdT>
 __device__ __forceinline__ void write_slot(unsigned f, unsigned n, int bucket, int pos, const int* base,
@@ -212,10 +229,7 @@ __device__ __forceinline__ void write_slot(unsigned f, unsigned n, int bucket, i
     o.row_map[j * (n / (unsigned)o.top_k) + t] = out;
   }
   if (o.w_out) {
-    // weights of a token divided by their sum (added up in slot order)
-    const float* w = o.w_in + f / (unsigned)o.top_k * (unsigned)o.top_k;
-    float sum = 0.f;
-    for (int j = 0; j < o.top_k; ++j) sum += __ldg(w + j);
+    const float sum = slot_weight_sum(o.w_in + f / (unsigned)o.top_k * (unsigned)o.top_k, o.top_k);
     o.w_out[f] = __ldg(o.w_in + f) / sum;
   }
 }

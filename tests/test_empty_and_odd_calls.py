@@ -208,3 +208,35 @@ def test_shapes_that_do_not_fit_are_refused():
     ops.topk_gating_bwd(ws, torch.float32, 6, 8, 2, 3, one, torch.ones(12, device=DEV))
     with pytest.raises(AssertionError):
         ops.topk_gating_bwd(ws, torch.float32, 6, 8, 2, 3, one, torch.ones(11, device=DEV))
+
+
+# ---- routing weights divided by their sum -------------------------------------------------------------------------
+@pytest.mark.gpu
+@pytest.mark.parametrize("top_k", [1, 2, 3, 4, 5, 6, 7, 8, 9, 12, 15, 16, 17, 24, 31, 32])
+@pytest.mark.parametrize("tokens", [1, 37, 3000])          # one block, one block with several ids per lane, chunks
+def test_plan_normalises_as_torch_does(tokens, top_k):
+    """Bit for bit: the expert-parallel path divides by torch's sum."""
+    from dlblas_b200 import _C
+    g = torch.Generator().manual_seed(tokens + top_k)
+    ids = torch.randint(0, 40, (tokens, top_k), generator=g).to(DEV)
+    w = torch.rand(tokens, top_k, generator=g).to(DEV)
+    lib, slots = _C.lib(), tokens * top_k
+    got, pos = torch.empty_like(w), torch.empty(slots, dtype=torch.int32, device=DEV)
+    max_tiles = slots // 128 + 40
+    tiles = torch.empty((max_tiles + 1) * 4, dtype=torch.int32, device=DEV)
+    ws = torch.empty(max(lib.dlb_sort_by_expert_workspace_size(slots, 40), 1), dtype=torch.uint8, device=DEV)
+    _C.check(lib.dlb_moe_plan(_C.ptr(ids), _C.DLB_I64, tokens, top_k, 40, 0, 40, 128, None, _C.ptr(pos), _C.ptr(tiles),
+                              max_tiles, _C.ptr(w), _C.ptr(got), _C.ptr(ws), ws.numel(), _C.stream()))
+    assert torch.equal(got, w / w.sum(-1, keepdim=True))
+
+
+@pytest.mark.gpu
+def test_layer_normalises_weights_of_any_layout():
+    from dlblas_b200.layers.moe.ep_moe import DlblasTritonFusedMoEBlockedF8Impl
+    x, logits, *weights = (t.to(DEV) for t in O.make_layer_inputs(50, 256, 256, 16, seed=8))
+    w, ids = (t.to(DEV) for t in O.softmax_topk(logits.cpu(), 6, False))
+    layer, plain = (DlblasTritonFusedMoEBlockedF8Impl(top_k=6, num_experts=16, renormalize=r, out_dtype=torch.bfloat16)
+                    for r in (True, False))
+    for given in (w, w.t().contiguous().t(), w.half(), w.half().t().contiguous().t()):
+        want = plain.forward(x, given / given.sum(-1, keepdim=True), ids, *weights)
+        assert torch.equal(layer.forward(x, given, ids, *weights), want)
