@@ -6,6 +6,7 @@ The shared library is built in-tree by ``python -m dlblas_b200.build`` (or
 """
 import ctypes
 import os
+import sys
 import threading
 
 import torch
@@ -119,6 +120,17 @@ def lib():
 
 
 _host_module = None
+HOST_PATH = os.path.join(_HERE, "_host.so")
+
+
+def host_tag() -> str:
+    """What _host.so is compiled for: it uses torch's C++ interface, which changes from one version to the next."""
+    return f"dlblas_b200 host for torch {torch.__version__}, Python {sys.version_info[0]}.{sys.version_info[1]};"
+
+
+def host_is_current(path: str = HOST_PATH) -> bool:
+    with open(path, "rb") as fh:
+        return host_tag().encode() in fh.read()
 
 
 def host():
@@ -128,11 +140,13 @@ def host():
         handle = lib()
         with _lock:
             if _host_module is None:
-                path = os.path.join(_HERE, "_host.so")
-                if not os.path.exists(path):
-                    raise RuntimeError(f"dlblas_b200: {path} is missing; build it with `python -m dlblas_b200.build`")
+                if not os.path.exists(HOST_PATH):
+                    raise RuntimeError(f"dlblas_b200: {HOST_PATH} is missing; build it with `python -m dlblas_b200.build`")
+                if not host_is_current():
+                    raise RuntimeError(f"dlblas_b200: {HOST_PATH} was built for another torch or Python than this "
+                                       f"({host_tag()}); build it again with `python -m dlblas_b200.build`")
                 import importlib.util
-                spec = importlib.util.spec_from_file_location("dlblas_b200._host", path)
+                spec = importlib.util.spec_from_file_location("dlblas_b200._host", HOST_PATH)
                 module = importlib.util.module_from_spec(spec)
                 spec.loader.exec_module(module)
                 module.bind({name: ctypes.cast(getattr(handle, name), ctypes.c_void_p).value for name in SIGNATURES})

@@ -14,6 +14,8 @@ import os
 import subprocess
 import sys
 
+from ._C import HOST_PATH, host_is_current, host_tag
+
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 OUT = os.path.join(PKG, "_dlblas_b200.so")
@@ -25,7 +27,6 @@ NVCC_FLAGS = [
 ]
 
 
-HOST_OUT = os.path.join(PKG, "_host.so")
 HOST_SOURCE = "host.cpp"
 
 
@@ -39,8 +40,9 @@ def _host_command(obj_source, out):
            os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
     lib = os.path.join(root, "lib")
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
-    return (["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
-             "-w"] + [f for d in inc for f in ("-isystem", d)] + [obj_source, "-o", out, "-L" + lib, "-Wl,-rpath," + lib,
+    return (["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-Wall", "-Wextra",
+             f"-D_GLIBCXX_USE_CXX11_ABI={abi}", f'-DDLB_HOST_TAG="{host_tag()}"'] +
+            [f for d in inc for f in ("-isystem", d)] + [obj_source, "-o", out, "-L" + lib, "-Wl,-rpath," + lib,
              "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"])
 
 
@@ -64,8 +66,9 @@ def build(force=False, verbose=False):
     hdrs = [os.path.normpath(os.path.join(CSRC, h)) for h in HEADERS]
     objs, procs = [], []
     host = os.path.join(CSRC, HOST_SOURCE)
-    if force or _stale(HOST_OUT, [host, hdrs[-1]]):
-        procs.append((HOST_SOURCE, subprocess.Popen(_host_command(host, HOST_OUT), stdout=subprocess.PIPE,
+    # torch's C++ interface is not stable: another torch, another build
+    if force or _stale(HOST_PATH, [host, hdrs[-1]]) or not host_is_current(HOST_PATH):
+        procs.append((HOST_SOURCE, subprocess.Popen(_host_command(host, HOST_PATH), stdout=subprocess.PIPE,
                                                     stderr=subprocess.STDOUT, text=True)))
     for src in SOURCES:
         s = os.path.join(CSRC, src)
@@ -77,8 +80,8 @@ def build(force=False, verbose=False):
     failed = False
     for src, p in procs:
         out, _ = p.communicate()
-        if p.returncode != 0 or verbose:
-            sys.stderr.write(f"--- nvcc {src} ---\n{out}\n")
+        if out.strip():                # errors and warnings; the registers of every kernel with `verbose`
+            sys.stderr.write(f"--- {src} ---\n{out}\n")
         failed = failed or p.returncode != 0
     if failed:
         raise RuntimeError("nvcc failed while building the dlblas_b200 extension")

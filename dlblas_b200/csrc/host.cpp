@@ -33,6 +33,9 @@
 
 #include "../../include/dlblas_b200.h"
 
+// What this file was compiled for (build.py); _C.host() looks for it before it loads the module.
+extern "C" __attribute__((used)) const char dlb_host_built_for[] = DLB_HOST_TAG;
+
 namespace {
 
 using at::Tensor;

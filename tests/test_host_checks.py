@@ -42,6 +42,28 @@ def test_registry_keeps_no_argument():
     assert len(r.quick) <= _QUICK_MAX
 
 
+def test_host_module_of_another_torch_is_refused_and_rebuilt(monkeypatch):
+    from dlblas_b200 import _C, build
+    assert _C.host() is not None and _C.host_is_current()
+    monkeypatch.setattr(torch, "__version__", torch.__version__ + "1")
+    monkeypatch.setattr(_C, "_host_module", None)
+    with pytest.raises(RuntimeError, match="another torch"):
+        _C.host()
+    started = []
+
+    class Started(Exception):
+        pass
+
+    def popen(command, **kwargs):
+        started.append(command)
+        raise Started
+
+    monkeypatch.setattr(build.subprocess, "Popen", popen)
+    with pytest.raises(Started):
+        build.build()
+    assert started[0][0] == "g++" and any(torch.__version__ in word for word in started[0])
+
+
 @pytest.mark.gpu
 def test_refused_on_the_device(monkeypatch):
     from dlblas_b200 import _C, ops
