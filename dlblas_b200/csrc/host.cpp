@@ -714,17 +714,33 @@ PyObject* py_moe_align_block_size(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // ---- capacity-limited gating --------------------------------------------------------------------------------------
-// ceil(T / E * capacity_factor), at least min_capacity, from the single-precision product that the reference forms
+// ceil(T / E * capacity_factor), at least min_capacity, from the single-precision product that the reference forms.  A product
+// that is no whole number of slots is an error, as it is for Python's math.ceil.  Needs the GIL.
 int64_t gating_capacity(int64_t tokens, int64_t experts, double factor, int64_t min_capacity) {
   require(experts > 0, "logits must have at least one expert");
   const float per_expert = (float)((double)tokens / (double)experts), f = (float)factor;
-  return std::max<int64_t>((int64_t)std::ceil(per_expert * f), min_capacity);
+  const double slots = std::ceil(per_expert * f);
+  if (std::isnan(slots) || std::isinf(slots) || slots >= 0x1p63) {
+    PyErr_Format(std::isnan(slots) ? PyExc_ValueError : PyExc_OverflowError, "topk_gating: the capacity is not a whole number");
+    throw PyFailed{};
+  }
+  return std::max<int64_t>((int64_t)std::max(slots, -0x1p62), min_capacity);
+}
+
+// int(o): a least capacity may be given as a float
+int64_t truncated(PyObject* o) {
+  PyObject* whole = PyNumber_Long(o);
+  if (whole == nullptr) throw PyFailed{};
+  const long long v = PyLong_AsLongLong(whole);
+  Py_DECREF(whole);
+  if (v == -1 && PyErr_Occurred()) throw PyFailed{};
+  return v;
 }
 
 PyObject* py_gating_capacity(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     need_args(n, 4);
-    return PyLong_FromLongLong(gating_capacity(integer(a[0]), integer(a[1]), real(a[2]), integer(a[3])));
+    return PyLong_FromLongLong(gating_capacity(integer(a[0]), integer(a[1]), real(a[2]), truncated(a[3])));
   });
 }
 
@@ -815,7 +831,7 @@ PyObject* py_topk_gating(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor& logits = tensor(a[0]);
     const int64_t k = integer(a[1]);
     require(logits.dim() == 2, "logits must be 2-D");
-    const int64_t capacity = gating_capacity(logits.size(0), logits.size(1), real(a[2]) * (double)k, integer(a[3]));
+    const int64_t capacity = gating_capacity(logits.size(0), logits.size(1), real(a[2]) * (double)k, truncated(a[3]));
     if (logits.requires_grad() && at::GradMode::is_enabled()) {
       auto r = GatingFunction::apply(logits, k, capacity, truth(a[4]));
       return wrap_tuple({&r[0], &r[1], &r[2], &r[3]});

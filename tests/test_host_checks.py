@@ -17,6 +17,18 @@ def test_refused_without_a_device():
         host().gating_capacity(16, 0, 1.0, 2)
 
 
+def test_gating_capacity_takes_and_refuses_what_python_would():
+    from dlblas_b200.kernels.topk_gating import _capacity
+    assert _capacity(64, 8, 1.25, 2) == 10 and _capacity(64, 8, 0.1, 4.7) == 4 and _capacity(64, 8, -3.0, 2) == 2
+    assert _capacity(64, 8, -1e30, 2) == 2
+    for factor, error in ((float("inf"), OverflowError), (float("-inf"), OverflowError), (1e39, OverflowError),
+                          (1e30, OverflowError), (float("nan"), ValueError)):
+        with pytest.raises(error):
+            _capacity(64, 8, factor, 2)
+    with pytest.raises(ValueError):
+        _capacity(64, 8, 1.0, float("nan"))
+
+
 def test_registry_keeps_no_argument():
     import gc
     import weakref
