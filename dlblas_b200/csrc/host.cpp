@@ -990,14 +990,18 @@ struct PermuteFunction : torch::autograd::Function<PermuteFunction> {
     ctx->save_for_backward({p.row_map});
     ctx->saved_data["t"] = t;
     ctx->saved_data["k"] = k;
+    ctx->saved_data["h"] = x.size(1);
+    ctx->saved_data["dtype"] = (int64_t)x.scalar_type();
     ctx->mark_non_differentiable({p.row_map});
     return {out, p.row_map};
   }
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
-    if (!grads[0].defined() || grads[0].numel() == 0) return {grads[0], Tensor()};
-    return {unpermute_rows(grads[0], ctx->get_saved_variables()[0], Tensor(), ctx->saved_data["t"].toInt(),
-                           ctx->saved_data["k"].toInt()),
-            Tensor()};
+    auto& s = ctx->saved_data;
+    const Tensor row_map = ctx->get_saved_variables()[0];
+    if (!grads[0].defined())       // the rows' consumer has no gradient for them; zeros for the row map are not wanted
+      return {at::zeros({s["t"].toInt(), s["h"].toInt()}, row_map.options().dtype((at::ScalarType)s["dtype"].toInt())), Tensor()};
+    if (grads[0].numel() == 0) return {grads[0], Tensor()};
+    return {unpermute_rows(grads[0], row_map, Tensor(), s["t"].toInt(), s["k"].toInt()), Tensor()};
   }
 };
 

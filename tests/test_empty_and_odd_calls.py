@@ -57,6 +57,25 @@ def test_permute_plan_without_tokens():
         assert out.shape == (0, 64) and got.shape == (0,) and order.shape == (0,) and order.dtype == torch.int64
 
 
+class _NoGradient(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x):
+        return x.sum()
+
+    @staticmethod
+    def backward(ctx, grad):
+        return None
+
+
+@pytest.mark.gpu
+def test_permute_whose_rows_get_no_gradient():
+    from dlblas_b200.kernels.permute import permute
+    x = torch.ones(5, 64, dtype=torch.bfloat16, device=DEV, requires_grad=True)
+    rows, _ = permute(x, torch.zeros(5, 2, dtype=torch.int32, device=DEV))
+    (grad,) = torch.autograd.grad(_NoGradient.apply(rows), x)
+    assert grad.shape == x.shape and grad.dtype == x.dtype and not grad.any()
+
+
 # ---- one-rank decode layer ---------------------------------------------------------------------------------------
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float64])
