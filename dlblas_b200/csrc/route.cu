@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(WARPS * 32) grouped_topk_lanes_kernel(const T*
     for (int i = 0; i < VPT; ++i) xf[i] = to_f32<T>(x[i]);
     sigmoid_row<VPT>(xf, sc);
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) ch[i] = sc[i] + __ldg(bias + lane * VPT + i);
+    for (int i = 0; i < VPT; ++i) ch[i] = fmaxf(sc[i] + __ldg(bias + lane * VPT + i), NEG_INF);   // a NaN is never chosen
   }
   // the two largest scores of the lane, then of its group
   float v1 = ch[0], v2 = NEG_INF;
@@ -328,9 +328,13 @@ __global__ void __launch_bounds__(WARPS * 32) grouped_topk_lanes_kernel(const T*
     const float s = __shfl_sync(0xffffffffu, gscore, g * group_lanes);
     better_groups += (s > gscore || (s == gscore && g < my_group)) ? 1 : 0;
   }
-  const bool kept = better_groups < topk_group;
+  // Groups of minus infinity (a bias that switches experts off) lose to all others.  Where there are not enough others, the
+  // rounds of the kernel above take the first group of the row again and again, and the first expert once no score is left.
+  const bool scored = gscore > NEG_INF;
+  const bool too_few = __popc(__ballot_sync(0xffffffffu, scored)) < topk_group * group_lanes;
+  const bool kept = (scored && better_groups < topk_group) || (too_few && my_group == 0);
   // best remaining expert of the lane
-  float best = NEG_INF, best_score = 0.f;
+  float best = NEG_INF, best_score = sc[0];
   int best_at = 0;
   auto scan = [&] {
     best = NEG_INF;
@@ -345,7 +349,7 @@ __global__ void __launch_bounds__(WARPS * 32) grouped_topk_lanes_kernel(const T*
       }
   };
   if (kept) scan();
-  uint32_t key = kept ? order_key(best) : 0u;
+  uint32_t key = order_key(best);
   float wsum = 0.f, my_w = 0.f;
   int my_id = 0;
   for (int j = 0; j < top_k; ++j) {
@@ -358,7 +362,7 @@ __global__ void __launch_bounds__(WARPS * 32) grouped_topk_lanes_kernel(const T*
       my_w = w;
       my_id = owner * VPT + at;
     }
-    if (lane == owner) {
+    if (lane == owner && kept) {
 #pragma unroll
       for (int i = 0; i < VPT; ++i)
         if (i == best_at) ch[i] = NEG_INF;

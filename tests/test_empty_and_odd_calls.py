@@ -259,3 +259,29 @@ def test_layer_normalises_weights_of_any_layout():
     for given in (w, w.t().contiguous().t(), w.half(), w.half().t().contiguous().t()):
         want = plain.forward(x, given / given.sum(-1, keepdim=True), ids, *weights)
         assert torch.equal(layer.forward(x, given, ids, *weights), want)
+
+
+# ---- routing scores that are no numbers, or minus infinity --------------------------------------------------------
+@pytest.mark.gpu
+@pytest.mark.parametrize("experts,groups", [(256, 8), (160, 8), (64, 8), (256, 32), (32, 1), (96, 8)])   # the last: general kernel
+@pytest.mark.parametrize("off", [0.02, 0.5, 0.9, 1.0])
+def test_grouped_routing_with_experts_switched_off(experts, groups, off):
+    """A bias of minus infinity switches an expert off, down to fewer experts and groups than are wanted; so does a NaN."""
+    from dlblas_b200 import ops
+    g = torch.Generator().manual_seed(int(100 * off) + experts + groups)
+    topk_group, top_k = max(groups // 2, 1), 6
+    x = torch.randn(200, experts, generator=g)
+    for trial in range(4):
+        bias = torch.randn(experts, generator=g) * 0.1
+        dead = torch.rand(experts, generator=g) < off
+        if trial == 1:
+            dead[0::experts // 32] = True                     # the first expert of every lane
+        bias[dead] = -float("inf")
+        want_w, want_ids = O.biased_grouped_topk(x, bias, top_k, False, groups, topk_group)
+        w, ids = ops.route_grouped_topk(x.to(DEV), bias.to(DEV), top_k, False, groups, topk_group)
+        assert torch.equal(ids.cpu(), want_ids) and torch.equal(w.cpu(), want_w)
+        if 2 * int(dead.sum()) <= experts:                    # enough left in any topk_group groups
+            nan = bias.masked_fill(dead, float("nan"))
+            w, ids = ops.route_grouped_topk(x.to(DEV), nan.to(DEV), top_k, False, groups, topk_group)
+            live = ~dead[want_ids.long()]
+            assert torch.equal(ids.cpu()[live], want_ids[live]) and torch.equal(w.cpu()[live], want_w[live])
