@@ -21,6 +21,7 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <array>
 #include <cctype>
 #include <cerrno>
 #include <climits>
@@ -79,6 +80,9 @@ struct Abi {
 struct AssertionFailed : std::runtime_error {
   using std::runtime_error::runtime_error;
 };
+struct BadValue : std::runtime_error {
+  using std::runtime_error::runtime_error;
+};
 void require(bool ok, const char* msg) {
   if (!ok) throw AssertionFailed(msg);
 }
@@ -90,7 +94,17 @@ void check(int rc) {
 }
 
 // ---- arguments ----------------------------------------------------------------------------------------------------
-struct PyFailed {};   // a Python error is already set
+struct PyFailed {};   // a Python error is already set (thrown with the GIL held only)
+
+// The work of a method, after its arguments are read and before its result is wrapped, runs without the GIL, as torch's own
+// operators do: an allocation or a launch into a full queue can wait for the GPU, and other threads go on meanwhile.
+template <typename F> auto without_gil(F&& f) {
+  struct Released {
+    PyThreadState* state = PyEval_SaveThread();
+    ~Released() { PyEval_RestoreThread(state); }
+  } released;
+  return f();
+}
 
 const Tensor& tensor(PyObject* o) {
   if (!THPVariable_Check(o)) {
@@ -147,6 +161,8 @@ template <typename F> PyObject* guarded(F&& f) {
     return nullptr;
   } catch (const AssertionFailed& e) {
     PyErr_SetString(PyExc_AssertionError, e.what());
+  } catch (const BadValue& e) {
+    PyErr_SetString(PyExc_ValueError, e.what());
   } catch (const c10::OutOfMemoryError& e) {
     // the type that torch's own allocations raise
     PyObject* torch = PyImport_ImportModule("torch");
@@ -239,10 +255,8 @@ int env_int(const char* name, int fallback) {
   errno = 0;
   const long n = std::strtol(v, &end, 10);
   while (end != v && std::isspace((unsigned char)*end)) ++end;
-  if (end == v || *end != 0 || errno != 0 || n < INT_MIN || n > INT_MAX) {
-    PyErr_Format(PyExc_ValueError, "%s must be a whole number, got '%s'", name, v);
-    throw PyFailed{};
-  }
+  if (end == v || *end != 0 || errno != 0 || n < INT_MIN || n > INT_MAX)
+    throw BadValue(std::string(name) + " must be a whole number, got '" + v + "'");
   return (int)n;
 }
 int tile_rows_env(const char* name, int fallback) {
@@ -280,31 +294,37 @@ std::pair<Tensor, Tensor> quant_fp8(const Tensor& x, int64_t group, int mode, do
 PyObject* py_quant_fp8(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     need_args(n, 8);
-    auto [q, s] = quant_fp8(tensor(a[0]), integer(a[1]), (int)integer(a[2]), real(a[3]), truth(a[4]), opt_tensor(a[5]),
-                            integer(a[6]), integer(a[7]));
+    const Tensor& x = tensor(a[0]);
+    const int64_t group = integer(a[1]), mode = integer(a[2]), fanout = integer(a[6]), rows_out = integer(a[7]);
+    const double eps = real(a[3]);
+    const bool column_major = truth(a[4]);
+    const std::optional<Tensor> dst_pos = opt_tensor(a[5]);
+    auto [q, s] = without_gil([&] { return quant_fp8(x, group, (int)mode, eps, column_major, dst_pos, fanout, rows_out); });
     return wrap_tuple({&q, &s});
   });
 }
 
 // per_token_group_quant_fp8: any leading dimensions
+std::pair<Tensor, Tensor> group_quant_fp8(const Tensor& x, int64_t group, double eps, bool column_major) {
+  require(x.dim() > 0 && x.stride(-1) == 1, "groups must be contiguous");
+  if (x.dim() == 2) return quant_fp8(x, group, DLB_QUANT_DIV_EPS, eps, column_major, std::nullopt, 1, -1);
+  require(!column_major, "column-major scales need a 2-D input");
+  auto [q, s] = quant_fp8(x.reshape({-1, x.size(-1)}), group, DLB_QUANT_DIV_EPS, eps, false, std::nullopt, 1, -1);
+  std::vector<int64_t> shape = x.sizes().vec();
+  Tensor qv = q.view(shape);
+  shape.back() /= group;
+  return {qv, s.view(shape)};
+}
+
 PyObject* py_group_quant_fp8(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     need_args(n, 4);
     const Tensor& x = tensor(a[0]);
     const int64_t group = integer(a[1]);
+    const double eps = real(a[2]);
     const bool column_major = truth(a[3]);
-    require(x.dim() > 0 && x.stride(-1) == 1, "groups must be contiguous");
-    if (x.dim() == 2) {
-      auto [q, s] = quant_fp8(x, group, DLB_QUANT_DIV_EPS, real(a[2]), column_major, std::nullopt, 1, -1);
-      return wrap_tuple({&q, &s});
-    }
-    require(!column_major, "column-major scales need a 2-D input");
-    auto [q, s] = quant_fp8(x.reshape({-1, x.size(-1)}), group, DLB_QUANT_DIV_EPS, real(a[2]), false, std::nullopt, 1, -1);
-    std::vector<int64_t> shape = x.sizes().vec();
-    Tensor qv = q.view(shape);
-    shape.back() /= group;
-    Tensor sv = s.view(shape);
-    return wrap_tuple({&qv, &sv});
+    auto [q, s] = without_gil([&] { return group_quant_fp8(x, group, eps, column_major); });
+    return wrap_tuple({&q, &s});
   });
 }
 
@@ -336,47 +356,62 @@ Tensor fp8_gemm(const Tensor& a, const Tensor& b, const Tensor& a_s, const Tenso
 PyObject* py_fp8_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     need_args(n, 6);
-    return wrap(fp8_gemm(tensor(a[0]), tensor(a[1]), tensor(a[2]), tensor(a[3]), dtype(a[4]), (int)integer(a[5])));
+    const Tensor &x = tensor(a[0]), &w = tensor(a[1]), &x_s = tensor(a[2]), &w_s = tensor(a[3]);
+    const at::ScalarType out = dtype(a[4]);
+    const int64_t tile_rows = integer(a[5]);
+    return wrap(without_gil([&] { return fp8_gemm(x, w, x_s, w_s, out, (int)tile_rows); }));
   });
 }
 
 // ---- routing ------------------------------------------------------------------------------------------------------
+std::pair<Tensor, Tensor> route_softmax_topk(const Tensor& logits, int64_t top_k, bool renormalize, at::ScalarType ids_dtype) {
+  require_cuda(logits);
+  require(logits.dim() == 2 && logits.is_contiguous(), "logits must be a contiguous 2-D tensor");
+  Call c(logits);
+  const int64_t t = logits.size(0);
+  Tensor w = empty({t, top_k}, at::kFloat, c), ids = empty({t, top_k}, ids_dtype, c);
+  check(abi.dlb_route_softmax_topk(logits.data_ptr(), code(logits.scalar_type()), t, (int)logits.size(1), (int)top_k,
+                                   renormalize, w.data_ptr<float>(), ids.data_ptr(), code(ids_dtype), c.stream));
+  return {w, ids};
+}
+
 PyObject* py_route_softmax_topk(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     need_args(n, 4);
     const Tensor& logits = tensor(a[0]);
     const int64_t top_k = integer(a[1]);
+    const bool renormalize = truth(a[2]);
     const at::ScalarType ids_dtype = dtype(a[3]);
-    require_cuda(logits);
-    require(logits.dim() == 2 && logits.is_contiguous(), "logits must be a contiguous 2-D tensor");
-    Call c(logits);
-    const int64_t t = logits.size(0);
-    Tensor w = empty({t, top_k}, at::kFloat, c), ids = empty({t, top_k}, ids_dtype, c);
-    check(abi.dlb_route_softmax_topk(logits.data_ptr(), code(logits.scalar_type()), t, (int)logits.size(1), (int)top_k,
-                                     truth(a[2]), w.data_ptr<float>(), ids.data_ptr(), code(ids_dtype), c.stream));
+    auto [w, ids] = without_gil([&] { return route_softmax_topk(logits, top_k, renormalize, ids_dtype); });
     return wrap_tuple({&w, &ids});
   });
+}
+
+std::pair<Tensor, Tensor> route_grouped_topk(const Tensor& given, const Tensor& given_bias, int64_t top_k, bool renormalize,
+                                             int64_t groups, int64_t topk_group) {
+  require_cuda(given);
+  require_cuda(given_bias);
+  require(given.dim() == 2, "logits must be 2-D");
+  Call c(given);
+  const Tensor logits = given.is_contiguous() ? given : given.contiguous();
+  Tensor bias = given_bias.scalar_type() == at::kFloat ? given_bias : given_bias.to(at::kFloat);
+  if (!bias.is_contiguous()) bias = bias.contiguous();
+  const int64_t t = logits.size(0), e = logits.size(1);
+  require(bias.numel() == e, "the bias must have one entry per expert");
+  Tensor w = empty({t, top_k}, at::kFloat, c), ids = empty({t, top_k}, at::kInt, c);
+  check(abi.dlb_route_grouped_topk(logits.data_ptr(), code(logits.scalar_type()), bias.data_ptr<float>(), t, (int)e, (int)groups,
+                                   (int)topk_group, (int)top_k, renormalize, w.data_ptr<float>(), ids.data_ptr<int32_t>(),
+                                   c.stream));
+  return {w, ids};
 }
 
 PyObject* py_route_grouped_topk(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     need_args(n, 6);
-    const Tensor& given = tensor(a[0]);
-    const Tensor& given_bias = tensor(a[1]);
-    const int64_t top_k = integer(a[2]);
-    require_cuda(given);
-    require_cuda(given_bias);
-    require(given.dim() == 2, "logits must be 2-D");
-    Call c(given);
-    const Tensor logits = given.is_contiguous() ? given : given.contiguous();
-    Tensor bias = given_bias.scalar_type() == at::kFloat ? given_bias : given_bias.to(at::kFloat);
-    if (!bias.is_contiguous()) bias = bias.contiguous();
-    const int64_t t = logits.size(0), e = logits.size(1);
-    require(bias.numel() == e, "the bias must have one entry per expert");
-    Tensor w = empty({t, top_k}, at::kFloat, c), ids = empty({t, top_k}, at::kInt, c);
-    check(abi.dlb_route_grouped_topk(logits.data_ptr(), code(logits.scalar_type()), bias.data_ptr<float>(), t, (int)e,
-                                     (int)integer(a[4]), (int)integer(a[5]), (int)top_k, truth(a[3]), w.data_ptr<float>(),
-                                     ids.data_ptr<int32_t>(), c.stream));
+    const Tensor &logits = tensor(a[0]), &bias = tensor(a[1]);
+    const int64_t top_k = integer(a[2]), groups = integer(a[4]), topk_group = integer(a[5]);
+    const bool renormalize = truth(a[3]);
+    auto [w, ids] = without_gil([&] { return route_grouped_topk(logits, bias, top_k, renormalize, groups, topk_group); });
     return wrap_tuple({&w, &ids});
   });
 }
@@ -480,7 +515,7 @@ PyObject* py_moe_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     MoeArgs g{opt_tensor(a[0]), opt_tensor(a[1]), opt_tensor(a[2]), tensor(a[3]), tensor(a[4]), tensor(a[5]), tensor(a[6]),
               tensor(a[7]), tensor(a[8]), integer(a[9]), dtype(a[10]), integer(a[11]), integer(a[12]), (int)integer(a[13]),
               truth(a[14]), truth(a[15]), truth(a[16])};
-    return wrap(moe_forward(g));
+    return wrap(without_gil([&] { return moe_forward(g); }));
   });
 }
 
@@ -540,8 +575,10 @@ Tensor low_latency_forward(const Tensor& x, const Tensor& topk_weights, const Te
 PyObject* py_low_latency_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     need_args(n, 8);
-    return wrap(low_latency_forward(tensor(a[0]), tensor(a[1]), tensor(a[2]), tensor(a[3]), tensor(a[4]), tensor(a[5]),
-                                    tensor(a[6]), dtype(a[7])));
+    const Tensor &x = tensor(a[0]), &weights = tensor(a[1]), &ids = tensor(a[2]), &w1 = tensor(a[3]), &w1_s = tensor(a[4]),
+                 &w2 = tensor(a[5]), &w2_s = tensor(a[6]);
+    const at::ScalarType out = dtype(a[7]);
+    return wrap(without_gil([&] { return low_latency_forward(x, weights, ids, w1, w1_s, w2, w2_s, out); }));
   });
 }
 
@@ -594,7 +631,9 @@ Tensor m_grouped_gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& size
 PyObject* py_m_grouped_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     need_args(n, 4);
-    return wrap(m_grouped_gemm(tensor(a[0]), tensor(a[1]), tensor(a[2]), truth(a[3])));
+    const Tensor &x = tensor(a[0]), &w = tensor(a[1]), &sizes = tensor(a[2]);
+    const bool trans_b = truth(a[3]);
+    return wrap(without_gil([&] { return m_grouped_gemm(x, w, sizes, trans_b); }));
   });
 }
 
@@ -627,7 +666,8 @@ Tensor k_grouped_gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& size
 PyObject* py_k_grouped_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     need_args(n, 3);
-    return wrap(k_grouped_gemm(tensor(a[0]), tensor(a[1]), tensor(a[2])));
+    const Tensor &x = tensor(a[0]), &y = tensor(a[1]), &sizes = tensor(a[2]);
+    return wrap(without_gil([&] { return k_grouped_gemm(x, y, sizes); }));
   });
 }
 
@@ -679,36 +719,44 @@ Tensor moe_forward_16bit(const Tensor& x, const Tensor& w1_in, const Tensor& w2_
 PyObject* py_moe_forward_16bit(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     need_args(n, 5);
-    return wrap(moe_forward_16bit(tensor(a[0]), tensor(a[1]), tensor(a[2]), tensor(a[3]), tensor(a[4])));
+    const Tensor &x = tensor(a[0]), &w1 = tensor(a[1]), &w2 = tensor(a[2]), &weights = tensor(a[3]), &ids = tensor(a[4]);
+    return wrap(without_gil([&] { return moe_forward_16bit(x, w1, w2, weights, ids); }));
   });
 }
 
 // ---- block-aligned token layout -----------------------------------------------------------------------------------
+std::array<Tensor, 3> moe_align_block_size(Tensor given, int64_t block, int64_t experts, int64_t local,
+                                           const std::optional<Tensor>& expert_map, bool pad) {
+  require_cuda(given);
+  require(given.scalar_type() == at::kInt || given.scalar_type() == at::kLong, "topk_ids must be int32 or int64");
+  require(block > 0 && experts > 0, "block_size and num_experts must be positive");
+  Call c(given);
+  Tensor ids = given.is_contiguous() ? given : given.contiguous();
+  const int64_t slots = ids.numel();
+  int64_t padded = slots + experts * (block - 1);
+  if (pad) padded = (padded + block - 1) / block * block;
+  const int64_t blocks = (padded + block - 1) / block;
+  Tensor sorted = empty({padded}, at::kInt, c), owner = empty({blocks}, at::kInt, c), total = empty({1}, at::kInt, c);
+  const size_t sort_bytes = abi.dlb_sort_by_expert_workspace_size(slots, (int)experts);
+  Workspace ws;
+  ws.take(sort_bytes);
+  ws.allocate(c);
+  check(abi.dlb_moe_align_block_size(ids.data_ptr(), code(ids.scalar_type()), slots, (int)experts, (int)local, (int)block,
+                                     sorted.data_ptr<int32_t>(), padded, owner.data_ptr<int32_t>(), (int)blocks,
+                                     total.data_ptr<int32_t>(), ws.at<void>(0), sort_bytes, c.stream));
+  if (!ids.is_same(given)) given.copy_(ids);      // negative ids are replaced in the caller's tensor
+  if (expert_map) owner = expert_map->index({owner.to(at::kLong)});
+  return {sorted, owner, total};
+}
+
 PyObject* py_moe_align_block_size(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     need_args(n, 6);
-    Tensor given = tensor(a[0]);
+    const Tensor& ids = tensor(a[0]);
     const int64_t block = integer(a[1]), experts = integer(a[2]), local = integer(a[3]);
     const std::optional<Tensor> expert_map = opt_tensor(a[4]);
-    require_cuda(given);
-    require(given.scalar_type() == at::kInt || given.scalar_type() == at::kLong, "topk_ids must be int32 or int64");
-    require(block > 0 && experts > 0, "block_size and num_experts must be positive");
-    Call c(given);
-    Tensor ids = given.is_contiguous() ? given : given.contiguous();
-    const int64_t slots = ids.numel();
-    int64_t padded = slots + experts * (block - 1);
-    if (truth(a[5])) padded = (padded + block - 1) / block * block;
-    const int64_t blocks = (padded + block - 1) / block;
-    Tensor sorted = empty({padded}, at::kInt, c), owner = empty({blocks}, at::kInt, c), total = empty({1}, at::kInt, c);
-    const size_t sort_bytes = abi.dlb_sort_by_expert_workspace_size(slots, (int)experts);
-    Workspace ws;
-    ws.take(sort_bytes);
-    ws.allocate(c);
-    check(abi.dlb_moe_align_block_size(ids.data_ptr(), code(ids.scalar_type()), slots, (int)experts, (int)local, (int)block,
-                                       sorted.data_ptr<int32_t>(), padded, owner.data_ptr<int32_t>(), (int)blocks,
-                                       total.data_ptr<int32_t>(), ws.at<void>(0), sort_bytes, c.stream));
-    if (!ids.is_same(given)) given.copy_(ids);      // negative ids are replaced in the caller's tensor
-    if (expert_map) owner = expert_map->index({owner.to(at::kLong)});
+    const bool pad = truth(a[5]);
+    auto [sorted, owner, total] = without_gil([&] { return moe_align_block_size(ids, block, experts, local, expert_map, pad); });
     return wrap_tuple({&sorted, &owner, &total});
   });
 }
@@ -809,7 +857,9 @@ struct GatingFunction : torch::autograd::Function<GatingFunction> {
 PyObject* py_gating_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     need_args(n, 4);
-    Gating g = gating_forward(tensor(a[0]), integer(a[1]), integer(a[2]));
+    const Tensor& logits = tensor(a[0]);
+    const int64_t k = integer(a[1]), capacity = integer(a[2]);
+    Gating g = without_gil([&] { return gating_forward(logits, k, capacity); });
     return truth(a[3]) ? wrap_tuple({&g.l_aux, &g.ec_idx, &g.weights, &g.select, &g.ws})
                        : wrap_tuple({&g.l_aux, &g.ec_idx, &g.weights, &g.select});
   });
@@ -819,8 +869,10 @@ PyObject* py_gating_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     need_args(n, 8);
     const std::optional<Tensor> gw = opt_tensor(a[7]);
-    return wrap(gating_backward(tensor(a[0]), dtype(a[1]), integer(a[2]), integer(a[3]), integer(a[4]), integer(a[5]),
-                                tensor(a[6]), gw ? *gw : Tensor()));
+    const Tensor &ws = tensor(a[0]), &gl = tensor(a[6]);
+    const at::ScalarType dt = dtype(a[1]);
+    const int64_t tokens = integer(a[2]), experts = integer(a[3]), k = integer(a[4]), capacity = integer(a[5]);
+    return wrap(without_gil([&] { return gating_backward(ws, dt, tokens, experts, k, capacity, gl, gw ? *gw : Tensor()); }));
   });
 }
 
@@ -833,10 +885,11 @@ PyObject* py_topk_gating(PyObject*, PyObject* const* a, Py_ssize_t n) {
     require(logits.dim() == 2, "logits must be 2-D");
     const int64_t capacity = gating_capacity(logits.size(0), logits.size(1), real(a[2]) * (double)k, truncated(a[3]));
     if (logits.requires_grad() && at::GradMode::is_enabled()) {
-      auto r = GatingFunction::apply(logits, k, capacity, truth(a[4]));
+      const bool higher_precision = truth(a[4]);
+      auto r = without_gil([&] { return GatingFunction::apply(logits, k, capacity, higher_precision); });
       return wrap_tuple({&r[0], &r[1], &r[2], &r[3]});
     }
-    Gating g = gating_forward(logits, k, capacity);
+    Gating g = without_gil([&] { return gating_forward(logits, k, capacity); });
     return wrap_tuple({&g.l_aux, &g.ec_idx, &g.weights, &g.select});
   });
 }
@@ -886,9 +939,7 @@ PermutePlan permute_plan(const Tensor& indices, int64_t dest_limit, bool want_so
                                with_stats ? (void*)events[dev].event() : nullptr, ws.at<void>(0), bytes, c.stream));
   };
   plan(PERMUTE_EXPERTS, true);
-  PyThreadState* others = PyGILState_Check() ? PyEval_SaveThread() : nullptr;   // the host may wait here: let others run
   const cudaError_t waited = cudaEventSynchronize(events[dev].event());
-  if (others != nullptr) PyEval_RestoreThread(others);
   if (waited != cudaSuccess) throw std::runtime_error(std::string("permute: ") + cudaGetErrorString(waited));
   const int64_t largest = stats[0];
   p.minus_one = stats[1];
@@ -910,7 +961,9 @@ void permute_rows(const Tensor& x, const PermutePlan& p, int64_t k, const Tensor
 PyObject* py_permute_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     need_args(n, 2);
-    PermutePlan p = permute_plan(tensor(a[0]), integer(a[1]), true);
+    const Tensor& indices = tensor(a[0]);
+    const int64_t dest_limit = integer(a[1]);
+    PermutePlan p = without_gil([&] { return permute_plan(indices, dest_limit, true); });
     return Py_BuildValue("(NNNLL)", wrap(p.sorted_idx), wrap(p.dest), wrap(p.row_map), (long long)p.minus_one,
                          (long long)p.negative);
   });
@@ -940,7 +993,9 @@ PyObject* py_unpermute_rows(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     need_args(n, 5);
     const std::optional<Tensor> probs = opt_tensor(a[2]);
-    return wrap(unpermute_rows(tensor(a[0]), tensor(a[1]), probs ? *probs : Tensor(), integer(a[3]), integer(a[4])));
+    const Tensor &x = tensor(a[0]), &row_map = tensor(a[1]);
+    const int64_t tokens = integer(a[3]), k = integer(a[4]);
+    return wrap(without_gil([&] { return unpermute_rows(x, row_map, probs ? *probs : Tensor(), tokens, k); }));
   });
 }
 
@@ -972,7 +1027,9 @@ std::pair<Tensor, Tensor> unpermute_backward(const Tensor& grad_in, const Tensor
 PyObject* py_unpermute_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     need_args(n, 5);
-    auto [act, prob] = unpermute_backward(tensor(a[0]), tensor(a[1]), tensor(a[2]), tensor(a[3]), dtype(a[4]));
+    const Tensor &grad = tensor(a[0]), &fwd = tensor(a[1]), &row_map = tensor(a[2]), &probs = tensor(a[3]);
+    const at::ScalarType act_dtype = dtype(a[4]);
+    auto [act, prob] = without_gil([&] { return unpermute_backward(grad, fwd, row_map, probs, act_dtype); });
     return wrap_tuple({&act, &prob});
   });
 }
@@ -1015,7 +1072,7 @@ PyObject* py_permute(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!x.is_cuda() || !indices.is_cuda()) throw std::runtime_error("permute needs CUDA tensors");
     if (x.size(0) != indices.size(0))
       throw std::runtime_error("token count mismatch: " + std::to_string(x.size(0)) + " vs " + std::to_string(indices.size(0)));
-    auto r = PermuteFunction::apply(x, indices);
+    auto r = without_gil([&] { return PermuteFunction::apply(x, indices); });
     return wrap_tuple({&r[0], &r[1]});
   });
 }
@@ -1047,7 +1104,9 @@ PyObject* py_unpermute(PyObject*, PyObject* const* a, Py_ssize_t n) {
     need_args(n, 3);
     const Tensor& x = tensor(a[0]);
     if (x.numel() == 0) return wrap(x);
-    return wrap(UnpermuteFunction::apply(x, tensor(a[1]), opt_tensor(a[2])));
+    const Tensor& row_map = tensor(a[1]);
+    const std::optional<Tensor> probs = opt_tensor(a[2]);
+    return wrap(without_gil([&] { return UnpermuteFunction::apply(x, row_map, probs); }));
   });
 }
 
@@ -1070,7 +1129,10 @@ PyObject* py_bind(PyObject*, PyObject* arg) {
 }
 
 PyObject* py_status_word(PyObject*, PyObject* arg) {
-  return guarded([&] { return wrap(status_word((at::DeviceIndex)integer(arg))); });
+  return guarded([&] {
+    const int64_t index = integer(arg);
+    return wrap(without_gil([&] { return status_word((at::DeviceIndex)index); }));
+  });
 }
 
 #define FAST(name, fn) {name, (PyCFunction)(void (*)(void))fn, METH_FASTCALL, nullptr}

@@ -285,3 +285,40 @@ def test_grouped_routing_with_experts_switched_off(experts, groups, off):
             w, ids = ops.route_grouped_topk(x.to(DEV), nan.to(DEV), top_k, False, groups, topk_group)
             live = ~dead[want_ids.long()]
             assert torch.equal(ids.cpu()[live], want_ids[live]) and torch.equal(w.cpu()[live], want_w[live])
+
+
+# ---- threads ------------------------------------------------------------------------------------------------------
+@pytest.mark.gpu
+def test_other_threads_run_while_a_launch_waits():
+    """Launches behind half a second of work fill the queue, and the next one waits for the GPU; torch's operators let other
+    threads run in the meantime, and so do these."""
+    import threading
+    import time
+
+    from dlblas_b200 import ops
+    x = torch.zeros(4, 128, dtype=torch.bfloat16, device=DEV)
+    ops.quant_fp8(x, 128)
+    torch.cuda.synchronize()
+    gaps, done = [], threading.Event()
+
+    def watch():
+        last = time.perf_counter()
+        while not done.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    thread = threading.Thread(target=watch)
+    thread.start()
+    torch.cuda._sleep(1_000_000_000)
+    begin = time.perf_counter()
+    for _ in range(4000):
+        ops.quant_fp8(x, 128)
+    queued = time.perf_counter() - begin
+    done.set()
+    thread.join()
+    torch.cuda.synchronize()
+    if queued < 0.3:
+        pytest.skip("the queue took all launches")
+    assert max(gaps) < 0.5 * queued, (max(gaps), queued)
