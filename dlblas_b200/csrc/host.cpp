@@ -18,6 +18,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -171,6 +172,8 @@ template <typename F> PyObject* guarded(F&& f) {
     PyErr_SetString(type != nullptr ? type : PyExc_MemoryError, e.what_without_backtrace());
     Py_XDECREF(type);
     Py_XDECREF(torch);
+  } catch (python_error& e) {      // of Python code that torch ran on the way, a saved-tensor hook say
+    e.restore();
   } catch (const c10::Error& e) {
     PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
   } catch (const std::exception& e) {

@@ -76,6 +76,24 @@ def test_permute_whose_rows_get_no_gradient():
     assert grad.shape == x.shape and grad.dtype == x.dtype and not grad.any()
 
 
+@pytest.mark.gpu
+def test_errors_of_saved_tensor_hooks_come_through():
+    import dlblas_b200
+    from dlblas_b200.kernels.permute import permute, unpermute
+
+    def pack(t):
+        raise KeyError("packed")
+
+    x = torch.ones(5, 64, dtype=torch.bfloat16, device=DEV, requires_grad=True)
+    ids = torch.zeros(5, 2, dtype=torch.int32, device=DEV)
+    rows, rmap = permute(x, ids)
+    logits = torch.ones(5, 8, device=DEV, requires_grad=True)
+    for call in (lambda: permute(x, ids), lambda: unpermute(rows, rmap, torch.ones(5, 2, device=DEV)),
+                 lambda: dlblas_b200.topk_gating(logits, 2)):
+        with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t), pytest.raises(KeyError, match="packed"):
+            call()
+
+
 # ---- one-rank decode layer ---------------------------------------------------------------------------------------
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float64])
