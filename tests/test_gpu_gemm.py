@@ -360,8 +360,10 @@ def test_fp8_gemm_narrow_tiles(m, n, k):
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("fuse", [True, False])
 def test_layer_tiles_of_few_rows(dtype, fuse):
-    """At most 32 rows per expert on average: tiles of at most 32 rows exchange the operands.  Segments around the 16-row
-    chunks, the 32-row line and whole tiles, every expert with one row, and both sides of the line of the rule."""
+    """At most 32 rows per expert on average.  Segments around the 16-row chunks, the 32-row line and whole tiles, every expert
+    with one row, and both sides of the line of the rule.  The first GEMM of the fused layer exchanges the operands of tiles
+    of at most 32 rows here; the other launches take narrower tiles, except with 160 experts (for them see
+    test_exchanged_operands_give_the_same_bits)."""
     from dlblas_b200.layers.moe.kernels.blocked_fp8_fused_moe import moe_expert_forward
     g = torch.Generator().manual_seed(41)
     for counts in ([1, 0, 15, 16, 17, 31, 32, 33, 49, 63, 64, 65, 127, 128, 129, 192, 193, 0, 2] + [0] * 20, [1] * 160, [32, 32],
@@ -379,3 +381,56 @@ def test_layer_tiles_of_few_rows(dtype, fuse):
             rows = ids[:, 0] == k
             if bool(rows.any()):
                 assert O.rel_frobenius(out[rows], ref[rows]) < 2e-2, (e, k)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("epilogue", ["store", "scatter", "swiglu"])
+def test_exchanged_operands_give_the_same_bits(epilogue, dtype):
+    """Enough tiles for 256 columns each (148) and at most 32 rows per expert on average: tiles of at most 32 rows exchange
+    the operands, the others between them do not.  Tiles of 256 rows never do, and products and sums keep their order."""
+    from dlblas_b200 import _C, ops
+    counts = [1, 0, 15, 16, 17, 31, 32, 33, 49, 63, 64, 65, 127, 128, 129, 160, 161, 193, 2] + [0, 5, 30, 24] * 10
+    e, rows, k, n = len(counts), sum(counts), 384, 1024 if epilogue == "swiglu" else 1152
+    assert rows <= 32 * e and (rows // 128 + e) * -(-n // 256) >= 148
+    g = torch.Generator().manual_seed(17)
+    a, a_s = O.quant_fp8(torch.randn(rows, k, generator=g).to(torch.bfloat16), 128)
+    b = torch.randn(e, n, k, generator=g).to(FP8)
+    b_s = torch.rand(e, n // 128, k // 128, generator=g) * 0.01 + 0.01
+    a, a_s, b, b_s = (t.to(DEV) for t in (a, a_s, b, b_s))
+    ends = torch.tensor(counts, dtype=torch.int64).cumsum(0)
+    starts = (ends - torch.tensor(counts)).to(DEV)
+    order = torch.randperm(rows, generator=g).to(DEV)
+    weights = (torch.rand(rows, generator=g) + 0.5).to(DEV)
+    out = []
+    for tile_rows in (128, 256):
+        mt = ops.max_tiles_for(rows, e, tile_rows)
+        tiles = ops.build_tiles(starts, ends.to(DEV), 0, e, mt, tile_rows)
+        if epilogue == "swiglu":
+            c, s = torch.zeros(rows, n // 2, device=DEV).to(FP8), torch.zeros(rows, n // 256, device=DEV)
+            ops.grouped_gemm(a, a_s, b, b_s, tiles, mt, _C.EPI_SWIGLU_QUANT, c, q_scale=s, round_dtype=dtype, tile_rows=tile_rows)
+            out.append((c.view(torch.uint8), s))
+        else:
+            c = torch.zeros(rows, n, dtype=dtype, device=DEV)
+            extra = {"sorted_idx": order, "weights": weights} if epilogue == "scatter" else {}
+            ops.grouped_gemm(a, a_s, b, b_s, tiles, mt, _C.EPI_SCATTER_WEIGHT if extra else _C.EPI_STORE, c,
+                             tile_rows=tile_rows, **extra)
+            out.append((c,))
+    _status_ok()
+    assert all(torch.equal(x, y) for x, y in zip(*out)) and bool(out[0][0].any())
+
+
+def test_decode_step_of_few_rows_per_expert():
+    """128 tokens over 256 experts, skewed: the direct step's GEMMs exchange the operands, those on the masked layout, which a
+    replaced step leads to, do not.  Same bits."""
+    from dlblas_b200.layers.moe.ep_moe import FusedMoELowLatency
+    x, logits, *weights = (t.to(DEV) for t in O.make_layer_inputs(128, 512, 256, 256, seed=12))
+    g = torch.Generator().manual_seed(12)
+    p = torch.arange(1, 257).float().pow(-1.2)
+    ids = torch.stack([torch.multinomial(p, 8, generator=g) for _ in range(128)]).to(DEV)
+    w = torch.rand(128, 8, generator=g).to(DEV)
+    layer = FusedMoELowLatency(1, None, 256, 512, 0)
+    out = layer.forward(x, w, ids, *weights)
+    layer.token_dispatcher.dispatch = layer.token_dispatcher.dispatch
+    ref = layer.forward(x, w, ids, *weights)
+    _status_ok()
+    assert torch.equal(out, ref) and bool(out.any())
