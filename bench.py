@@ -701,7 +701,7 @@ def run_profile_bandwidth(args):
 
     add("grouped_topk (8192 x 256 fp32 logits -> ids, weights)", lambda: ops.route_grouped_topk(
         logits, bias, TOPK, True, GROUPS, TOPK_GROUP), 4.0 * t * E + 8.0 * t * TOPK)
-    add("sort_by_expert (73 728 slots, 257 experts; 4 kernels)", lambda: ops.sort_by_expert(
+    add("sort_by_expert (73 728 slots, 257 experts; 2 kernels)", lambda: ops.sort_by_expert(
         ids9, E + 1, want_pos=True), 8.0 * s_rows * 2 + 12.0 * s_rows + 16.0 * (E + 1))
     add("quant_fp8, fan-out 9 (x bf16 -> a1 e4m3 + scales in expert order)", lambda: ops.quant_fp8(
         x, 128, _C.QUANT_RECIP_MUL, 0.0, False, pos, k, s_rows), 2.0 * t * H + k * t * H * (1 + 4 / 128))
