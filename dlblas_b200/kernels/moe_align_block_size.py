@@ -4,8 +4,8 @@ dlblas/kernels/moe_align_block_size.py:138-210).
 Every expert's slots are laid out contiguously and padded to a multiple of `block_size`:
 sorted_ids int32 [max padded] holds flat slot indices (t * top_k + j) grouped by expert in ascending slot
 order, padding entries = topk_ids.numel(); expert_ids int32 [blocks] = expert of every block (0 for blocks
-past the end); num_tokens_post_pad int32 [1].  The library's stable sort writes the layout itself (one or two kernels, no
-host round trip).
+past the end); num_tokens_post_pad int32 [1].  The library's stable sort writes the layout itself (one kernel up to 4096 slots,
+two up to 327680, three beyond; no host round trip).  Without slots everything is padding: zeros.
 """
 from typing import Optional, Tuple
 
