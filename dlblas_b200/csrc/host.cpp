@@ -250,21 +250,30 @@ Tensor status_word(at::DeviceIndex index) {
 }
 int32_t* status_ptr(const Call& c) { return status_word(c.device.index()).data_ptr<int32_t>(); }
 
-// A whole number from the environment; text that is none is an error, as Python's int() makes it.
-int env_int(const char* name, int fallback) {
-  const char* v = std::getenv(name);
-  if (v == nullptr) return fallback;
-  char* end = nullptr;
-  errno = 0;
-  const long n = std::strtol(v, &end, 10);
-  while (end != v && std::isspace((unsigned char)*end)) ++end;
-  if (end == v || *end != 0 || errno != 0 || n < INT_MIN || n > INT_MAX)
-    throw BadValue(std::string(name) + " must be a whole number, got '" + v + "'");
-  return (int)n;
-}
-int tile_rows_env(const char* name, int fallback) {
-  const int rows = env_int(name, fallback);
-  if (rows != 128 && rows != 256) throw AssertionFailed(std::string(name) + " must be 128 or 256");
+// A setting from the environment.  The text is read with the GIL held, which os.environ's writers hold too, and understood
+// where it is wanted.
+struct Setting {
+  const char* name;
+  std::optional<std::string> text;
+  explicit Setting(const char* n) : name(n) {
+    if (const char* v = std::getenv(n)) text = v;
+  }
+  // a whole number; text that is none is an error, as Python's int() makes it
+  int value(int fallback) const {
+    if (!text) return fallback;
+    const char* v = text->c_str();
+    char* end = nullptr;
+    errno = 0;
+    const long n = std::strtol(v, &end, 10);
+    while (end != v && std::isspace((unsigned char)*end)) ++end;
+    if (end == v || *end != 0 || errno != 0 || n < INT_MIN || n > INT_MAX)
+      throw BadValue(std::string(name) + " must be a whole number, got '" + *text + "'");
+    return (int)n;
+  }
+};
+int tile_rows_of(const Setting& setting, int fallback) {
+  const int rows = setting.value(fallback);
+  if (rows != 128 && rows != 256) throw AssertionFailed(std::string(setting.name) + " must be 128 or 256");
   return rows;
 }
 
@@ -332,9 +341,9 @@ PyObject* py_group_quant_fp8(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 Tensor fp8_gemm(const Tensor& a, const Tensor& b, const Tensor& a_s, const Tensor& b_s, at::ScalarType out_dtype,
-                int tile_rows) {
+                int tile_rows, const Setting& fp8_tile_rows) {
   for (const Tensor* t : {&a, &b, &a_s, &b_s}) require_cuda(*t);
-  if (tile_rows < 0) tile_rows = env_int("DLBLAS_FP8_TILE_ROWS", 0);
+  if (tile_rows < 0) tile_rows = fp8_tile_rows.value(0);
   if (out_dtype == at::kFloat) tile_rows = 128;
   require(a.is_contiguous() && b.is_contiguous(), "Input tensors must be contiguous");
   require(a_s.is_contiguous() && b_s.is_contiguous(), "Scaling factor tensors must be contiguous");
@@ -362,7 +371,8 @@ PyObject* py_fp8_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor &x = tensor(a[0]), &w = tensor(a[1]), &x_s = tensor(a[2]), &w_s = tensor(a[3]);
     const at::ScalarType out = dtype(a[4]);
     const int64_t tile_rows = integer(a[5]);
-    return wrap(without_gil([&] { return fp8_gemm(x, w, x_s, w_s, out, (int)tile_rows); }));
+    const Setting fp8_tile_rows("DLBLAS_FP8_TILE_ROWS");
+    return wrap(without_gil([&] { return fp8_gemm(x, w, x_s, w_s, out, (int)tile_rows, fp8_tile_rows); }));
   });
 }
 
@@ -430,6 +440,7 @@ struct MoeArgs {
   int64_t expert_offset, num_experts;
   int quant_mode;
   bool skip_unrouted, renormalize, fuse_swiglu;
+  Setting fp8_tile_rows{"DLBLAS_FP8_TILE_ROWS"};
 };
 
 Tensor moe_forward(const MoeArgs& g) {
@@ -458,7 +469,7 @@ Tensor moe_forward(const MoeArgs& g) {
     weights = weights.to(at::kFloat);
   }
   if (!weights.is_contiguous()) weights = weights.contiguous();
-  int tile_rows = env_int("DLBLAS_FP8_TILE_ROWS", 0);
+  int tile_rows = g.fp8_tile_rows.value(0);
   if (tile_rows == 0 || g.out_dtype == at::kFloat) tile_rows = 128;
   require(tile_rows == 128 || tile_rows == 256, "DLBLAS_FP8_TILE_ROWS must be 0, 128 or 256");
   const bool fused = g.fuse_swiglu && n % 256 == 0;
@@ -527,7 +538,8 @@ PyObject* py_moe_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // rows that exist: with a single rank the exchange is a permutation, so the rows go straight into expert order instead of a
 // [experts, max tokens, hidden] layout, and the layer is six launches of which two stream the weights.
 Tensor low_latency_forward(const Tensor& x, const Tensor& topk_weights, const Tensor& topk_ids, const Tensor& w1,
-                           const Tensor& w1_s, const Tensor& w2, const Tensor& w2_s, at::ScalarType out_dtype) {
+                           const Tensor& w1_s, const Tensor& w2, const Tensor& w2_s, at::ScalarType out_dtype,
+                           const Setting& sm_margin) {
   require_cuda({&x, &w1, &w1_s, &w2, &w2_s, &topk_weights, &topk_ids});
   require(topk_weights.scalar_type() == at::kFloat, "topk_weights must be fp32");
   require(w1.dim() == 3, "w1 must be [experts, 2 * intermediate, hidden]");
@@ -559,7 +571,7 @@ Tensor low_latency_forward(const Tensor& x, const Tensor& topk_weights, const Te
   check(abi.dlb_quant_fp8(x.data_ptr(), code(x.scalar_type()), m, h, x.stride(0), 128, DLB_QUANT_DIV_EPS, 1e-10f,
                           ws.at<void>(o_a), ws.at<float>(o_as), h / 128, 1, pos, (int)top_k, c.stream));
   // SMs left to kernels of other streams (a shared expert's small GEMMs): the weights stream at the memory rate from fewer
-  const int margin = env_int("DLBLAS_DECODE_SM_MARGIN", 0);
+  const int margin = sm_margin.value(0);
   auto gemm = [&](size_t a, size_t a_s, int64_t nn, int64_t kk, const Tensor& b, const Tensor& b_s, size_t dst) {
     check(abi.dlb_moe_grouped_gemm_window(ws.at<void>(a), ws.at<float>(a_s), slots, b.data_ptr(), b_s.data_ptr<float>(),
                                           (int)e, nn, kk, tiles, max_tiles, 128, DLB_EPI_STORE, ws.at<void>(dst),
@@ -581,15 +593,19 @@ PyObject* py_low_latency_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor &x = tensor(a[0]), &weights = tensor(a[1]), &ids = tensor(a[2]), &w1 = tensor(a[3]), &w1_s = tensor(a[4]),
                  &w2 = tensor(a[5]), &w2_s = tensor(a[6]);
     const at::ScalarType out = dtype(a[7]);
-    return wrap(without_gil([&] { return low_latency_forward(x, weights, ids, w1, w1_s, w2, w2_s, out); }));
+    const Setting sm_margin("DLBLAS_DECODE_SM_MARGIN");
+    return wrap(without_gil([&] { return low_latency_forward(x, weights, ids, w1, w1_s, w2, w2_s, out, sm_margin); }));
   });
 }
 
 // ---- 16-bit grouped GEMMs and the unquantised expert layer --------------------------------------------------------
 // pairs of CTAs on 256-row tiles when the groups are large enough to fill them (decided from the shapes, no look at the
 // group sizes on the host); DLBLAS_GEMM16_TILE_ROWS = 128 / 256 overrides
-int gemm16_tile_rows(int64_t rows, int64_t groups) {
-  return tile_rows_env("DLBLAS_GEMM16_TILE_ROWS", rows >= 512 * groups ? 256 : 128);
+struct Gemm16Rows : Setting {
+  Gemm16Rows() : Setting("DLBLAS_GEMM16_TILE_ROWS") {}
+};
+int gemm16_tile_rows(const Gemm16Rows& setting, int64_t rows, int64_t groups) {
+  return tile_rows_of(setting, rows >= 512 * groups ? 256 : 128);
 }
 
 Tensor group_sizes(const Tensor& sizes) {
@@ -597,7 +613,7 @@ Tensor group_sizes(const Tensor& sizes) {
   return s.is_contiguous() ? s : s.contiguous();
 }
 
-Tensor m_grouped_gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& sizes_in, bool trans_b) {
+Tensor m_grouped_gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& sizes_in, bool trans_b, const Gemm16Rows& setting) {
   require(a_in.dim() == 2, "A must be 2-D");
   require(b_in.dim() == 3, "B must be 3-D");
   for (const Tensor* t : {&a_in, &b_in, &sizes_in}) require_cuda(*t);
@@ -617,7 +633,7 @@ Tensor m_grouped_gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& size
   Tensor out = empty({m, n}, a.scalar_type(), c);
   if (m == 0) return out;
   const Tensor sizes = group_sizes(sizes_in);
-  const int tile_rows = gemm16_tile_rows(m, groups);
+  const int tile_rows = gemm16_tile_rows(setting, m, groups);
   const int max_tiles = (int)(m / tile_rows + groups);
   Workspace ws;
   ws.take((size_t)(max_tiles + 1) * 16);
@@ -636,11 +652,12 @@ PyObject* py_m_grouped_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     need_args(n, 4);
     const Tensor &x = tensor(a[0]), &w = tensor(a[1]), &sizes = tensor(a[2]);
     const bool trans_b = truth(a[3]);
-    return wrap(without_gil([&] { return m_grouped_gemm(x, w, sizes, trans_b); }));
+    const Gemm16Rows setting;
+    return wrap(without_gil([&] { return m_grouped_gemm(x, w, sizes, trans_b, setting); }));
   });
 }
 
-Tensor k_grouped_gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& sizes_in) {
+Tensor k_grouped_gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& sizes_in, const Gemm16Rows& setting) {
   require(a_in.dim() == 2, "A must be 2-D");
   require(b_in.dim() == 2, "B must be 2-D");
   for (const Tensor* t : {&a_in, &b_in, &sizes_in}) require_cuda(*t);
@@ -657,7 +674,7 @@ Tensor k_grouped_gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& size
   Tensor sizes = group_sizes(sizes_in);
   if (sizes.scalar_type() != at::kLong) sizes = sizes.to(at::kLong);
   // pairs of CTAs on 256-row tiles of C unless M is smaller than one; DLBLAS_GEMM16_TILE_ROWS = 128 / 256 overrides
-  const int tile_rows = tile_rows_env("DLBLAS_GEMM16_TILE_ROWS", m >= 256 ? 256 : 128);
+  const int tile_rows = tile_rows_of(setting, m >= 256 ? 256 : 128);
   const int64_t need = abi.dlb_k_grouped_gemm_workspace_bytes(k, m, n, (int)groups, tile_rows);
   require(need > 0, "k_grouped_gemm: bad sizes");
   const Tensor work = empty({need}, at::kByte, c);
@@ -670,13 +687,14 @@ PyObject* py_k_grouped_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     need_args(n, 3);
     const Tensor &x = tensor(a[0]), &y = tensor(a[1]), &sizes = tensor(a[2]);
-    return wrap(without_gil([&] { return k_grouped_gemm(x, y, sizes); }));
+    const Gemm16Rows setting;
+    return wrap(without_gil([&] { return k_grouped_gemm(x, y, sizes, setting); }));
   });
 }
 
 // rows copied into expert order -> w1 GEMM -> silu(gate) * up -> w2 GEMM -> fp32 weighted sum over the slots
 Tensor moe_forward_16bit(const Tensor& x, const Tensor& w1_in, const Tensor& w2_in, const Tensor& weights_in,
-                         const Tensor& ids_in) {
+                         const Tensor& ids_in, const Gemm16Rows& setting) {
   require(x.scalar_type() == at::kBFloat16 || x.scalar_type() == at::kHalf,
           "the unquantised mode takes bf16 or fp16 activations");
   require(w1_in.scalar_type() == x.scalar_type() && w2_in.scalar_type() == x.scalar_type(),
@@ -697,7 +715,7 @@ Tensor moe_forward_16bit(const Tensor& x, const Tensor& w1_in, const Tensor& w2_
   const Tensor w1 = w1_in.is_contiguous() ? w1_in : w1_in.contiguous(), w2 = w2_in.is_contiguous() ? w2_in : w2_in.contiguous();
   Tensor weights = weights_in.scalar_type() == at::kFloat ? weights_in : weights_in.to(at::kFloat);
   if (!weights.is_contiguous()) weights = weights.contiguous();
-  const int tile_rows = gemm16_tile_rows(slots, e), max_tiles = (int)(slots / tile_rows + e), dt = code(x.scalar_type());
+  const int tile_rows = gemm16_tile_rows(setting, slots, e), max_tiles = (int)(slots / tile_rows + e), dt = code(x.scalar_type());
   const size_t sort_bytes = abi.dlb_sort_by_expert_workspace_size(slots, (int)e);
   Workspace ws;
   const size_t o_pos = ws.take(slots * 4), o_tiles = ws.take((max_tiles + 1) * 16), o_sort = ws.take(sort_bytes),
@@ -723,7 +741,8 @@ PyObject* py_moe_forward_16bit(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
     need_args(n, 5);
     const Tensor &x = tensor(a[0]), &w1 = tensor(a[1]), &w2 = tensor(a[2]), &weights = tensor(a[3]), &ids = tensor(a[4]);
-    return wrap(without_gil([&] { return moe_forward_16bit(x, w1, w2, weights, ids); }));
+    const Gemm16Rows setting;
+    return wrap(without_gil([&] { return moe_forward_16bit(x, w1, w2, weights, ids, setting); }));
   });
 }
 
