@@ -340,3 +340,41 @@ def test_other_threads_run_while_a_launch_waits():
     if queued < 0.3:
         pytest.skip("the queue took all launches")
     assert max(gaps) < 0.5 * queued, (max(gaps), queued)
+
+
+@pytest.mark.gpu
+def test_threads_on_their_own_streams():
+    """Four threads at once, each with its own sizes and stream: the results of one thread alone."""
+    import threading
+
+    from dlblas_b200.kernels.permute import permute, unpermute
+    from dlblas_b200.layers.moe.ep_moe import DlblasTritonFusedMoEBlockedF8Impl
+    layer = DlblasTritonFusedMoEBlockedF8Impl(top_k=2, num_experts=8, renormalize=True, out_dtype=torch.bfloat16)
+    jobs, results = [], {}
+    for i, tokens in enumerate((3, 70, 500, 2100)):
+        x, logits, *weights = (t.to(DEV) for t in O.make_layer_inputs(tokens, 256, 256, 8, seed=i))
+        w, ids = (t.to(DEV) for t in O.softmax_topk(logits.cpu(), 2, False))
+        jobs.append((x, w, ids, weights))
+    torch.cuda.synchronize()
+
+    def run(i):
+        x, w, ids, weights = jobs[i]
+        a = x.detach().requires_grad_(True)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(20):
+                a.grad = None
+                rows, rmap = permute(a, ids)
+                y = unpermute(rows, rmap, w)
+                y.backward(x)
+                out = layer.forward(x, w, ids, *weights)
+            torch.cuda.current_stream().synchronize()
+        return out, y.detach(), rmap, a.grad
+
+    alone = [run(i) for i in range(4)]
+    threads = [threading.Thread(target=lambda i=i: results.__setitem__(i, run(i))) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for i in range(4):
+        assert all(torch.equal(p, q) for p, q in zip(alone[i], results[i])), i
