@@ -55,8 +55,8 @@ constexpr int TMEM_COLS = 512;
 // tensor core's tile are columns of C, its columns the rows of A, 16 at a time.  A tile with a handful of rows otherwise
 // multiplies and promotes 128 all the same; the weights' way from DRAM bounds such a launch, and in repeated passes that
 // work costs the clocks and with them the memory rate.  (Up to 64 rows per tile this way: 2 % slower on those steps.)
-// Registers: the promotion warps hold both forms, and spill 132 bytes of stores and 204 of loads in the scatter epilogue, 44 / 116
-// in the plain one and 40 / 96 in the fused one, where the kernel without the exchanged form spills 0, 0 and 24 / 68 (ptxas).
+// Registers: the promotion warps hold both forms, and spill 36 bytes of stores and 104 of loads in the scatter epilogue, 28 / 92 in
+// the plain and the fused one, where the kernel without the exchanged form spills 0, 0 and 28 / 80 (ptxas).
 constexpr int SWAP_ROWS = 32;
 constexpr int CHUNK = 16;                    // rows of A per box and per step of N
 constexpr int CHUNKS = SWAP_ROWS / CHUNK;
@@ -96,7 +96,7 @@ template <int BN, int CTAS = 1> struct Cfg {
   static constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
   static constexpr int STAGES = (BN == 256) ? (CTAS == 2 ? 4 : 3) : (BN == 128 ? 5 : 8);
   static constexpr int TMEM_BUFS = TMEM_COLS / BN;
-  static constexpr int SEG = BN / 4;  // columns per thread segment (two segments per thread)
+  static constexpr int COLS = BN / 2;  // columns per promotion thread: the first warpgroup has the first half
   // Staging tile of the epilogue: BM rows of BN 16-bit values.  Rows are padded by 16 bytes so
   // that the 16-byte stores of 32 threads holding 32 different rows spread over all banks.
   static constexpr int STAGING_ROW_BYTES = BN * 2 + 16;
@@ -338,7 +338,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   } else if (warp == MMA_WARP) {
     {
       constexpr uint32_t idesc = make_idesc(BN, CTAS);
-      uint32_t it = 0;
+      uint32_t s = 0, s_phase = 0, b = 0, b_phase = 1;   // stage and accumulator of the next K block
+      bool ready = false;                                // both are known to be there
       bool ok = true;
       for (int t = worker; t < total_tiles && ok && rank == 0; t += workers) {
         uint32_t idesc_swap = 0;
@@ -346,11 +347,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           const Tile ti = decode_tile<BN, MODE, CTAS>(g, num_m_tiles, t, (int)rank);
           if (swapped(ti)) idesc_swap = make_idesc(CHUNK * chunks_of(ti));
         }
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
-          const int s = it % C::STAGES;
-          const int b = it % C::TMEM_BUFS;
-          if (!mbar_wait(full_bar(s), (it / C::STAGES) & 1u, abort_flag, limit) ||
-              !mbar_wait(tempty_bar(b), ((it / C::TMEM_BUFS) & 1u) ^ 1u, abort_flag, limit)) {
+        for (int kb = 0; kb < kblocks; ++kb) {
+          if (!ready && (!mbar_wait(full_bar(s), s_phase, abort_flag, limit) ||
+                         !mbar_wait(tempty_bar(b), b_phase, abort_flag, limit))) {
             ok = false;
             break;
           }
@@ -358,36 +357,47 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           const uint32_t a_addr = smem_base + s * C::STAGE_BYTES;
           const uint64_t a_desc = make_smem_desc(a_addr);
           const uint64_t b_desc = make_smem_desc(a_addr + A_STAGE_BYTES);
-          const uint32_t d_tmem = tmem_base + (uint32_t)(b * BN);
-          if constexpr (PAIR) {
-            if (elect_one()) {
+          const uint32_t d_tmem = tmem_base + b * BN;
+          const uint32_t done_stage = empty_bar(s), done_acc = tfull_bar(b);
+          if (++s == C::STAGES) { s = 0; s_phase ^= 1u; }
+          if (++b == C::TMEM_BUFS) { b = 0; b_phase ^= 1u; }
+          // +32 bytes along K inside the 128 B swizzle row == +2 in the (addr >> 4) field
+          auto mma = [&](int kk) {
+            if constexpr (PAIR) tc_mma_f8_pair(d_tmem, a_desc + 2u * kk, b_desc + 2u * kk, idesc, kk > 0 ? 1u : 0u);
+            else tc_mma_f8(d_tmem, a_desc + 2u * kk, b_desc + 2u * kk, idesc, kk > 0 ? 1u : 0u);
+          };
+          const bool swap = SWAP && idesc_swap != 0;
+          if (elect_one()) {
+            if (swap) {
 #pragma unroll
               for (int kk = 0; kk < BK / 32; ++kk)
-                tc_mma_f8_pair(d_tmem, a_desc + 2u * kk, b_desc + 2u * kk, idesc, kk > 0 ? 1u : 0u);
-              tc_commit_pair(empty_bar(s));   // both CTAs' stages
-              tc_commit_pair(tfull_bar(b));   // both CTAs' promotion warps
+                tc_mma_f8(d_tmem, b_desc + 2u * kk, a_desc + 2u * kk, idesc_swap, kk > 0 ? 1u : 0u);
+            } else {
+              mma(0);
+              mma(1);
             }
-          } else {
-            if (SWAP && idesc_swap != 0) {
-              if (elect_one()) {
-                const uint64_t b2_desc = make_smem_desc(a_addr + A_STAGE_BYTES + BM * BK);
+          }
+          __syncwarp();
+          // The tensor core's queue holds two to three instructions: the next K block's barriers are asked about while
+          // those of this one are in it.  Asked after the last, the answers left the pipe idle for some 300 cycles a block.
+          ready = mbar_test(full_bar(s), s_phase);
+          ready = mbar_test(tempty_bar(b), b_phase) && ready;
+          if (elect_one()) {
+            if (swap) {
+              const uint64_t b2_desc = make_smem_desc(a_addr + A_STAGE_BYTES + BM * BK);
 #pragma unroll
-                for (int kk = 0; kk < BK / 32; ++kk)
-                  tc_mma_f8(d_tmem, b_desc + 2u * kk, a_desc + 2u * kk, idesc_swap, kk > 0 ? 1u : 0u);
-#pragma unroll
-                for (int kk = 0; kk < BK / 32; ++kk)
-                  tc_mma_f8(d_tmem + BM, b2_desc + 2u * kk, a_desc + 2u * kk, idesc_swap, kk > 0 ? 1u : 0u);
-                tc_commit(empty_bar(s));
-                tc_commit(tfull_bar(b));
-              }
-            } else if (elect_one()) {
-#pragma unroll
-              for (int kk = 0; kk < BK / 32; ++kk) {
-                // +32 bytes along K inside the 128 B swizzle row == +2 in the (addr >> 4) field
-                tc_mma_f8(d_tmem, a_desc + 2u * kk, b_desc + 2u * kk, idesc, kk > 0 ? 1u : 0u);
-              }
-              tc_commit(empty_bar(s));   // smem stage reusable once these MMAs retire
-              tc_commit(tfull_bar(b));   // accumulator ready for the promotion warps
+              for (int kk = 0; kk < BK / 32; ++kk)
+                tc_mma_f8(d_tmem + BM, b2_desc + 2u * kk, a_desc + 2u * kk, idesc_swap, kk > 0 ? 1u : 0u);
+            } else {
+              mma(2);
+              mma(3);
+            }
+            if constexpr (PAIR) {
+              tc_commit_pair(done_stage);   // both CTAs' stages
+              tc_commit_pair(done_acc);     // both CTAs' promotion warps
+            } else {
+              tc_commit(done_stage);   // smem stage reusable once these MMAs retire
+              tc_commit(done_acc);     // accumulator ready for the promotion warps
             }
           }
           __syncwarp();
@@ -494,16 +504,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     const int wg = warp >> 2;                 // 0 or 1
     const int quad = warp & 3;                // TMEM lane quadrant of this warp
     const int r = quad * 32 + lane;           // row inside the tile
-    constexpr int SEG = C::SEG;
-    // TMEM column offsets of this thread's two segments, and matching output columns
-    int seg_col[2];
-    if constexpr (MODE == DLB_EPI_SWIGLU_QUANT) {
-      seg_col[0] = wg * SEG;                  // gate columns
-      seg_col[1] = BN / 2 + wg * SEG;         // up columns
-    } else {
-      seg_col[0] = wg * 2 * SEG;
-      seg_col[1] = wg * 2 * SEG + SEG;
-    }
+    constexpr int COLS = C::COLS;
+    const int col0 = wg * COLS;               // this thread's columns of the tile (SWIGLU: gate | up)
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
     uint32_t it = 0;
     uint32_t tile_no = 0;
@@ -515,23 +517,12 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       // threads without a row read the scales of a row that exists (a pair's second CTA can hold an empty
       // half tile whose first row lies beyond the end of A)
       const float* as_ptr = g.a_s + (row_ok ? p : (long long)min(ti.row0, g.m - 1)) * g.a_s_rs;
-      // scale blocks of the two segments
-      const float* bs_ptr[2];
+      // scale block of this thread's columns
+      const float* bs_ptr;
       {
-        const float* be = g.b_s + (long long)ti.e * g.b_s_es;
-        int nb0, nb1;
-        if constexpr (MODE == DLB_EPI_SWIGLU_QUANT) {
-          nb0 = ti.n0 / 128;
-          nb1 = (g.n_half + ti.n0) / 128;
-        } else {
-          nb0 = (ti.n0 + seg_col[0]) / 128;
-          nb1 = (ti.n0 + seg_col[1]) / 128;
-          const int nb_max = (g.n + 127) / 128 - 1;
-          nb0 = min(nb0, nb_max);
-          nb1 = min(nb1, nb_max);
-        }
-        bs_ptr[0] = be + (long long)nb0 * kblocks;
-        bs_ptr[1] = be + (long long)nb1 * kblocks;
+        const int nb = MODE == DLB_EPI_SWIGLU_QUANT ? (wg * g.n_half + ti.n0) / 128
+                                                    : min((ti.n0 + col0) / 128, (g.n + 127) / 128 - 1);
+        bs_ptr = g.b_s + (long long)ti.e * g.b_s_es + (long long)nb * kblocks;
       }
       if constexpr (SWAP) {
         if (swapped(ti)) {
@@ -539,7 +530,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           // Lanes 0-15 (and 16-31 again) fetch the scales of a chunk's 16 rows, two K blocks ahead.  The products and their
           // order are those of the other form.
           const int chunks = chunks_of(ti);
-          const float* bs = bs_ptr[MODE == DLB_EPI_SWIGLU_QUANT ? wg : 0];
+          const float* bs = bs_ptr;
           const float* as = g.a_s + (long long)min(ti.row0, g.m - 1) * g.a_s_rs;
           int a_off[CHUNKS];                       // less than SWAP_ROWS rows' worth of scales
           float a0[CHUNKS], a1[CHUNKS], a2[CHUNKS];
@@ -633,9 +624,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           continue;
         }
       }
-      uint64_t acc2[SEG];                 // 2 * SEG fp32 accumulators, packed in pairs
+      uint64_t acc2[COLS / 2];            // COLS fp32 accumulators, packed in pairs
 #pragma unroll
-      for (int j = 0; j < SEG; ++j) acc2[j] = 0ull;
+      for (int j = 0; j < COLS / 2; ++j) acc2[j] = 0ull;
       // row / weight of the scatter epilogue, fetched now so that the two dependent loads are
       // long done when the tile's last K block arrives
       long long crow = p;
@@ -649,30 +640,27 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 
       // scales are fetched two K blocks ahead: under full TMA load an L2 round trip can take
       // longer than one K block
-      float a_sc = __ldg(as_ptr), b_sc0 = __ldg(bs_ptr[0]), b_sc1 = __ldg(bs_ptr[1]);
-      float a_n1 = 0.f, b0_n1 = 0.f, b1_n1 = 0.f;
+      float a_sc = __ldg(as_ptr), b_sc = __ldg(bs_ptr);
+      float a_n1 = 0.f, b_n1 = 0.f;
       if (kblocks > 1) {
         a_n1 = __ldg(as_ptr + g.a_s_ks);
-        b0_n1 = __ldg(bs_ptr[0] + 1);
-        b1_n1 = __ldg(bs_ptr[1] + 1);
+        b_n1 = __ldg(bs_ptr + 1);
       }
-      // Two 32-column staging buffers.  A K block is drained in NB batches of two loads; the
-      // loads of the next batch (or of the next K block's first batch) are issued as soon as a
-      // staging buffer has been folded into the accumulators, so a load is always in flight.
-      constexpr int CH = 2 * SEG / 32;   // 32-column chunks per thread and K block (1, 2 or 4)
-      constexpr int NB = (CH + 1) / 2;
-      constexpr bool TWO = CH > 1;       // one chunk (BN = 64): both segments lie in one scale block, s1 stays unused
-      auto chunk_col = [&](int c) { return (c * 32 < SEG) ? seg_col[0] + c * 32 : seg_col[1] + c * 32 - SEG; };
-      uint32_t s0[32], s1[32];
-      bool pending = false;              // first batch of the current K block already issued
+      // Two 32-column staging buffers: while one is folded into the accumulators, the load of the next 32 columns (or of
+      // the next K block's first 32) is in flight into the other.  This and the early questions for the barriers (here and
+      // in the MMA warp) took 8192 x 4096 x 7168 from 287 to 257 us in repeated passes at the power limit (1675 -> 1869
+      // TFLOP/s, 1600 -> 1480 MHz), 4096 x 7168 x 2048 from 84 to 76, 8192 x 24576 x 1536 from 405 to 369; the promotion
+      // warp's question alone is two thirds of that.
+      constexpr int CH = COLS / 32;      // 32-column chunks per thread and K block (1, 2 or 4)
+      uint32_t stage[2][32];
+      bool pending = false;              // first chunk of the current K block already issued
       for (int kb = 0; kb < kblocks && ok; ++kb, ++it) {
         const int b = it % C::TMEM_BUFS;
-        const uint32_t buf_addr = lane_addr + (uint32_t)(b * BN);
-        float a_n2 = 0.f, b0_n2 = 0.f, b1_n2 = 0.f;
+        const uint32_t buf_addr = lane_addr + (uint32_t)(b * BN + col0);
+        float a_n2 = 0.f, b_n2 = 0.f;
         if (kb + 2 < kblocks) {
           a_n2 = __ldg(as_ptr + (long long)(kb + 2) * g.a_s_ks);
-          b0_n2 = __ldg(bs_ptr[0] + kb + 2);
-          b1_n2 = __ldg(bs_ptr[1] + kb + 2);
+          b_n2 = __ldg(bs_ptr + kb + 2);
         }
         if (!pending) {
           if (!mbar_wait(tfull_bar(b), (it / C::TMEM_BUFS) & 1u, abort_flag, limit)) {
@@ -680,80 +668,60 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
             break;
           }
           tc_fence_after();
-          tmem_ld32(buf_addr + chunk_col(0), s0);
-          if constexpr (TWO) tmem_ld32(buf_addr + chunk_col(1), s1);
+          tmem_ld32(buf_addr, stage[0]);
         }
         pending = false;
-        const float sc0f = a_sc * b_sc0, sc1f = a_sc * b_sc1;
-        const uint64_t sc0 = pack2(sc0f, sc0f);
-        const uint64_t sc1 = pack2(sc1f, sc1f);
-        const bool has_next = kb + 1 < kblocks;
-        const int nb_buf = (it + 1) % C::TMEM_BUFS;
-        const uint32_t next_addr = lane_addr + (uint32_t)(nb_buf * BN);
+        const float scf = a_sc * b_sc;
+        const uint64_t sc = pack2(scf, scf);
+        const int nb = (it + 1) % C::TMEM_BUFS;
+        const uint32_t nb_phase = ((it + 1) / C::TMEM_BUFS) & 1u;
+        bool next_full = false;
 #pragma unroll
-        for (int q = 0; q < NB; ++q) {
-          if constexpr (TWO) tmem_ld_wait(s0, s1);
-          else tmem_ld_wait(s0);
-          const bool last = (q == NB - 1);
-          if (last) {
+        for (int q = 0; q < CH; ++q) {
+          tmem_ld_wait(stage[q & 1]);
+          if (q < CH - 1) {
+            tmem_ld32(buf_addr + (q + 1) * 32, stage[(q + 1) & 1]);
+            // the next K block's accumulator is asked about under the FMAs below
+            if (q == CH - 2) next_full = mbar_test(tfull_bar(nb), nb_phase);
+          } else {
             // every column of this accumulator is in registers: hand it back to the MMA warp
             tc_fence_before();
             __syncwarp();
             if (lane == 0) {
               if (rank == 0) mbar_arrive(tempty_bar(b));
-              else mbar_arrive_cluster(mapa(tempty_bar(b), 0));
+              else mbar_arrive_cluster_no_release(mapa(tempty_bar(b), 0));
+            }
+            if (CH > 1 && kb + 1 < kblocks) {
+              if (!next_full && !mbar_wait(tfull_bar(nb), nb_phase, abort_flag, limit)) {
+                ok = false;
+              } else {
+                tc_fence_after();
+                tmem_ld32(lane_addr + (uint32_t)(nb * BN + col0), stage[0]);
+                pending = true;
+              }
             }
           }
-          {
-            const uint64_t sc = ((2 * q) * 32 < SEG) ? sc0 : sc1;
 #pragma unroll
-            for (int j = 0; j < 16; ++j) fma2(acc2[(2 * q) * 16 + j], s0[2 * j], s0[2 * j + 1], sc);
-          }
-          if (!last) {
-            tmem_ld32(buf_addr + chunk_col(2 * q + 2), s0);
-          } else if (has_next) {
-            if (!mbar_wait(tfull_bar(nb_buf), ((it + 1) / C::TMEM_BUFS) & 1u, abort_flag, limit)) {
-              ok = false;
-            } else {
-              tc_fence_after();
-              tmem_ld32(next_addr + chunk_col(0), s0);
-              if constexpr (!TWO) pending = true;
-            }
-          }
-          if constexpr (TWO) {
-            const uint64_t sc = ((2 * q + 1) * 32 < SEG) ? sc0 : sc1;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) fma2(acc2[(2 * q + 1) * 16 + j], s1[2 * j], s1[2 * j + 1], sc);
-          }
-          if constexpr (TWO) {
-            if (!last) {
-              tmem_ld32(buf_addr + chunk_col(2 * q + 3), s1);
-            } else if (has_next && ok) {
-              tmem_ld32(next_addr + chunk_col(1), s1);
-              pending = true;
-            }
-          }
+          for (int j = 0; j < 16; ++j) fma2(acc2[q * 16 + j], stage[q & 1][2 * j], stage[q & 1][2 * j + 1], sc);
         }
         if (!ok) {
           tmem_ld_wait_plain();
           break;
         }
         a_sc = a_n1;
-        b_sc0 = b0_n1;
-        b_sc1 = b1_n1;
+        b_sc = b_n1;
         a_n1 = a_n2;
-        b0_n1 = b0_n2;
-        b1_n1 = b1_n2;
+        b_n1 = b_n2;
       }
       if (!ok) break;
 
       // ---- hand the tile over ------------------------------------------------
-      float acc[2 * SEG];
+      float acc[COLS];
 #pragma unroll
-      for (int j = 0; j < SEG; ++j) unpack2(acc2[j], acc[2 * j], acc[2 * j + 1]);
+      for (int j = 0; j < COLS / 2; ++j) unpack2(acc2[j], acc[2 * j], acc[2 * j + 1]);
       if constexpr (MODE == DLB_EPI_SCATTER_WEIGHT) {
 #pragma unroll
-        for (int j = 0; j < 2 * SEG; ++j) acc[j] *= row_w;
+        for (int j = 0; j < COLS; ++j) acc[j] *= row_w;
       }
       if constexpr (STAGED) {
         // the staging tile must have been emptied by the epilogue warps (previous tile)
@@ -761,20 +729,15 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           ok = false;
           break;
         }
-        uint8_t* srow = staging + r * C::STAGING_ROW_BYTES;
-        // byte offsets of this thread's two segments inside the staging row; the fused w13
-        // epilogue wants all gate columns first, then all up columns
-        const int off0 = (MODE == DLB_EPI_SWIGLU_QUANT) ? wg * SEG * 2 : seg_col[0] * 2;
-        const int off1 = (MODE == DLB_EPI_SWIGLU_QUANT) ? BN + wg * SEG * 2 : seg_col[1] * 2;
+        uint8_t* srow = staging + r * C::STAGING_ROW_BYTES + col0 * 2;
 #pragma unroll
-        for (int j = 0; j < 2 * SEG; j += 8) {
+        for (int j = 0; j < COLS; j += 8) {
           uint4 v;
           v.x = Pack<OutT>::two(acc[j], acc[j + 1]);
           v.y = Pack<OutT>::two(acc[j + 2], acc[j + 3]);
           v.z = Pack<OutT>::two(acc[j + 4], acc[j + 5]);
           v.w = Pack<OutT>::two(acc[j + 6], acc[j + 7]);
-          const int off = (j < SEG) ? off0 + j * 2 : off1 + (j - SEG) * 2;
-          *reinterpret_cast<uint4*>(srow + off) = v;
+          *reinterpret_cast<uint4*>(srow + j * 2) = v;
         }
         // the rows leave through the async proxy (bulk copies): order these writes before it
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -782,10 +745,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         if (lane == 0) mbar_arrive(staged_bar);
       } else {
         if (row_ok) {
-          const int col0 = ti.n0 + seg_col[0];
-          OutT* dst = reinterpret_cast<OutT*>(g.c) + crow * g.ldc + col0;
-          const int ncols = min(2 * SEG, g.n - col0);   // n % 8 == 0
-          store_row<OutT, 2 * SEG>(dst, acc, ncols);
+          OutT* dst = reinterpret_cast<OutT*>(g.c) + crow * g.ldc + ti.n0 + col0;
+          store_row<OutT, COLS>(dst, acc, min(COLS, g.n - ti.n0 - col0));   // n % 8 == 0
         }
       }
     }
@@ -870,12 +831,14 @@ int launch_typed(int bn, int ctas, bool swap, int c_dtype, const CUtensorMap& ma
   return fail(DLB_ERR_INVALID, "unsupported output dtype %d for this GEMM epilogue", c_dtype);
 }
 
-// Columns per tile: 256 feed the tensor cores best; 128 where those would leave SMs idle; 64 where they still make one wave.
-// Quantiser and GEMM of 100 rows, 128 -> 64 columns: 7168 x 2048 17.4 -> 16.4 us, 512 x 7168 30.7 -> 28.7, 7168 x 512
-// 13.3 -> 12.3; one row, 512 x 7168 28.7 -> 26.6.
+// Columns per tile: the narrowest that still makes one wave, else 256.  A K block of a wave takes about the same time on 64
+// and 128 columns and a third more on 256, so a second wave costs more than the wider tile.  Repeated GEMMs alone, one wave
+// of 256 against two of 128: 1000 x 4096 x 7168 37.8 / 48.5 us, 300 x 7168 x 2048 17.4 / 21.1;
+// one of 128 against one of 256: 128 x 12288 x 7168 31.0 / 39.4; one of 64 against one of 128: 64 x 7168 x 2048
+// 13.7 / 14.8; with more waves on either side 256 is never behind (1000 x 12288 x 7168, 2.6 against 5.2 waves, 104 / 136).
 int tile_width(long long m_tiles, int64_t n, int sms, int c_dtype) {
-  if (m_tiles * ceil_div(n, (int64_t)256) >= sms) return 256;
-  return c_dtype != DLB_F32 && m_tiles * ceil_div(n, (int64_t)64) <= sms ? 64 : 128;
+  if (c_dtype != DLB_F32 && m_tiles * ceil_div(n, (int64_t)64) <= sms) return 64;
+  return m_tiles * ceil_div(n, (int64_t)128) <= sms ? 128 : 256;
 }
 
 }  // namespace
@@ -902,9 +865,9 @@ extern "C" int dlb_fp8_gemm(const void* a, const void* b, const float* a_s, int6
   DLB_REQUIRE(tile_rows == 0 || tile_rows == 128 || tile_rows == 256, DLB_ERR_INVALID,
               "fp8_gemm: tile_rows must be 0 (choose), 128 or 256");
   const int sms = sm_count();
-  // Pairs of CTAs only on request: with one hand-shake per K block between the MMA warp of the leader and the
-  // promotion warps of both CTAs, the cluster-wide signalling doubles the K-block period (measured: 1.04 against
-  // 1.96 PFLOP/s on 8192 x 4096 x 7168), although the MMAs themselves get cheaper.
+  // Pairs of CTAs only on request: they move a third less through L2 and shared memory, but what bounds a K block is the
+  // hand-over between the MMA warp and the promotion warps, which crosses CTAs there: 8192 x 4096 x 7168 256 us against 257,
+  // 4096 x 7168 x 2048 78 against 76, 64 groups of about 256 rows 916 against 821 (tiles of 256 rows fill worse).
   const int ctas = tile_rows == 256 ? 2 : 1;
   const int m_tiles = (int)ceil_div(m, (int64_t)(ctas * BM));
   int bn = 256;

@@ -434,3 +434,23 @@ def test_decode_step_of_few_rows_per_expert():
     ref = layer.forward(x, w, ids, *weights)
     _status_ok()
     assert torch.equal(out, ref) and bool(out.any())
+
+
+@pytest.mark.parametrize("k", [128, 256, 384])
+@pytest.mark.parametrize("per_sm,extra", [(64, 0), (64, 8), (128, 0), (128, 8), (256, 0), (256, 8)])
+def test_fp8_gemm_where_the_tile_width_changes(per_sm, extra, k):
+    """One tile per SM of 64, 128 and 256 columns, and one tile more; one, two and three K blocks (the hand-over of the
+    accumulators starts and ends differently)."""
+    from dlblas_b200 import ops
+    m, n = 3, torch.cuda.get_device_properties(DEV).multi_processor_count * per_sm + extra
+    g = torch.Generator().manual_seed(per_sm + extra + k)
+    a, a_s = O.quant_fp8(torch.randn(m, k, generator=g).to(torch.bfloat16), 128)
+    b = torch.randn(n, k, generator=g).to(FP8)
+    b_s = torch.rand((n + 127) // 128, k // 128, generator=g) + 0.5
+    c = ops.fp8_gemm(a.to(DEV), b.to(DEV), a_s.to(DEV), b_s.to(DEV), torch.float32)
+    cb = ops.fp8_gemm(a.to(DEV), b.to(DEV), a_s.to(DEV), b_s.to(DEV), torch.bfloat16)
+    _status_ok()
+    ref = O.fp8_gemm(a, b, a_s, b_s, torch.float32)
+    assert O.rel_frobenius(c.cpu(), ref) < 1e-5
+    # the same products in the same order at every width: one rounding apart
+    assert torch.equal(cb, c.to(torch.bfloat16))
