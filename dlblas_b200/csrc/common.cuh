@@ -7,6 +7,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <utility>
+
 #include "../../include/dlblas_b200.h"
 
 namespace dlb {
@@ -36,6 +38,61 @@ bool withhold_loads();  // dlb_set_wait_policy(): the GEMMs' load role issues no
   do {                                               \
     if (!(cond)) return dlb::fail(code, __VA_ARGS__); \
   } while (0)
+
+// ---- launches that overlap ------------------------------------------------- //
+// Kernels of one operator follow one another on a stream, and most of them are short: from the end of one to the first
+// instructions of the next 1.5 to 2 us pass.  after_predecessor() launches a kernel while its predecessor in the stream is
+// still running (programmatic stream serialization); its blocks take up SMs as they become free, and
+// wait_for_predecessor(), the first thing that every thread does (after a set-up that touches no global memory), returns when
+// the predecessor has completed and its writes are visible.  Only then does a kernel let its own successor be launched, so
+// one that starts early knows that everything up to its predecessor's predecessor is complete.  After kernels that know
+// nothing of this (torch's, the peer-to-peer ones) the launch waits for their end as always.
+// Passes among others, before -> after: expert layer of 64 tokens (six kernels) 36.9 -> 22.8 us, quantiser and GEMM of 100
+// rows 16.4 -> 11.9, routing and aligned layout of 20000 tokens 45.1 -> 40.0, 16-bit expert layer of 500 tokens 203 -> 194,
+// decode step of 128 tokens and 256 experts 478 -> 465, permutation both ways 525 -> 515.
+// A kernel that runs for long and fills the SMs (the GEMMs) calls start_successor() when a block has nothing left but its
+// end: with the successor waiting in line from the start, they were 1 to 2 % slower and the short ones no faster.
+#ifdef __CUDACC__
+__device__ __forceinline__ void start_successor() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// The answer is always true.  The loads behind it hang on the branch, so that the compiler cannot move those it may take
+// for constant (ld.global.nc) in front of the wait.
+__device__ __forceinline__ bool wait_for_predecessor(bool then_start_successor = true) {
+  uint32_t done;
+  asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, 1;" : "=r"(done)::"memory");
+  if (then_start_successor) start_successor();
+  return done != 0;
+}
+template <typename... P> struct LaunchAfterPredecessor {
+  void (*kernel)(P...);
+  dim3 grid, block;
+  size_t smem;
+  cudaStream_t stream;
+  int cluster;
+  template <typename... A> cudaError_t operator()(A&&... args) const {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+  }
+};
+// after_predecessor(kernel, grid, block, shared memory, stream)(arguments); errors as after a <<<>>> launch
+template <typename... P>
+LaunchAfterPredecessor<P...> after_predecessor(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                                               cudaStream_t stream, int cluster = 1) {
+  return {kernel, grid, block, smem, stream, cluster};
+}
+#endif
 
 __host__ __device__ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 

@@ -206,12 +206,6 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
   const int worker = blockIdx.x / CTAS;                   // CTA or pair index
   const int workers = gridDim.x / CTAS;
   const int kblocks = (g.k_bytes + UMMA_BK_BYTES - 1) / UMMA_BK_BYTES;
-  const int num_m_tiles = g.tiles != nullptr ? __ldg(reinterpret_cast<const int*>(g.tiles)) : g.num_m_tiles_static;
-  const int total_tiles = num_m_tiles * g.num_n_tiles;
-  const int my_tiles = g.sched != nullptr ? __ldg(g.sched_count + worker)
-                                          : (worker < total_tiles ? (total_tiles - worker + workers - 1) / workers : 0);
-  const int* my_sched = g.sched != nullptr ? g.sched + (long long)worker * g.sched_stride : nullptr;
-  auto nth_tile = [&](int i) { return my_sched != nullptr ? __ldg(my_sched + i) : worker + i * workers; };
   const unsigned long long limit = g.timeout_cycles;
 
   if (threadIdx.x == 0) {
@@ -231,6 +225,10 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     abort_flag[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == PRODUCER_WARP && elect_one()) {
+    prefetch_map(&tmap_a);
+    prefetch_map(&tmap_b);
   }
   if (warp == MMA_WARP) {
     if constexpr (PAIR) {
@@ -252,6 +250,13 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
   if constexpr (PAIR) cluster_sync();   // both CTAs' barriers exist before anything remote touches them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  if (!wait_for_predecessor(false)) return;
+  const int num_m_tiles = g.tiles != nullptr ? __ldg(reinterpret_cast<const int*>(g.tiles)) : g.num_m_tiles_static;
+  const int total_tiles = num_m_tiles * g.num_n_tiles;
+  const int my_tiles = g.sched != nullptr ? __ldg(g.sched_count + worker)
+                                          : (worker < total_tiles ? (total_tiles - worker + workers - 1) / workers : 0);
+  const int* my_sched = g.sched != nullptr ? g.sched + (long long)worker * g.sched_stride : nullptr;
+  auto nth_tile = [&](int i) { return my_sched != nullptr ? __ldg(my_sched + i) : worker + i * workers; };
 
   if (warp == PRODUCER_WARP) {
     uint32_t it = 0;
@@ -518,6 +523,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     }
   }
 
+  start_successor();
   tc_fence_before();
   __syncthreads();
   if constexpr (PAIR) cluster_sync();   // no CTA leaves while its partner may still signal its barriers
@@ -545,25 +551,8 @@ int launch16(const CUtensorMap& ma, const CUtensorMap& mb, const Args16& g, int 
     if (rc != DLB_OK) return rc;
     configured[dev] = true;
   }
-  if constexpr (CTAS == 1) {
-    kern<<<grid, NUM_THREADS, SMEM_BYTES, st>>>(ma, mb, g);
-    DLB_CHECK_LAUNCH("gemm16_kernel");
-  } else {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(NUM_THREADS);
-    cfg.dynamicSmemBytes = SMEM_BYTES;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int rc = check_cuda(cudaLaunchKernelEx(&cfg, kern, ma, mb, g), "cudaLaunchKernelEx(gemm16_kernel, pairs)");
-    if (rc != DLB_OK) return rc;
-  }
+  after_predecessor(kern, grid, NUM_THREADS, SMEM_BYTES, st, CTAS)(ma, mb, g);
+  DLB_CHECK_LAUNCH("gemm16_kernel");
   count_launch();
   return DLB_OK;
 }
@@ -596,6 +585,7 @@ constexpr int KG_CHUNK = 1024;   // groups whose K ranges are worked out at a ti
 __global__ void __launch_bounds__(KG_MAX_WORKERS)
 k_group_plan_kernel(const long long* __restrict__ sizes, int groups, long long k_total, int tiles_per_group, int workers,
                     int4* __restrict__ kseg, int* __restrict__ sched, int sched_stride, int* __restrict__ sched_count) {
+  if (!wait_for_predecessor()) return;
   // per rank, double-buffered so that a group needs one barrier: when the worker becomes free, which one it is, and the
   // tiles it holds (a worker changes rank from group to group, its tile count travels with it)
   __shared__ long long free_at[2][KG_MAX_WORKERS];
@@ -822,7 +812,7 @@ extern "C" int dlb_k_grouped_gemm_16bit(const void* a, const void* b, int dtype,
   const int workers = (int)(all_tiles < max_workers ? all_tiles : max_workers);   // as run_gemm16 sizes its grid
   DLB_REQUIRE(workers <= KG_MAX_WORKERS, DLB_ERR_INVALID, "k_grouped_gemm_16bit: more than %d workers", KG_MAX_WORKERS);
   const int sched_stride = (int)(num_groups * (per_group / workers + 1));
-  k_group_plan_kernel<<<1, (workers + 31) / 32 * 32, 0, (cudaStream_t)stream>>>(
+  after_predecessor(k_group_plan_kernel, 1, (workers + 31) / 32 * 32, 0, (cudaStream_t)stream)(
       reinterpret_cast<const long long*>(group_sizes), num_groups, k_total, (int)per_group, workers, kseg, sched,
       sched_stride, sched_count);
   if ((rc = check_cuda(cudaGetLastError(), "k_group_plan_kernel")) != DLB_OK) return rc;

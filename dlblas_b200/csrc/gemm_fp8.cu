@@ -227,8 +227,6 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   const int worker = blockIdx.x / CTAS;                   // CTA or pair index
   const int workers = gridDim.x / CTAS;
   const int kblocks = g.k / BK;
-  const int num_m_tiles = g.tiles != nullptr ? __ldg(reinterpret_cast<const int*>(g.tiles)) : g.num_m_tiles_static;
-  const int total_tiles = num_m_tiles * g.num_n_tiles;
   const unsigned long long limit = g.timeout_cycles;
 
   if (threadIdx.x == 0) {
@@ -247,6 +245,11 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     abort_flag[1] = 0;   // private flag of the drain waits
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == PRODUCER_WARP && elect_one()) {
+    prefetch_map(&tmap_a);
+    prefetch_map(&tmap_b);
+    if constexpr (SWAP) prefetch_map(&tmap_a16);
   }
   if (warp == MMA_WARP) {
     if constexpr (PAIR) {
@@ -268,6 +271,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   if constexpr (PAIR) cluster_sync();   // both CTAs' barriers exist before anything remote touches them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  if (!wait_for_predecessor(false)) return;
+  const int num_m_tiles = g.tiles != nullptr ? __ldg(reinterpret_cast<const int*>(g.tiles)) : g.num_m_tiles_static;
+  const int total_tiles = num_m_tiles * g.num_n_tiles;
 
   if (warp >= EPI_WARPS) {
     // third warpgroup: give registers away, then run the producer / MMA roles
@@ -753,6 +759,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   }
 
   // ---- teardown ----------------------------------------------------------------
+  start_successor();
   tc_fence_before();
   __syncthreads();
   if constexpr (PAIR) cluster_sync();   // no CTA leaves while its partner may still signal its barriers
@@ -780,25 +787,8 @@ int launch_one(const CUtensorMap& ma, const CUtensorMap& ma16, const CUtensorMap
     if (rc != DLB_OK) return rc;
     configured[dev] = true;
   }
-  if constexpr (CTAS == 1) {
-    kern<<<grid, NUM_THREADS, SMEM, st>>>(ma, ma16, mb, g);
-    DLB_CHECK_LAUNCH("gemm_fp8_kernel");
-  } else {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(NUM_THREADS);
-    cfg.dynamicSmemBytes = SMEM;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int rc = check_cuda(cudaLaunchKernelEx(&cfg, kern, ma, ma16, mb, g), "cudaLaunchKernelEx(gemm_fp8_kernel, pairs)");
-    if (rc != DLB_OK) return rc;
-  }
+  after_predecessor(kern, grid, NUM_THREADS, SMEM, st, CTAS)(ma, ma16, mb, g);
+  DLB_CHECK_LAUNCH("gemm_fp8_kernel");
   count_launch();
   return DLB_OK;
 }

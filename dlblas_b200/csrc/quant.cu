@@ -124,6 +124,7 @@ __global__ void __launch_bounds__(THREADS) quant_fp8_kernel(const T* __restrict_
                                                             uint8_t* __restrict__ q, float* __restrict__ scales,
                                                             long long s_rs, long long s_gs,
                                                             const int* __restrict__ dst_pos, int fanout) {
+  if (!wait_for_predecessor()) return;
   const long long k = (long long)vec_per_row.d * 16;
   for (uint32_t u0 = blockIdx.x * THREADS; u0 < total; u0 += gridDim.x * THREADS) {
     const uint32_t u = u0 + threadIdx.x;
@@ -186,6 +187,7 @@ __global__ void __launch_bounds__(THREADS) permute_rows_kernel(const uint4* __re
                                                                const float* __restrict__ scales, uint32_t groups,
                                                                uint32_t total, const int* __restrict__ dst_pos, int fanout,
                                                                uint4* __restrict__ out_q, float* __restrict__ out_s) {
+  if (!wait_for_predecessor()) return;
   for (uint32_t u = blockIdx.x * THREADS + threadIdx.x; u < total; u += gridDim.x * THREADS) {
     const uint32_t row = vec_per_row.quot(u);
     const uint32_t c = u - row * vec_per_row.d;
@@ -217,6 +219,7 @@ template <typename T>
 __global__ void __launch_bounds__(THREADS) silu_and_mul_kernel(const T* __restrict__ in, uint32_t total,
                                                                FastDiv vec_per_row, long long ld_in,
                                                                T* __restrict__ out, long long ld_out) {
+  if (!wait_for_predecessor()) return;
   const long long n = (long long)vec_per_row.d * 8;
   for (uint32_t u = blockIdx.x * THREADS + threadIdx.x; u < total; u += gridDim.x * THREADS) {
     const uint32_t r = vec_per_row.quot(u);
@@ -242,6 +245,7 @@ __global__ void __launch_bounds__(THREADS) silu_mul_quant_kernel(const T* __rest
                                                                  const int* __restrict__ masked_m, int experts,
                                                                  long long rows_per_expert, uint8_t* __restrict__ q,
                                                                  float* __restrict__ scales) {
+  if (!wait_for_predecessor()) return;
   __shared__ int prefix[MASKED_MAX_EXPERTS + 1];
   const long long n = (long long)vec_per_row.d * 8;
   const long long groups = n / 128;
@@ -302,6 +306,7 @@ __global__ void __launch_bounds__(THREADS) sum_topk_kernel(const T* __restrict__
                                                            int top_k, long long h, const IdT* __restrict__ ids,
                                                            long long id_lo, long long id_hi, int skip_unrouted,
                                                            T* __restrict__ out) {
+  if (!wait_for_predecessor()) return;
   const int lane = threadIdx.x & 31;
   for (uint32_t w = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5); w < units; w += gridDim.x * (THREADS / 32)) {
     const uint32_t t = chunks.quot(w);
@@ -344,6 +349,7 @@ __global__ void __launch_bounds__(THREADS) ep_gather_kernel(const T* __restrict_
                                                             const IdxT* __restrict__ ids, const IdxT* __restrict__ index,
                                                             const float* __restrict__ weights, uint32_t units,
                                                             FastDiv chunks, int top_k, T* __restrict__ out) {
+  if (!wait_for_predecessor()) return;
   const int lane = threadIdx.x & 31;
   for (uint32_t w = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5); w < units; w += gridDim.x * (THREADS / 32)) {
     const uint32_t t = chunks.quot(w);
@@ -383,6 +389,7 @@ __global__ void __launch_bounds__(THREADS) ep_gather_kernel(const T* __restrict_
 __global__ void __launch_bounds__(1024) scatter_layout_kernel(const int* __restrict__ counts, int num_experts,
                                                               int* __restrict__ start_loc, int* __restrict__ m_indices,
                                                               long long m_indices_len) {
+  if (!wait_for_predecessor()) return;
   extern __shared__ int s_start[];  // [num_experts + 1]
   if (threadIdx.x == 0) {
     int run = 0;
@@ -404,6 +411,7 @@ template <typename IdxT>
 __global__ void __launch_bounds__(THREADS) scatter_index_kernel(const IdxT* __restrict__ ids, const int* __restrict__ rank,
                                                                 const int* __restrict__ start_loc, long long slots,
                                                                 IdxT* __restrict__ output_index, int* __restrict__ dst_pos) {
+  if (!wait_for_predecessor()) return;
   for (long long f = (long long)blockIdx.x * THREADS + threadIdx.x; f < slots; f += (long long)gridDim.x * THREADS) {
     const long long e = (long long)ids[f];
     int d = -1;
@@ -418,6 +426,7 @@ __global__ void __launch_bounds__(THREADS) scatter_index_kernel(const IdxT* __re
 template <typename IdxT>
 __global__ void __launch_bounds__(THREADS) dest_ranks_kernel(const IdxT* __restrict__ ids, long long tokens, int top_k,
                                                              int num_local, int world, int* __restrict__ dest) {
+  if (!wait_for_predecessor()) return;
   const long long total = tokens * world;
   for (long long u = (long long)blockIdx.x * THREADS + threadIdx.x; u < total; u += (long long)gridDim.x * THREADS) {
     const long long t = u / world;
@@ -474,6 +483,7 @@ __global__ void __launch_bounds__(THREADS) unpermute_kernel(const T* __restrict_
                                                             const float* __restrict__ probs, uint32_t tokens,
                                                             uint32_t units, FastDiv chunks, int top_k, long long h,
                                                             T* __restrict__ out) {
+  if (!wait_for_predecessor()) return;
   const int lane = threadIdx.x & 31;
   for (uint32_t w = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5); w < units; w += gridDim.x * (THREADS / 32)) {
     const uint32_t t = chunks.quot(w);
@@ -517,6 +527,7 @@ __global__ void __launch_bounds__(THREADS) unpermute_kernel(const T* __restrict_
 // Rows that some slot refers to (a row without one gets a zero gradient).
 __global__ void __launch_bounds__(THREADS) mark_rows_kernel(const int* __restrict__ row_id_map, uint32_t slots,
                                                             uint8_t* __restrict__ marks) {
+  if (!wait_for_predecessor()) return;
   for (uint32_t i = blockIdx.x * THREADS + threadIdx.x; i < slots; i += gridDim.x * THREADS) {
     const int row = __ldg(row_id_map + i);
     if (row >= 0) marks[row] = 1;
@@ -538,6 +549,7 @@ __global__ void __launch_bounds__(THREADS) unpermute_bwd_kernel(const T* __restr
                                                                 int top_k, long long h, const uint8_t* __restrict__ marks,
                                                                 uint32_t rows, OutT* __restrict__ act_grad,
                                                                 float* __restrict__ prob_grad) {
+  if (!wait_for_predecessor()) return;
   constexpr int R = GATHER_ROWS<T>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   if (blockIdx.x >= tokens) {
@@ -652,8 +664,10 @@ extern "C" int dlb_quant_fp8(const void* x, int x_dtype, int64_t m, int64_t k, i
     float* ss = scales + (dst_pos == nullptr ? r0 * scale_row_stride : 0);
     const int* dp = dst_pos == nullptr ? nullptr : dst_pos + r0 * fanout;
     auto launch = [&](auto* xp) {
-      quant_fp8_kernel<<<grid, THREADS, 0, st>>>(xp + r0 * ldx, total, vpr, ldx, group_size / 16, mode, eps, qq, ss,
-                                                 scale_row_stride, scale_group_stride, dp, fanout);
+      using T = std::remove_const_t<std::remove_pointer_t<decltype(xp)>>;
+      after_predecessor(quant_fp8_kernel<T>, grid, THREADS, 0, st)(xp + r0 * ldx, total, vpr, ldx, group_size / 16, mode,
+                                                                   eps, qq, ss, scale_row_stride, scale_group_stride, dp,
+                                                                   fanout);
     };
     if (x_dtype == DLB_BF16) launch(reinterpret_cast<const __nv_bfloat16*>(x));
     else if (x_dtype == DLB_F16) launch(reinterpret_cast<const __half*>(x));
@@ -679,7 +693,7 @@ extern "C" int dlb_permute_rows(const void* q, int64_t row_bytes, const float* s
   const long long slab = slab_rows(vpr);
   for (long long r0 = 0; r0 < m; r0 += slab) {
     const uint32_t total = (uint32_t)(std::min<long long>(slab, m - r0) * vpr);
-    permute_rows_kernel<<<grid_for(total), THREADS, 0, (cudaStream_t)stream>>>(
+    after_predecessor(permute_rows_kernel, grid_for(total), THREADS, 0, (cudaStream_t)stream)(
         reinterpret_cast<const uint4*>(q) + r0 * vpr, FastDiv((uint32_t)vpr),
         scales == nullptr ? nullptr : scales + r0 * groups, (uint32_t)groups, total, dst_pos + r0 * fanout, fanout,
         reinterpret_cast<uint4*>(out_q), out_scales);
@@ -706,8 +720,9 @@ extern "C" int dlb_silu_and_mul(const void* gate_up, int dtype, int64_t rows, in
   for (long long r0 = 0; r0 < rows; r0 += slab) {
     const uint32_t total = (uint32_t)(std::min<long long>(slab, rows - r0) * (n / 8));
     auto launch = [&](auto* in, auto* o) {
-      silu_and_mul_kernel<<<grid_for(total), THREADS, 0, st>>>(in + r0 * ld_in, total, FastDiv((uint32_t)(n / 8)), ld_in,
-                                                               o + r0 * ld_out, ld_out);
+      using T = std::remove_pointer_t<decltype(o)>;
+      after_predecessor(silu_and_mul_kernel<T>, grid_for(total), THREADS, 0, st)(
+          in + r0 * ld_in, total, FastDiv((uint32_t)(n / 8)), ld_in, o + r0 * ld_out, ld_out);
     };
     if (dtype == DLB_BF16) launch(reinterpret_cast<const __nv_bfloat16*>(gate_up), reinterpret_cast<__nv_bfloat16*>(out));
     else if (dtype == DLB_F16) launch(reinterpret_cast<const __half*>(gate_up), reinterpret_cast<__half*>(out));
@@ -746,8 +761,10 @@ extern "C" int dlb_silu_mul_quant(const void* gate_up, int dtype, int64_t rows, 
     int grid = grid_for(here * (n / 8));
     if (masked_m != nullptr) grid = std::min(grid, 4 * sm_count());   // the valid rows are few; every block pays for the sums
     auto launch = [&](auto* in) {
-      silu_mul_quant_kernel<<<grid, THREADS, 0, st>>>(in, (uint32_t)r0, (uint32_t)here, FastDiv((uint32_t)(n / 8)), quant_mode,
-                                                      eps, round_silu, masked_m, experts, rows_per_expert, qq, scales);
+      using T = std::remove_const_t<std::remove_pointer_t<decltype(in)>>;
+      after_predecessor(silu_mul_quant_kernel<T>, grid, THREADS, 0, st)(
+          in, (uint32_t)r0, (uint32_t)here, FastDiv((uint32_t)(n / 8)), quant_mode, eps, round_silu, masked_m, experts,
+          rows_per_expert, qq, scales);
     };
     if (dtype == DLB_BF16) launch(reinterpret_cast<const __nv_bfloat16*>(gate_up));
     else launch(reinterpret_cast<const __half*>(gate_up));
@@ -774,7 +791,8 @@ int launch_sum_topk(const void* y, int64_t tokens, int top_k, int64_t h, const v
     const uint32_t units = (uint32_t)(std::min<long long>(slab, tokens - t0) * chunks.d);
     auto launch = [&](auto* idp) {
       with_rows_in_flight<T>(top_k, [&](auto r) {
-        sum_topk_kernel<T, r.value><<<gather_grid(units), THREADS, 0, st>>>(
+        using IdT = std::remove_const_t<std::remove_pointer_t<decltype(idp)>>;
+        after_predecessor(sum_topk_kernel<T, r.value, IdT>, gather_grid(units), THREADS, 0, st)(
             reinterpret_cast<const T*>(y) + t0 * top_k * h, units, chunks, top_k, h,
             idp == nullptr ? idp : idp + t0 * top_k, lo, hi, skip, reinterpret_cast<T*>(out) + t0 * h);
       });
@@ -818,7 +836,8 @@ int launch_gather(const void* in, int64_t h, const void* ids, const void* index,
     const long long s0 = t0 * top_k;
     auto launch = [&](auto* idp, auto* ixp) {
       with_rows_in_flight<T>(top_k, [&](auto r) {
-        ep_gather_kernel<T, r.value><<<gather_grid(units), THREADS, 0, st>>>(
+        using IdxT = std::remove_const_t<std::remove_pointer_t<decltype(idp)>>;
+        after_predecessor(ep_gather_kernel<T, r.value, IdxT>, gather_grid(units), THREADS, 0, st)(
             reinterpret_cast<const T*>(in), h, idp + s0, ixp + s0, weights + s0, units, chunks, top_k,
             reinterpret_cast<T*>(out) + t0 * h);
       });
@@ -868,8 +887,9 @@ extern "C" int dlb_ep_scatter(const void* x, int64_t row_bytes, const float* x_s
   DLB_REQUIRE(row_bytes > 0 && row_bytes % 16 == 0, DLB_ERR_INVALID, "ep_scatter: row_bytes must be a multiple of 16");
   DLB_REQUIRE(counts && expert_start_loc && m_indices, DLB_ERR_INVALID, "ep_scatter: null pointer");
   cudaStream_t st = (cudaStream_t)stream;
-  scatter_layout_kernel<<<1, 1024, (size_t)(num_experts + 1) * 4, st>>>(counts, num_experts, expert_start_loc, m_indices,
-                                                                        m_indices_len);
+  after_predecessor(scatter_layout_kernel, 1, 1024, (size_t)(num_experts + 1) * 4, st)(counts, num_experts,
+                                                                                       expert_start_loc, m_indices,
+                                                                                       m_indices_len);
   count_launch();
   DLB_CHECK_LAUNCH("scatter_layout_kernel");
   if (tokens == 0) return DLB_OK;
@@ -886,14 +906,13 @@ extern "C" int dlb_ep_scatter(const void* x, int64_t row_bytes, const float* x_s
                           workspace_bytes - 2 * align256((size_t)slots * 4), st);
   if (rc != DLB_OK) return rc;
   if (idx_dtype == DLB_I32)
-    scatter_index_kernel<int><<<grid_for(slots), THREADS, 0, st>>>(reinterpret_cast<const int*>(ids), rank,
+    after_predecessor(scatter_index_kernel<int>, grid_for(slots), THREADS, 0, st)(reinterpret_cast<const int*>(ids), rank,
                                                                   expert_start_loc, slots,
                                                                   reinterpret_cast<int*>(output_index), dst_pos);
   else
-    scatter_index_kernel<long long><<<grid_for(slots), THREADS, 0, st>>>(reinterpret_cast<const long long*>(ids), rank,
-                                                                        expert_start_loc, slots,
-                                                                        reinterpret_cast<long long*>(output_index),
-                                                                        dst_pos);
+    after_predecessor(scatter_index_kernel<long long>, grid_for(slots), THREADS, 0, st)(
+        reinterpret_cast<const long long*>(ids), rank, expert_start_loc, slots,
+        reinterpret_cast<long long*>(output_index), dst_pos);
   count_launch();
   DLB_CHECK_LAUNCH("scatter_index_kernel");
   return dlb_permute_rows(x, row_bytes, x_scale, groups, tokens, dst_pos, top_k, out_x, out_scale, stream);
@@ -908,11 +927,11 @@ extern "C" int dlb_ep_dest_ranks(const void* ids, int ids_dtype, int64_t tokens,
   const int grid = grid_for(tokens * world);
   cudaStream_t st = (cudaStream_t)stream;
   if (ids_dtype == DLB_I32)
-    dest_ranks_kernel<int><<<grid, THREADS, 0, st>>>(reinterpret_cast<const int*>(ids), tokens, top_k, num_local_experts,
-                                                    world, dest);
+    after_predecessor(dest_ranks_kernel<int>, grid, THREADS, 0, st)(
+        reinterpret_cast<const int*>(ids), tokens, top_k, num_local_experts, world, dest);
   else
-    dest_ranks_kernel<long long><<<grid, THREADS, 0, st>>>(reinterpret_cast<const long long*>(ids), tokens, top_k,
-                                                          num_local_experts, world, dest);
+    after_predecessor(dest_ranks_kernel<long long>, grid, THREADS, 0, st)(
+        reinterpret_cast<const long long*>(ids), tokens, top_k, num_local_experts, world, dest);
   count_launch();
   DLB_CHECK_LAUNCH("dest_ranks_kernel");
   return DLB_OK;
@@ -934,8 +953,8 @@ extern "C" int dlb_unpermute(const void* in, int dtype, const int32_t* row_id_ma
   auto launch = [&](auto* ip, auto* op) {
     using T = std::remove_pointer_t<decltype(op)>;
     with_rows_in_flight<T>(top_k, [&](auto r) {
-      unpermute_kernel<T, r.value><<<gather_grid(units), THREADS, 0, st>>>(ip, row_id_map, probs, (uint32_t)tokens, units,
-                                                                          chunks, top_k, h, op);
+      after_predecessor(unpermute_kernel<T, r.value>, gather_grid(units), THREADS, 0, st)(
+          ip, row_id_map, probs, (uint32_t)tokens, units, chunks, top_k, h, op);
     });
   };
   if (dtype == DLB_BF16) launch(reinterpret_cast<const __nv_bfloat16*>(in), reinterpret_cast<__nv_bfloat16*>(out));
@@ -969,7 +988,8 @@ static int unpermute_bwd(const void* grad_out, const void* fwd_in, int dtype, co
   if (marks != nullptr && rows > 0) {
     int rc = check_cuda(cudaMemsetAsync(marks, 0, (size_t)rows, st), "cudaMemsetAsync(unpermute_bwd)");
     if (rc != DLB_OK) return rc;
-    mark_rows_kernel<<<grid_for(tokens * top_k), THREADS, 0, st>>>(row_id_map, (uint32_t)(tokens * top_k), marks);
+    after_predecessor(mark_rows_kernel, grid_for(tokens * top_k), THREADS, 0, st)(
+        row_id_map, (uint32_t)(tokens * top_k), marks);
     count_launch();
     DLB_CHECK_LAUNCH("mark_rows_kernel");
   }
@@ -978,7 +998,8 @@ static int unpermute_bwd(const void* grad_out, const void* fwd_in, int dtype, co
   const int zero_blocks = marks == nullptr ? 0 : (int)std::min<long long>(ceil_div(rows, 8ll * 32), sm_count());
   auto launch = [&](auto* go, auto* ag) {
     using T = std::remove_const_t<std::remove_pointer_t<decltype(go)>>;
-    unpermute_bwd_kernel<T><<<(int)tokens + zero_blocks, threads, 0, st>>>(
+    using O = std::remove_pointer_t<decltype(ag)>;
+    after_predecessor(unpermute_bwd_kernel<T, O>, (int)tokens + zero_blocks, threads, 0, st)(
         go, reinterpret_cast<const T*>(fwd_in), row_id_map, probs, (uint32_t)tokens, top_k, h, marks, (uint32_t)rows, ag,
         prob_grad);
   };

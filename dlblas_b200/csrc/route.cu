@@ -67,6 +67,7 @@ template <typename T, int VPT, typename IdT>
 __global__ void __launch_bounds__(WARPS * 32) softmax_topk_kernel(const T* __restrict__ logits, long long tokens,
                                                                   int experts, int top_k, int renorm,
                                                                   float* __restrict__ weights, IdT* __restrict__ ids) {
+  if (!wait_for_predecessor()) return;
   const int lane = threadIdx.x & 31;
   const long long t = (long long)blockIdx.x * WARPS + (threadIdx.x >> 5);
   if (t >= tokens) return;
@@ -193,6 +194,7 @@ __global__ void __launch_bounds__(WARPS * 32) grouped_topk_kernel(const T* __res
                                                                   int experts, int num_groups, int topk_group, int top_k,
                                                                   int renorm, float* __restrict__ weights,
                                                                   int* __restrict__ ids) {
+  if (!wait_for_predecessor()) return;
   const int lane = threadIdx.x & 31;
   const long long t = (long long)blockIdx.x * WARPS + (threadIdx.x >> 5);
   if (t >= tokens) return;
@@ -286,6 +288,7 @@ __global__ void __launch_bounds__(WARPS * 32) grouped_topk_lanes_kernel(const T*
                                                                         int num_groups, int group_lanes, int topk_group,
                                                                         int top_k, int renorm, float* __restrict__ weights,
                                                                         int* __restrict__ ids) {
+  if (!wait_for_predecessor()) return;
   const int lane = threadIdx.x & 31;
   const long long t = (long long)blockIdx.x * WARPS + (threadIdx.x >> 5);
   if (t >= tokens) return;
@@ -391,6 +394,7 @@ __global__ void __launch_bounds__(WARPS * 32) gating_part1_kernel(const T* __res
                                                                   int* __restrict__ ids_km, float* __restrict__ gate_km,
                                                                   float* __restrict__ psum, int* __restrict__ pcnt,
                                                                   int* __restrict__ ticket) {
+  if (!wait_for_predecessor()) return;
   extern __shared__ float sm[];
   float* s_sum = sm;                                            // [WARPS][experts]
   int* s_cnt = reinterpret_cast<int*>(sm + WARPS * experts);    // [experts]
@@ -512,6 +516,7 @@ __global__ void __launch_bounds__(64) gating_part3_kernel(const int* __restrict_
                                                           float* __restrict__ ce_out, int* __restrict__ ticket,
                                                           T* __restrict__ l_aux, int* __restrict__ ec_idx,
                                                           T* __restrict__ out_w, long long* __restrict__ select) {
+  if (!wait_for_predecessor()) return;
   if ((int)blockIdx.x >= token_blocks) {
     gating_expert_part<T>(ids_km, counts, psum, pcnt, part_blocks, tokens, experts, top_k, capacity,
                           blockIdx.x - token_blocks, gridDim.x - token_blocks, res, ce_out, ticket, l_aux, select);
@@ -579,13 +584,13 @@ template <int VPT> struct SoftmaxLauncher {
   template <typename T> static void go(const SoftmaxArgs& a) {
     const int grid = (int)ceil_div(a.tokens, WARPS);
     if (a.ids_dtype == DLB_I32)
-      softmax_topk_kernel<T, VPT, int><<<grid, WARPS * 32, 0, a.st>>>(reinterpret_cast<const T*>(a.logits), a.tokens,
-                                                                     a.experts, a.top_k, a.renorm, a.weights,
-                                                                     reinterpret_cast<int*>(a.ids));
+      after_predecessor(softmax_topk_kernel<T, VPT, int>, grid, WARPS * 32, 0, a.st)(
+          reinterpret_cast<const T*>(a.logits), a.tokens, a.experts, a.top_k, a.renorm, a.weights,
+          reinterpret_cast<int*>(a.ids));
     else
-      softmax_topk_kernel<T, VPT, long long><<<grid, WARPS * 32, 0, a.st>>>(reinterpret_cast<const T*>(a.logits),
-                                                                           a.tokens, a.experts, a.top_k, a.renorm,
-                                                                           a.weights, reinterpret_cast<long long*>(a.ids));
+      after_predecessor(softmax_topk_kernel<T, VPT, long long>, grid, WARPS * 32, 0, a.st)(
+          reinterpret_cast<const T*>(a.logits), a.tokens, a.experts, a.top_k, a.renorm, a.weights,
+          reinterpret_cast<long long*>(a.ids));
   }
   static int run(SoftmaxArgs a) {
     if (a.dtype == DLB_F32) go<float>(a);
@@ -614,16 +619,16 @@ template <int VPT> struct GroupedLauncher {
     if (a.experts == 32 * VPT && per_group % VPT == 0 && (lanes & (lanes - 1)) == 0) {
       const int grid = (int)ceil_div(a.tokens, WARPS);
       if ((uintptr_t)a.logits % 16 == 0)   // every row then is, too
-        grouped_topk_lanes_kernel<T, VPT, true><<<grid, WARPS * 32, 0, a.st>>>(
+        after_predecessor(grouped_topk_lanes_kernel<T, VPT, true>, grid, WARPS * 32, 0, a.st)(
             reinterpret_cast<const T*>(a.logits), a.bias, a.tokens, a.num_groups, lanes, a.topk_group, a.top_k, a.renorm,
             a.weights, a.ids);
       else
-        grouped_topk_lanes_kernel<T, VPT, false><<<grid, WARPS * 32, 0, a.st>>>(
+        after_predecessor(grouped_topk_lanes_kernel<T, VPT, false>, grid, WARPS * 32, 0, a.st)(
             reinterpret_cast<const T*>(a.logits), a.bias, a.tokens, a.num_groups, lanes, a.topk_group, a.top_k, a.renorm,
             a.weights, a.ids);
       return;
     }
-    grouped_topk_kernel<T, VPT><<<(int)ceil_div(a.tokens, WARPS), WARPS * 32, 0, a.st>>>(
+    after_predecessor(grouped_topk_kernel<T, VPT>, (int)ceil_div(a.tokens, WARPS), WARPS * 32, 0, a.st)(
         reinterpret_cast<const T*>(a.logits), a.bias, a.tokens, a.experts, a.num_groups, a.topk_group, a.top_k, a.renorm,
         a.weights, a.ids);
   }
@@ -656,11 +661,11 @@ template <int VPT> struct GatingLauncher {
     const int grid = gating_blocks(a.tokens);
     const size_t smem = (size_t)(WARPS + 1) * a.experts * 4;    // at most 36 KB
     if (a.dtype == DLB_F32)
-      gating_part1_kernel<float, VPT><<<grid, WARPS * 32, smem, a.st>>>(
+      after_predecessor(gating_part1_kernel<float, VPT>, grid, WARPS * 32, smem, a.st)(
           reinterpret_cast<const float*>(a.logits), a.tokens, a.experts, a.top_k, a.gates, a.ids_km, a.gate_km, a.psum,
           a.pcnt, a.ticket);
     else
-      gating_part1_kernel<__half, VPT><<<grid, WARPS * 32, smem, a.st>>>(
+      after_predecessor(gating_part1_kernel<__half, VPT>, grid, WARPS * 32, smem, a.st)(
           reinterpret_cast<const __half*>(a.logits), a.tokens, a.experts, a.top_k, a.gates, a.ids_km, a.gate_km, a.psum,
           a.pcnt, a.ticket);
     count_launch();
@@ -685,6 +690,7 @@ __global__ void __launch_bounds__(WARPS * 32) gating_bwd_kernel(const float* __r
                                                                 int experts, int top_k, long long capacity,
                                                                 const T* __restrict__ grad_l_aux,
                                                                 const T* __restrict__ grad_w, T* __restrict__ grad_logits) {
+  if (!wait_for_predecessor()) return;
   const int lane = threadIdx.x & 31;
   const long long t = (long long)blockIdx.x * WARPS + (threadIdx.x >> 5);
   if (t >= tokens) return;
@@ -757,7 +763,7 @@ struct GatingBwdArgs {
 };
 template <int VPT> struct GatingBwdLauncher {
   template <typename T> static void go(const GatingBwdArgs& a) {
-    gating_bwd_kernel<T, VPT><<<(int)ceil_div(a.tokens, WARPS), WARPS * 32, 0, a.st>>>(
+    after_predecessor(gating_bwd_kernel<T, VPT>, (int)ceil_div(a.tokens, WARPS), WARPS * 32, 0, a.st)(
         a.gates, a.ce, a.ids_km, a.gate_km, a.rank, a.tokens, a.experts, a.top_k, a.capacity,
         reinterpret_cast<const T*>(a.grad_l_aux), reinterpret_cast<const T*>(a.grad_w), reinterpret_cast<T*>(a.grad_logits));
   }
@@ -802,6 +808,7 @@ __global__ void __launch_bounds__(EPLB_THREADS) eplb_map_hash_kernel(const IdT* 
                                                                 const int* __restrict__ logcnt, long long slots,
                                                                 int top_k, int num_logical, int max_replica,
                                                                 uint32_t seed, int* __restrict__ out) {
+  if (!wait_for_predecessor()) return;
   for (long long i = (long long)blockIdx.x * EPLB_THREADS + threadIdx.x; i < slots; i += (long long)gridDim.x * EPLB_THREADS) {
     const long long e = (long long)topk_idx[i];
     int phy = -1;
@@ -839,12 +846,13 @@ extern "C" int dlb_eplb_map_hash(const void* topk_idx, int ids_dtype, const int3
   const int grid = (int)std::min<long long>(ceil_div(slots, (long long)EPLB_THREADS), (long long)sm_count() * 16);
   cudaStream_t st = (cudaStream_t)stream;
   if (ids_dtype == DLB_I32) {
-    eplb_map_hash_kernel<int><<<grid, EPLB_THREADS, 0, st>>>(reinterpret_cast<const int*>(topk_idx), log2phy, logcnt, slots,
-                                                        top_k, num_logical, max_replica, seed, physical_idx);
+    after_predecessor(eplb_map_hash_kernel<int>, grid, EPLB_THREADS, 0, st)(
+        reinterpret_cast<const int*>(topk_idx), log2phy, logcnt, slots, top_k, num_logical, max_replica, seed,
+        physical_idx);
   } else if (ids_dtype == DLB_I64) {
-    eplb_map_hash_kernel<long long><<<grid, EPLB_THREADS, 0, st>>>(reinterpret_cast<const long long*>(topk_idx), log2phy,
-                                                              logcnt, slots, top_k, num_logical, max_replica, seed,
-                                                              physical_idx);
+    after_predecessor(eplb_map_hash_kernel<long long>, grid, EPLB_THREADS, 0, st)(
+        reinterpret_cast<const long long*>(topk_idx), log2phy, logcnt, slots, top_k, num_logical, max_replica, seed,
+        physical_idx);
   } else {
     return fail(DLB_ERR_INVALID, "eplb_map_hash: ids must be int32 or int64 (got %d)", ids_dtype);
   }
@@ -932,7 +940,8 @@ extern "C" int dlb_topk_gating(const void* logits, int dtype, int64_t tokens, in
   if (rc != DLB_OK) return rc;
   const int token_blocks = (int)ceil_div(tokens, 64), expert_blocks = (int)ceil_div(experts, 2);
   auto part3 = [&](auto* out_l_aux, auto* out_w) {
-    gating_part3_kernel<<<token_blocks + expert_blocks, 64, 0, st>>>(
+    using T = std::remove_pointer_t<decltype(out_w)>;
+    after_predecessor(gating_part3_kernel<T>, token_blocks + expert_blocks, 64, 0, st)(
         ids_km, gate_km, rank, counts, psum, pcnt, gating_blocks(tokens), tokens, experts, top_k, capacity, token_blocks, res,
         reinterpret_cast<float*>(ws + w.ce), ticket, out_l_aux, ec_idx, out_w, reinterpret_cast<long long*>(select));
   };

@@ -238,6 +238,7 @@ __device__ __forceinline__ void write_slot(unsigned f, unsigned n, int bucket, i
 template <typename IdT, int ITEMS>
 __global__ void __launch_bounds__(MAX_WARPS * 32) sort_one_block_kernel(const IdT* __restrict__ ids, unsigned n,
                                                                         int num_experts, SortOut o) {
+  if (!wait_for_predecessor()) return;
   extern __shared__ int sm[];
   const int nb = num_experts + 2;
   const int stride = hist_stride(num_experts);
@@ -286,6 +287,7 @@ template <typename IdT>
 __global__ void __launch_bounds__(512) sort_count_kernel(const IdT* __restrict__ ids, unsigned n, int num_experts,
                                                          unsigned chunk, int negative_as, int* __restrict__ cnt,
                                                          int* __restrict__ stats, int* __restrict__ run) {
+  if (!wait_for_predecessor()) return;
   extern __shared__ int sm[];
   __shared__ int stats_s[3];
   const int nb = num_experts + 2;
@@ -320,6 +322,7 @@ __global__ void __launch_bounds__(512) sort_count_kernel(const IdT* __restrict__
 
 // One CTA per bucket: exclusive prefix over chunks (in place) and the bucket total.
 __global__ void __launch_bounds__(256) sort_scan_chunks_kernel(int* cnt, int num_chunks, int nb, int* total) {
+  if (!wait_for_predecessor()) return;
   __shared__ int warp_sums[8];
   __shared__ int carry_s;
   const int b = blockIdx.x;
@@ -354,6 +357,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32) sort_scatter_kernel(const IdT*
                                                                       int num_experts, unsigned chunk,
                                                                       const int* __restrict__ cnt,
                                                                       const int* __restrict__ total_in, SortOut o) {
+  if (!wait_for_predecessor()) return;
   extern __shared__ int sm[];
   const int nb = num_experts + 2, stride = hist_stride(num_experts);
   uint32_t* hist = reinterpret_cast<uint32_t*>(sm);   // [MAX_WARPS][stride]
@@ -473,7 +477,7 @@ int launch_one_block(const IdT* ids, long long n, int num_experts, const SortOut
                         "cudaFuncSetAttribute(sort_one_block_kernel)");
     if (rc != DLB_OK) return rc;
   }
-  sort_one_block_kernel<IdT, ITEMS><<<1, p.warps * 32, p.smem, st>>>(ids, (unsigned)n, num_experts, o);
+  after_predecessor(sort_one_block_kernel<IdT, ITEMS>, 1, p.warps * 32, p.smem, st)(ids, (unsigned)n, num_experts, o);
   count_launch();
   DLB_CHECK_LAUNCH("sort_one_block_kernel");
   if (o.stats_event != nullptr) return check_cuda(cudaEventRecord((cudaEvent_t)o.stats_event, st), "cudaEventRecord");
@@ -505,8 +509,8 @@ int run_sort(const IdT* ids, long long n, int num_experts, const SortOut& o, voi
     cudaMemsetAsync(run, 0xff, 4, st);
     cudaMemsetAsync(run + 1, 0, 12, st);
   }
-  sort_count_kernel<IdT><<<p.num_chunks, 512, (size_t)(nb + 1) * 4, st>>>(ids, (unsigned)n, num_experts, (unsigned)p.chunk, o.negative_as, cnt,
-                                                                         o.stats, run);
+  after_predecessor(sort_count_kernel<IdT>, p.num_chunks, 512, (size_t)(nb + 1) * 4, st)(
+      ids, (unsigned)n, num_experts, (unsigned)p.chunk, o.negative_as, cnt, o.stats, run);
   count_launch();
   DLB_CHECK_LAUNCH("sort_count_kernel");
   if (o.stats_event != nullptr) {
@@ -515,7 +519,7 @@ int run_sort(const IdT* ids, long long n, int num_experts, const SortOut& o, voi
   }
   const bool scan = p.num_chunks > DIRECT_CHUNKS;
   if (scan) {
-    sort_scan_chunks_kernel<<<nb, 256, 0, st>>>(cnt, p.num_chunks, nb, total);
+    after_predecessor(sort_scan_chunks_kernel, nb, 256, 0, st)(cnt, p.num_chunks, nb, total);
     count_launch();
     DLB_CHECK_LAUNCH("sort_scan_chunks_kernel");
   }
@@ -525,8 +529,8 @@ int run_sort(const IdT* ids, long long n, int num_experts, const SortOut& o, voi
                         "cudaFuncSetAttribute(sort_scatter_kernel)");
     if (rc != DLB_OK) return rc;
   }
-  sort_scatter_kernel<IdT><<<p.num_chunks, MAX_WARPS * 32, p.smem, st>>>(ids, (unsigned)n, num_experts, (unsigned)p.chunk, cnt,
-                                                                        scan ? total : nullptr, o);
+  after_predecessor(sort_scatter_kernel<IdT>, p.num_chunks, MAX_WARPS * 32, p.smem, st)(
+      ids, (unsigned)n, num_experts, (unsigned)p.chunk, cnt, scan ? total : nullptr, o);
   count_launch();
   DLB_CHECK_LAUNCH("sort_scatter_kernel");
   return DLB_OK;
@@ -538,6 +542,7 @@ __global__ void __launch_bounds__(1024) build_tiles_kernel(const long long* exp_
                                                            const int* masked_m, int expert_offset, int num_local,
                                                            int rows_per_expert, int tile_rows, int4* tiles,
                                                            int max_tiles) {
+  if (!wait_for_predecessor()) return;
   __shared__ int warp_sums[32];
   __shared__ int carry_s;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -588,6 +593,7 @@ template <typename SizeT>
 __global__ void __launch_bounds__(1024) build_tiles_sizes_kernel(const SizeT* __restrict__ sizes, int groups,
                                                                  long long total_rows, int tile_rows,
                                                                  int4* __restrict__ tiles, int max_tiles) {
+  if (!wait_for_predecessor()) return;
   __shared__ long long warp_rows[32];
   __shared__ int warp_tiles[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -759,7 +765,7 @@ extern "C" int dlb_moe_build_tiles(const int64_t* exp_start, const int64_t* exp_
   DLB_REQUIRE(exp_start && exp_end && tiles, DLB_ERR_INVALID, "build_tiles: null pointer");
   DLB_REQUIRE(num_local_experts > 0 && expert_offset >= 0 && max_tiles >= 0, DLB_ERR_INVALID, "build_tiles: bad sizes");
   DLB_REQUIRE((uintptr_t)tiles % 16 == 0, DLB_ERR_INVALID, "build_tiles: tiles must be 16-byte aligned");
-  build_tiles_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(reinterpret_cast<const long long*>(exp_start),
+  after_predecessor(build_tiles_kernel, 1, 1024, 0, (cudaStream_t)stream)(reinterpret_cast<const long long*>(exp_start),
                                                            reinterpret_cast<const long long*>(exp_end), nullptr,
                                                            expert_offset, num_local_experts, 0, 128,
                                                            reinterpret_cast<int4*>(tiles), max_tiles);
@@ -776,7 +782,7 @@ extern "C" int dlb_moe_build_tiles_rows(const int64_t* exp_start, const int64_t*
               "build_tiles_rows: bad sizes");
   DLB_REQUIRE(tile_rows == 128 || tile_rows == 256, DLB_ERR_INVALID, "build_tiles_rows: tile_rows must be 128 or 256");
   DLB_REQUIRE((uintptr_t)tiles % 16 == 0, DLB_ERR_INVALID, "build_tiles_rows: tiles must be 16-byte aligned");
-  build_tiles_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(reinterpret_cast<const long long*>(exp_start),
+  after_predecessor(build_tiles_kernel, 1, 1024, 0, (cudaStream_t)stream)(reinterpret_cast<const long long*>(exp_start),
                                                            reinterpret_cast<const long long*>(exp_end), nullptr,
                                                            expert_offset, num_local_experts, 0, tile_rows,
                                                            reinterpret_cast<int4*>(tiles), max_tiles);
@@ -791,7 +797,7 @@ extern "C" int dlb_moe_build_tiles_masked(const int32_t* masked_m, int num_local
   DLB_REQUIRE(num_local_experts > 0 && rows_per_expert > 0 && max_tiles >= 0, DLB_ERR_INVALID,
               "build_tiles_masked: bad sizes");
   DLB_REQUIRE((uintptr_t)tiles % 16 == 0, DLB_ERR_INVALID, "build_tiles_masked: tiles must be 16-byte aligned");
-  build_tiles_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(nullptr, nullptr, masked_m, 0, num_local_experts,
+  after_predecessor(build_tiles_kernel, 1, 1024, 0, (cudaStream_t)stream)(nullptr, nullptr, masked_m, 0, num_local_experts,
                                                            rows_per_expert, 128, reinterpret_cast<int4*>(tiles),
                                                            max_tiles);
   count_launch();
@@ -811,11 +817,11 @@ extern "C" int dlb_moe_build_tiles_sizes(const void* sizes, int sizes_dtype, int
   const int threads = num_groups >= 1024 ? 1024 : (num_groups + 31) / 32 * 32;
   int4* out = reinterpret_cast<int4*>(tiles);
   if (sizes_dtype == DLB_I32)
-    build_tiles_sizes_kernel<<<1, threads, 0, (cudaStream_t)stream>>>(reinterpret_cast<const int*>(sizes), num_groups,
-                                                                      total_rows, tile_rows, out, max_tiles);
+    after_predecessor(build_tiles_sizes_kernel<int>, 1, threads, 0, (cudaStream_t)stream)(
+        reinterpret_cast<const int*>(sizes), num_groups, total_rows, tile_rows, out, max_tiles);
   else
-    build_tiles_sizes_kernel<<<1, threads, 0, (cudaStream_t)stream>>>(reinterpret_cast<const long long*>(sizes), num_groups,
-                                                                      total_rows, tile_rows, out, max_tiles);
+    after_predecessor(build_tiles_sizes_kernel<long long>, 1, threads, 0, (cudaStream_t)stream)(
+        reinterpret_cast<const long long*>(sizes), num_groups, total_rows, tile_rows, out, max_tiles);
   count_launch();
   DLB_CHECK_LAUNCH("build_tiles_sizes_kernel");
   return DLB_OK;

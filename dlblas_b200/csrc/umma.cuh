@@ -78,6 +78,11 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
+// The map's descriptor is on its way before the first load asks for it (it lies among the kernel's parameters).
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+}
+
 // Order of the tiles of a persistent launch.  band = 1: n tile by n tile, then the next m tile.  band > 1: bands of that
 // many m tiles, each walked n tile by n tile with the m tiles innermost, so that the tiles in flight share their operands: in
 // the first order a launch of 112 n tiles holds one or two m tiles at a time, and the weights (117 MB an expert) come from

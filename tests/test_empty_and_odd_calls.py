@@ -378,3 +378,50 @@ def test_threads_on_their_own_streams():
         t.join()
     for i in range(4):
         assert all(torch.equal(p, q) for p, q in zip(alone[i], results[i])), i
+
+
+@pytest.mark.gpu
+def test_operators_in_a_row_wait_for_one_another():
+    """Every kernel is launched while its predecessor runs.  Inputs overwritten by torch right before and right after each
+    chain, no synchronisation in between, against the same chain with one after every operator."""
+    from dlblas_b200 import ops
+    from dlblas_b200.kernels.fp8 import per_token_group_quant_fp8
+    from dlblas_b200.kernels.moe import biased_grouped_topk
+    from dlblas_b200.kernels.permute import permute, unpermute
+    g = torch.Generator(device=DEV).manual_seed(5)
+    t, h, e, k, rounds = 300, 512, 64, 4, 24
+    xs = torch.randn(rounds, t, h, device=DEV, generator=g, dtype=torch.bfloat16)
+    ls = torch.randn(rounds, t, e, device=DEV, generator=g)
+    bias = torch.randn(e, device=DEV, generator=g) * 0.01
+    w = torch.randn(640, h, device=DEV, generator=g).to(torch.float8_e4m3fn)
+    ws = torch.rand(5, h // 128, device=DEV, generator=g) + 0.5
+    x, logits = torch.empty_like(xs[0]), torch.empty_like(ls[0])
+
+    def chain(sync):
+        wait = torch.cuda.synchronize if sync else (lambda: None)
+        weights, ids = biased_grouped_topk(x, logits, bias, k, True, 8, 4)
+        wait()
+        rows, row_map = permute(x, ids)
+        wait()
+        back = unpermute(rows, row_map, weights)
+        wait()
+        q, s = per_token_group_quant_fp8(back, 128)
+        wait()
+        y = ops.fp8_gemm(q, w, s, ws, torch.bfloat16)
+        wait()
+        return ids, rows, back, q.view(torch.uint8), y
+
+    def run(sync):
+        out = []
+        for i in range(rounds):
+            x.copy_(xs[i])
+            logits.copy_(ls[i])
+            out.append(chain(sync))
+            x.zero_()
+            logits.zero_()
+        torch.cuda.synchronize()
+        return out
+
+    for got, want in zip(run(False), run(True)):
+        for a, b in zip(got, want):
+            assert torch.equal(a, b)
