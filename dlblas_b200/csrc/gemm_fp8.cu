@@ -14,7 +14,8 @@
 //   warps 10-11         epilogue: rows of the staging tile leave with one bulk copy each
 //                       (store / scatter), or are turned into silu(gate)*up, quantised per 128
 //                       columns and stored as e4m3 (fused w13 epilogue), while the other roles
-//                       already work on the next tile.  (With fp32 output the tile does not fit
+//                       already work on the next tile.  (Tiles of 64 and 128 columns are emptied by the
+//                       promotion warps, see store_rows.  With fp32 output the tile does not fit
 //                       the staging buffer and the promotion warps store it themselves.)
 //
 // (A 16-warp variant, four promotion warps per scheduler partition with 64 accumulator columns
@@ -55,7 +56,7 @@ constexpr int TMEM_COLS = 512;
 // tensor core's tile are columns of C, its columns the rows of A, 16 at a time.  A tile with a handful of rows otherwise
 // multiplies and promotes 128 all the same; the weights' way from DRAM bounds such a launch, and in repeated passes that
 // work costs the clocks and with them the memory rate.  (Up to 64 rows per tile this way: 2 % slower on those steps.)
-// Registers: the promotion warps hold both forms, and spill 36 bytes of stores and 104 of loads in the scatter epilogue, 28 / 92 in
+// Registers: the promotion warps hold both forms, and spill 40 bytes of stores and 108 of loads in the scatter epilogue, 36 / 104 in
 // the plain and the fused one, where the kernel without the exchanged form spills 0, 0 and 28 / 80 (ptxas).
 constexpr int SWAP_ROWS = 32;
 constexpr int CHUNK = 16;                    // rows of A per box and per step of N
@@ -96,16 +97,22 @@ template <int BN, int CTAS = 1> struct Cfg {
   static constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
   static constexpr int STAGES = (BN == 256) ? (CTAS == 2 ? 4 : 3) : (BN == 128 ? 5 : 8);
   static constexpr int TMEM_BUFS = TMEM_COLS / BN;
+  // accumulators are handed back in order, so the last of RUN free ones says that all of them are
+  static constexpr int RUN = TMEM_BUFS / 2;
   static constexpr int COLS = BN / 2;  // columns per promotion thread: the first warpgroup has the first half
   // Staging tile of the epilogue: BM rows of BN 16-bit values.  Rows are padded by 16 bytes so
   // that the 16-byte stores of 32 threads holding 32 different rows spread over all banks.
   static constexpr int STAGING_ROW_BYTES = BN * 2 + 16;
   static constexpr int STAGING_BYTES = BM * STAGING_ROW_BYTES;
-  // dynamic smem: stages | staging tile | barriers (full, empty, tmem_full, tmem_empty, drain,
-  // staged, staging_free) | misc
+  // dynamic smem: stages | staging tile | barriers (full, done, tmem_empty, drain, staged, staging_free) | misc
   static constexpr int STAGING_OFF = STAGES * STAGE_BYTES;
   static constexpr int BAR_OFF = STAGING_OFF + STAGING_BYTES;
-  static constexpr int NUM_BARS = 2 * STAGES + 2 * TMEM_BUFS + 3;
+  // One commit per K block (each holds the MMA warp for about 45 cycles, and so does a question
+  // for a barrier, of which narrow tiles ask one in RUN less): its barrier (the stage's) tells the producer that the
+  // stage is free and the promotion warps that the accumulator is full.  A stage's next use but one cannot be over before
+  // this one's accumulator has been drained.
+  static_assert(STAGES >= TMEM_BUFS, "a promotion warp could miss a phase of the stage's barrier");
+  static constexpr int NUM_BARS = 2 * STAGES + TMEM_BUFS + 3;
   static constexpr int MISC_OFF = BAR_OFF + NUM_BARS * 8;
   static constexpr int SMEM_BYTES = MISC_OFF + 16 + 1024;  // + slack for 1024 B alignment
 };
@@ -207,14 +214,14 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t bar_base = smem_base + C::BAR_OFF;
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
-  auto empty_bar = [&](int s) { return bar_base + 8u * (C::STAGES + s); };
-  auto tfull_bar = [&](int b) { return bar_base + 8u * (2 * C::STAGES + b); };
-  auto tempty_bar = [&](int b) { return bar_base + 8u * (2 * C::STAGES + C::TMEM_BUFS + b); };
-  const uint32_t drain_bar = bar_base + 8u * (2 * C::STAGES + 2 * C::TMEM_BUFS);
+  auto done_bar = [&](int s) { return bar_base + 8u * (C::STAGES + s); };   // stage free, its K block's accumulator full
+  auto tempty_bar = [&](int b) { return bar_base + 8u * (2 * C::STAGES + b); };
+  const uint32_t drain_bar = bar_base + 8u * (2 * C::STAGES + C::TMEM_BUFS);
   const uint32_t staged_bar = drain_bar + 8u;   // promotion warps -> epilogue warps: tile is in the staging buffer
   const uint32_t sfree_bar = drain_bar + 16u;   // epilogue warps -> promotion warps: staging buffer may be reused
   uint8_t* staging = smem + C::STAGING_OFF;
   constexpr bool STAGED = sizeof(OutT) == 2;
+  constexpr bool SELF_DRAIN = STAGED && BN < 256;   // the promotion warps empty the staging tile
   static_assert(!SWAP || (BN == 256 && !PAIR && STAGED), "the exchanged form fills the staging tile of one CTA");
   auto swapped = [](const Tile& ti) { return SWAP && ti.rows <= SWAP_ROWS; };
   auto chunks_of = [](const Tile& ti) { return max(1, (ti.rows + CHUNK - 1) / CHUNK); };   // of a swapped tile
@@ -232,15 +239,13 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
       mbar_init(full_bar(s), 1);
-      mbar_init(empty_bar(s), 1);
+      mbar_init(done_bar(s), 1);
     }
-    for (int b = 0; b < C::TMEM_BUFS; ++b) {
-      mbar_init(tfull_bar(b), 1);
+    for (int b = 0; b < C::TMEM_BUFS; ++b)
       mbar_init(tempty_bar(b), CTAS * EPI_WARPS);   // pair: the promotion warps of both CTAs release the leader's
-    }
     mbar_init(drain_bar, 1);
     mbar_init(staged_bar, EPI_WARPS);
-    mbar_init(sfree_bar, STORE_WARPS);
+    mbar_init(sfree_bar, SELF_DRAIN ? EPI_WARPS : STORE_WARPS);
     abort_flag[0] = 0;
     abort_flag[1] = 0;   // private flag of the drain waits
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -275,6 +280,25 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   const int num_m_tiles = g.tiles != nullptr ? __ldg(reinterpret_cast<const int*>(g.tiles)) : g.num_m_tiles_static;
   const int total_tiles = num_m_tiles * g.num_n_tiles;
 
+  // Narrow tiles are chosen for launches of one tile per CTA, so nothing follows that could hide the staging tile's way out:
+  // the promotion warps empty it themselves with ordinary 16-byte stores, warp w of EPI_WARPS its share of the rows.  (A bulk
+  // copy per row holds its lane for some 70 cycles: 100 rows of 64 columns took two warps 5100 of the kernel's 18300 cycles;
+  // quantiser and GEMM of 100 x 7168 x 2048 11.9 -> 9.6 us with the single commit.  256 columns keep the two epilogue warps and the bulk copies, which
+  // run beside the next tile: with these lines for the last tile only, 8192 x 4096 x 7168 lost 3 %.)
+  auto store_rows = [&](const Tile& ti, int w) {
+    constexpr int VECS = BN / 8, ROWS = 32 / VECS;       // vectors of a row, rows of a pass
+    const int vec = lane % VECS, in_pass = lane / VECS;
+    const bool there = ti.n0 + vec * 8 < g.n;            // n % 8 == 0
+#pragma unroll 4
+    for (int row = w * ROWS + in_pass; row < ti.rows; row += EPI_WARPS * ROWS) {
+      long long crow = (long long)ti.row0 + row;
+      if constexpr (MODE == DLB_EPI_SCATTER_WEIGHT) crow = __ldg(g.sorted_idx + crow);
+      if (there)
+        *reinterpret_cast<uint4*>(reinterpret_cast<OutT*>(g.c) + crow * g.ldc + ti.n0 + vec * 8) =
+            *reinterpret_cast<const uint4*>(staging + row * C::STAGING_ROW_BYTES + vec * 16);
+    }
+  };
+
   if (warp >= EPI_WARPS) {
     // third warpgroup: give registers away, then run the producer / MMA roles
     reg_dec<REGS_OTHER>();
@@ -293,7 +317,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         for (int kb = 0; kb < kblocks; ++kb, ++it) {
           const int s = it % C::STAGES;
           const uint32_t ph = (it / C::STAGES) & 1u;
-          if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, limit)) {
+          if (!mbar_wait(done_bar(s), ph ^ 1u, abort_flag, limit)) {
             ok = false;
             break;
           }
@@ -354,8 +378,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           if (swapped(ti)) idesc_swap = make_idesc(CHUNK * chunks_of(ti));
         }
         for (int kb = 0; kb < kblocks; ++kb) {
+          const bool new_run = b % C::RUN == 0;
           if (!ready && (!mbar_wait(full_bar(s), s_phase, abort_flag, limit) ||
-                         !mbar_wait(tempty_bar(b), b_phase, abort_flag, limit))) {
+                         (new_run && !mbar_wait(tempty_bar(b + C::RUN - 1), b_phase, abort_flag, limit)))) {
             ok = false;
             break;
           }
@@ -364,7 +389,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           const uint64_t a_desc = make_smem_desc(a_addr);
           const uint64_t b_desc = make_smem_desc(a_addr + A_STAGE_BYTES);
           const uint32_t d_tmem = tmem_base + b * BN;
-          const uint32_t done_stage = empty_bar(s), done_acc = tfull_bar(b);
+          const uint32_t done = done_bar(s);
           if (++s == C::STAGES) { s = 0; s_phase ^= 1u; }
           if (++b == C::TMEM_BUFS) { b = 0; b_phase ^= 1u; }
           // +32 bytes along K inside the 128 B swizzle row == +2 in the (addr >> 4) field
@@ -387,7 +412,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           // The tensor core's queue holds two to three instructions: the next K block's barriers are asked about while
           // those of this one are in it.  Asked after the last, the answers left the pipe idle for some 300 cycles a block.
           ready = mbar_test(full_bar(s), s_phase);
-          ready = mbar_test(tempty_bar(b), b_phase) && ready;
+          if (b % C::RUN == 0) ready = mbar_test(tempty_bar(b + C::RUN - 1), b_phase) && ready;
           if (elect_one()) {
             if (swap) {
               const uint64_t b2_desc = make_smem_desc(a_addr + A_STAGE_BYTES + BM * BK);
@@ -399,11 +424,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
               mma(3);
             }
             if constexpr (PAIR) {
-              tc_commit_pair(done_stage);   // both CTAs' stages
-              tc_commit_pair(done_acc);     // both CTAs' promotion warps
+              tc_commit_pair(done);   // both CTAs
             } else {
-              tc_commit(done_stage);   // smem stage reusable once these MMAs retire
-              tc_commit(done_acc);     // accumulator ready for the promotion warps
+              tc_commit(done);   // once these MMAs retire
             }
           }
           __syncwarp();
@@ -421,7 +444,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         mbar_wait(drain_bar, 0, abort_flag + 1, 40000000ull);
       }
     }
-  } else if (STAGED) {
+  } else if (STAGED && !SELF_DRAIN) {
     // ---- epilogue warps: empty the staging tile while the next tile is being computed ----
     const int ew = warp - STORE_WARP0;
     uint32_t tile_no = 0;
@@ -562,7 +585,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
                 if (i < chunks) a2[i] = __ldg(as + (long long)(kb + 2) * g.a_s_ks + a_off[i]);
               b2 = __ldg(bs + kb + 2);
             }
-            if (!mbar_wait(tfull_bar(b), (it / C::TMEM_BUFS) & 1u, abort_flag, limit)) {
+            if (!mbar_wait(done_bar(it % C::STAGES), (it / C::STAGES) & 1u, abort_flag, limit)) {
               ok = false;
               break;
             }
@@ -669,7 +692,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           b_n2 = __ldg(bs_ptr + kb + 2);
         }
         if (!pending) {
-          if (!mbar_wait(tfull_bar(b), (it / C::TMEM_BUFS) & 1u, abort_flag, limit)) {
+          if (!mbar_wait(done_bar(it % C::STAGES), (it / C::STAGES) & 1u, abort_flag, limit)) {
             ok = false;
             break;
           }
@@ -680,7 +703,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         const float scf = a_sc * b_sc;
         const uint64_t sc = pack2(scf, scf);
         const int nb = (it + 1) % C::TMEM_BUFS;
-        const uint32_t nb_phase = ((it + 1) / C::TMEM_BUFS) & 1u;
+        const uint32_t next_done = done_bar((it + 1) % C::STAGES), next_phase = ((it + 1) / C::STAGES) & 1u;
         bool next_full = false;
 #pragma unroll
         for (int q = 0; q < CH; ++q) {
@@ -688,7 +711,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           if (q < CH - 1) {
             tmem_ld32(buf_addr + (q + 1) * 32, stage[(q + 1) & 1]);
             // the next K block's accumulator is asked about under the FMAs below
-            if (q == CH - 2) next_full = mbar_test(tfull_bar(nb), nb_phase);
+            if (q == CH - 2) next_full = mbar_test(next_done, next_phase);
           } else {
             // every column of this accumulator is in registers: hand it back to the MMA warp
             tc_fence_before();
@@ -698,7 +721,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
               else mbar_arrive_cluster_no_release(mapa(tempty_bar(b), 0));
             }
             if (CH > 1 && kb + 1 < kblocks) {
-              if (!next_full && !mbar_wait(tfull_bar(nb), nb_phase, abort_flag, limit)) {
+              if (!next_full && !mbar_wait(next_done, next_phase, abort_flag, limit)) {
                 ok = false;
               } else {
                 tc_fence_after();
@@ -749,6 +772,12 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(staged_bar);
+        if constexpr (SELF_DRAIN) {
+          if (!mbar_wait(staged_bar, tile_no & 1u, abort_flag, limit)) break;   // all promotion warps' parts are there
+          store_rows(ti, warp);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(sfree_bar);
+        }
       } else {
         if (row_ok) {
           OutT* dst = reinterpret_cast<OutT*>(g.c) + crow * g.ldc + ti.n0 + col0;

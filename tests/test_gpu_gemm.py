@@ -454,3 +454,22 @@ def test_fp8_gemm_where_the_tile_width_changes(per_sm, extra, k):
     assert O.rel_frobenius(c.cpu(), ref) < 1e-5
     # the same products in the same order at every width: one rounding apart
     assert torch.equal(cb, c.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("kblocks", [1, 4, 7, 8, 9, 17])
+@pytest.mark.parametrize("m,n", [(1, 8), (33, 72), (100, 200), (128, 64), (129, 1032)])
+def test_narrow_tiles_leave_whole(m, n, kblocks):
+    """Tiles of 64 columns, which the promotion warps store themselves: ragged rows and columns, K blocks around the number of
+    stages and accumulators (8).  The fp32 output goes another way, through 128 columns and no staging tile."""
+    from dlblas_b200 import ops
+    k = 128 * kblocks
+    g = torch.Generator().manual_seed(m + n + k)
+    a, a_s = O.quant_fp8(torch.randn(m, k, generator=g).to(torch.bfloat16), 128)
+    b = torch.randn(n, k, generator=g).to(FP8)
+    b_s = torch.rand((n + 127) // 128, k // 128, generator=g) + 0.5
+    args = (a.to(DEV), b.to(DEV), a_s.to(DEV), b_s.to(DEV))
+    c = ops.fp8_gemm(*args, torch.float32)
+    assert O.rel_frobenius(c.cpu(), O.fp8_gemm(a, b, a_s, b_s, torch.float32)) < 1e-5
+    for dtype in (torch.bfloat16, torch.float16):
+        assert torch.equal(ops.fp8_gemm(*args, dtype), c.to(dtype))
+    _status_ok()
