@@ -56,8 +56,8 @@ constexpr int TMEM_COLS = 512;
 // tensor core's tile are columns of C, its columns the rows of A, 16 at a time.  A tile with a handful of rows otherwise
 // multiplies and promotes 128 all the same; the weights' way from DRAM bounds such a launch, and in repeated passes that
 // work costs the clocks and with them the memory rate.  (Up to 64 rows per tile this way: 2 % slower on those steps.)
-// Registers: the promotion warps hold both forms, and spill 40 bytes of stores and 108 of loads in the scatter epilogue, 36 / 104 in
-// the plain and the fused one, where the kernel without the exchanged form spills 0, 0 and 28 / 80 (ptxas).
+// Registers: the promotion warps hold both forms without a spill, but for 24 bytes of stores and 72 of loads in the fused epilogue,
+// where the kernel without the exchanged form spills 24 / 64 (ptxas).
 constexpr int SWAP_ROWS = 32;
 constexpr int CHUNK = 16;                    // rows of A per box and per step of N
 constexpr int CHUNKS = SWAP_ROWS / CHUNK;
@@ -370,6 +370,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       constexpr uint32_t idesc = make_idesc(BN, CTAS);
       uint32_t s = 0, s_phase = 0, b = 0, b_phase = 1;   // stage and accumulator of the next K block
       bool ready = false;                                // both are known to be there
+      // One lane issues; elected once, as the warp is whole wherever it acts.  (Two elections per K block and lanes that
+      // branch on their own answers: 64 x 4096 x 7168 18.3 us, votes with two elections 18.6, votes and this 17.1.)
+      const bool lead = elect_one();
       bool ok = true;
       for (int t = worker; t < total_tiles && ok && rank == 0; t += workers) {
         uint32_t idesc_swap = 0;
@@ -398,7 +401,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
             else tc_mma_f8(d_tmem, a_desc + 2u * kk, b_desc + 2u * kk, idesc, kk > 0 ? 1u : 0u);
           };
           const bool swap = SWAP && idesc_swap != 0;
-          if (elect_one()) {
+          if (lead) {
             if (swap) {
 #pragma unroll
               for (int kk = 0; kk < BK / 32; ++kk)
@@ -408,12 +411,11 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
               mma(1);
             }
           }
-          __syncwarp();
           // The tensor core's queue holds two to three instructions: the next K block's barriers are asked about while
           // those of this one are in it.  Asked after the last, the answers left the pipe idle for some 300 cycles a block.
           ready = mbar_test(full_bar(s), s_phase);
           if (b % C::RUN == 0) ready = mbar_test(tempty_bar(b + C::RUN - 1), b_phase) && ready;
-          if (elect_one()) {
+          if (lead) {
             if (swap) {
               const uint64_t b2_desc = make_smem_desc(a_addr + A_STAGE_BYTES + BM * BK);
 #pragma unroll
@@ -429,11 +431,11 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
               tc_commit(done);   // once these MMAs retire
             }
           }
-          __syncwarp();
+          ready = __all_sync(WHOLE_WARP, ready);
         }
       }
       if (!ok) {
-        if (elect_one()) {
+        if (lead) {
           if constexpr (PAIR)
             asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(drain_bar)
                          : "memory");
@@ -721,7 +723,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
               else mbar_arrive_cluster_no_release(mapa(tempty_bar(b), 0));
             }
             if (CH > 1 && kb + 1 < kblocks) {
-              if (!next_full && !mbar_wait(next_done, next_phase, abort_flag, limit)) {
+              if (!__all_sync(WHOLE_WARP, next_full) && !mbar_wait(next_done, next_phase, abort_flag, limit)) {
                 ok = false;
               } else {
                 tc_fence_after();

@@ -473,3 +473,33 @@ def test_narrow_tiles_leave_whole(m, n, kblocks):
     for dtype in (torch.bfloat16, torch.float16):
         assert torch.equal(ops.fp8_gemm(*args, dtype), c.to(dtype))
     _status_ok()
+
+
+@pytest.mark.parametrize("m,n,k,tile_rows,dtype", [
+    (100, 2048, 2176, 128, torch.bfloat16),      # 64 columns
+    (128, 12288, 1152, 128, torch.bfloat16),     # 128
+    (1000, 12288, 1152, 128, torch.bfloat16),    # 256, several tiles per CTA
+    (1000, 4096, 1152, 128, torch.float32),      # stored by the promotion warps
+    (1000, 12288, 1152, 256, torch.bfloat16),    # pairs of CTAs
+])
+def test_gemm_beside_copies(m, n, k, tile_rows, dtype):
+    """A copy on another stream takes memory and SM time, so that the kernel's early questions for its barriers are answered
+    now with yes, now with no.  Same bits as alone, every time."""
+    from dlblas_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(m + n)
+    a, b = (torch.randn(*s, generator=g, device=DEV).to(FP8) for s in ((m, k), (n, k)))
+    a_s, b_s = torch.rand(m, k // 128, generator=g, device=DEV), torch.rand((n + 127) // 128, k // 128, generator=g, device=DEV)
+    alone = ops.fp8_gemm(a, b, a_s, b_s, dtype, tile_rows=tile_rows)
+    assert O.rel_frobenius(alone[:8].float().cpu(), O.fp8_gemm(a[:8].cpu(), b.cpu(), a_s[:8].cpu(), b_s.cpu(),
+                                                               torch.float32)) < 4e-3
+    src = torch.randn(32 << 20, device=DEV)
+    dst, side, out = torch.empty_like(src), torch.cuda.Stream(), []
+    torch.cuda.synchronize()
+    for _ in range(20):
+        with torch.cuda.stream(side):
+            dst.copy_(src)
+        for _ in range(3):
+            out.append(ops.fp8_gemm(a, b, a_s, b_s, dtype, tile_rows=tile_rows))
+    torch.cuda.synchronize()
+    _status_ok()
+    assert all(torch.equal(alone, c) for c in out)
