@@ -496,7 +496,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
           __syncwarp();
           if (lane == 0) {
             if (rank == 0) mbar_arrive(tempty_bar(b));
-            else mbar_arrive_cluster_no_release(mapa(tempty_bar(b), 0));
+            else mbar_arrive_cluster_relaxed(mapa(tempty_bar(b), 0));
           }
         }
 #pragma unroll

@@ -720,7 +720,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
             __syncwarp();
             if (lane == 0) {
               if (rank == 0) mbar_arrive(tempty_bar(b));
-              else mbar_arrive_cluster_no_release(mapa(tempty_bar(b), 0));
+              else mbar_arrive_cluster_relaxed(mapa(tempty_bar(b), 0));
             }
             if (CH > 1 && kb + 1 < kblocks) {
               if (!__all_sync(WHOLE_WARP, next_full) && !mbar_wait(next_done, next_phase, abort_flag, limit)) {

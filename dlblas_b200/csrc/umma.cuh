@@ -227,11 +227,13 @@ __device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// The same for handing an accumulator back: nothing but TMEM reads has to come before it, and those are ordered by the
-// tcgen05 fence in front.  A release at cluster scope first waits for all the warp's earlier memory operations; one per K
-// block made the FP8 kernel's pairs half as fast (4096 x 7168 x 2048: 870 against 1464 TFLOP/s).
-__device__ __forceinline__ void mbar_arrive_cluster_no_release(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+// The same for handing an accumulator back: relaxed, it orders no access to shared or global memory and must not publish any.
+// Only TMEM reads have to come before it; tcgen05.wait::ld has seen their values arrive, and the tcgen05 fences on both sides
+// order them against the MMAs that follow.  A release at cluster scope first waits for all the warp's earlier memory
+// operations; one per K block made the FP8 kernel's pairs half as fast (4096 x 7168 x 2048: 870 against 1464 TFLOP/s).  The
+// 16-bit kernel's pairs, with one per tile, do not notice (16384 x 4096 x 3072 in 16 groups: 361 us both ways).
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");

@@ -177,3 +177,31 @@ def test_m_grouped_gemm_narrow_tiles(groups, n):
         _C.check_status()
         ref = utils.gmm(a.float(), b.float(), sizes.cpu(), trans_b=True)
         assert float((out.float() - ref).norm() / ref.norm()) < 1e-3     # one rounding to fp16
+
+
+@pytest.mark.parametrize("tile_rows", [128, 256])
+def test_m_grouped_gemm_beside_copies(tile_rows, monkeypatch):
+    """Several tiles per CTA or pair, so that accumulators are handed back and used again, beside a copy on another stream:
+    same bits as alone, every time."""
+    monkeypatch.setenv("DLBLAS_GEMM16_TILE_ROWS", str(tile_rows))
+    from dlblas_b200 import _C
+    from dlblas_b200.kernels.grouped_gemm.BF16 import m_grouped_gemm, utils
+    g = torch.Generator(device=DEV).manual_seed(6)
+    sizes = torch.tensor([1500, 0, 700, 2300, 1], device=DEV)
+    m, n, k = int(sizes.sum()), 6144, 192
+    a = torch.randn(m, k, generator=g, device=DEV, dtype=torch.bfloat16)
+    b = torch.randn(5, n, k, generator=g, device=DEV, dtype=torch.bfloat16)
+    alone = m_grouped_gemm(a, b, sizes, trans_b=True)
+    ref = utils.gmm(a.float(), b.float(), sizes.cpu(), trans_b=True)
+    assert float((alone.float() - ref).norm() / ref.norm()) < 3e-3
+    src = torch.randn(32 << 20, device=DEV)
+    dst, side, out = torch.empty_like(src), torch.cuda.Stream(), []
+    torch.cuda.synchronize()
+    for _ in range(20):
+        with torch.cuda.stream(side):
+            dst.copy_(src)
+        for _ in range(3):
+            out.append(m_grouped_gemm(a, b, sizes, trans_b=True))
+    torch.cuda.synchronize()
+    _C.check_status()
+    assert all(torch.equal(alone, c) for c in out)
