@@ -34,6 +34,7 @@
 // All mbarrier waits are bounded (about 2 s of SM clock cycles): a wait that exceeds its limit raises a CTA-wide
 // abort flag, every role leaves its loop, the status word is set to DLB_STATUS_TIMEOUT
 // and the kernel returns after draining what it issued.
+#include "tile_width.h"
 #include "umma.cuh"
 
 namespace dlb {
@@ -280,11 +281,12 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   const int num_m_tiles = g.tiles != nullptr ? __ldg(reinterpret_cast<const int*>(g.tiles)) : g.num_m_tiles_static;
   const int total_tiles = num_m_tiles * g.num_n_tiles;
 
-  // Narrow tiles are chosen for launches of one tile per CTA, so nothing follows that could hide the staging tile's way out:
-  // the promotion warps empty it themselves with ordinary 16-byte stores, warp w of EPI_WARPS its share of the rows.  (A bulk
-  // copy per row holds its lane for some 70 cycles: 100 rows of 64 columns took two warps 5100 of the kernel's 18300 cycles;
-  // quantiser and GEMM of 100 x 7168 x 2048 11.9 -> 9.6 us with the single commit.  256 columns keep the two epilogue warps and the bulk copies, which
-  // run beside the next tile: with these lines for the last tile only, 8192 x 4096 x 7168 lost 3 %.)
+  // Narrow tiles are chosen for launches that probably have one tile per CTA, so nothing follows that could hide the staging
+  // tile's way out: the promotion warps empty it themselves with ordinary 16-byte stores, warp w of EPI_WARPS its share of the
+  // rows.  (A bulk copy per row holds its lane for some 70 cycles: 100 rows of 64 columns took two warps 5100 of the kernel's
+  // 18300 cycles; 100 x 7168 x 2048 alone 11.1 -> 9.0 us by these stores, 128 x 12288 x 2048 12.2 -> 10.8.  256 columns keep
+  // the two epilogue warps and the bulk copies, which run beside the next tile: with these lines for the last tile only,
+  // 8192 x 4096 x 7168 lost 3 %.)
   auto store_rows = [&](const Tile& ti, int w) {
     constexpr int VECS = BN / 8, ROWS = 32 / VECS;       // vectors of a row, rows of a pass
     const int vec = lane % VECS, in_pass = lane / VECS;
@@ -852,16 +854,6 @@ int launch_typed(int bn, int ctas, bool swap, int c_dtype, const CUtensorMap& ma
   return fail(DLB_ERR_INVALID, "unsupported output dtype %d for this GEMM epilogue", c_dtype);
 }
 
-// Columns per tile: the narrowest that still makes one wave, else 256.  A K block of a wave takes about the same time on 64
-// and 128 columns and a third more on 256, so a second wave costs more than the wider tile.  Repeated GEMMs alone, one wave
-// of 256 against two of 128: 1000 x 4096 x 7168 37.8 / 48.5 us, 300 x 7168 x 2048 17.4 / 21.1;
-// one of 128 against one of 256: 128 x 12288 x 7168 31.0 / 39.4; one of 64 against one of 128: 64 x 7168 x 2048
-// 13.7 / 14.8; with more waves on either side 256 is never behind (1000 x 12288 x 7168, 2.6 against 5.2 waves, 104 / 136).
-int tile_width(long long m_tiles, int64_t n, int sms, int c_dtype) {
-  if (c_dtype != DLB_F32 && m_tiles * ceil_div(n, (int64_t)64) <= sms) return 64;
-  return m_tiles * ceil_div(n, (int64_t)128) <= sms ? 128 : 256;
-}
-
 }  // namespace
 }  // namespace dlb
 
@@ -892,7 +884,7 @@ extern "C" int dlb_fp8_gemm(const void* a, const void* b, const float* a_s, int6
   const int ctas = tile_rows == 256 ? 2 : 1;
   const int m_tiles = (int)ceil_div(m, (int64_t)(ctas * BM));
   int bn = 256;
-  if (ctas == 1) bn = tile_width(m_tiles, n, sms, c_dtype);
+  if (ctas == 1) bn = fp8_tile_width(m_tiles, m_tiles, n, sms, c_dtype != DLB_F32);
   if ((rc = make_map_box(&mb, b, (uint64_t)n, (uint64_t)k, bn < 128 ? bn : 128)) != DLB_OK) return rc;
   GemmArgs g = {};
   g.a_s = a_s;
@@ -986,7 +978,8 @@ static int moe_grouped_gemm(const void* a, const float* a_s, int64_t rows_a, con
     if (epilogue == DLB_EPI_SCATTER_WEIGHT)
       DLB_REQUIRE(sorted_idx && weights, DLB_ERR_INVALID, "grouped_gemm: scatter epilogue needs sorted_idx and weights");
     DLB_REQUIRE(ldc % 8 == 0, DLB_ERR_INVALID, "grouped_gemm: ldc must be a multiple of 8");
-    if (!window && ctas == 1) bn = tile_width(max_tiles, n, sms, c_dtype);
+    if (!window && ctas == 1)
+      bn = fp8_tile_width(max_tiles, likely_tiles(rows_a, num_local_experts, max_tiles), n, sms, c_dtype != DLB_F32);
     g.num_n_tiles = (int)ceil_div(n_count, bn);
     g.n_tile0 = (int)(n_begin / bn);
   }

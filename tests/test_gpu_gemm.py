@@ -503,3 +503,39 @@ def test_gemm_beside_copies(m, n, k, tile_rows, dtype):
     torch.cuda.synchronize()
     _status_ok()
     assert all(torch.equal(alone, c) for c in out)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("epilogue", ["store", "scatter"])
+def test_more_tiles_than_expected(epilogue, dtype):
+    """Tiles of 128 columns are chosen for the likely number of tiles, 8 x 16; here there are as many as there can be, 11 x 16, so
+    that some CTAs have two, and the staging tile is filled and emptied more than once.  The bits are those of 256-row tiles."""
+    from dlblas_b200 import _C, ops
+    counts = [1, 129, 3, 129, 1, 129, 5, 1]
+    e, rows, k, n = len(counts), sum(counts), 1152, 2048
+    sms = torch.cuda.get_device_properties(DEV).multi_processor_count
+    assert sum(-(-c // 128) for c in counts) == rows // 128 + e and (rows // 128 + e) * n // 128 > sms >= e * n // 128
+    g = torch.Generator().manual_seed(23)
+    a, a_s = O.quant_fp8(torch.randn(rows, k, generator=g).to(torch.bfloat16), 128)
+    b = torch.randn(e, n, k, generator=g).to(FP8)
+    b_s = torch.rand(e, n // 128, k // 128, generator=g) * 0.01 + 0.01
+    ends = torch.tensor(counts).cumsum(0)
+    order = torch.randperm(rows, generator=g)
+    weights = torch.rand(rows, generator=g) + 0.5
+    extra = {"sorted_idx": order.to(DEV), "weights": weights.to(DEV)} if epilogue == "scatter" else {}
+    out = []
+    for tile_rows in (128,) if dtype == torch.float32 else (128, 256):
+        most = ops.max_tiles_for(rows, e, tile_rows)
+        tiles = ops.build_tiles((ends - torch.tensor(counts)).to(DEV), ends.to(DEV), 0, e, most, tile_rows)
+        c = torch.zeros(rows, n, dtype=dtype, device=DEV)
+        ops.grouped_gemm(a.to(DEV), a_s.to(DEV), b.to(DEV), b_s.to(DEV), tiles, most,
+                         _C.EPI_SCATTER_WEIGHT if extra else _C.EPI_STORE, c, tile_rows=tile_rows, **extra)
+        out.append(c)
+    _status_ok()
+    assert torch.equal(out[0], out[-1])
+    for i in range(e):
+        sl = slice(int(ends[i]) - counts[i], int(ends[i]))
+        ref = O.fp8_gemm(a[sl], b[i], a_s[sl], b_s[i], torch.float32)
+        got = out[0].cpu().float()
+        got = got[order[sl]] / weights[order[sl], None] if extra else got[sl]
+        assert O.rel_frobenius(got, ref) < (1e-5 if dtype == torch.float32 else 4e-3), i
