@@ -225,3 +225,31 @@ def test_exchange_kernels_in_between(captured):
     _same(got, want)
     if captured:
         graph.reset()
+
+
+def test_default_stream_and_a_blocking_stream():
+    """The legacy default stream waits for streams that were created without the non-blocking flag, and they for it, without an
+    event.  An operator on the default stream, right behind another one, reads what such a stream wrote in between."""
+    import ctypes
+
+    from dlblas_b200.kernels.fp8 import per_token_group_quant_fp8
+    handle = ctypes.c_void_p()
+    assert int(torch.cuda.cudart().cudaStreamCreate(ctypes.addressof(handle))) == 0
+    blocking = torch.cuda.ExternalStream(handle.value)
+    x, other = (torch.zeros(2048, 512, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    xs = torch.randn(6, 2048, 512, device=DEV, dtype=torch.bfloat16)
+    want = [per_token_group_quant_fp8(t, 128) for t in xs]
+    torch.cuda.synchronize()
+    got = []
+    for t in xs:
+        per_token_group_quant_fp8(other, 128)
+        with torch.cuda.stream(blocking):
+            torch.cuda._sleep(SLOW)
+            x.copy_(t)
+        got.append(per_token_group_quant_fp8(x, 128))
+        with torch.cuda.stream(blocking):
+            x.zero_()
+    torch.cuda.synchronize()
+    _same([[q.view(torch.uint8), s] for q, s in got], [[q.view(torch.uint8), s] for q, s in want])
+    del blocking
+    assert int(torch.cuda.cudart().cudaStreamDestroy(handle.value)) == 0
