@@ -57,8 +57,8 @@ constexpr int TMEM_COLS = 512;
 // tensor core's tile are columns of C, its columns the rows of A, 16 at a time.  A tile with a handful of rows otherwise
 // multiplies and promotes 128 all the same; the weights' way from DRAM bounds such a launch, and in repeated passes that
 // work costs the clocks and with them the memory rate.  (Up to 64 rows per tile this way: 2 % slower on those steps.)
-// Registers: the promotion warps hold both forms without a spill, but for 24 bytes of stores and 72 of loads in the fused epilogue,
-// where the kernel without the exchanged form spills 24 / 64 (ptxas).
+// Registers: the promotion warps hold both forms without a spill, but for 24 bytes of stores and 72 of loads in the fused
+// epilogue, where the kernel without the exchanged form spills 24 / 64 (ptxas).
 constexpr int SWAP_ROWS = 32;
 constexpr int CHUNK = 16;                    // rows of A per box and per step of N
 constexpr int CHUNKS = SWAP_ROWS / CHUNK;
@@ -108,10 +108,11 @@ template <int BN, int CTAS = 1> struct Cfg {
   // dynamic smem: stages | staging tile | barriers (full, done, tmem_empty, drain, staged, staging_free) | misc
   static constexpr int STAGING_OFF = STAGES * STAGE_BYTES;
   static constexpr int BAR_OFF = STAGING_OFF + STAGING_BYTES;
-  // One commit per K block (each holds the MMA warp for about 45 cycles, and so does a question
-  // for a barrier, of which narrow tiles ask one in RUN less): its barrier (the stage's) tells the producer that the
-  // stage is free and the promotion warps that the accumulator is full.  A stage's next use but one cannot be over before
-  // this one's accumulator has been drained.
+  // One commit per K block: its barrier (the stage's) tells the producer that the stage is free and the promotion warps that
+  // the accumulator is full.  (A commit holds the MMA warp for about 45 cycles, and a question for a barrier for as long:
+  // narrow tiles ask about the accumulators once in RUN K blocks.)  The promotion warps wait by parity, so none may miss a
+  // phase.  K block it + STAGES uses the stage next; its MMAs are issued only after every promotion warp has drained K block
+  // it + STAGES - TMEM_BUFS, and with it, STAGES being no less than TMEM_BUFS, K block it, whose phase it waited for.
   static_assert(STAGES >= TMEM_BUFS, "a promotion warp could miss a phase of the stage's barrier");
   static constexpr int NUM_BARS = 2 * STAGES + TMEM_BUFS + 3;
   static constexpr int MISC_OFF = BAR_OFF + NUM_BARS * 8;
@@ -683,7 +684,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       // the next K block's first 32) is in flight into the other.  This and the early questions for the barriers (here and
       // in the MMA warp) took 8192 x 4096 x 7168 from 287 to 257 us in repeated passes at the power limit (1675 -> 1869
       // TFLOP/s, 1600 -> 1480 MHz), 4096 x 7168 x 2048 from 84 to 76, 8192 x 24576 x 1536 from 405 to 369; the promotion
-      // warp's question alone is two thirds of that.
+      // warp's question alone is two thirds of that.  (With whole-warp answers 247, 73 and 362.)
       constexpr int CH = COLS / 32;      // 32-column chunks per thread and K block (1, 2 or 4)
       uint32_t stage[2][32];
       bool pending = false;              // first chunk of the current K block already issued
@@ -808,7 +809,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 }
 
 template <int BN, int MODE, typename OutT, int CTAS = 1, bool SWAP = false>
-int launch_one(const CUtensorMap& ma, const CUtensorMap& ma16, const CUtensorMap& mb, const GemmArgs& g, int grid, cudaStream_t st) {
+int launch_one(const CUtensorMap& ma, const CUtensorMap& ma16, const CUtensorMap& mb, const GemmArgs& g, int grid,
+               cudaStream_t st) {
   auto kern = gemm_fp8_kernel<BN, MODE, OutT, CTAS, SWAP>;
   constexpr int SMEM = Cfg<BN, CTAS>::SMEM_BYTES;
   static bool configured[64] = {};
@@ -827,8 +829,8 @@ int launch_one(const CUtensorMap& ma, const CUtensorMap& ma16, const CUtensorMap
 }
 
 template <int MODE>
-int launch_typed(int bn, int ctas, bool swap, int c_dtype, const CUtensorMap& ma, const CUtensorMap& ma16, const CUtensorMap& mb, const GemmArgs& g,
-                 int grid, cudaStream_t st) {
+int launch_typed(int bn, int ctas, bool swap, int c_dtype, const CUtensorMap& ma, const CUtensorMap& ma16,
+                 const CUtensorMap& mb, const GemmArgs& g, int grid, cudaStream_t st) {
   if (ctas == 2) {
     // pairs exist for 256-wide tiles with a 16-bit output (the ones that go through the staging tile)
     if (bn == 256 && c_dtype == DLB_BF16) return launch_one<256, MODE, __nv_bfloat16, 2>(ma, ma16, mb, g, grid, st);
@@ -879,8 +881,8 @@ extern "C" int dlb_fp8_gemm(const void* a, const void* b, const float* a_s, int6
               "fp8_gemm: tile_rows must be 0 (choose), 128 or 256");
   const int sms = sm_count();
   // Pairs of CTAs only on request: they move a third less through L2 and shared memory, but what bounds a K block is the
-  // hand-over between the MMA warp and the promotion warps, which crosses CTAs there: 8192 x 4096 x 7168 256 us against 257,
-  // 4096 x 7168 x 2048 78 against 76, 64 groups of about 256 rows 916 against 821 (tiles of 256 rows fill worse).
+  // hand-over between the MMA warp and the promotion warps, which crosses CTAs there: 8192 x 4096 x 7168 252 us against 247,
+  // 4096 x 7168 x 2048 75 against 73, 64 groups of about 256 rows 943 against 830 (tiles of 256 rows fill worse).
   const int ctas = tile_rows == 256 ? 2 : 1;
   const int m_tiles = (int)ceil_div(m, (int64_t)(ctas * BM));
   int bn = 256;

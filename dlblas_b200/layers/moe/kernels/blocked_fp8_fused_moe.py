@@ -61,9 +61,9 @@ def moe_expert_forward(hidden: Optional[torch.Tensor], x_q: Optional[torch.Tenso
     if weights.dtype != torch.float32:
         weights = weights.float()
     sorted_idx, exp_start, exp_end, pos = ops.sort_by_expert(ids, num_experts, want_pos=True)
-    # DLBLAS_FP8_TILE_ROWS=256 runs the GEMMs on pairs of CTAs with 256-row tiles (tcgen05 cta_group::2).  Off by
-    # default: the per-K-block hand-shake across the two CTAs costs more than the cheaper MMAs win (0.94 against
-    # 1.85 PFLOP/s on 32 experts of 2048 rows); the variant is kept, bit-identical, for kernels with fewer hand-shakes.
+    # DLBLAS_FP8_TILE_ROWS=256 runs the GEMMs on pairs of CTAs with 256-row tiles (tcgen05 cta_group::2), bit-identical.
+    # Off by default: 2 to 3 % slower on large dense problems, and more on ragged segments, whose ends fill tiles of 256 rows
+    # worse (64 experts of about 256 rows: 943 against 830 us).
     tile_rows = int(os.environ.get("DLBLAS_FP8_TILE_ROWS", "0")) or 128
     if out_dtype == torch.float32:
         tile_rows = 128
